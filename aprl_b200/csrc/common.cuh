@@ -8,11 +8,19 @@
 //     (k + zbase_c) mod nz_c.  The moving-window shift
 //     (src/moving_window_fields.cpp:439-518) then only decrements zbase and
 //     rewrites the one inserted plane instead of moving the volume.
-//   * Two E buffers: E^n ("old", read by the orbit-averaged gather) and
-//     E* ("star", the zero-current preview with its boundary applied).  The
-//     trial candidate E* - dt/eps0 J is never stored: every gather forms it
-//     from E* and J, so a fixed-point trial touches the grid only through J.
-//   * J is not ring-buffered: it is cleared before every trial.
+//   * Two E buffers: E^n ("old") and E* ("star", the zero-current preview
+//     with its boundary applied).  The trial candidate E* - dt/eps0 J is never
+//     stored.
+//   * The wide part of the particle shapes lives on the grid.  A deposit or
+//     gather weight of either shape is a narrow weight (linear in x, y, z for
+//     linear-binomial3; linear in x, y and the plain B-spline in z for
+//     quintic-compensated) convolved with a fixed filter: [1/4, 1/2, 1/4] in
+//     x and in z, or the seven compensation coefficients in z.  Particles
+//     therefore deposit the narrow weights into the RAW current (12 nodes a
+//     piece instead of 64, 44 instead of 92) and gather from the FILTERED
+//     orbit sum and B; grid passes apply the filter (J = filter(raw)).  Both
+//     are plain (not ring-buffered) arrays of one geometry, padded by the
+//     filter's reach: one node on either side in x, jpad planes in z.
 //   * CPML convolution histories keep the reference's [slot][k][row] order
 //     (src/eb_cpml.cpp:42-96) with the same z ring as their component.
 #pragma once
@@ -121,7 +129,9 @@ struct GridT {
   double* e_old[3];      // E^n  (ring)
   double* e_star[3];     // E*   (ring)
   double* b[3];          // B    (ring)
-  F* j[3];               // J    (plain)
+  F* j[3];               // raw current (plain, padded)
+  int jpad;              // its z padding: 1 (linear-binomial3) or 3 (quintic)
+  double inv_h[3];       // 1/dx, 1/dy, 1/dz, each rounded once
   int zb_e[3];           // ring bases of Ex Ey Ez
   int zb_b[3];           // ring bases of Bx By Bz
   F jcoef;               // (-1*dt)/eps0, applyCurrentSource(-1) scale
@@ -193,13 +203,28 @@ __device__ __forceinline__ size_t b_index(const GridT<F>& g, int c, int i, int j
   return ((size_t)ring(k, g.zb_b[c], nzc) * b_ny(g, c) + j) * b_nx(g, c) + i;
 }
 
+// The raw current and the filtered orbit sum of E component c: nodes
+// -1 <= i <= e_nx, 0 <= j < e_ny, -jpad <= k < e_nz + jpad.
 template <class F>
 __device__ __forceinline__ size_t j_index(const GridT<F>& g, int c, int i, int j, int k) {
-  APRL_NODE_CHECK(g, i, j, k, e_nx(g, c), e_ny(g, c), e_nz(g, c), 7 + c);
-  return ((size_t)k * e_ny(g, c) + j) * e_nx(g, c) + i;
+  APRL_NODE_CHECK(g, i + 1, j, k + g.jpad, e_nx(g, c) + 2, e_ny(g, c), e_nz(g, c) + 2 * g.jpad,
+                  7 + c);
+  return ((size_t)(k + g.jpad) * e_ny(g, c) + j) * (e_nx(g, c) + 2) + (i + 1);
+}
+template <class F>
+__device__ __forceinline__ size_t j_count(const GridT<F>& g, int c) {
+  return (size_t)(e_nx(g, c) + 2) * e_ny(g, c) * (e_nz(g, c) + 2 * g.jpad);
 }
 
-// Elements of E component c (also of J and of the orbit sum) and of B component c.
+// The filtered B of component c: nodes -1 <= i <= b_nx, 0 <= j < b_ny,
+// -1 <= k <= b_nz.
+template <class F>
+__device__ __forceinline__ size_t bf_index(const GridT<F>& g, int c, int i, int j, int k) {
+  APRL_NODE_CHECK(g, i + 1, j, k + 1, b_nx(g, c) + 2, b_ny(g, c), b_nz(g, c) + 2, 27 + c);
+  return ((size_t)(k + 1) * b_ny(g, c) + j) * (b_nx(g, c) + 2) + (i + 1);
+}
+
+// Elements of E component c and of B component c.
 template <class F>
 __device__ __forceinline__ size_t e_count(const GridT<F>& g, int c) {
   return (size_t)e_nx(g, c) * e_ny(g, c) * e_nz(g, c);
@@ -217,15 +242,19 @@ __device__ __forceinline__ bool current_mask(const GridT<F>& g, int c, int i, in
   return i > 0 && i < g.nx && j > 0 && j < g.ny;
 }
 
-// Trial candidate E* - dt/eps0 J at a native node (applyCurrentSource(-1)).
-template <class F>
-__device__ __forceinline__ F e_candidate(const GridT<F>& g, int c, int i, int j, int k) {
-  F v = F(g.e_star[c][e_index(g, c, i, j, k)]);
-  if (current_mask(g, c, i, j, k)) {
-    const F jc = g.j[c][j_index(g, c, i, j, k)];
-    if (jc != F(0.)) v += g.jcoef * jc;
-  }
-  return v;
+// x / h for a divisor whose reciprocal `inv` = RN(1/h) is at hand: Markstein's
+// correction (P. W. Markstein, IBM J. Res. Dev. 34, 1990).  q = x * inv is
+// within an ulp of the quotient, the remainder x - q h is exact in a fused
+// multiply-add, and adding its share gives the correctly rounded quotient --
+// the same bits as x / h away from overflow and the subnormal range, in three
+// operations instead of the division's loop.
+__device__ __forceinline__ double divide_by(double x, double h, double inv) {
+  const double q = x * inv;
+  return fma(fma(-q, h, x), inv, q);
+}
+__device__ __forceinline__ float divide_by(float x, float h, float inv) {
+  const float q = x * inv;
+  return fmaf(fmaf(-q, h, x), inv, q);
 }
 
 // ---------------------------------------------------------------------------
@@ -312,20 +341,9 @@ constexpr double c[7] = {-d / 64.,
 static __constant__ double kQuinticC64[7] = {
     quintic_detail::c[0], quintic_detail::c[1], quintic_detail::c[2], quintic_detail::c[3],
     quintic_detail::c[4], quintic_detail::c[5], quintic_detail::c[6]};
-static __constant__ float kQuinticC32[7] = {
-    float(quintic_detail::c[0]), float(quintic_detail::c[1]), float(quintic_detail::c[2]),
-    float(quintic_detail::c[3]), float(quintic_detail::c[4]), float(quintic_detail::c[5]),
-    float(quintic_detail::c[6])};
-
 template <class F>
-__device__ __forceinline__ F quintic_coefficient(int k);
-template <>
-__device__ __forceinline__ double quintic_coefficient<double>(int k) {
-  return kQuinticC64[k];
-}
-template <>
-__device__ __forceinline__ float quintic_coefficient<float>(int k) {
-  return kQuinticC32[k];
+__device__ __forceinline__ F quintic_coefficient(int k) {
+  return F(kQuinticC64[k]);
 }
 
 // basis(z, edge, QuinticCompensated) (src/longitudinal_shape.h:48-54): the
@@ -342,24 +360,13 @@ __device__ __forceinline__ void quintic_compensate(const F* n, unsigned degree, 
     for (unsigned k = 0; k < 7; ++k) r.v[j + k] += n[j] * quintic_coefficient<F>(k);
 }
 
-// Node q of quintic_compensate's result alone: the same products, summed in
-// the same order (spline index j rising), so the value is bit for bit
-// quintic_compensate's r.v[q].
-template <class F>
-__device__ __forceinline__ F quintic_compensated_at(const F* n, int degree, int q) {
-  F v = F(0.);
-#pragma unroll
-  for (int j = 0; j <= 5; ++j)
-    if (j <= degree && q - j >= 0 && q - j < 7) v += n[j] * quintic_coefficient<F>(q - j);
-  return v;
-}
-
 // The B-spline recursion on f = z - floor(z) up to `degree`.
 template <class F>
 __device__ __forceinline__ void quintic_spline_level(F n[6], F f, unsigned j) {
   F saved = F(0.);
+#pragma unroll
   for (unsigned k = 0; k < j; ++k) {
-    const F t = n[k] / F(j);
+    const F t = divide_by(n[k], F(j), F(1.) / F(j));
     n[k] = saved + (F(k + 1) - f) * t;
     saved = (f + F(j) - F(k) - F(1)) * t;
   }
@@ -372,32 +379,10 @@ __device__ __forceinline__ void quintic_basis(double z, bool edge, Basis<F>& r) 
   const double cell = floor(z);
   const F f = F(z - cell);
   F n[6] = {F(1.), F(0.), F(0.), F(0.), F(0.), F(0.)};
-  for (unsigned j = 1; j <= degree; ++j) quintic_spline_level(n, f, j);
+#pragma unroll
+  for (unsigned j = 1; j <= 5; ++j)
+    if (j <= degree) quintic_spline_level(n, f, j);
   quintic_compensate(n, degree, cell, r);
-}
-
-// Both spline sets of one point: the edge basis (degree 4) is the node
-// basis's recursion (degree 5) stopped after its fourth level, so one pass
-// yields the values quintic_basis computes for either.
-template <class F>
-struct QuinticSplines {
-  double cell;
-  F edge[5];
-  F node[6];
-};
-
-template <class F>
-__device__ __forceinline__ void quintic_splines(double z, QuinticSplines<F>& s) {
-  s.cell = floor(z);
-  const F f = F(z - s.cell);
-  F n[6] = {F(1.), F(0.), F(0.), F(0.), F(0.), F(0.)};
-#pragma unroll
-  for (unsigned j = 1; j <= 4; ++j) quintic_spline_level(n, f, j);
-#pragma unroll
-  for (int q = 0; q < 5; ++q) s.edge[q] = n[q];
-  quintic_spline_level(n, f, 5);
-#pragma unroll
-  for (int q = 0; q < 6; ++q) s.node[q] = n[q];
 }
 
 // BoostFrameTransform::gammaFromProperVelocity (src/boostframe.cpp:74-87).

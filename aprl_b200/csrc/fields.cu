@@ -7,8 +7,7 @@
 // expression keeps the reference's operation order; the library is compiled
 // without FMA contraction, so these kernels reproduce the reference's
 // translation units bit for bit.  The kernels are templated on the type F of
-// the current J (double, or float in the FP32-mixed mode), which only the
-// commit reads.
+// the current J, which only the filter passes read.
 #include "common.cuh"
 #include "dd.cuh"
 #include "fields.cuh"
@@ -262,16 +261,6 @@ __device__ __forceinline__ double bval(const GridT<F>& g, int c, int i, int j, i
 // the same B), PEC on the x/y faces, and the inlet Ex/Ey overwrite at k=0.
 // Reads E^n from e_old, writes E* to e_star.
 template <class F>
-__device__ __forceinline__ void preview_orbit(const PreviewArgs<F>& a, int c, size_t n,
-                                              double e_star, double e_old) {
-  // orbit_sum_kernel without current: S = W(E* + E^n), the same expression.
-  if (a.orbit_float)
-    static_cast<float*>(a.orbit[c])[n] = float(e_star + e_old);
-  else
-    static_cast<double*>(a.orbit[c])[n] = e_star + e_old;
-}
-
-template <class F>
 __global__ void electric_preview_kernel(PreviewArgs<F> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -323,7 +312,7 @@ __global__ void electric_preview_kernel(PreviewArgs<F> a) {
       v = inlet_value(a.inlet, 0, i, j);
     }
     g.e_star[0][n0] = v;
-    if (a.orbit[0]) preview_orbit(a, 0, n0, v, old0);
+    if (a.sum[0]) a.sum[0][n0] = v + old0;
   }
   if (has_y) {  // Ey (nx+1, ny, nz+1)
     double v = old1;
@@ -344,7 +333,7 @@ __global__ void electric_preview_kernel(PreviewArgs<F> a) {
       v = inlet_value(a.inlet, 1, i, j);
     }
     g.e_star[1][n1] = v;
-    if (a.orbit[0]) preview_orbit(a, 1, n1, v, old1);
+    if (a.sum[0]) a.sum[1][n1] = v + old1;
   }
   if (has_z) {  // Ez (nx+1, ny+1, nz)
     double v = old2;
@@ -365,37 +354,7 @@ __global__ void electric_preview_kernel(PreviewArgs<F> a) {
     }
     if (i == 0 || i == g.nx || j == 0 || j == g.ny) v = 0.0;
     g.e_star[2][n2] = v;
-    if (a.orbit[0]) preview_orbit(a, 2, n2, v, old2);
-  }
-}
-
-// commitConservativeElectric (src/simulation_source_coupling.cpp:61-65): the
-// previewed boundary already holds the committed CPML/PEC/inlet values, so
-// E^{n+1} = E* - dt/eps0 J on the applyCurrentSource mask, in place.
-template <class F>
-__global__ void electric_commit_kernel(GridT<F> g) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (i > g.nx || j > g.ny || k > g.nz) return;
-  // The three J reads are issued before the first update of E* (which may
-  // alias them as far as the compiler knows), so their latencies overlap.
-  F jc[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    jc[c] = F(0.);
-    if (i < e_nx(g, c) && j < e_ny(g, c) && k < e_nz(g, c) && current_mask(g, c, i, j, k))
-      jc[c] = g.j[c][j_index(g, c, i, j, k)];
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (jc[c] != F(0.)) {
-      // binary64 J: g.jcoef is -dt/eps0 itself.  A binary32 J is widened and
-      // scaled by the binary64 coefficient.
-      const double jcoef =
-          sizeof(F) == sizeof(double) ? (double)g.jcoef : -1. * g.dt / kEpsilon0;
-      g.e_star[c][e_index(g, c, i, j, k)] += jcoef * (double)jc[c];
-    }
+    if (a.sum[0]) a.sum[2][n2] = v + old2;
   }
 }
 
@@ -465,54 +424,188 @@ __global__ void shift_insert_kernel(ShiftArgs<F> a) {
   }
 }
 
-// The orbit sum the electric gathers read, one pass per trial:
-// S = E_new + E^n at every E node, with E_new = E* - dt/eps0 J on the
-// applyCurrentSource mask (with_current) or E* (the first-trial guess, before
-// any current).  In binary64 this is exactly the sum the orbit-averaged
-// gather forms node by node (Impl::electric, src/source_coupling.cpp:31-39),
-// so the gather is unchanged bit for bit; W = float rounds it once.
-template <class W>
-__global__ void orbit_sum_kernel(GridT<double> g, W* s0, W* s1, W* s2, int with_current) {
-  if (trial_skipped(g)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  W* s[3] = {s0, s1, s2};
-  // Every read of the node is issued before its first store (which may
-  // alias them as far as the compiler knows), so their latencies overlap.
-  bool in[3];
-  size_t n[3];
-  double star[3], old[3], jc[3];
+// The particle shape's filter, applied on the grid once per trial instead of
+// once per particle and node.  With raw J the narrow deposits,
+//   J = filter(raw J)                       (linear-binomial3: x and z;
+//                                            quintic-compensated: z)
+//   E_new = E* - dt/eps0 J                  (applyCurrentSource's mask)
+//   S = E_new + E^n = S0 - dt/eps0 J        (S0 = E* + E^n from the preview)
+// and the gathers read filter(S).  A deposit or gather over the wide stencil
+// skips the nodes outside a component, so both filters take zero there.
+//
+// A warp owns 32 x nodes of one row (j) of one component and marches z: the
+// x filter takes its neighbours by shuffle (28 of the 32 lanes write, the
+// filter reaching two nodes in all), the z filter keeps the last planes in
+// registers.  Nothing couples rows in y, and every array is read and written
+// once, but for the planes a chunk shares with its neighbours.
+__device__ __forceinline__ double lane_filter(double v) {
+  const double lo = __shfl_up_sync(0xffffffffu, v, 1), hi = __shfl_down_sync(0xffffffffu, v, 1);
+  return fma(0.25, lo + hi, 0.5 * v);
+}
+
+// z filter of S = 0: the three planes' values oldest first; S = 1: seven.
+template <int S>
+struct ZWindow {
+  static constexpr int R = S == 0 ? 1 : 3, N = 2 * R + 1;
+  double v[N];
+  __device__ __forceinline__ void clear() {
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    in[c] = i < e_nx(g, c) && j < e_ny(g, c) && k < e_nz(g, c);
-    n[c] = in[c] ? e_index(g, c, i, j, k) : 0;
-    star[c] = in[c] ? g.e_star[c][n[c]] : 0.;
-    old[c] = in[c] ? g.e_old[c][n[c]] : 0.;
-    jc[c] = in[c] && with_current && current_mask(g, c, i, j, k)
-                ? g.j[c][j_index(g, c, i, j, k)]
-                : 0.;
+    for (int t = 0; t < N; ++t) v[t] = 0.;
   }
+  __device__ __forceinline__ void push(double x) {
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    if (!in[c]) continue;
-    double v = star[c];
-    if (jc[c] != 0.) v += g.jcoef * jc[c];
-    s[c][n[c]] = W(v + old[c]);
+    for (int t = 0; t + 1 < N; ++t) v[t] = v[t + 1];
+    v[N - 1] = x;
+  }
+  __device__ __forceinline__ double value() const {  // at the window's middle plane
+    if constexpr (S == 0) {
+      return fma(0.25, v[0] + v[2], 0.5 * v[1]);
+    } else {
+      double r = kQuinticC64[3] * v[3];
+      r = fma(kQuinticC64[2], v[2] + v[4], r);
+      r = fma(kQuinticC64[1], v[1] + v[5], r);
+      return fma(kQuinticC64[0], v[0] + v[6], r);
+    }
+  }
+};
+
+template <int S, int MODE, class W>
+__global__ void current_filter_kernel(FilterArgs a) {
+  const GridT<double>& g = a.g;
+  if (trial_skipped(g)) return;
+  constexpr int R = ZWindow<S>::R;
+  constexpr bool kOrbit = MODE == kFilterGuess || MODE == kFilterOrbit;
+  constexpr bool kRaw = MODE != kFilterGuess;
+  const int lane = threadIdx.x & 31;
+  const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  // Select by branch: a run-time index into the parameter arrays would copy
+  // them to local memory.
+  const int c = blockIdx.z / a.chunks;
+  const int nxc = e_nx(g, c), nyc = e_ny(g, c), nzc = e_nz(g, c);
+  const int zb = c == 0 ? g.zb_e[0] : (c == 1 ? g.zb_e[1] : g.zb_e[2]);
+  const double* raw = c == 0 ? g.j[0] : (c == 1 ? g.j[1] : g.j[2]);
+  const double* sum = c == 0 ? a.sum[0] : (c == 1 ? a.sum[1] : a.sum[2]);
+  double* star = c == 0 ? g.e_star[0] : (c == 1 ? g.e_star[1] : g.e_star[2]);
+  void* out = c == 0 ? a.out[0] : (c == 1 ? a.out[1] : a.out[2]);
+  // Tiles: kFilterLanes nodes from -1 on for the orbit modes (lanes 2..29
+  // write), 30 from 0 on otherwise (lanes 1..30).
+  constexpr int kHalo = kOrbit ? 2 : 1, kWritten = 32 - 2 * kHalo;
+  const int i = tile * kWritten + lane - kHalo - (kOrbit ? 1 : 0);
+  if (tile * kWritten - (kOrbit ? 1 : 0) > nxc || j >= nyc) return;  // whole warps
+  const bool inside = i >= 0 && i < nxc;
+  const bool raw_in = i >= -1 && i <= nxc;
+  const bool writes = lane >= kHalo && lane < 32 - kHalo && (kOrbit ? raw_in : inside);
+  const bool column = inside && (c == 0 ? (j > 0 && j < g.ny)
+                                        : (c == 1 ? (i > 0 && i < g.nx)
+                                                  : (i > 0 && i < g.nx && j > 0 && j < g.ny)));
+  const int zlo = (c != 2) ? 1 : 0, zhi = (c != 2) ? nzc - 2 : nzc - 1;  // the mask's planes
+  // Output planes [k0, k1): the padded array's for the orbit modes.
+  const int first = kOrbit ? -g.jpad : 0, last = kOrbit ? nzc + g.jpad : nzc;
+  const int k0 = first + (int)(blockIdx.z % a.chunks) * a.planes;
+  const int k1 = min(k0 + a.planes, last);
+  if (k0 >= k1) return;
+  const size_t row = (size_t)j * (nxc + 2) + (i + 1), plane = (size_t)nyc * (nxc + 2);
+  const size_t node = (size_t)j * nxc + i, nplane = (size_t)nyc * nxc;
+  ZWindow<S> wj, ws;
+  wj.clear();
+  ws.clear();
+  const int s0 = kOrbit ? k0 - R : k0;  // first plane of the (candidate) sum
+  auto raw_at = [&](int k) -> double {
+    if (!(raw_in && k >= -g.jpad && k < nzc + g.jpad)) return 0.;
+    return raw[APRL_BOUNDED(g.status, (size_t)(k + g.jpad) * plane + row, j_count(g, c), 33 + c)];
+  };
+  auto sum_at = [&](int k) -> double {
+    if (!(inside && k >= 0 && k < nzc)) return 0.;
+    return sum[APRL_BOUNDED(g.status, (size_t)ring(k, zb, nzc) * nplane + node, e_count(g, c),
+                            36 + c)];
+  };
+  if constexpr (kRaw) {
+#pragma unroll
+    for (int t = -R; t < R; ++t) {
+      double v = raw_at(s0 + t);
+      if constexpr (S == 0) v = lane_filter(v);
+      wj.push(v);
+    }
+  }
+  const int s1 = kOrbit ? k1 + R : k1;
+  // The next plane's reads are issued before this plane's arithmetic.
+  double raw_next = kRaw ? raw_at(s0 + R) : 0.;
+  double sum_next = kOrbit ? sum_at(s0) : 0.;
+  for (int k = s0; k < s1; ++k) {
+    double v = raw_next;
+    const double base = sum_next;
+    if (k + 1 < s1) {
+      if constexpr (kRaw) raw_next = raw_at(k + 1 + R);
+      if constexpr (kOrbit) sum_next = sum_at(k + 1);
+    }
+    double current = 0.;
+    if constexpr (kRaw) {
+      if constexpr (S == 0) v = lane_filter(v);
+      wj.push(v);
+      current = wj.value();
+    }
+    const bool masked = column && k >= zlo && k <= zhi;
+    if constexpr (MODE == kFilterCommit) {
+      if (writes && masked && current != 0.) {
+        const size_t n = APRL_BOUNDED(g.status, (size_t)ring(k, zb, nzc) * nplane + node,
+                                      e_count(g, c), 39 + c);
+        star[n] += g.jcoef * current;
+      }
+    } else if constexpr (MODE == kFilterCurrent) {
+      if (writes) static_cast<double*>(out)[(size_t)k * nplane + node] = current;
+    } else {
+      double s = base;
+      if (masked && current != 0.) s += g.jcoef * current;
+      if constexpr (S == 0) s = lane_filter(s);
+      ws.push(s);
+      const int ko = k - R;
+      if (ko >= k0 && writes)
+        static_cast<W*>(out)[APRL_BOUNDED(g.status, (size_t)(ko + g.jpad) * plane + row,
+                                          j_count(g, c), 42 + c)] = W(ws.value());
+    }
   }
 }
 
-// Binary32 copy of B (same ring layout) for the FP32-mixed gathers; one
-// launch for the three components (blockIdx.y).
-__global__ void b_shadow_kernel(BShadowArgs a) {
-  const int c = blockIdx.y;
-  // Select by branch: a run-time index into the parameter arrays would copy
-  // them to local memory in every thread.
-  const double* b = c == 0 ? a.b[0] : (c == 1 ? a.b[1] : a.b[2]);
-  float* out = c == 0 ? a.out[0] : (c == 1 ? a.out[1] : a.out[2]);
-  const long long n = c == 0 ? a.n[0] : (c == 1 ? a.n[1] : a.n[2]);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = (float)b[i];
+// The x-z filtered B of the linear-binomial3 gathers, one pass per step:
+// binomialXZMagneticSample clamps its nodes to the component (open faces), so
+// the filter does, and the output covers one node beyond in x and z.
+template <class W>
+__global__ void magnetic_filter_kernel(BFilterArgs a) {
+  const GridT<double>& g = a.g;
+  const int lane = threadIdx.x & 31;
+  const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int c = blockIdx.z / a.chunks;
+  const int nxc = b_nx(g, c), nyc = b_ny(g, c), nzc = b_nz(g, c);
+  const int zb = c == 0 ? g.zb_b[0] : (c == 1 ? g.zb_b[1] : g.zb_b[2]);
+  const double* b = c == 0 ? g.b[0] : (c == 1 ? g.b[1] : g.b[2]);
+  W* out = static_cast<W*>(c == 0 ? a.out[0] : (c == 1 ? a.out[1] : a.out[2]));
+  if (tile * 30 - 1 > nxc || j >= nyc) return;
+  const int i = tile * 30 + lane - 2;  // lanes 1..30 write nodes -1..nxc
+  const int ic = min(max(i, 0), nxc - 1);
+  const bool writes = lane >= 1 && lane < 31 && i <= nxc;
+  const int k0 = -1 + (int)(blockIdx.z % a.chunks) * a.planes;
+  const int k1 = min(k0 + a.planes, nzc + 1);
+  if (k0 >= k1) return;
+  const size_t node = (size_t)j * nxc + ic, nplane = (size_t)nyc * nxc;
+  const size_t row = (size_t)j * (nxc + 2) + (i + 1), plane = (size_t)nyc * (nxc + 2);
+  auto at = [&](int k) -> double {
+    const int kc = min(max(k, 0), nzc - 1);
+    return b[APRL_BOUNDED(g.status, (size_t)ring(kc, zb, nzc) * nplane + node, b_count(g, c),
+                          45 + c)];
+  };
+  ZWindow<0> w;
+  w.clear();
+  w.push(lane_filter(at(k0 - 1)));
+  w.push(lane_filter(at(k0)));
+  double next = at(k0 + 1);
+  for (int k = k0; k < k1; ++k) {
+    const double v = next;
+    if (k + 1 < k1) next = at(k + 2);
+    w.push(lane_filter(v));
+    if (writes) out[(size_t)(k + 1) * plane + row] = W(w.value());
+  }
 }
 
 // Lab detector field plane (src/lab_detectors.cpp:39-99, 2836-2905).
@@ -589,12 +682,21 @@ __global__ void detector_plane_kernel(DetectorArgs<F> a) {
 #define APRL_FIELD_KERNELS(F)                                                  \
   template __global__ void cowan_magnetic_kernel<F>(CowanArgs<F>);            \
   template __global__ void electric_preview_kernel<F>(PreviewArgs<F>);        \
-  template __global__ void electric_commit_kernel<F>(GridT<F>);               \
   template __global__ void shift_insert_kernel<F>(ShiftArgs<F>);              \
   template __global__ void detector_plane_kernel<F>(DetectorArgs<F>);
 APRL_FIELD_KERNELS(double)
-template __global__ void orbit_sum_kernel<double>(GridT<double>, double*, double*, double*, int);
-template __global__ void orbit_sum_kernel<float>(GridT<double>, float*, float*, float*, int);
+#define APRL_FILTER_KERNELS(S)                                                       \
+  template __global__ void current_filter_kernel<S, kFilterGuess, double>(FilterArgs);  \
+  template __global__ void current_filter_kernel<S, kFilterGuess, float>(FilterArgs);   \
+  template __global__ void current_filter_kernel<S, kFilterOrbit, double>(FilterArgs);  \
+  template __global__ void current_filter_kernel<S, kFilterOrbit, float>(FilterArgs);   \
+  template __global__ void current_filter_kernel<S, kFilterCommit, double>(FilterArgs); \
+  template __global__ void current_filter_kernel<S, kFilterCurrent, double>(FilterArgs);
+APRL_FILTER_KERNELS(0)
+APRL_FILTER_KERNELS(1)
+template __global__ void magnetic_filter_kernel<double>(BFilterArgs);
+template __global__ void magnetic_filter_kernel<float>(BFilterArgs);
+#undef APRL_FILTER_KERNELS
 #undef APRL_FIELD_KERNELS
 
 // TransverseReferenceCurrent::prepare's values (src/transverse_reference_current.cpp:
@@ -616,10 +718,13 @@ __global__ void surface_prepare_kernel(SurfaceArgs a) {
 
 // TransverseReferenceCurrent::apply (src/transverse_reference_current.cpp:104-118):
 // Jz(i, j, k) += the lerp of the prepared planes at offset + k - beta*step.
+// The current is the same in every trial of a step, so it goes into E* (and
+// its orbit sum) once, after the first trial's current-free gather; a
+// read-out of J adds it to Jz.
 __global__ void surface_add_kernel(SurfaceArgs a) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const DGrid& g = a.g;
-  if (trial_skipped(g) || n >= a.count * g.nz) return;
+  if (n >= a.count * g.nz) return;
   const int k = (int)(n / a.count);
   const long long p = n % a.count;
   const double z = static_cast<double>(a.offset + k) - a.beta * static_cast<double>(a.step);
@@ -629,7 +734,14 @@ __global__ void surface_add_kernel(SurfaceArgs a) {
   const double low = a.table[lo * a.count + p], high = a.table[hi * a.count + p];
   const double value = fraction == 0. ? low : (1. - fraction) * low + fraction * high;
   const int i = (int)a.points[2 * p], j = (int)a.points[2 * p + 1];
-  g.j[2][j_index(g, 2, i, j, k)] += value;
+  if (a.jz) {
+    a.jz[((size_t)k * (g.ny + 1) + j) * (g.nx + 1) + i] += value;
+    return;
+  }
+  if (!current_mask(g, 2, i, j, k)) return;
+  const size_t at = e_index(g, 2, i, j, k);
+  g.e_star[2][at] += g.jcoef * value;
+  if (a.sum) a.sum[at] += g.jcoef * value;
 }
 
 }  // namespace aprl_gpu

@@ -60,11 +60,9 @@ struct PreviewArgs {
   CpmlHistory h[4];      // electric histories 6 (Ex,y) 9 (Ey,x) 10 (Ez,x) 11 (Ez,y)
   InletTable inlet;      // reference(a, i, j, offset, step+1)
   double* pre_inlet[2];  // when set: Ex, Ey of plane 0 before the inlet overwrite
-  // When set: the first trial's orbit sum S = E* + E^n (the current-free pass
-  // of orbit_sum_kernel), written here from the values already in hand;
-  // binary32 when orbit_float, else binary64.
-  void* orbit[3];
-  int orbit_float;
+  // When set: the current-free orbit sum S0 = E* + E^n (ring layout of E),
+  // written here from the values already in hand.
+  double* sum[3];
 };
 
 // ChargeMatchedInlet::complete (src/charge_matched_inlet.h:55-71): Ez of the
@@ -127,18 +125,33 @@ struct DetectorArgs {
 constexpr int kCowanTileX = 32, kCowanTileY = 8, kCowanChunk = APRL_COWAN_CHUNK;
 template <class F> __global__ void cowan_magnetic_kernel(CowanArgs<F> a);
 template <class F> __global__ void electric_preview_kernel(PreviewArgs<F> a);
-template <class F> __global__ void electric_commit_kernel(GridT<F> g);
 __global__ void inlet_lower_kernel(InletPlaneArgs a);
 template <class F> __global__ void shift_insert_kernel(ShiftArgs<F> a);
 template <class F> __global__ void detector_plane_kernel(DetectorArgs<F> a);
-template <class W>
-__global__ void orbit_sum_kernel(GridT<double> g, W* s0, W* s1, W* s2, int with_current);
-struct BShadowArgs {
-  const double* b[3];
-  float* out[3];
-  long long n[3];
+// The particle shape's filter on the grid (common.cuh).
+struct FilterArgs {
+  GridT<double> g;
+  const double* sum[3];   // S0 = E* + E^n (ring layout of E)
+  void* out[3];           // kFilterOrbit*: W, layout of j_index; kFilterCurrent: J, native layout
+  int planes;             // output planes marched by one warp
+  int chunks;             // z chunks (blockIdx.z = component * chunks + chunk)
 };
-__global__ void b_shadow_kernel(BShadowArgs a);
+enum FilterMode {
+  kFilterGuess = 0,    // out = filter(S0)
+  kFilterOrbit = 1,    // out = filter(S0 - dt/eps0 filter(raw J)), on the current mask
+  kFilterCommit = 2,   // E* += -dt/eps0 filter(raw J), on the current mask
+  kFilterCurrent = 3   // out = filter(raw J)
+};
+constexpr int kFilterLanes = 28;  // x nodes written by a warp of kFilterOrbit*
+template <int S, int MODE, class W> __global__ void current_filter_kernel(FilterArgs a);
+
+// The filtered B the linear-binomial3 gathers read (layout of bf_index).
+struct BFilterArgs {
+  GridT<double> g;
+  void* out[3];
+  int planes, chunks;
+};
+template <class W> __global__ void magnetic_filter_kernel(BFilterArgs a);
 
 // The reference's equivalent surface current (TransverseReferenceCurrent).
 struct SurfaceArgs {
@@ -149,7 +162,9 @@ struct SurfaceArgs {
   int nx, ny;
   double dx, dy;
   DeviceStatus* status;
-  GridT<double> g;          // J of the trial, for the addition
+  GridT<double> g;          // E* of the step, for the addition
+  double* sum;              // its orbit sum S0 of Ez, when formed
+  double* jz;               // for a read-out: Jz, native layout
   long long offset;
   unsigned long long step;  // step + 1 of the trial
   double beta;

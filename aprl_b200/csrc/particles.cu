@@ -4,12 +4,14 @@
 // lab magnets, charge-conserving deposition, particle-boundary events with
 // CPML current carriers, the fixed-point residual, and stable compaction.
 //
-// One thread owns one particle; its gathers and weights run in the
-// reference's visit order, so in FP64 (no FMA contraction) the per-particle
-// arithmetic matches the reference, except that the quintic shape's four
-// Gauss points of a cut piece are summed per node before the gather's read
-// and the deposit's atomic.  Deposition accumulates with atomics into J; the
-// summation order of J differs from the reference.
+// One thread owns one particle.  The wide part of either shape is a filter
+// of the grid (common.cuh): a cut piece of a chord deposits its narrow
+// weights into the raw current and gathers with them from the filtered orbit
+// sum and B, which are the reference's sums over the wide stencil with the
+// terms in another order.  A sparse run's first-trial gather reads the wide
+// stencil directly, in the reference's visit order (no FMA contraction), so
+// there the gathered fields are the reference's bits.  Deposition accumulates
+// with atomics; the summation order of J differs from the reference.
 //
 // The walkers are templated on the type F of J and of the weight
 // arithmetic.  Positions, chord cuts and cell indices are always binary64,
@@ -78,60 +80,90 @@ __device__ __forceinline__ void binomial_xz_segment(const GridT<G>& g, const dou
     }
 }
 
-// Four-point Gauss quadrature of the quintic-compensated shape over one cut
-// piece of the chord (the quintic branch of longitudinal_shape::weights).
+// The narrow weights of binomialXZSegment: with wx = lx * [1/4, 1/2, 1/4] and
+// slope = (-1, 1) * [1/4, 1/2, 1/4] (convolutions), the 4x2x4 stencil's
+// weights are those of this 12-node one -- linear along the two axes across
+// the component, the component's own cell along it -- filtered in x and z.
 template <class G, class V>
-__device__ __forceinline__ void quintic_segment(const GridT<G>& g, const double x[3],
-                                                const double v[3], double lower,
-                                                double upper, double width, V& visit) {
+__device__ __forceinline__ void binomial_linear_segment(const GridT<G>& g, const double s[3],
+                                                        const double d[3], double first,
+                                                        double last, V& visit) {
   using F = typename V::Weight;
-  const double q[4] = {-.8611363115940525752, -.3399810435848562648,
-                       .3399810435848562648, .8611363115940525752};
-  const double qw[4] = {.3478548451374538574, .6521451548625461426,
-                        .6521451548625461426, .3478548451374538574};
-  for (int t = 0; t < 4; ++t) {
-    const double u = .5 * (upper + lower + width * q[t]), xx = x[0] + u * v[0],
-                 yy = x[1] + u * v[1], zz = x[2] + u * v[2];
-    const F factor = F(.5 * width * qw[t]);
-    long long i = (long long)floor(xx), j = (long long)floor(yy);
-    if (i == (long long)g.nx) --i;
-    if (j == (long long)g.ny) --j;
-    const F fx = F(xx - i), fy = F(yy - j);
-    QuinticSplines<F> spline;
-    quintic_splines(zz, spline);
-    Basis<F> nodes, edge;
-    quintic_compensate(spline.node, 5, spline.cell, nodes);
-    quintic_compensate(spline.edge, 4, spline.cell, edge);
-    for (int k = 0; k < nodes.count; ++k) {
-      const F w = factor * nodes.v[k];
-      if (w == F(0.)) continue;
-      for (int b = 0; b < 2; ++b) visit(0, i, j + b, nodes.first + k, w * (b ? fy : F(1.) - fy));
-      for (int a = 0; a < 2; ++a) visit(1, i + a, j, nodes.first + k, w * (a ? fx : F(1.) - fx));
+  const F width = F(last - first);
+  const double mid = (first + last) * 0.5;
+  const double x = s[0] + mid * d[0], y = s[1] + mid * d[1], z = s[2] + mid * d[2];
+  long long i = (long long)floor(x), j = (long long)floor(y);
+  const long long k = (long long)floor(z);
+  if (i == (long long)g.nx) --i;
+  if (j == (long long)g.ny) --j;
+  const F fx = F(x - i), fy = F(y - j), fz = F(z - k);
+  const F lx[2] = {F(1.) - fx, fx}, ly[2] = {F(1.) - fy, fy}, lz[2] = {F(1.) - fz, fz};
+  const F curvature = width * width / F(12.);
+  const F xy = curvature * F(d[0]) * F(d[1]);
+  const F xz = curvature * F(d[0]) * F(d[2]);
+  const F yz = curvature * F(d[1]) * F(d[2]);
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      visit(0, i, j + b, k + c, width * (ly[b] * lz[c] + (b == c ? yz : -yz)));
+      visit(1, i + b, j, k + c, width * (lx[b] * lz[c] + (b == c ? xz : -xz)));
+      visit(2, i + b, j + c, k, width * (lx[b] * ly[c] + (b == c ? xy : -xy)));
     }
-    for (int k = 0; k < edge.count; ++k) {
-      const F w = factor * edge.v[k];
-      if (w == F(0.)) continue;
-      for (int b = 0; b < 2; ++b)
-        for (int a = 0; a < 2; ++a)
-          visit(2, i + a, j + b, edge.first + k,
-                w * (a ? fx : F(1.) - fx) * (b ? fy : F(1.) - fy));
-    }
-  }
 }
 
-// quintic_segment for the deposit and the electric gather: every Gauss point
-// of a cut piece lies in the same cell, so the 4 x 92 node visits fall on 92
-// nodes; each node's four weights are summed first and visited once (a
-// quarter of the atomics or S reads).  The weights are quintic_segment's;
-// only their summation order changes.  The
-// walk is node by node: a Gauss point's compensated value at a node is formed
-// once (quintic_compensated_at, the same sums as quintic_compensate) and
-// shared by the component's transverse corners, so a node keeps four live
-// sums and the 12-node loop stays rolled.  A piece whose Gauss points
-// straddle a cell (only possible through rounding at a cut) is visited point
-// by point.
+// B-spline values on f = z - floor(z): degree 4 (the edge basis, n[0..4]) and
+// its next level, degree 5 (the node basis, n[0..5]).
+template <class F>
+__device__ __forceinline__ void spline_edge(F f, F n[6]) {
+  n[0] = F(1.);
+#pragma unroll
+  for (int q = 1; q < 6; ++q) n[q] = F(0.);
+#pragma unroll
+  for (unsigned j = 1; j <= 4; ++j) quintic_spline_level(n, f, j);
+}
+
+// One Gauss point at parameter u of the chord, weighted by `factor`, visited
+// on its own (the rare piece whose points straddle a cell).
 template <class G, class V>
-__device__ __forceinline__ void quintic_segment_summed(const GridT<G>& g, const double x[3],
+__device__ __noinline__ void quintic_linear_point(const GridT<G>& g, const double x[3],
+                                                  const double v[3], double u,
+                                                  typename V::Weight factor, V& visit) {
+  using F = typename V::Weight;
+  const double xx = x[0] + u * v[0], yy = x[1] + u * v[1], zz = x[2] + u * v[2];
+  long long i = (long long)floor(xx), j = (long long)floor(yy);
+  const long long k = (long long)floor(zz);
+  if (i == (long long)g.nx) --i;
+  if (j == (long long)g.ny) --j;
+  const F fx = F(xx - i), fy = F(yy - j), fz = F(zz - k);
+  F n[6];
+  spline_edge(fz, n);
+#pragma unroll 1
+  for (int m = 0; m < 5; ++m)
+#pragma unroll 1
+    for (int t = 0; t < 4; ++t)
+      visit(2, i + (t & 1), j + (t >> 1), k - 2 + m,
+            factor * n[m] * (t & 1 ? fx : F(1.) - fx) * (t >> 1 ? fy : F(1.) - fy));
+  quintic_spline_level(n, fz, 5);
+#pragma unroll 1
+  for (int m = 0; m < 6; ++m)
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+      visit(0, i, j + c, k - 2 + m, factor * n[m] * (c ? fy : F(1.) - fy));
+      visit(1, i + c, j, k - 2 + m, factor * n[m] * (c ? fx : F(1.) - fx));
+    }
+}
+
+// Four-point Gauss quadrature of the quintic-compensated shape over one cut
+// piece of the chord (the quintic branch of longitudinal_shape::weights), in
+// its narrow form: the compensated basis is the plain B-spline convolved in z
+// with the seven compensation coefficients, which the grid passes apply, so a
+// piece reaches 6 z nodes of Jx and Jy and 5 of Jz.  Every Gauss point of a
+// cut piece lies in the same cell, so the four points' weights are summed per
+// node first and each node visited once.  A piece whose Gauss points straddle
+// a cell (only possible through rounding at a cut) is visited point by point.
+template <class G, class V>
+__device__ __forceinline__ void quintic_linear_segment(const GridT<G>& g, const double x[3],
                                                        const double v[3], double lower,
                                                        double upper, double width, V& visit) {
   using F = typename V::Weight;
@@ -139,81 +171,77 @@ __device__ __forceinline__ void quintic_segment_summed(const GridT<G>& g, const 
                        .3399810435848562648, .8611363115940525752};
   const double qw[4] = {.3478548451374538574, .6521451548625461426,
                         .6521451548625461426, .3478548451374538574};
-  double zz[4];
-  F factor[4], fx[4], fy[4];
-  long long i = 0, j = 0, kz = 0;
+  F factor[4], fx[4], fy[4], fz[4];
+  long long i = 0, j = 0, k = 0;
   bool same = true;
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const double u = .5 * (upper + lower + width * q[t]), xx = x[0] + u * v[0],
-                 yy = x[1] + u * v[1];
-    zz[t] = x[2] + u * v[2];
+                 yy = x[1] + u * v[1], zz = x[2] + u * v[2];
     factor[t] = F(.5 * width * qw[t]);
     long long it = (long long)floor(xx), jt = (long long)floor(yy);
+    const long long kt = (long long)floor(zz);
     if (it == (long long)g.nx) --it;
     if (jt == (long long)g.ny) --jt;
-    const long long kt = (long long)floor(zz[t]);
     fx[t] = F(xx - it);
     fy[t] = F(yy - jt);
+    fz[t] = F(zz - kt);
     if (t == 0) {
       i = it;
       j = jt;
-      kz = kt;
-    } else if (it != i || jt != j || kt != kz) {
-      same = false;
+      k = kt;
     }
+    same = same && it == i && jt == j && kt == k;
   }
   if (!same) {
-    quintic_segment(g, x, v, lower, upper, width, visit);
+    V copy = visit;  // the call takes an address; the visitor itself stays in registers
+#pragma unroll 1
+    for (int t = 0; t < 4; ++t)
+      quintic_linear_point(g, x, v, .5 * (upper + lower + width * q[t]), F(.5 * width * qw[t]),
+                           copy);
+    visit = copy;
     return;
   }
-  // Each Gauss point's spline recursion once.
-  QuinticSplines<F> spline[4];
+  F n[4][6];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) quintic_splines(zz[t], spline[t]);
-  const long long first = (long long)spline[0].cell - 5;
-  // Jx at (i, j + c) and Jy at (i + c, j): node basis, 12 nodes.
-#pragma unroll 1
-  for (int k = 0; k < 12; ++k) {
+  for (int t = 0; t < 4; ++t) spline_edge(fz[t], n[t]);
+  // Jz at (i + a, j + c): edge basis, 5 nodes.
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
     F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
-    bool hit = false;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const F w = factor[t] * quintic_compensated_at(spline[t].node, 5, k);
-      if (w == F(0.)) continue;
-      hit = true;
+      const F w = factor[t] * n[t][m];
+      const F wx = w * fx[t], wo = w * (F(1.) - fx[t]);
+      acc[0] += wo * (F(1.) - fy[t]);
+      acc[1] += wx * (F(1.) - fy[t]);
+      acc[2] += wo * fy[t];
+      acc[3] += wx * fy[t];
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int a = 0; a < 2; ++a) visit(2, i + a, j + c, k - 2 + m, acc[2 * c + a]);
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t) quintic_spline_level(n[t], fz[t], 5);
+  // Jx at (i, j + c) and Jy at (i + c, j): node basis, 6 nodes.
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const F w = factor[t] * n[t][m];
       acc[0] += w * (F(1.) - fy[t]);
       acc[1] += w * fy[t];
       acc[2] += w * (F(1.) - fx[t]);
       acc[3] += w * fx[t];
     }
-    if (!hit) continue;
-    visit(0, i, j, first + k, acc[0]);
-    visit(0, i, j + 1, first + k, acc[1]);
-    visit(1, i, j, first + k, acc[2]);
-    visit(1, i + 1, j, first + k, acc[3]);
-  }
-  // Jz at (i + a, j + c): edge basis, 11 nodes.
-#pragma unroll 1
-  for (int k = 0; k < 11; ++k) {
-    F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
-    bool hit = false;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const F w = factor[t] * quintic_compensated_at(spline[t].edge, 4, k);
-      if (w == F(0.)) continue;
-      hit = true;
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-          acc[2 * c + a] += w * (a ? fx[t] : F(1.) - fx[t]) * (c ? fy[t] : F(1.) - fy[t]);
+    for (int c = 0; c < 2; ++c) {
+      visit(0, i, j + c, k - 2 + m, acc[c]);
+      visit(1, i + c, j, k - 2 + m, acc[2 + c]);
     }
-    if (!hit) continue;
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-#pragma unroll
-      for (int a = 0; a < 2; ++a) visit(2, i + a, j + c, first + k, acc[2 * c + a]);
   }
 }
 
@@ -222,78 +250,93 @@ __device__ __forceinline__ void quintic_segment_summed(const GridT<G>& g, const 
 // when the chord exceeds the 64-cut crossing budget.
 // lattice_shape_weights takes the chord in lattice units: start
 // x = (begin - origin)/h and extent v = (end - begin)/h per axis.
-template <int S, class F, class V>
-__device__ int lattice_shape_weights(const GridT<F>& g, const double x[3], const double v[3],
-                                     V& visit);
-
-template <int S, class F, class V>
-__device__ __forceinline__ int shape_weights(const GridT<F>& g, const double begin[3],
-                                             const double end[3], V& visit) {
-  const double h[3] = {g.dx, g.dy, g.dz};
-  double x[3], v[3];
-  for (int a = 0; a < 3; ++a) {
-    x[a] = (begin[a] - g.origin[a]) / h[a];
-    v[a] = (end[a] - begin[a]) / h[a];
+//
+// The cell-boundary cuts of the chord, ascending.  Along each axis the cuts
+// (j - x)/v of the crossed lattice planes j are already monotone, so a
+// three-way merge yields the sorted cut sequence of the reference (same
+// values, ties give zero-width pieces) without a cut array.  The axes' states
+// are separate scalars: indexed by a run-time axis they would live in local
+// memory.
+struct AxisCuts {
+  double x, v, next;
+  int plane, left, dir;
+  __device__ __forceinline__ double init(double x0, double v0) {  // the number of cuts
+    x = x0;
+    v = v0;
+    next = INFINITY;
+    plane = left = 0;
+    dir = 1;
+    if (v == 0.) return 0.;
+    const double lo = fmin(x, x + v), hi = fmax(x, x + v);
+    const double first = floor(lo) + 1., last = ceil(hi) - 1.;
+    const double count = last >= first ? last - first + 1. : 0.;
+    if (count > 0. && count <= 62.) {
+      left = (int)count;
+      dir = v > 0. ? 1 : -1;
+      plane = (int)(v > 0. ? first : last);
+      next = (plane - x) / v;
+    }
+    return count;
   }
-  return lattice_shape_weights<S>(g, x, v, visit);
-}
+  __device__ __forceinline__ double take() {  // this axis's next cut
+    const double cut = next;
+    plane += dir;
+    next = --left ? (plane - x) / v : INFINITY;
+    return cut;
+  }
+};
 
 template <int S, class F, class V>
 __device__ __forceinline__ int lattice_shape_weights(const GridT<F>& g, const double x[3],
                                                      const double v[3], V& visit) {
-  // The cell-boundary cuts of the chord, ascending.  Along each axis the cuts
-  // (j - x)/v of the crossed lattice planes j are already monotone, so a
-  // three-way merge yields the sorted cut sequence of the reference (same
-  // values, ties give zero-width pieces) without a cut array.
-  double next[3];
-  long long plane[3], left[3];
-  int dir[3];
-  long long total = 0;
-  for (int a = 0; a < 3; ++a) {
-    left[a] = 0;
-    if (v[a] != 0.) {
-      const double lo = fmin(x[a], x[a] + v[a]), hi = fmax(x[a], x[a] + v[a]);
-      const long long first = (long long)floor(lo) + 1, last = (long long)ceil(hi) - 1;
-      left[a] = last >= first ? last - first + 1 : 0;
-      dir[a] = v[a] > 0. ? 1 : -1;
-      plane[a] = v[a] > 0. ? first : last;
-      if (left[a]) next[a] = (plane[a] - x[a]) / v[a];
-    }
-    total += left[a];
-  }
-  if (total > 62) return -1;  // more than 64 cuts with the chord ends
+  AxisCuts a0, a1, a2;
+  if (a0.init(x[0], v[0]) + a1.init(x[1], v[1]) + a2.init(x[2], v[2]) > 62.)
+    return -1;  // more than 64 cuts with the chord ends
   int segments = 0;
   double lower = 0.;
-  for (;;) {
-    int axis = -1;
-    for (int a = 0; a < 3; ++a)
-      if (left[a] && (axis < 0 || next[a] < next[axis])) axis = a;
+  for (bool more = true; more;) {
     double upper = 1.;
-    if (axis >= 0) {
-      upper = next[axis];
-      plane[axis] += dir[axis];
-      if (--left[axis]) next[axis] = (plane[axis] - x[axis]) / v[axis];
-    }
+    if (a0.left && !(a1.next < a0.next) && !(a2.next < a0.next)) upper = a0.take();
+    else if (a1.left && !(a2.next < a1.next)) upper = a1.take();
+    else if (a2.left) upper = a2.take();
+    else more = false;
     const double width = upper - lower;
     const double piece_lower = lower;
     lower = upper;
     if (width > 0.) {
       ++segments;
       if constexpr (S == 0) {
-        if constexpr (V::kF3Segment)
-          visit.f3_segment(g, x, v, piece_lower, upper);
+        if constexpr (V::kOwnSegment)
+          visit.segment(g, x, v, piece_lower, upper);
         else
-          binomial_xz_segment(g, x, v, piece_lower, upper, visit);
+          binomial_linear_segment(g, x, v, piece_lower, upper, visit);
       } else {
-        if constexpr (V::kQuinticSummed)
-          quintic_segment_summed(g, x, v, piece_lower, upper, width, visit);
-        else
-          quintic_segment(g, x, v, piece_lower, upper, width, visit);
+        quintic_linear_segment(g, x, v, piece_lower, upper, width, visit);
       }
     }
-    if (axis < 0) break;
   }
   return segments;
+}
+
+// A chord in lattice units: start x = (begin - origin)/h and extent
+// v = (end - begin)/h per axis.
+template <class F>
+__device__ __forceinline__ void lattice_chord(const GridT<F>& g, const double begin[3],
+                                              const double end[3], double x[3], double v[3]) {
+  const double h[3] = {g.dx, g.dy, g.dz};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    x[a] = divide_by(begin[a] - g.origin[a], h[a], g.inv_h[a]);
+    v[a] = divide_by(end[a] - begin[a], h[a], g.inv_h[a]);
+  }
+}
+
+template <int S, class F, class V>
+__device__ __forceinline__ int shape_weights(const GridT<F>& g, const double begin[3],
+                                             const double end[3], V& visit) {
+  double x[3], v[3];
+  lattice_chord(g, begin, end, x, v);
+  return lattice_shape_weights<S>(g, x, v, visit);
 }
 
 // ---------------------------------------------------------------------------
@@ -318,7 +361,8 @@ __device__ __forceinline__ bool clip_open_orbit(const GridT<F>& g, const double 
     o.end[a] = e[a];
   }
   for (int a = 0; a < 3; ++a) {
-    const double x = (b[a] - g.origin[a]) / ds[a], d = (e[a] - b[a]) / ds[a];
+    const double x = divide_by(b[a] - g.origin[a], ds[a], g.inv_h[a]);
+    const double d = divide_by(e[a] - b[a], ds[a], g.inv_h[a]);
     if (!isfinite(x) || !isfinite(d)) return false;
     if (d == 0.) {
       if (x < 0. || x > size[a]) o.valid = false;
@@ -358,49 +402,28 @@ struct Ptr3 {
 // The cut pieces of a chord in lattice units, one at a time, in the order
 // and with the cut values of shape_weights (longitudinal_shape::weights).
 struct CutWalker {
-  double x[3], v[3], next[3], lower;
-  long long plane[3], left[3];
-  int dir[3];
+  AxisCuts a0, a1, a2;
+  double lower;
   bool done;
   // The chord's lattice coordinates; false beyond the 64-cut budget.
-  __device__ bool init(const double begin[3], const double end[3], const double origin[3],
-                       const double h[3]) {
-    long long total = 0;
-    for (int a = 0; a < 3; ++a) {
-      x[a] = (begin[a] - origin[a]) / h[a];
-      v[a] = (end[a] - begin[a]) / h[a];
-      left[a] = 0;
-      dir[a] = 1;
-      plane[a] = 0;
-      next[a] = 0.;
-      if (v[a] != 0.) {
-        const double lo = fmin(x[a], x[a] + v[a]), hi = fmax(x[a], x[a] + v[a]);
-        const long long first = (long long)floor(lo) + 1, last = (long long)ceil(hi) - 1;
-        left[a] = last >= first ? last - first + 1 : 0;
-        dir[a] = v[a] > 0. ? 1 : -1;
-        plane[a] = v[a] > 0. ? first : last;
-        if (left[a]) next[a] = (plane[a] - x[a]) / v[a];
-      }
-      total += left[a];
-    }
+  template <class F>
+  __device__ __forceinline__ bool init(const GridT<F>& g, const double begin[3],
+                                       const double end[3]) {
+    double x[3], v[3];
+    lattice_chord(g, begin, end, x, v);
+    const double total = a0.init(x[0], v[0]) + a1.init(x[1], v[1]) + a2.init(x[2], v[2]);
     lower = 0.;
     done = false;
-    return total <= 62;
+    return total <= 62.;
   }
   // The next piece of nonzero width, as shape_weights cuts the chord.
-  __device__ bool advance(double& first, double& last) {
+  __device__ __forceinline__ bool advance(double& first, double& last) {
     while (!done) {
-      int axis = -1;
-      for (int a = 0; a < 3; ++a)
-        if (left[a] && (axis < 0 || next[a] < next[axis])) axis = a;
       double upper = 1.;
-      if (axis >= 0) {
-        upper = next[axis];
-        plane[axis] += dir[axis];
-        if (--left[axis]) next[axis] = (plane[axis] - x[axis]) / v[axis];
-      } else {
-        done = true;
-      }
+      if (a0.left && !(a1.next < a0.next) && !(a2.next < a0.next)) upper = a0.take();
+      else if (a1.left && !(a2.next < a1.next)) upper = a1.take();
+      else if (a2.left) upper = a2.take();
+      else done = true;
       const double width = upper - lower;
       first = lower;
       last = upper;
@@ -411,29 +434,95 @@ struct CutWalker {
   }
 };
 
+// The electric gather over the narrow stencil, from the filtered orbit sum
+// (layout of j_index; W is both its type and the arithmetic's).
 template <class W, class F>
-struct ElectricVisitor {
-  static constexpr bool kF3Segment = true;
-  // Quintic pieces arrive with each node's four Gauss-point weights summed:
-  // the gather is linear in the weights, so this reads each S node once
-  // instead of four times; the per-particle sum then differs from the
-  // reference's point-by-point order in the last bits (binomial3 pieces keep
-  // the reference's order exactly).
-  static constexpr bool kQuinticSummed = true;
+struct FilteredVisitor {
+  static constexpr bool kOwnSegment = true;
   using Weight = W;
   const GridT<F>* g;
-  Ptr3<W> s;             // orbit sum S = E_new + E^n per E node (ring layout)
+  Ptr3<W> s;
+  W r[3];
+  // .5*w*S at a node, skipped outside the padded array (where every wide
+  // node the entry stands for is outside the component).
+  __device__ __forceinline__ void operator()(int d, long long i, long long j, long long k, W w) {
+    const GridT<F>& G = *g;
+    if (i < -1 || j < 0 || i > e_nx(G, d) || j >= e_ny(G, d)) return;
+    if (k < -G.jpad || k >= e_nz(G, d) + G.jpad) return;
+    r[d] += W(.5) * w * s.p[d][j_index(G, d, (int)i, (int)j, (int)k)];
+  }
+  __device__ __forceinline__ W at(int d, size_t n) const {
+    return s.p[d][APRL_BOUNDED(g->status, n, j_count(*g, d), 24 + d)];
+  }
+  // One linear-binomial3 piece.  12 reads; in the 4x2x4 form it was 64 and
+  // the reads' latency bound the kernel.
+  __device__ __forceinline__ void segment(const GridT<F>& G, const double s0[3],
+                                          const double d[3], double first, double last) {
+    const double mid = (first + last) * 0.5;
+    const double x = s0[0] + mid * d[0], y = s0[1] + mid * d[1], z = s0[2] + mid * d[2];
+    const double fi = floor(x), fj = floor(y), fk = floor(z);
+    if (!(fi >= 0. && fi < (double)G.nx && fj >= 0. && fj < (double)G.ny && fk >= 0. &&
+          fk < (double)G.nz)) {
+      binomial_linear_segment(G, s0, d, first, last, *this);
+      return;
+    }
+    const int i = (int)fi, j = (int)fj, k = (int)fk;
+    const W fx = W(x - fi), fy = W(y - fj), fz = W(z - fk);
+    const W lx[2] = {W(1.) - fx, fx}, ly[2] = {W(1.) - fy, fy}, lz[2] = {W(1.) - fz, fz};
+    const W width = W(last - first), half = W(.5) * width;
+    const W curvature = width * width * W(1. / 12.);
+    const W xy = curvature * W(d[0]) * W(d[1]);
+    const W xz = curvature * W(d[0]) * W(d[2]);
+    const W yz = curvature * W(d[1]) * W(d[2]);
+    const size_t p0 = (size_t)G.nx + 2, p1 = p0 + 1;  // row pitches of Ex and of Ey, Ez
+    const size_t n0 = ((size_t)(k + G.jpad) * (G.ny + 1) + j) * p0 + (i + 1);
+    const size_t n1 = ((size_t)(k + G.jpad) * G.ny + j) * p1 + (i + 1);
+    const size_t n2 = ((size_t)(k + G.jpad) * (G.ny + 1) + j) * p1 + (i + 1);
+    const size_t z0 = p0 * (G.ny + 1), z1 = p1 * G.ny;
+    W e0[4], e1[4], e2[4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        e0[2 * c + b] = at(0, n0 + (b ? p0 : 0) + (c ? z0 : 0));
+        e1[2 * c + b] = at(1, n1 + b + (c ? z1 : 0));
+        e2[2 * c + b] = at(2, n2 + b + (c ? p1 : 0));
+      }
+    W t0 = W(0.), t1 = W(0.), t2 = W(0.);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        t0 = fma(fma(ly[b], lz[c], b == c ? yz : -yz), e0[2 * c + b], t0);
+        t1 = fma(fma(lx[b], lz[c], b == c ? xz : -xz), e1[2 * c + b], t1);
+        t2 = fma(fma(lx[b], ly[c], b == c ? xy : -xy), e2[2 * c + b], t2);
+      }
+    r[0] = fma(half, t0, r[0]);
+    r[1] = fma(half, t1, r[1]);
+    r[2] = fma(half, t2, r[2]);
+  }
+};
+
+// The electric gather over the wide linear-binomial3 stencil, in the
+// reference's visit order, from the unfiltered orbit sum S = E_new + E^n
+// (binary64, ring layout; rounded to W as it is read).
+template <class W, class F>
+struct DirectVisitor {
+  static constexpr bool kOwnSegment = true;
+  using Weight = W;
+  const GridT<F>* g;
+  Ptr3<double> s;
   W r[3];
   __device__ __forceinline__ void operator()(int d, long long i, long long j, long long k, W w) {
     const GridT<F>& G = *g;
     if (i < 0 || j < 0 || i >= e_nx(G, d) || j >= e_ny(G, d)) return;
     if (k < 0 || k >= e_nz(G, d)) return;
-    r[d] += W(.5) * w * s.p[d][e_index(G, d, (int)i, (int)j, (int)k)];
+    r[d] += W(.5) * w * W(s.p[d][e_index(G, d, (int)i, (int)j, (int)k)]);
   }
 
   // One accumulation .5*w*(E_new + E^n) at the ring offset n of a node.
-  __device__ __forceinline__ W term(int d, size_t n, size_t, W w) const {
-    return W(.5) * w * s.p[d][APRL_BOUNDED(g->status, n, e_count(*g, d), 24 + d)];
+  __device__ __forceinline__ W term(int d, size_t n, W w) const {
+    return W(.5) * w * W(s.p[d][APRL_BOUNDED(g->status, n, e_count(*g, d), 24 + d)]);
   }
 
   // binomialXZSegment specialised for the gather.  When the whole 4x2x4
@@ -442,8 +531,8 @@ struct ElectricVisitor {
   // row is addressed once and its nodes read back to back; otherwise the
   // generic visits run.  Per component the accumulation order is the
   // reference's (Ex: k, y, x; Ey: k, x; Ez: y, x, k).
-  __device__ __forceinline__ void f3_segment(const GridT<F>& G, const double s[3],
-                                             const double d[3], double first, double last) {
+  __device__ __forceinline__ void segment(const GridT<F>& G, const double s[3],
+                                          const double d[3], double first, double last) {
     const W width = W(last - first);
     const double mid = (first + last) * 0.5;
     const double x = s[0] + mid * d[0], y = s[1] + mid * d[1], z = s[2] + mid * d[2];
@@ -473,14 +562,12 @@ struct ElectricVisitor {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const size_t plane = (size_t)ring(K - 1 + c, G.zb_e[0], nzc) * nyc;
-        const size_t jplane = (size_t)(K - 1 + c) * nyc;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
           const W weight = width * (wy[b] * wz[c] + yz * sy[b] * slope[c]);
           const size_t n0 = (plane + J + b) * nxc + (I - 1);
-          const size_t j0 = (jplane + J + b) * nxc + (I - 1);
 #pragma unroll
-          for (int a = 0; a < 3; ++a) r[0] += term(0, n0 + a, j0 + a, weight * edge[a]);
+          for (int a = 0; a < 3; ++a) r[0] += term(0, n0 + a, weight * edge[a]);
         }
       }
     }
@@ -490,21 +577,17 @@ struct ElectricVisitor {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const size_t n0 = ((size_t)ring(K - 1 + c, G.zb_e[1], nzc) * nyc + J) * nxc + (I - 1);
-        const size_t j0 = ((size_t)(K - 1 + c) * nyc + J) * nxc + (I - 1);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
-          r[1] += term(1, n0 + a, j0 + a, width * (wx[a] * wz[c] + xz * slope[a] * slope[c]));
+          r[1] += term(1, n0 + a, width * (wx[a] * wz[c] + xz * slope[a] * slope[c]));
       }
     }
     // Ez (nx+1, ny+1, nz): nodes x I-1..I+2, y J..J+1, z K-1..K+1
     {
       const int nxc = G.nx + 1, nyc = G.ny + 1, nzc = G.nz;
-      size_t plane[3], jplane[3];
+      size_t plane[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        plane[c] = (size_t)ring(K - 1 + c, G.zb_e[2], nzc) * nyc;
-        jplane[c] = (size_t)(K - 1 + c) * nyc;
-      }
+      for (int c = 0; c < 3; ++c) plane[c] = (size_t)ring(K - 1 + c, G.zb_e[2], nzc) * nyc;
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
@@ -512,16 +595,15 @@ struct ElectricVisitor {
           const W weight = width * (wx[a] * wy[b] + xy * slope[a] * sy[b]);
 #pragma unroll
           for (int c = 0; c < 3; ++c)
-            r[2] += term(2, (plane[c] + J + b) * nxc + (I - 1 + a),
-                         (jplane[c] + J + b) * nxc + (I - 1 + a), weight * edge[c]);
+            r[2] += term(2, (plane[c] + J + b) * nxc + (I - 1 + a), weight * edge[c]);
         }
     }
   }
 };
 
 template <class W, class F>
-__device__ __forceinline__ W open_b(const GridT<F>& g, const Ptr3<W>& bsrc, int a, long long i,
-                                    long long j, long long k) {
+__device__ __forceinline__ W open_b(const GridT<F>& g, int a, long long i, long long j,
+                                    long long k) {
   const long long nxc = b_nx(g, a), nyc = b_ny(g, a), nzc = b_nz(g, a);
   if (i < 0) i = 0;
   if (i > nxc - 1) i = nxc - 1;
@@ -529,19 +611,15 @@ __device__ __forceinline__ W open_b(const GridT<F>& g, const Ptr3<W>& bsrc, int 
   if (j > nyc - 1) j = nyc - 1;
   if (k < 0) k = 0;
   if (k >= nzc) k = nzc - 1;
-  return bsrc.p[a][b_index(g, a, (int)i, (int)j, (int)k)];
+  return W(g.b[a][b_index(g, a, (int)i, (int)j, (int)k)]);
 }
 
 // binomialXZMagneticSample (src/source_coupling_math.h:142-167).  Rows of
 // the 4x2x4 stencil that lie inside the component are read without the
 // open-face clamps; the clamped form runs otherwise.  Same order either way.
 template <class W, class F>
-__device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const Ptr3<W>& bsrc,
-                                                     const double p[3], double value[3]) {
-  const double h[3] = {g.dx, g.dy, g.dz};
-  // the point in lattice units, shared by the three components' staggerings
-  double lattice[3];
-  for (int d = 0; d < 3; ++d) lattice[d] = (p[d] - g.origin[d]) / h[d];
+__device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const double lattice[3],
+                                                     double value[3]) {
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     long long cell[3];
@@ -559,7 +637,7 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const Pt
     W v = W(0.);
     if (cell[0] >= 1 && cell[0] + 2 <= nxc - 1 && cell[1] >= 0 && cell[1] + 1 <= nyc - 1 &&
         cell[2] >= 1 && cell[2] + 2 <= nzc - 1) {
-      const W* base = bsrc.p[a];
+      const double* base = g.b[a];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const size_t plane = (size_t)ring((int)cell[2] - 1 + k, g.zb_b[a], (int)nzc) * nyc;
@@ -569,7 +647,7 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const Pt
           W r = W(0.);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            r += wx[i] * base[APRL_BOUNDED(g.status, row + i, b_count(g, a), 27 + a)];
+            r += wx[i] * W(base[APRL_BOUNDED(g.status, row + i, b_count(g, a), 27 + a)]);
           v += wz[k] * wy[j] * r;
         }
       }
@@ -578,7 +656,7 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const Pt
         for (int j = 0; j < 2; ++j) {
           W row = W(0.);
           for (int i = 0; i < 4; ++i)
-            row += wx[i] * open_b(g, bsrc, a, cell[0] - 1 + i, cell[1] + j, cell[2] - 1 + k);
+            row += wx[i] * open_b<W>(g, a, cell[0] - 1 + i, cell[1] + j, cell[2] - 1 + k);
           v += wz[k] * wy[j] * row;
         }
     }
@@ -586,16 +664,53 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const Pt
   }
 }
 
+// binomialXZMagneticSample from the filtered B (layout of bf_index): the
+// 4x2x4 stencil is the trilinear one filtered in x and z, the open faces'
+// clamped nodes included.  8 reads a component instead of 32.
+template <class W, class F>
+__device__ __forceinline__ void filtered_magnetic(const GridT<F>& g, const Ptr3<W>& bf,
+                                                  const double lattice[3], double value[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int nxc = b_nx(g, a), nyc = b_ny(g, a), nzc = b_nz(g, a);
+    int cell[3];
+    W f[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double pos = lattice[d] - (a == d ? 0. : 0.5);
+      const double whole = floor(pos);
+      cell[d] = (int)whole;
+      f[d] = W(pos - whole);
+    }
+    const int i0 = min(max(cell[0], -1), nxc), i1 = min(max(cell[0] + 1, -1), nxc);
+    const int j0 = min(max(cell[1], 0), nyc - 1), j1 = min(max(cell[1] + 1, 0), nyc - 1);
+    const int k0 = min(max(cell[2], -1), nzc), k1 = min(max(cell[2] + 1, -1), nzc);
+    const W* base = bf.p[a];
+    W plane[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      W row[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const W lo = base[bf_index(g, a, i0, j ? j1 : j0, k ? k1 : k0)];
+        const W hi = base[bf_index(g, a, i1, j ? j1 : j0, k ? k1 : k0)];
+        row[j] = fma(f[0], hi, (W(1.) - f[0]) * lo);
+      }
+      plane[k] = fma(f[1], row[1], (W(1.) - f[1]) * row[0]);
+    }
+    value[a] = double(fma(f[2], plane[1], (W(1.) - f[2]) * plane[0]));
+  }
+}
+
 // magneticSample(bounds=false, halo, openFaces=true) (src/source_coupling_math.h:122-138).
 template <class W, class F>
-__device__ __forceinline__ void trilinear_magnetic(const GridT<F>& g, const Ptr3<W>& bsrc,
-                                                   const double p[3], double value[3]) {
-  const double ds[3] = {g.dx, g.dy, g.dz};
+__device__ __forceinline__ void trilinear_magnetic(const GridT<F>& g, const double lattice[3],
+                                                   double value[3]) {
   int cell[2][3];
   double fraction[2][3];
   for (int half = 0; half < 2; ++half)
     for (int d = 0; d < 3; ++d) {
-      const double x = (p[d] - g.origin[d]) / ds[d] - .5 * half;
+      const double x = lattice[d] - .5 * half;
       cell[half][d] = (int)floor(x);
       fraction[half][d] = x - cell[half][d];
     }
@@ -609,7 +724,7 @@ __device__ __forceinline__ void trilinear_magnetic(const GridT<F>& g, const Ptr3
                   y = W(j ? fraction[hy][1] : 1 - fraction[hy][1]),
                   z = W(k ? fraction[hz][2] : 1 - fraction[hz][2]);
           v += x * y * z *
-               open_b(g, bsrc, axis, cell[hx][0] + i, cell[hy][1] + j, cell[hz][2] + k);
+               open_b<W>(g, axis, cell[hx][0] + i, cell[hy][1] + j, cell[hz][2] + k);
         }
     value[axis] = double(v);
   }
@@ -619,24 +734,73 @@ __device__ __forceinline__ void trilinear_magnetic(const GridT<F>& g, const Ptr3
 // (src/source_coupling.cpp:31-51) of one chord a -> b: both clip the chord
 // with clipOpenOrbit, which is done once here; the electric error (crossing
 // budget) skips the magnetic gather, as the reference's call order does.
-template <int S, class W, class F>
+//
+// A chord whose ends lie so far inside the domain that every face test of
+// clipOpenOrbit leaves it whole (the tests below are the ones its quotients
+// would decide, without the quotients) keeps its own ends.
+//
+// DE: the wide electric stencil from the unfiltered S; else the filtered one.
+// DB: the wide magnetic stencil from B; else the filtered B (linear-binomial3).
+template <class W>
+struct GatherSource {
+  Ptr3<W> filtered;       // filtered orbit sum
+  Ptr3<double> sum;       // unfiltered orbit sum S0 = E* + E^n (DE)
+  Ptr3<W> magnetic;       // filtered B (unless DB)
+};
+
+template <class W>
+__device__ __forceinline__ GatherSource<W> gather_source(const GatherArrays& a) {
+  GatherSource<W> s;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    s.filtered.p[d] = static_cast<const W*>(a.filtered[d]);
+    s.sum.p[d] = a.sum[d];
+    s.magnetic.p[d] = static_cast<const W*>(a.magnetic[d]);
+  }
+  return s;
+}
+
+template <int S, bool DE, bool DB, class W, class F>
 __device__ __forceinline__ unsigned gather_fields(const GridT<F>& g, const double a[3],
-                                                  const double b[3], const Ptr3<W>& orbit,
-                                                  const Ptr3<W>& bsrc, double e_out[3],
-                                                  double b_out[3]) {
-  OpenOrbit path;
-  if (!clip_open_orbit(g, a, b, path)) return kErrNonFinite;
-  if (!path.valid) return kErrOrbitOutside;
-  double middle[3];
-  for (int d = 0; d < 3; ++d) middle[d] = (path.begin[d] + path.end[d]) * .5;
-  const double fraction = path.last - path.first;
-  ElectricVisitor<W, F> ev{&g, orbit, {W(0.), W(0.), W(0.)}};
-  if (shape_weights<S>(g, path.begin, path.end, ev) < 0) return kErrCrossingBudget;
-  for (int d = 0; d < 3; ++d) e_out[d] = double(ev.r[d]) * fraction;
-  if constexpr (S == 0)
-    binomial_xz_magnetic(g, bsrc, middle, b_out);
+                                                  const double b[3], const GatherSource<W>& src,
+                                                  double e_out[3], double b_out[3]) {
+  const double size[3] = {(double)g.nx, (double)g.ny, (double)g.nz};
+  double x[3], v[3], middle[3], fraction = 1.;
+  lattice_chord(g, a, b, x, v);
+  bool whole = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    whole = whole && x[d] >= 0. && size[d] - x[d] >= 0. &&
+            (v[d] >= 0. ? size[d] - x[d] >= v[d] : x[d] >= -v[d]);
+  if (whole) {
+    for (int d = 0; d < 3; ++d) middle[d] = (a[d] + b[d]) * .5;
+  } else {
+    OpenOrbit path;
+    if (!clip_open_orbit(g, a, b, path)) return kErrNonFinite;
+    if (!path.valid) return kErrOrbitOutside;
+    for (int d = 0; d < 3; ++d) middle[d] = (path.begin[d] + path.end[d]) * .5;
+    fraction = path.last - path.first;
+    lattice_chord(g, path.begin, path.end, x, v);
+  }
+  if constexpr (DE) {
+    DirectVisitor<W, F> ev{&g, src.sum, {W(0.), W(0.), W(0.)}};
+    if (lattice_shape_weights<S>(g, x, v, ev) < 0) return kErrCrossingBudget;
+    for (int d = 0; d < 3; ++d) e_out[d] = double(ev.r[d]) * fraction;
+  } else {
+    FilteredVisitor<W, F> ev{&g, src.filtered, {W(0.), W(0.), W(0.)}};
+    if (lattice_shape_weights<S>(g, x, v, ev) < 0) return kErrCrossingBudget;
+    for (int d = 0; d < 3; ++d) e_out[d] = double(ev.r[d]) * fraction;
+  }
+  const double h[3] = {g.dx, g.dy, g.dz};
+  double lattice[3];
+  for (int d = 0; d < 3; ++d)
+    lattice[d] = divide_by(middle[d] - g.origin[d], h[d], g.inv_h[d]);
+  if constexpr (S != 0)
+    trilinear_magnetic<W>(g, lattice, b_out);
+  else if constexpr (DB)
+    binomial_xz_magnetic<W>(g, lattice, b_out);
   else
-    trilinear_magnetic(g, bsrc, middle, b_out);
+    filtered_magnetic(g, src.magnetic, lattice, b_out);
   return kErrNone;
 }
 
@@ -646,8 +810,7 @@ __device__ __forceinline__ unsigned gather_fields(const GridT<F>& g, const doubl
 // of binary64 atomics into J.
 template <class F, bool Q>
 struct DepositVisitor {
-  static constexpr bool kF3Segment = false;
-  static constexpr bool kQuinticSummed = true;
+  static constexpr bool kOwnSegment = false;
   using Weight = F;
   const GridT<F>* g;
   F scale[3];
@@ -656,7 +819,9 @@ struct DepositVisitor {
   __device__ __forceinline__ void operator()(int a, long long i, long long j, long long k, F w) {
     if (scale[a] == F(0.)) return;
     const GridT<F>& G = *g;
-    if (i < 0 || i >= e_nx(G, a)) {
+    // linear-binomial3: a raw node one step outside still reaches the
+    // component through the x filter; the x support may leave the grid.
+    if (smooth_x ? i < -1 || i > e_nx(G, a) : i < 0 || i >= e_nx(G, a)) {
       if (!smooth_x) error = kErrSupportX;
       return;
     }
@@ -664,7 +829,7 @@ struct DepositVisitor {
       error = kErrSupportY;
       return;
     }
-    if (k < 0 || k >= e_nz(G, a)) return;
+    if (k < -G.jpad || k >= e_nz(G, a) + G.jpad) return;
     const size_t at = j_index(G, a, (int)i, (int)j, (int)k);
     if constexpr (Q) {
       // Order-free integer sum, converted to J once per trial.
@@ -691,11 +856,14 @@ __device__ __forceinline__ unsigned validate_segment(const GridT<F>& g, const do
   return kErrNone;
 }
 
+// Longitudinal-shape Current::deposit without the depositor's endpoint
+// validation (src/longitudinal_shape.h:175-187): the upstream part of an
+// admitted held particle and the frozen source support
+// (src/source_coupling.cpp:73-78) deposit this way.  Not inlined: the kernels
+// call it from several places, and the quintic walk is long.
 template <int S, bool Q, class F>
-__device__ unsigned deposit_segment(const GridT<F>& g, const double b[3],
-                                    const double e[3], double charge) {
-  const unsigned invalid = validate_segment(g, b, e, charge);
-  if (invalid) return invalid;
+__device__ __noinline__ unsigned deposit_current(const GridT<F>& g, const double b[3],
+                                                 const double e[3], double charge) {
   DepositVisitor<F, Q> v;
   v.g = &g;
   v.smooth_x = S == 0;
@@ -704,6 +872,13 @@ __device__ unsigned deposit_segment(const GridT<F>& g, const double b[3],
     v.scale[a] = F(charge * (e[a] - b[a]) / (g.dx * g.dy * g.dz * g.dt));
   if (shape_weights<S>(g, b, e, v) < 0) return kErrCrossingBudget;
   return v.error;
+}
+
+template <int S, bool Q, class F>
+__device__ __forceinline__ unsigned deposit_segment(const GridT<F>& g, const double b[3],
+                                                    const double e[3], double charge) {
+  const unsigned invalid = validate_segment(g, b, e, charge);
+  return invalid ? invalid : deposit_current<S, Q>(g, b, e, charge);
 }
 
 // ---------------------------------------------------------------------------
@@ -1017,7 +1192,7 @@ __device__ unsigned carrier_segment(const GridT<F>& g, const DRegion& r,
 // (src/simulation.cpp:4531-4537).  Carriers deposit with the run's shape,
 // like every ChargeConservingCurrentDepositor call.
 template <class F, int S, bool Q>
-__global__ void carrier_kernel(CarrierArgs<F> a) {
+__global__ void carrier_kernel(const __grid_constant__ CarrierArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
@@ -1081,23 +1256,6 @@ __device__ unsigned coupling_push(const PushArgs<F>& a, long long n, double pos[
   return kErrNone;
 }
 
-// Longitudinal-shape Current::deposit without the depositor's endpoint
-// validation (src/longitudinal_shape.h:175-187): the upstream part of an
-// admitted held particle and the frozen source support
-// (src/source_coupling.cpp:73-78) deposit this way.
-template <int S, bool Q, class F>
-__device__ unsigned deposit_current(const GridT<F>& g, const double b[3],
-                                    const double e[3], double charge) {
-  DepositVisitor<F, Q> v;
-  v.g = &g;
-  v.smooth_x = S == 0;
-  v.error = kErrNone;
-  for (int a = 0; a < 3; ++a)
-    v.scale[a] = F(charge * (e[a] - b[a]) / (g.dx * g.dy * g.dz * g.dt));
-  if (shape_weights<S>(g, b, e, v) < 0) return kErrCrossingBudget;
-  return v.error;
-}
-
 // Where the coupled push of one particle starts this step: prepareParticle
 // with hold_transverse_until_activation (src/simulation.cpp:4919-5035).  An
 // active particle is pushed from the step start over dt; a held particle
@@ -1152,8 +1310,8 @@ __device__ __forceinline__ SlotPlan plan_slot(const GridT<F>& g, const DFrame& f
 // (Impl::Slot::guess, src/source_coupling.cpp:92-95), gathered from E*
 // before any current of the trial is deposited; the push reads them as the
 // previous residual's fields.
-template <class W, class F, int S>
-__global__ void APRL_GATHER_BOUNDS guess_gather_kernel(PushArgs<F> a) {
+template <class W, class F, int S, bool D>
+__global__ void APRL_GATHER_BOUNDS guess_gather_kernel(const __grid_constant__ PushArgs<F> a) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
   const double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
@@ -1167,11 +1325,8 @@ __global__ void APRL_GATHER_BOUNDS guess_gather_kernel(PushArgs<F> a) {
   const double guess[3] = {s.start[0] + sc * u[0], s.start[1] + sc * u[1],
                            s.start[2] + sc * u[2]};
   double ne[3], nb[3];
-  const Ptr3<W> orbit{{static_cast<const W*>(a.orbit[0]), static_cast<const W*>(a.orbit[1]),
-                       static_cast<const W*>(a.orbit[2])}};
-  const Ptr3<W> bsrc{{static_cast<const W*>(a.bgather[0]), static_cast<const W*>(a.bgather[1]),
-                      static_cast<const W*>(a.bgather[2])}};
-  const unsigned err = gather_fields<S>(a.g, s.start, guess, orbit, bsrc, ne, nb);
+  const unsigned err =
+      gather_fields<S, D, D>(a.g, s.start, guess, gather_source<W>(a.src), ne, nb);
   if (err) raise_error(a.status, err, (unsigned long long)n);
   double* next_e = const_cast<double*>(a.next_e);
   double* next_b = const_cast<double*>(a.next_b);
@@ -1188,7 +1343,7 @@ __global__ void APRL_GATHER_BOUNDS guess_gather_kernel(PushArgs<F> a) {
 // with Simulation::firstMovingWindowEntry
 // (src/simulation_moving_window.cpp:380-395).
 template <class F, int S, bool Q>
-__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(PushArgs<F> a) {
+__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(const __grid_constant__ PushArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
@@ -1366,18 +1521,16 @@ __global__ void APRL_PUSH_BOUNDS push_deposit_kernel(PushArgs<F> a) {
 // ---------------------------------------------------------------------------
 // The deposit of the main chords of linear-binomial3 particles
 // (Current::deposit, src/longitudinal_shape.h:175-187, with the cut pieces of
-// weights() and binomialXZSegment, :61-117), one thread per particle with the
-// warp converged.  The warp walks the cut pieces of its lanes' chords in
-// step: at each step every lane holds at most one piece, whose 4x2x4 node
-// block is fixed by the piece's cell (i, j, k).  Particles are stored in cell
-// order, so lanes holding pieces of the same cell sit side by side; such a
-// run of lanes adds its 32 stencil weights (8 Jx, 16 Jy, 8 Jz products of
-// the x, y and z factors; the edge smoothing [1/4, 1/2, 1/4] of Jx along x
-// and of Jz along z is applied after the sum) with a segmented shuffle scan,
-// and the run's last lane issues the 64 reductions for all of them.  A lone
-// lane adds its own weights.  The weights are binomialXZSegment's; only the
-// order of the floating-point additions into J differs from one reduction
-// per particle and node.
+// weights() and binomialXZSegment, :61-117) into the raw current, one thread
+// per particle with the warp converged.  The warp walks the cut pieces of its
+// lanes' chords in step: at each step every lane holds at most one piece,
+// whose 12 narrow weights (binomial_linear_segment) fall on the 2x2 nodes of
+// each component around the piece's cell (i, j, k).  Particles are stored in
+// cell order, so lanes holding pieces of the same cell sit side by side; such
+// a run of lanes adds its weights with a segmented shuffle scan, and the
+// run's last lane issues the reductions for all of them.  A lone lane adds
+// its own weights.  Only the order of the floating-point additions into J
+// differs from one reduction per particle and node.
 // Inclusive sum of v over the lanes from `head` (the first lane of this
 // lane's run) to this lane; `span` = the longest run in the warp.
 __device__ __forceinline__ double run_sum(double v, int lane, int head, unsigned span) {
@@ -1388,43 +1541,10 @@ __device__ __forceinline__ double run_sum(double v, int lane, int head, unsigned
   return v;
 }
 
-// The 4x2x4 node block of component `ax` around a piece in cell (i, j, k):
-// nodes (i-1+x, j+b, k-1+c), with in-range masks per x, b and c.
-struct ChordBlock {
-  long long base, row, plane;
-  unsigned xok, yok, zok;
-  __device__ __forceinline__ bool in(int c, int b) const {
-    return ((zok >> c) & 1u) && ((yok >> b) & 1u);
-  }
-  __device__ __forceinline__ size_t at(int c, int b, int x) const {
-    return (size_t)(base + c * plane + b * row + x);
-  }
-};
-
-// `levels`: z levels k-1 .. k-2+levels.
-__device__ __forceinline__ ChordBlock chord_block(const DGrid& g, int ax, long long i,
-                                                  long long j, long long k, int levels) {
-  const long long nxc = e_nx(g, ax), nyc = e_ny(g, ax), nzc = e_nz(g, ax);
-  ChordBlock s;
-  s.row = nxc;
-  s.plane = nxc * nyc;
-  s.base = ((k - 1) * nyc + j) * nxc + (i - 1);
-  s.xok = s.yok = s.zok = 0u;
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-    if (i - 1 + x >= 0 && i - 1 + x < nxc) s.xok |= 1u << x;
-#pragma unroll
-  for (int b = 0; b < 2; ++b)
-    if (j + b >= 0 && j + b < nyc) s.yok |= 1u << b;
-#pragma unroll
-  for (int c = 0; c < 5; ++c)
-    if (c < levels && k - 1 + c >= 0 && k - 1 + c < nzc) s.zok |= 1u << c;
-  return s;
-}
-
 template <bool Q>
 __device__ __forceinline__ void chord_add(const DGrid& g, int a, size_t at, double v,
                                           unsigned& err) {
+  at = APRL_BOUNDED(g.status, at, j_count(g, a), 30 + a);
   if constexpr (Q) {
     if (!fixed_add(g.jq[a] + 2 * at, v, g.jq_scale)) err = kErrFixedRange;
   } else {
@@ -1432,10 +1552,10 @@ __device__ __forceinline__ void chord_add(const DGrid& g, int a, size_t at, doub
   }
 }
 
-// One cut piece's cell and binomialXZSegment factors.
+// One cut piece's cell and narrow factors.
 struct PieceGeometry {
-  long long i, j, k;
-  double wx[4], wz[4], wy[2];
+  int i, j, k;
+  double fx, fy, fz;
   double width, xy, xz, yz;
 };
 
@@ -1443,23 +1563,35 @@ __device__ __forceinline__ void piece_geometry(const DGrid& g, const CutWalker& 
                                                double last, PieceGeometry& p) {
   p.width = last - first;
   const double mid = (first + last) * 0.5;
-  const double px = w.x[0] + mid * w.v[0], py = w.x[1] + mid * w.v[1], pz = w.x[2] + mid * w.v[2];
-  p.i = (long long)floor(px);
-  p.j = (long long)floor(py);
-  p.k = (long long)floor(pz);
-  if (p.i == (long long)g.nx) --p.i;
-  if (p.j == (long long)g.ny) --p.j;
-  node_weights(px - p.i, p.wx);
-  node_weights(pz - p.k, p.wz);
-  p.wy[0] = 1. - (py - p.j);
-  p.wy[1] = py - p.j;
+  const double px = w.a0.x + mid * w.a0.v, py = w.a1.x + mid * w.a1.v,
+               pz = w.a2.x + mid * w.a2.v;
+  // the endpoints are inside the domain to roundoff (validate_segment)
+  p.i = (int)floor(px);
+  p.j = (int)floor(py);
+  p.k = (int)floor(pz);
+  if (p.i == g.nx) --p.i;
+  if (p.j == g.ny) --p.j;
+  p.fx = px - p.i;
+  p.fy = py - p.j;
+  p.fz = pz - p.k;
   const double curvature = p.width * p.width / 12.;
-  p.xy = curvature * w.v[0] * w.v[1];
-  p.xz = curvature * w.v[0] * w.v[2];
-  p.yz = curvature * w.v[1] * w.v[2];
+  p.xy = curvature * w.a0.v * w.a1.v;
+  p.xz = curvature * w.a0.v * w.a2.v;
+  p.yz = curvature * w.a1.v * w.a2.v;
 }
 
-__device__ __forceinline__ unsigned long long piece_key(long long i, long long j, long long k,
+// The 2x2 narrow weights of a piece over two directions, index 2 * second +
+// first, for fractions f (first) and h (second).
+__device__ __forceinline__ void piece_weights(double width, double f, double h, double cross,
+                                              double scale, double out[4]) {
+  const double s = scale * width, g = 1. - f, d = 1. - h;
+  out[0] = s * (g * d + cross);
+  out[1] = s * (f * d - cross);
+  out[2] = s * (g * h - cross);
+  out[3] = s * (f * h + cross);
+}
+
+__device__ __forceinline__ unsigned long long piece_key(int i, int j, int k,
                                                         unsigned long long kind) {
   return (kind << 63) | ((unsigned long long)(k + 2) << 42) |
          ((unsigned long long)(j + 2) << 21) | (unsigned long long)(i + 2);
@@ -1503,172 +1635,61 @@ __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(ChordArgs a) {
     }
     const double q = a.q[n];
     for (int d = 0; d < 3; ++d) scale[d] = q * (e[d] - b[d]) / (g.dx * g.dy * g.dz * g.dt);
-    const double h[3] = {g.dx, g.dy, g.dz};
-    if (!w.init(b, e, g.origin, h)) {
+    if (!w.init(g, b, e)) {
       err = kErrCrossingBudget;
       alive = false;
     }
   }
-  const double edge[3] = {0.25, 0.5, 0.25};
-  const double slope[4] = {-0.25, -0.25, 0.25, 0.25};
-  const double sy[2] = {-1., 1.};
-  // ---- chords of exactly two pieces in z-neighbouring cells of one (i, j)
-  // column (a chord crossing one z plane: nearly every chord of a beam that
-  // moves about a cell per step along z).  Their stencils overlap, so the two
-  // pieces are added per node of the union before the reductions: 82 nodes
-  // instead of 2 x 64.
-  double f0 = 0., l0 = 0., f1 = 0., l1 = 0.;
-  bool pair = false;
-  if (alive) {
-    const bool two = w.advance(f0, l0) && w.advance(f1, l1);
-    double fx, lx;
-    if (two && !w.advance(fx, lx)) {
-      PieceGeometry p0, p1;
-      piece_geometry(g, w, f0, l0, p0);
-      piece_geometry(g, w, f1, l1, p1);
-      pair = p0.i == p1.i && p0.j == p1.j && (p1.k - p0.k == 1 || p0.k - p1.k == 1);
-      if (pair && p1.k < p0.k) {  // lower piece first
-        double t = f0; f0 = f1; f1 = t;
-        t = l0; l0 = l1; l1 = t;
-      }
-    }
-    if (!pair) {  // the general walk below starts over
-      double b[3], e[3];
-      for (int d = 0; d < 3; ++d) {
-        b[d] = a.b[d][n];
-        e[d] = a.e[d][n];
-      }
-      const double h[3] = {g.dx, g.dy, g.dz};
-      w.init(b, e, g.origin, h);
-    }
-  }
-  if (__any_sync(0xffffffffu, pair)) {
-    PieceGeometry lo, up;
-    unsigned long long key = ~0ull - (unsigned long long)lane;
-    if (pair) {
-      piece_geometry(g, w, f0, l0, lo);
-      piece_geometry(g, w, f1, l1, up);
-      key = piece_key(lo.i, lo.j, lo.k, 1);
-    } else {
-      lo = PieceGeometry{};
-      up = PieceGeometry{};
-    }
-    const Runs runs = lane_runs(key, lane);
-    const bool adds = pair && runs.last;
-    const long long i = lo.i, j = lo.j, k = lo.k;
-    // Node blocks of the union: z levels k-1 .. k+3 (Jx, Jy) and k-1 .. k+2 (Jz).
-    const ChordBlock bx = chord_block(g, 0, i, j, k, 5), by = chord_block(g, 1, i, j, k, 5),
-                     bz = chord_block(g, 2, i, j, k, 4);
-    if (pair) {
-      if (scale[0] != 0. && (bx.xok & 7u) && (bx.yok & 3u) != 3u) err = kErrSupportY;
-      if (scale[1] != 0. && (by.xok & 15u) && !(by.yok & 1u)) err = kErrSupportY;
-      if (scale[2] != 0. && (bz.xok & 15u) && (bz.yok & 3u) != 3u) err = kErrSupportY;
-    }
-    // Jx: level zz takes the lower piece's c = zz and the upper's c = zz - 1.
-#pragma unroll
-    for (int zz = 0; zz < 5; ++zz) {
-#pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        double v = 0.;
-        if (zz < 4) v += lo.width * (lo.wy[b] * lo.wz[zz] + lo.yz * sy[b] * slope[zz]);
-        if (zz >= 1)
-          v += up.width * (up.wy[b] * up.wz[zz - 1] + up.yz * sy[b] * slope[zz - 1]);
-        const double total = run_sum(scale[0] * v, lane, runs.head, runs.span);
-        if (adds && total != 0. && bx.in(zz, b))
-#pragma unroll
-          for (int x = 0; x < 3; ++x)
-            if ((bx.xok >> x) & 1u) chord_add<Q>(g, 0, bx.at(zz, b, x), total * edge[x], err);
-      }
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        double v = 0.;
-        if (zz < 4) v += lo.width * (lo.wx[x] * lo.wz[zz] + lo.xz * slope[x] * slope[zz]);
-        if (zz >= 1)
-          v += up.width * (up.wx[x] * up.wz[zz - 1] + up.xz * slope[x] * slope[zz - 1]);
-        const double total = run_sum(scale[1] * v, lane, runs.head, runs.span);
-        if (adds && total != 0. && by.in(zz, 0) && ((by.xok >> x) & 1u))
-          chord_add<Q>(g, 1, by.at(zz, 0, x), total, err);
-      }
-    }
-    // Jz: each piece's weight is smoothed over three z nodes (its k-1, k,
-    // k+1), so the lower piece covers levels 0..2 and the upper 1..3.
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const double vl = lo.width * (lo.wx[x] * lo.wy[b] + lo.xy * slope[x] * sy[b]);
-        const double vu = up.width * (up.wx[x] * up.wy[b] + up.xy * slope[x] * sy[b]);
-        const double tl = run_sum(scale[2] * vl, lane, runs.head, runs.span);
-        const double tu = run_sum(scale[2] * vu, lane, runs.head, runs.span);
-        if (adds && ((bz.xok >> x) & 1u) && ((bz.yok >> b) & 1u)) {
-          const double level[4] = {tl * edge[0], tl * edge[1] + tu * edge[0],
-                                   tl * edge[2] + tu * edge[1], tu * edge[2]};
-#pragma unroll
-          for (int zz = 0; zz < 4; ++zz)
-            if (((bz.zok >> zz) & 1u) && level[zz] != 0.)
-              chord_add<Q>(g, 2, bz.at(zz, b, x), level[zz], err);
-        }
-      }
-  }
-  if (pair) alive = false;
-  // ---- every other chord, one piece per lane per round
+  const long long p0 = g.nx + 2, p1 = g.nx + 3;  // row pitches of Jx and of Jy, Jz
+  const long long z0 = p0 * (g.ny + 1), z1 = p1 * g.ny;
+  // ---- one piece per lane per round; a chord of a beam that moves about a
+  // cell per step along z has two, in z-neighbouring cells.
   while (__any_sync(0xffffffffu, alive)) {
     double first = 0., last = 0.;
     const bool have = alive && w.advance(first, last);
     if (!have) alive = false;
     // A lane without a piece takes a key no other lane has and adds nothing.
-    PieceGeometry p;
+    PieceGeometry p{};
     unsigned long long key = ~0ull - (unsigned long long)lane;
     if (have) {
       piece_geometry(g, w, first, last, p);
       key = piece_key(p.i, p.j, p.k, 0);
-    } else {
-      p = PieceGeometry{};
     }
     const Runs runs = lane_runs(key, lane);
-    const bool adds = have && runs.last;
-    const long long i = p.i, j = p.j, k = p.k;
-    // The three node blocks of the piece, with the visitor's support rules
-    // for this lane: x outside is skipped (the F3 x-support may leave the
-    // grid), y outside is an error when the lane carries current on that
-    // axis, z outside is skipped.  The run's sums are added by its last lane.
-    const ChordBlock bx = chord_block(g, 0, i, j, k, 4), by = chord_block(g, 1, i, j, k, 4),
-                     bz = chord_block(g, 2, i, j, k, 4);
-    if (have) {
-      if (scale[0] != 0. && (bx.xok & 7u) && (bx.yok & 3u) != 3u) err = kErrSupportY;
-      if (scale[1] != 0. && (by.xok & 15u) && !(by.yok & 1u)) err = kErrSupportY;
-      if (scale[2] != 0. && (bz.xok & 15u) && (bz.yok & 3u) != 3u) err = kErrSupportY;
+    // The visitor's support rules: x outside is skipped (the F3 x support may
+    // leave the grid; the raw array holds the nodes one step outside, which
+    // still reach it), y outside is an error when the lane carries current on
+    // that axis, z outside the padding is skipped.
+    const bool y_inside = p.j >= 0 && p.j < g.ny;
+    if (have && !y_inside && (scale[0] != 0. || scale[1] != 0. || scale[2] != 0.))
+      err = kErrSupportY;
+    const bool adds = have && runs.last && y_inside && p.i >= -1 && p.i <= g.nx && p.k >= -1 &&
+                      p.k <= g.nz;
+    const long long n0 = ((p.k + 1) * (long long)(g.ny + 1) + p.j) * p0 + (p.i + 1);
+    const long long n1 = ((p.k + 1) * (long long)g.ny + p.j) * p1 + (p.i + 1);
+    const long long n2 = ((p.k + 1) * (long long)(g.ny + 1) + p.j) * p1 + (p.i + 1);
+    double v[4];
+    piece_weights(p.width, p.fy, p.fz, p.yz, scale[0], v);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {  // Jx: y, z
+      const double total = run_sum(v[t], lane, runs.head, runs.span);
+      if (adds && total != 0.)
+        chord_add<Q>(g, 0, n0 + (t & 1 ? p0 : 0) + (t & 2 ? z0 : 0), total, err);
     }
+    piece_weights(p.width, p.fx, p.fz, p.xz, scale[1], v);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const double weight = p.width * (p.wy[b] * p.wz[c] + p.yz * sy[b] * slope[c]);
-        const double total = run_sum(scale[0] * weight, lane, runs.head, runs.span);
-        if (adds && total != 0. && bx.in(c, b))
-#pragma unroll
-          for (int x = 0; x < 3; ++x)
-            if ((bx.xok >> x) & 1u) chord_add<Q>(g, 0, bx.at(c, b, x), total * edge[x], err);
-      }
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const double weight = p.width * (p.wx[x] * p.wz[c] + p.xz * slope[x] * slope[c]);
-        const double total = run_sum(scale[1] * weight, lane, runs.head, runs.span);
-        if (adds && total != 0. && by.in(c, 0) && ((by.xok >> x) & 1u))
-          chord_add<Q>(g, 1, by.at(c, 0, x), total, err);
-      }
+    for (int t = 0; t < 4; ++t) {  // Jy: x, z
+      const double total = run_sum(v[t], lane, runs.head, runs.span);
+      if (adds && total != 0.)
+        chord_add<Q>(g, 1, n1 + (t & 1) + (t & 2 ? z1 : 0), total, err);
     }
+    piece_weights(p.width, p.fx, p.fy, p.xy, scale[2], v);
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const double weight = p.width * (p.wx[x] * p.wy[b] + p.xy * slope[x] * sy[b]);
-        const double total = run_sum(scale[2] * weight, lane, runs.head, runs.span);
-        if (adds && total != 0. && ((bz.xok >> x) & 1u) && ((bz.yok >> b) & 1u))
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            if ((bz.zok >> c) & 1u) chord_add<Q>(g, 2, bz.at(c, b, x), total * edge[c], err);
-      }
+    for (int t = 0; t < 4; ++t) {  // Jz: x, y
+      const double total = run_sum(v[t], lane, runs.head, runs.span);
+      if (adds && total != 0.)
+        chord_add<Q>(g, 2, n2 + (t & 1) + (t & 2 ? p1 : 0), total, err);
+    }
   }
   if (err) raise_error(a.status, err, (unsigned long long)n);
 }
@@ -1725,8 +1746,8 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-template <class W, class F, int S>
-__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(ResidualArgs<F> a) {
+template <class W, class F, int S, bool DB>
+__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ ResidualArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double force = 0.0, defect = 0.0, scale = 0.0;
@@ -1743,13 +1764,8 @@ __global__ void APRL_RESIDUAL_BOUNDS residual_kernel(ResidualArgs<F> a) {
     }
     const double last[3] = {a.x1[n], a.y1[n], a.z1[n]};
     double ne[3], nb[3];
-    const Ptr3<W> orbit{{static_cast<const W*>(a.orbit[0]),
-                         static_cast<const W*>(a.orbit[1]),
-                         static_cast<const W*>(a.orbit[2])}};
-    const Ptr3<W> bsrc{{static_cast<const W*>(a.bgather[0]),
-                        static_cast<const W*>(a.bgather[1]),
-                        static_cast<const W*>(a.bgather[2])}};
-    const unsigned err = gather_fields<S>(a.g, first, last, orbit, bsrc, ne, nb);
+    const unsigned err =
+        gather_fields<S, false, DB>(a.g, first, last, gather_source<W>(a.src), ne, nb);
     if (err) {
       raise_error(a.status, err, (unsigned long long)n);
       for (int d = 0; d < 3; ++d) ne[d] = nb[d] = 0.0;
@@ -2118,7 +2134,7 @@ __global__ void admit_kernel(DParticles out, long long first_slot, DPending src,
 // src/simulation.cpp:4170-4172, src/source_coupling.cpp:73-78): each
 // deposits its held chord of this step without endpoint validation.
 template <class F, int S, bool Q>
-__global__ void frozen_support_kernel(SupportArgs<F> a) {
+__global__ void frozen_support_kernel(const __grid_constant__ SupportArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.count) return;
@@ -2231,7 +2247,7 @@ __global__ void trial_clear_kernel(GridT<double> g, TrialCounters* counters, Res
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (int c = 0; c < 3 && clear_current; ++c) {
-    const long long count = (long long)e_nx(g, c) * e_ny(g, c) * e_nz(g, c);
+    const long long count = (long long)j_count(g, c);
     if (clear_current == 2) {
       ulonglong2* pairs = reinterpret_cast<ulonglong2*>(g.jq[c]);
       for (long long n = first; n < count; n += stride) pairs[n] = make_ulonglong2(0ull, 0ull);
@@ -2250,7 +2266,7 @@ __global__ void current_convert_kernel(GridT<double> g, double unscale) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (int c = 0; c < 3; ++c) {
-    const long long count = (long long)e_nx(g, c) * e_ny(g, c) * e_nz(g, c);
+    const long long count = (long long)j_count(g, c);
     const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(g.jq[c]);
     for (long long n = first; n < count; n += stride) {
       const ulonglong2 v = pairs[n];
@@ -2284,18 +2300,23 @@ __global__ void trial_verdict_kernel(const ResidualSums* sums, unsigned iteratio
 // 1 quintic-compensated), so a kernel carries the registers and local
 // memory of its own shape's weights only.
 #define APRL_SHAPE_KERNELS(S)                                                        \
-  template __global__ void push_deposit_kernel<double, S, false>(PushArgs<double>);  \
-  template __global__ void push_deposit_kernel<double, S, true>(PushArgs<double>);   \
-  template __global__ void carrier_kernel<double, S, false>(CarrierArgs<double>);    \
-  template __global__ void carrier_kernel<double, S, true>(CarrierArgs<double>);     \
-  template __global__ void frozen_support_kernel<double, S, false>(SupportArgs<double>); \
-  template __global__ void frozen_support_kernel<double, S, true>(SupportArgs<double>); \
-  template __global__ void guess_gather_kernel<double, double, S>(PushArgs<double>); \
-  template __global__ void guess_gather_kernel<float, double, S>(PushArgs<double>);  \
-  template __global__ void residual_kernel<double, double, S>(ResidualArgs<double>); \
-  template __global__ void residual_kernel<float, double, S>(ResidualArgs<double>);
+  template __global__ void push_deposit_kernel<double, S, false>(const __grid_constant__ PushArgs<double>);  \
+  template __global__ void push_deposit_kernel<double, S, true>(const __grid_constant__ PushArgs<double>);   \
+  template __global__ void carrier_kernel<double, S, false>(const __grid_constant__ CarrierArgs<double>);    \
+  template __global__ void carrier_kernel<double, S, true>(const __grid_constant__ CarrierArgs<double>);     \
+  template __global__ void frozen_support_kernel<double, S, false>(const __grid_constant__ SupportArgs<double>); \
+  template __global__ void frozen_support_kernel<double, S, true>(const __grid_constant__ SupportArgs<double>); \
+  template __global__ void guess_gather_kernel<double, double, S, false>(const __grid_constant__ PushArgs<double>); \
+  template __global__ void guess_gather_kernel<float, double, S, false>(const __grid_constant__ PushArgs<double>);  \
+  template __global__ void residual_kernel<double, double, S, false>(const __grid_constant__ ResidualArgs<double>); \
+  template __global__ void residual_kernel<float, double, S, false>(const __grid_constant__ ResidualArgs<double>);
 APRL_SHAPE_KERNELS(0)
 APRL_SHAPE_KERNELS(1)
+// the wide stencils of linear-binomial3, for sparse runs
+template __global__ void guess_gather_kernel<double, double, 0, true>(const __grid_constant__ PushArgs<double>);
+template __global__ void guess_gather_kernel<float, double, 0, true>(const __grid_constant__ PushArgs<double>);
+template __global__ void residual_kernel<double, double, 0, true>(const __grid_constant__ ResidualArgs<double>);
+template __global__ void residual_kernel<float, double, 0, true>(const __grid_constant__ ResidualArgs<double>);
 template __global__ void chord_deposit_kernel<false>(ChordArgs);
 template __global__ void chord_deposit_kernel<true>(ChordArgs);
 #undef APRL_SHAPE_KERNELS

@@ -80,16 +80,20 @@ struct DSlots {
   unsigned char* seen;
 };
 
+// What the gathers read.  W is the arithmetic type of the gathers.
+struct GatherArrays {
+  const void* filtered[3];   // W: the filtered orbit sum (layout of j_index)
+  const double* sum[3];      // the unfiltered current-free orbit sum (ring layout of E)
+  const void* magnetic[3];   // W: the filtered B (layout of bf_index), when dense
+};
+
 // The argument blocks of the particle kernels are templated on the type F
 // of J in the grid view (binary64 in both modes of this library).  Particle
 // state, the push, the deposit and the boundary logic are binary64.
 template <class F>
 struct PushArgs {
   GridT<F> g;
-  // What the gathers read, in their arithmetic type: the orbit sum
-  // S = E_new + E^n per E node and B, both in the ring layout of E and B.
-  const void* orbit[3];
-  const void* bgather[3];
+  GatherArrays src;
   DFrame frame;
   DRegion region;
   DMagnet magnets[kMaxMagnets];
@@ -138,8 +142,7 @@ struct CarrierArgs {
 template <class F>
 struct ResidualArgs {
   GridT<F> g;
-  const void* orbit[3];     // as in PushArgs
-  const void* bgather[3];
+  GatherArrays src;
   int shape;
   long long count;
   DParticles p;
@@ -224,14 +227,15 @@ struct ChordArgs {
 
 // W: arithmetic of the gathers (double, or float in the FP32-mixed mode).
 // S: the particle shape, 0 linear-binomial3, 1 quintic-compensated.
-template <class W, class F, int S> __global__ void guess_gather_kernel(PushArgs<F> a);
+// D, DB: read the wide stencils directly (linear-binomial3, sparse runs).
+template <class W, class F, int S, bool D> __global__ void guess_gather_kernel(const __grid_constant__ PushArgs<F> a);
 // Q: the deterministic mode's fixed-point current sum.
 template <class F, int S, bool Q>
-__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(PushArgs<F> a);
-template <class F, int S, bool Q> __global__ void carrier_kernel(CarrierArgs<F> a);
+__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(const __grid_constant__ PushArgs<F> a);
+template <class F, int S, bool Q> __global__ void carrier_kernel(const __grid_constant__ CarrierArgs<F> a);
 template <bool Q> __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(ChordArgs a);
-template <class W, class F, int S>
-__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(ResidualArgs<F> a);
+template <class W, class F, int S, bool DB>
+__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ ResidualArgs<F> a);
 
 // RelativisticBorisPusher::push of `count` particles (SoA, in place) with
 // per-particle E and B (3 values each).
@@ -297,7 +301,7 @@ struct SupportArgs {
   double held_distance_per_beta; // c*dt
   DeviceStatus* status;
 };
-template <class F, int S, bool Q> __global__ void frozen_support_kernel(SupportArgs<F> a);
+template <class F, int S, bool Q> __global__ void frozen_support_kernel(const __grid_constant__ SupportArgs<F> a);
 __global__ void crop_flags_kernel(DCarriers c, long long n, double upper,
                                   double lower, unsigned char* keep,
                                   TrialCounters* counters, DeviceStatus* status);

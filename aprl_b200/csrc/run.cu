@@ -58,7 +58,7 @@ enum Kernel : unsigned {
   kResidual, kElectricCommit, kFlagCount, kBlockScan, kGatherParticles,
   kGatherCarriers, kShiftInsert, kCropFlags, kInletCheck, kDetectorPlane,
   kSortKey, kChunkScan, kChunkAdd, kRadixScatter, kAdmit, kFrozenSupport,
-  kGuessGather, kOrbitSum, kBShadow, kLedgerPartial, kLedgerFinish,
+  kGuessGather, kOrbitSum, kMagneticFilter, kLedgerPartial, kLedgerFinish,
   kGaussDeposit, kGaussResidual, kGaussFinish, kTrialClear, kTrialVerdict,
   kSfMoments, kSfFinish, kSfDeposit, kSfSource, kSfApply, kSfUpdate,
   kSfDirection, kSfSmooth, kSfElectric, kSfMagnetic, kSfClear, kSfGauss, kSfEnergy,
@@ -72,7 +72,7 @@ const char* kKernelNames[kKernelCount] = {
   "block_offset_scan", "gather_particles", "gather_carriers",
   "shift_insert", "crop_flags", "inlet_check", "detector_plane",
   "sort_key", "chunk_scan", "chunk_add", "radix_scatter", "admit",
-  "frozen_support", "guess_gather", "orbit_sum", "b_shadow", "ledger_partial",
+  "frozen_support", "guess_gather", "orbit_filter", "magnetic_filter", "ledger_partial",
   "ledger_finish", "gauss_deposit", "gauss_residual", "gauss_finish", "trial_clear",
   "trial_verdict", "sf_moments", "sf_finish", "sf_deposit", "sf_source", "sf_apply",
   "sf_update", "sf_direction", "sf_smooth", "sf_electric", "sf_magnetic",
@@ -284,18 +284,27 @@ struct aprl_run {
   int cur = 0;  // e[cur] = E^n (committed), e[1-cur] = E*
   double* b[3]{};
   void* jc[3]{};
-  // J is known to be zero everywhere (set by a clear, kept by a trial that
-  // deposits nothing): the next clear and the commit's pass over J are
-  // skipped, which is most of a field-only step's work besides the field
-  // updates.
+  // The raw current (jc) is known to be zero everywhere (set by a clear, kept
+  // by a trial that deposits nothing): the next clear and the commit's pass
+  // over it are skipped, which is most of a field-only step's work besides
+  // the field updates.
   bool j_zero = true;
-  // The preview of this step wrote the current-free orbit sum.
-  bool orbit_from_preview = false;
+  // J as set by aprl_run_set_field, until the next step clears it.
+  double* j_set[3]{};
+  // The equivalent surface current that the current step's E* holds, for a
+  // read-out of J.
+  bool surface_in_j = false;
+  int64_t surface_offset = 0;
+  uint64_t surface_step = 0;
+  // This step's gathers read filtered arrays (see dense_gathers).
+  bool dense = false;
   double* lower[3]{};
-  // What the gathers read: the orbit sum S = E_new + E^n per E node (binary64,
-  // or binary32 in the FP32-mixed mode) and, in that mode, a binary32 B.
-  void* orbit[3]{};
-  float* bshadow[3]{};
+  // What the gathers read: S0 = E* + E^n per E node (binary64), and in the
+  // arithmetic of the gathers (binary32 in the FP32-mixed mode) the filtered
+  // orbit sum of the trial and, for dense linear-binomial3 runs, the filtered B.
+  double* sum[3]{};
+  void* filtered[3]{};
+  void* bfilter[3]{};
   int zb_e[3]{}, zb_b[3]{};
   double* ref[6]{};
   bool ref_set[6]{};
@@ -544,6 +553,15 @@ size_t e_count(const aprl_run_config& g, int c) {
 size_t b_count(const aprl_run_config& g, int c) {
   return (size_t)(g.nx + (c == 0)) * (g.ny + (c == 1)) * (g.nz + (c == 2));
 }
+// z padding and size of component c of the raw current and of the filtered
+// orbit sum (j_index), and size of the filtered B (bf_index).
+int raw_pad(const aprl_run_config& g) { return g.shape == APRL_SHAPE_LINEAR_BINOMIAL3 ? 1 : 3; }
+size_t raw_count(const aprl_run_config& g, int c) {
+  return (size_t)(g.nx + (c != 0) + 2) * (g.ny + (c != 1)) * (g.nz + (c != 2) + 2 * raw_pad(g));
+}
+size_t bfilter_count(const aprl_run_config& g, int c) {
+  return (size_t)(g.nx + (c == 0) + 2) * (g.ny + (c == 1)) * (g.nz + (c == 2) + 2);
+}
 void comp_shape(const aprl_run_config& g, unsigned a, size_t s[3]) {
   const bool electric = a < 3 || a >= 6;
   const unsigned axis = a % 3;
@@ -633,7 +651,7 @@ aprl_status launch(aprl_run* r, unsigned id, K kernel, dim3 grid, dim3 block, Ar
 // ---- autotuner -------------------------------------------------------------
 // The launch shapes of the grid kernels are chosen by measurement, per device
 // and grid extent: the Cowan magnetic kernel's z planes per block and the
-// thread-block shape of the preview, orbit-sum and commit kernels.  Every
+// thread-block shape of the preview, orbit-filter and commit kernels.  Every
 // candidate computes each node exactly as the others do (one thread per node,
 // or the same plane ring over a different split of z), so a choice changes
 // timing only, never a bit of a result.  While a grid extent has no choice
@@ -779,6 +797,10 @@ GridT<F> make_grid(const aprl_run* r) {
     g.zb_e[a] = r->zb_e[a];
     g.zb_b[a] = r->zb_b[a];
   }
+  g.jpad = raw_pad(r->cfg);
+  g.inv_h[0] = 1. / g.dx;
+  g.inv_h[1] = 1. / g.dy;
+  g.inv_h[2] = 1. / g.dz;
   g.jcoef = F(-1. * r->cfg.dt / kEpsilon0);
   g.status = r->d_status;
   if (r->deterministic) {
@@ -1403,8 +1425,13 @@ aprl_status advance_magnetic_t(aprl_run* r) {
   const aprl_run_config& c = r->cfg;
   if (!r->j_zero)
     for (int a = 0; a < 3; ++a)
-      CUDA_TRY(cudaMemsetAsync(r->jc[a], 0, e_count(c, a) * sizeof(F), r->stream));
+      CUDA_TRY(cudaMemsetAsync(r->jc[a], 0, raw_count(c, a) * sizeof(F), r->stream));
   r->j_zero = true;
+  r->surface_in_j = false;
+  for (int a = 0; a < 3; ++a) {
+    device_free(r, r->j_set[a]);
+    r->j_set[a] = nullptr;
+  }
   InletPlaneArgs ia{};
   ia.nx = (int)c.nx;
   ia.ny = (int)c.ny;
@@ -1458,6 +1485,65 @@ aprl_status do_advance_magnetic(aprl_run* r) {
   return advance_magnetic_t<double>(r);
 }
 
+// Whether this step's linear-binomial3 gathers read the filtered B and, in
+// the first trial, the filtered current-free sum.  The two grid passes cost
+// about 28 B of traffic a cell; the wide stencils cost a particle some 220
+// reads more.  Below one particle per 16 cells the direct reads are the
+// cheaper side.  The quintic shape always gathers from the filtered sum.  A run that cannot have
+// the filtered B's memory reads the wide stencils.
+constexpr size_t kDenseCells = 16;
+
+bool dense_gathers(aprl_run* r) {
+  const aprl_run_config& c = r->cfg;
+  if (!r->np) return false;
+  if (c.shape != APRL_SHAPE_LINEAR_BINOMIAL3) return true;
+  if (r->np * kDenseCells < (size_t)c.nx * c.ny * c.nz) return false;
+  const size_t w = r->fp32 ? sizeof(float) : sizeof(double);
+  for (int a = 0; a < 3; ++a)
+    if (!r->bfilter[a] &&
+        cudaMallocFromPoolAsync(&r->bfilter[a], bfilter_count(c, a) * w, r->pool, r->stream) !=
+            cudaSuccess) {
+      r->bfilter[a] = nullptr;
+      (void)cudaGetLastError();
+      return false;
+    }
+  return true;
+}
+
+// Launch grid of the filter kernels: `written` x nodes per warp, the z planes
+// (nz + 1 + 2 * reach) in chunks of `planes`: long marches share fewer planes
+// between chunks, short ones give a small grid enough warps (about 24 an SM).
+dim3 filter_grid(const aprl_run_config& c, dim3 block, unsigned written, int pad, int& planes,
+                 int& chunks) {
+  const unsigned tiles = blocks_for(c.nx + 3, written);
+  const size_t total = c.nz + 1 + 2 * (size_t)pad;
+  const size_t rows = (size_t)tiles * (c.ny + 1) * 3;
+  planes = 32;
+  while (planes > 8 && rows * ((total + planes - 1) / planes) < 148 * 24) planes /= 2;
+  chunks = (int)((total + planes - 1) / planes);
+  return dim3(blocks_for(tiles, block.x / 32), blocks_for(c.ny + 1, block.y), 3 * chunks);
+}
+
+// One filter pass over the raw current and the orbit sum, launched with the
+// thread block `block` (a multiple of 32 wide).
+template <int MODE, class W>
+aprl_status filter_pass(aprl_run* r, unsigned id, const GridT<double>& g, dim3 block,
+                        void* const out[3]) {
+  FilterArgs a{};
+  a.g = g;
+  for (int d = 0; d < 3; ++d) {
+    a.sum[d] = r->sum[d];
+    a.out[d] = out ? out[d] : nullptr;
+  }
+  const bool orbit = MODE == kFilterGuess || MODE == kFilterOrbit;
+  const dim3 grid = filter_grid(r->cfg, block, orbit ? kFilterLanes : 30, orbit ? g.jpad : 0,
+                                a.planes, a.chunks);
+  return launch(r, id,
+                r->cfg.shape == APRL_SHAPE_LINEAR_BINOMIAL3 ? current_filter_kernel<0, MODE, W>
+                                                           : current_filter_kernel<1, MODE, W>,
+                grid, block, a);
+}
+
 template <class F>
 aprl_status preview_electric_t(aprl_run* r) {
   if (r->stage != 1) return fail(APRL_ERR_RUNTIME, "Moving-window electric phase mismatch");
@@ -1468,27 +1554,25 @@ aprl_status preview_electric_t(aprl_run* r) {
   pa.ey_prof = r->eprof[1].view();
   for (int h = 0; h < 4; ++h) pa.h[h] = r->hist[4 + h].view();
   for (int a = 0; a < 2; ++a) pa.pre_inlet[a] = r->ledger_on ? r->ledger_pre[a] : nullptr;
-  // With particles to gather, the first trial's current-free orbit sum is
-  // written by the preview itself (E* and E^n are in its registers there).
-  r->orbit_from_preview = r->np != 0;
-  for (int a = 0; a < 3; ++a) pa.orbit[a] = r->orbit_from_preview ? r->orbit[a] : nullptr;
-  pa.orbit_float = r->fp32 ? 1 : 0;
+  // With particles to gather, the current-free orbit sum is written by the
+  // preview itself (E* and E^n are in its registers there).
+  for (int a = 0; a < 3; ++a) pa.sum[a] = r->np ? r->sum[a] : nullptr;
   TRY(inlet_table(r, r->offset, r->step + 1, pa.inlet));
   TuneLaunch tl;
   TRY(tune_begin(r, kTunePreview, tl));
   const dim3 block = kGridBlocks[tl.candidate];
   TRY(launch(r, kElectricPreview, electric_preview_kernel<F>, grid3(c, block), block, pa));
   TRY(tune_end(r, tl));
-  if (r->fp32 && r->np) {  // B is final for the step: its binary32 copy for the gathers
-    BShadowArgs sa{};
-    size_t most = 0;
-    for (int a = 0; a < 3; ++a) {
-      sa.b[a] = r->b[a];
-      sa.out[a] = r->bshadow[a];
-      sa.n[a] = (long long)b_count(c, a);
-      most = std::max(most, b_count(c, a));
-    }
-    TRY(launch(r, kBShadow, b_shadow_kernel, dim3(blocks_for(most, 256), 3), dim3(256), sa));
+  r->dense = dense_gathers(r);
+  if (r->dense && c.shape == APRL_SHAPE_LINEAR_BINOMIAL3) {  // B is final for the step
+    BFilterArgs fa{};
+    fa.g = make_grid<double>(r);
+    for (int a = 0; a < 3; ++a) fa.out[a] = r->bfilter[a];
+    const dim3 fblock(32, 8);
+    const dim3 fgrid = filter_grid(c, fblock, 30, 2, fa.planes, fa.chunks);
+    TRY(launch(r, kMagneticFilter,
+               r->fp32 ? magnetic_filter_kernel<float> : magnetic_filter_kernel<double>, fgrid,
+               fblock, fa));
   }
   if (r->np)
     CUDA_TRY(cudaMemcpyAsync(r->slot_order, r->p.order, r->np * 8, cudaMemcpyDeviceToDevice,
@@ -1556,14 +1640,20 @@ aprl_status surface_current_prepare(aprl_run* r) {
   return APRL_OK;
 }
 
-aprl_status surface_current_add(aprl_run* r, const GridT<double>& g) {
+// Into E* and S0 of the step (jz null), or into a read-out of Jz.
+aprl_status surface_current_add(aprl_run* r, const GridT<double>& g, double* jz) {
   TRY(surface_current_prepare(r));
   const aprl_run_config& c = r->cfg;
+  if (!jz) {
+    r->surface_offset = r->offset;
+    r->surface_step = r->step + 1;
+  }
   // The reference's range check (src/transverse_reference_current.cpp:109-110),
   // for the first and last window planes (z grows with k).
-  const double step = static_cast<double>(r->step + 1);
-  const double z0 = static_cast<double>(r->offset) - c.translation_beta * step;
-  const double z1 = static_cast<double>(r->offset + (int64_t)c.nz - 1) - c.translation_beta * step;
+  const double step = static_cast<double>(r->surface_step);
+  const double z0 = static_cast<double>(r->surface_offset) - c.translation_beta * step;
+  const double z1 = static_cast<double>(r->surface_offset + (int64_t)c.nz - 1) -
+                    c.translation_beta * step;
   if (!std::isfinite(z0) || z0 < 0. || z1 > static_cast<double>(c.reference_nz) - 1.)
     return fail(APRL_ERR_OUT_OF_RANGE, "Reference surface-current query outside domain");
   SurfaceArgs a{};
@@ -1571,10 +1661,13 @@ aprl_status surface_current_add(aprl_run* r, const GridT<double>& g) {
   a.table = r->surface_table;
   a.count = (long long)r->surface_count;
   a.planes = (long long)c.reference_nz;
-  a.offset = r->offset;
-  a.step = r->step + 1;
+  a.offset = r->surface_offset;
+  a.step = r->surface_step;
   a.beta = c.translation_beta;
   a.g = g;
+  a.jz = jz;
+  a.sum = r->np ? r->sum[2] : nullptr;
+  r->surface_in_j = true;
   return launch(r, kSurfaceCurrent, surface_add_kernel,
                 dim3(blocks_for(r->surface_count * c.nz, 256)), dim3(256), a);
 }
@@ -1598,7 +1691,7 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
   }
   const bool deposits = r->np || r->nc || (r->queue.extracted && frozen_end > r->queue.cursor);
   size_t most = 0;
-  for (int a = 0; a < 3; ++a) most = std::max(most, e_count(c, a));
+  for (int a = 0; a < 3; ++a) most = std::max(most, raw_count(c, a));
   const unsigned grid_blocks = std::min<unsigned>(blocks_for(most, 256), 148 * 8);
   // Deterministic mode: the deposits of the trial go into J's fixed-point
   // pairs, and J is written from them once they are all done.
@@ -1612,9 +1705,9 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
                r->d_sums, clear_current));
   }
   const bool surface = c.reference_surface_current != 0;
-  r->j_zero = !deposits && !surface;
-  // J complete for the trial: the fixed-point pairs converted (deterministic
-  // mode), then the reference's equivalent surface current added.
+  r->j_zero = !deposits;
+  // The raw current complete for the trial: the fixed-point pairs converted
+  // (deterministic mode).
   bool converted = false;
   auto convert_current = [&]() -> aprl_status {
     if (converted) return APRL_OK;
@@ -1622,7 +1715,6 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     if (convert)
       TRY(launch(r, kCurrentConvert, current_convert_kernel, dim3(grid_blocks), dim3(256), g,
                  1.0 / r->jq_scale));
-    if (surface) TRY(surface_current_add(r, g));
     return APRL_OK;
   };
   const DRegion region = make_region(r);
@@ -1727,22 +1819,23 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     pa.key_base = (unsigned long long)(r->step + 1) << 32;
     pa.counters = r->d_counters;
     pa.status = r->d_status;
-    W* orbit[3] = {static_cast<W*>(r->orbit[0]), static_cast<W*>(r->orbit[1]),
-                   static_cast<W*>(r->orbit[2])};
+    const bool direct = binomial && !r->dense;
     for (int a = 0; a < 3; ++a) {
-      pa.orbit[a] = orbit[a];
-      pa.bgather[a] = r->fp32 ? static_cast<const void*>(r->bshadow[a])
-                              : static_cast<const void*>(r->b[a]);
+      pa.src.filtered[a] = r->filtered[a];
+      pa.src.sum[a] = r->sum[a];
+      pa.src.magnetic[a] = r->bfilter[a];
     }
-    const dim3 oblock(32, 4);
     if (r->trials == 0) {
-      if (!r->orbit_from_preview)
-        TRY(launch(r, kOrbitSum, orbit_sum_kernel<W>, grid3(c, oblock), oblock, g, orbit[0],
-                   orbit[1], orbit[2], 0));
+      if (!direct)
+        TRY((filter_pass<kFilterGuess, W>(r, kOrbitSum, g, dim3(32, 8), r->filtered)));
       TRY(launch(r, kGuessGather,
-                 binomial ? guess_gather_kernel<W, F, 0> : guess_gather_kernel<W, F, 1>,
+                 binomial ? (direct ? guess_gather_kernel<W, F, 0, true>
+                                    : guess_gather_kernel<W, F, 0, false>)
+                          : guess_gather_kernel<W, F, 1, false>,
                  dim3(blocks_for(r->np, 128)),
                  dim3(128), pa));
+      // The step's surface current joins E* and S0 after the current-free gather.
+      if (surface) TRY(surface_current_add(r, g, nullptr));
     }
     TRY(launch(r, kPushDeposit,
                r->deterministic
@@ -1776,17 +1869,13 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
       } else {
         tl.candidate = std::max(0, r->tune_choice[kTuneOrbit]);
       }
-      const dim3 sblock = kGridBlocks[tl.candidate];
-      TRY(launch(r, kOrbitSum, orbit_sum_kernel<W>, grid3(c, sblock), sblock, g, orbit[0],
-                 orbit[1], orbit[2], 1));
+      TRY((filter_pass<kFilterOrbit, W>(r, kOrbitSum, g, kGridBlocks[tl.candidate],
+                                        r->filtered)));
       TRY(tune_end(r, tl));
     }
     ResidualArgs<F> ra{};
     ra.g = g;
-    for (int a = 0; a < 3; ++a) {
-      ra.orbit[a] = pa.orbit[a];
-      ra.bgather[a] = pa.bgather[a];
-    }
+    ra.src = pa.src;
     ra.shape = c.shape;
     ra.count = (long long)r->np;
     ra.p = r->p;
@@ -1801,8 +1890,12 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     ra.partial = r->res_partial;
     ra.ticket = r->res_ticket;
     ra.status = r->d_status;
-    TRY(launch(r, kResidual, binomial ? residual_kernel<W, F, 0> : residual_kernel<W, F, 1>,
+    TRY(launch(r, kResidual,
+               binomial ? (direct ? residual_kernel<W, F, 0, true> : residual_kernel<W, F, 0, false>)
+                        : residual_kernel<W, F, 1, false>,
                dim3(blocks_for(r->np, 128)), dim3(128), ra));
+  } else if (surface && r->trials == 0) {
+    TRY(surface_current_add(r, g, nullptr));
   }
   TRY(join_carriers());
   TRY(convert_current());
@@ -1855,15 +1948,14 @@ aprl_status do_trial(aprl_run* r, double residual[4]) {
 
 aprl_status do_commit(aprl_run* r) {
   if (r->stage != 3) return fail(APRL_ERR_RUNTIME, "Commit requires a completed coupling trial");
-  const aprl_run_config& c = r->cfg;
   // E^{n+1} = E* - dt/eps0 J, in place where J is nonzero: nothing to do
   // when J is known to be zero.
   if (!r->j_zero) {
     TuneLaunch tl;
     TRY(tune_begin(r, kTuneCommit, tl));
     const dim3 block = kGridBlocks[tl.candidate];
-    TRY(launch(r, kElectricCommit, electric_commit_kernel<double>, grid3(c, block), block,
-               make_grid<double>(r)));
+    TRY((filter_pass<kFilterCommit, double>(r, kElectricCommit, make_grid<double>(r), block,
+                                            nullptr)));
     TRY(tune_end(r, tl));
   }
   r->cur = 1 - r->cur;
@@ -2180,15 +2272,14 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
     }
     if ((s = device_alloc(r, &r->b[a], b_count(c, a))) != APRL_OK) return cleanup(s);
     cudaMemsetAsync(r->b[a], 0, b_count(c, a) * 8, r->stream);
-    if ((s = device_alloc_bytes(r, &r->jc[a], e_count(c, a) * fes)) != APRL_OK) return cleanup(s);
-    cudaMemsetAsync(r->jc[a], 0, e_count(c, a) * fes, r->stream);
+    if ((s = device_alloc_bytes(r, &r->jc[a], raw_count(c, a) * fes)) != APRL_OK) return cleanup(s);
+    cudaMemsetAsync(r->jc[a], 0, raw_count(c, a) * fes, r->stream);
     const size_t plane = (size_t)(c.nx + (a != 0)) * (c.ny + (a != 1));
     if ((s = device_alloc(r, &r->lower[a], plane)) != APRL_OK) return cleanup(s);
     const size_t gather_bytes = r->fp32 ? sizeof(float) : sizeof(double);
-    if ((s = device_alloc_bytes(r, &r->orbit[a], e_count(c, a) * gather_bytes)) != APRL_OK)
+    if ((s = device_alloc_bytes(r, &r->filtered[a], raw_count(c, a) * gather_bytes)) != APRL_OK)
       return cleanup(s);
-    if (r->fp32 && (s = device_alloc(r, &r->bshadow[a], b_count(c, a))) != APRL_OK)
-      return cleanup(s);
+    if ((s = device_alloc(r, &r->sum[a], e_count(c, a))) != APRL_OK) return cleanup(s);
     r->max_rate[a] = maximum_rate(c, a);
   }
   // CPML profiles (x, y) for magnetic (half-integer) and electric nodes.
@@ -2236,8 +2327,8 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
   r->deterministic = c.deterministic != 0;
   if (r->deterministic) {
     for (int a = 0; a < 3; ++a) {
-      if ((s = device_alloc(r, &r->jq[a], 2 * e_count(c, a))) != APRL_OK) return cleanup(s);
-      cudaMemsetAsync(r->jq[a], 0, 2 * e_count(c, a) * sizeof(unsigned long long), r->stream);
+      if ((s = device_alloc(r, &r->jq[a], 2 * raw_count(c, a))) != APRL_OK) return cleanup(s);
+      cudaMemsetAsync(r->jq[a], 0, 2 * raw_count(c, a) * sizeof(unsigned long long), r->stream);
     }
     if (c.inlet_charge_match &&
         (s = device_alloc(r, &r->inlet_rho_pairs, 2 * (size_t)(c.nx + 1) * (c.ny + 1))) != APRL_OK)
@@ -2323,8 +2414,10 @@ aprl_status aprl_run_destroy(aprl_run* r) {
   for (int a = 0; a < 3; ++a) {
     device_free(r, r->e[0][a]); device_free(r, r->e[1][a]); device_free(r, r->b[a]); device_free(r, r->jc[a]);
     device_free(r, r->lower[a]);
-    device_free(r, r->orbit[a]);
-    device_free(r, r->bshadow[a]);
+    device_free(r, r->sum[a]);
+    device_free(r, r->filtered[a]);
+    device_free(r, r->bfilter[a]);
+    device_free(r, r->j_set[a]);
   }
   for (int a = 0; a < 6; ++a) device_free(r, r->ref[a]);
   for (int a = 0; a < 2; ++a) {
@@ -2464,6 +2557,22 @@ aprl_status aprl_run_field_shape(const aprl_run* r, unsigned a, uint64_t shape[3
   return APRL_OK;
 }
 
+// J of the last trial (component c): the filtered raw current, and for Jz the
+// equivalent surface current that the step's E* holds.
+static aprl_status current_out(aprl_run* r, int c, double* out, size_t plane, size_t layers) {
+  double* j[3] = {};
+  aprl_status s = APRL_OK;
+  for (int a = 0; a < 3 && s == APRL_OK; ++a) s = device_alloc(r, &j[a], e_count(r->cfg, a));
+  if (s == APRL_OK)
+    s = filter_pass<kFilterCurrent, double>(r, kOrbitSum, make_grid<double>(r), dim3(32, 8),
+                                            reinterpret_cast<void* const*>(j));
+  if (s == APRL_OK && c == 2 && r->surface_in_j)
+    s = surface_current_add(r, make_grid<double>(r), j[2]);
+  if (s == APRL_OK) s = copy_ring(r, j[c], nullptr, out, plane, layers, 0);
+  for (int a = 0; a < 3; ++a) device_free(r, j[a]);
+  return s;
+}
+
 static aprl_status field_io(aprl_run* r, unsigned a, const double* in, double* out, size_t count) {
   if (!r || a >= 9) return fail(APRL_ERR_OUT_OF_RANGE, "Field component");
   size_t s[3];
@@ -2474,8 +2583,12 @@ static aprl_status field_io(aprl_run* r, unsigned a, const double* in, double* o
     return fail(APRL_ERR_RUNTIME, "Fields can only be replaced between steps");
   const size_t plane = s[0] * s[1];
   if (a >= 6) {
-    if (in) r->j_zero = false;
-    return copy_ring(r, static_cast<double*>(r->jc[a - 6]), in, out, plane, s[2], 0);
+    if (in) {
+      if (!r->j_set[a - 6]) TRY(device_alloc(r, &r->j_set[a - 6], count));
+      return copy_ring(r, r->j_set[a - 6], in, nullptr, plane, s[2], 0);
+    }
+    if (r->j_set[a - 6]) return copy_ring(r, r->j_set[a - 6], nullptr, out, plane, s[2], 0);
+    return current_out(r, (int)a - 6, out, plane, s[2]);
   }
   if (a < 3) return copy_ring(r, r->e[r->cur][a], in, out, plane, s[2], r->zb_e[a]);
   return copy_ring(r, r->b[a - 3], in, out, plane, s[2], r->zb_b[a - 3]);
