@@ -1206,6 +1206,12 @@ __global__ void carrier_kernel(const __grid_constant__ CarrierArgs<F> a) {
   bool kept = false;
   const unsigned err = carrier_segment<S, Q>(a.g, a.region, c, start, 0.0, a.counters, kept);
   if (err) raise_error(a.status, err, (unsigned long long)n);
+  const bool cropped = kept && c.pos[2] >= a.crop_upper;
+  if (cropped) {
+    kept = false;
+    atomicAdd(&a.counters->cropped, 1ull);
+    atomicAdd(&a.counters->cropped_charge, c.q * c.w);
+  }
   count_lanes(&a.counters->carriers_kept, kept);
   a.keep[n] = kept ? 1 : 0;
   a.out.px[n] = c.pos[0]; a.out.py[n] = c.pos[1]; a.out.pz[n] = c.pos[2];
@@ -1224,8 +1230,8 @@ __device__ unsigned coupling_push(const PushArgs<F>& a, long long n, double pos[
                                   double q, double m, double time, double dt, double used_e[3],
                                   double used_b[3], double& abs_work) {
   for (int d = 0; d < 3; ++d) {
-    used_e[d] = a.next_e[3 * n + d];
-    used_b[d] = a.next_b[3 * n + d];
+    used_e[d] = a.used_e[3 * n + d];
+    used_b[d] = a.used_b[3 * n + d];
   }
   abs_work = 0.0;
   const double h = dt / a.substeps;
@@ -1328,169 +1334,57 @@ __global__ void APRL_GATHER_BOUNDS guess_gather_kernel(const __grid_constant__ P
   const unsigned err =
       gather_fields<S, D, D>(a.g, s.start, guess, gather_source<W>(a.src), ne, nb);
   if (err) raise_error(a.status, err, (unsigned long long)n);
-  double* next_e = const_cast<double*>(a.next_e);
-  double* next_b = const_cast<double*>(a.next_b);
   for (int d = 0; d < 3; ++d) {
-    next_e[3 * n + d] = ne[d];
-    next_b[3 * n + d] = nb[d];
+    a.used_e[3 * n + d] = ne[d];
+    a.used_b[3 * n + d] = nb[d];
   }
 }
 
 // One fixed-point trial of one particle of the list: prepareParticle
-// (src/simulation.cpp:4919-5035), then the deposit and boundary pass
-// (src/simulation.cpp:5083-5368): upstream admission clip, the frozen part
-// up to an activation kink (4684-4756) and processActiveSegment (4760-4917)
-// with Simulation::firstMovingWindowEntry
-// (src/simulation_moving_window.cpp:380-395).
-template <class F, int S, bool Q>
-__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(const __grid_constant__ PushArgs<F> a) {
+// (src/simulation.cpp:4919-5035) and the push.  Nearly every particle then
+// stays inside the physical region, short of the exit plane, on one chord
+// from its step start to its new position: chord_deposit_kernel deposits that
+// chord.  The others -- a boundary crossing, an upstream or frozen leading
+// piece, any error -- go on a list for push_events_kernel: handled here their
+// long serial path held their warps (and its registers every warp) while the
+// rest waited.
+template <class F>
+__global__ void APRL_PUSH_BOUNDS push_kernel(const __grid_constant__ PushArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
   const GridT<F>& g = a.g;
-  const double t = a.time, dt = g.dt;
-  double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
+  const double t = a.time;
+  const double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
   double u[3] = {a.p.ux[n], a.p.uy[n], a.p.uz[n]};
-  const double q = a.p.q[n], m = a.p.m[n];
   const bool frozen0 = a.p.frozen[n] != 0;
   const SlotPlan s = plan_slot(g, a.frame, a.activation_plane_lab_z, t, start, frozen0,
                                frozen0 ? a.p.beta[n] : 0.0);
   unsigned err = s.err;
   const bool frozen1 = frozen0 && !s.released;
   double pos[3] = {s.start[0], s.start[1], frozen1 ? s.held_z : s.start[2]};
-  double used_e[3] = {0., 0., 0.}, used_b[3] = {0., 0., 0.};
   double abs_work = 0.0;
-  if (!err && s.seen)
-    err = coupling_push(a, n, pos, u, q, m, s.time, s.dt, used_e, used_b, abs_work);
-  if (!err && s.released) atomicAdd(&a.counters->activations, 1ull);
-  // An optional leading piece, then the main segment: the upstream part of
-  // an admitted held particle (deposited without validation), or the frozen
-  // part up to an activation kink (which may not cross a boundary).
-  double seg_frac = 0.0;
-  bool has_pre = false, pre_validate = false, has_main = true;
-  double pre_end[3] = {pos[0], pos[1], pos[2]};
-  double pre_start[3] = {start[0], start[1], start[2]};
-  if (!err && start[2] < g.origin[2]) {
-    if (!frozen0 || !frozen1) {
-      err = kErrAdmission;
-    } else if (pos[2] < g.origin[2]) {
-      has_pre = true;
-      has_main = false;
-    } else {
-      const double fraction = (g.origin[2] - start[2]) / (pos[2] - start[2]);
-      if (!(fraction >= 0.0 && fraction <= 1.0) || !isfinite(fraction)) {
-        err = kErrAdmission;
-      } else {
-        for (int d = 0; d < 3; ++d) pre_end[d] = start[d] + fraction * (pos[d] - start[d]);
-        pre_end[2] = g.origin[2];
-        has_pre = true;
-        seg_frac = fraction;
-        for (int d = 0; d < 3; ++d) start[d] = pre_end[d];
-      }
-    }
-  } else if (!err && s.released && s.time > t && s.time < t + dt) {
-    Hit hc, ho;
-    bool enters = false, exits = false;
-    err = cpml_first_entry(a.region, start, s.start, hc, enters);
-    if (!err) err = outer_first_exit(a.region, start, s.start, ho, exits);
-    if (!err && (enters || exits)) err = kErrHeldBoundary;
-    for (int d = 0; d < 3; ++d) pre_end[d] = s.start[d];
-    has_pre = true;
-    pre_validate = true;
-    for (int d = 0; d < 3; ++d) start[d] = s.start[d];
-    seg_frac = (s.time - t) / dt;
+  if (!err && s.seen) {
+    double used_e[3], used_b[3];
+    err = coupling_push(a, n, pos, u, a.p.q[n], a.p.m[n], s.time, s.dt, used_e, used_b, abs_work);
+  } else {
+    for (int d = 0; d < 3; ++d) a.used_e[3 * n + d] = a.used_b[3 * n + d] = 0.0;
   }
-  unsigned char action = 0;
-  bool deferred = false;
-  Hit selected;
-  for (int piece = has_pre ? 0 : 1; piece < (has_main ? 2 : 1) && !err; ++piece) {
-    double b[3], e[3];
-    bool validate = true;
-    if (piece == 0) {
-      for (int d = 0; d < 3; ++d) {
-        b[d] = pre_start[d];
-        e[d] = pre_end[d];
-      }
-      validate = pre_validate;
-    } else {
-      // firstMovingWindowEntry = CPML first entry + fixed-lab exit plane
-      Hit cpml_hit, outer_hit;
-      bool enters = false, exits = false;
-      err = cpml_first_entry(a.region, start, pos, cpml_hit, enters);
-      if (!err) {
-        const double za = lab_z_from_box_zt(a.frame, start[2], t + seg_frac * dt) - a.exit_lab_z;
-        const double zb = lab_z_from_box_zt(a.frame, pos[2], t + dt) - a.exit_lab_z;
-        if (za >= 0.) err = kErrBeyondExit;
-        else if (zb >= 0. && zb > za) {
-          const double fraction = -za / (zb - za);
-          if (!enters || fraction < cpml_hit.fraction) {
-            for (int d = 0; d < 3; ++d) cpml_hit.position[d] = start[d] + fraction * (pos[d] - start[d]);
-            cpml_hit.fraction = fraction;
-            cpml_hit.face = 5;
-            enters = true;
-          }
-        }
-      }
-      if (!err) err = outer_first_exit(a.region, start, pos, outer_hit, exits);
-      if (err) break;
-      if (enters && (!exits || cpml_hit.fraction <= outer_hit.fraction + 64.0 * kEpsilon)) {
-        action = 1;
-        selected = cpml_hit;
-      } else if (exits) {
-        action = 2;
-        selected = outer_hit;
-      }
-      for (int d = 0; d < 3; ++d) {
-        b[d] = start[d];
-        e[d] = action ? selected.position[d] : pos[d];
-      }
-    }
-    if constexpr (S == 0) {
-      // The main chord of a linear-binomial3 particle is validated here and
-      // deposited by chord_deposit_kernel, whose converged warps merge the
-      // stencils of particles in the same cell before the reductions.
-      if (piece == 1) {
-        err = validate_segment(g, b, e, q);
-        if (!err) {
-          for (int d = 0; d < 3; ++d) {
-            a.dep_b[d][n] = b[d];
-            a.dep_e[d][n] = e[d];
-          }
-          deferred = true;
-        }
-        continue;
-      }
-    }
-    err = validate ? deposit_segment<S, Q>(g, b, e, q) : deposit_current<S, Q>(g, b, e, q);
+  // Plain: both ends strictly inside every boundary's tests (false for NaN).
+  bool plain = !err && !s.released && lab_z_from_box_zt(a.frame, start[2], t) < a.exit_lab_z &&
+               lab_z_from_box_zt(a.frame, pos[2], t + g.dt) < a.exit_lab_z;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double lo = fmax(a.region.physical_lower[d], a.region.global_lower[d]);
+    const double hi = fmin(a.region.physical_upper[d], a.region.global_upper[d]);
+    plain = plain && start[d] >= lo && start[d] <= hi && pos[d] >= lo && pos[d] <= hi;
   }
-  bool born_kept = false;
-  CarrierState born;
-  if (!err && has_main && action == 1) {
-    if (selected.face == 5) {
-      atomicAdd(&a.counters->exits, 1ull);
-      atomicAdd(&a.counters->exit_charge, q);
-    } else {
-      atomicAdd(&a.counters->cpml[selected.face], 1ull);
-      atomicAdd(&a.counters->cpml_charge[selected.face], q);
-    }
-    for (int d = 0; d < 3; ++d) born.pos[d] = pos[d];
-    const double gamma = gamma_u(u[0], u[1], u[2]);
-    const double sv = kC / gamma;
-    for (int d = 0; d < 3; ++d) born.vel[d] = u[d] * sv;
-    born.q = q;
-    born.w = 1.0;
-    const double global_end = seg_frac + selected.fraction * (1.0 - seg_frac);
-    err = carrier_segment<S, Q>(g, a.region, born, selected.position, global_end, a.counters,
-                          born_kept);
-  } else if (!err && has_main && action == 2) {
-    atomicAdd(&a.counters->direct[selected.face], 1ull);
-    atomicAdd(&a.counters->direct_charge[selected.face], q);
+  plain = plain && start[2] >= g.origin[2];
+  if (!plain) {
+    a.events[atomicAdd(&a.counters->events, 1u)] = (unsigned)n;
+    if (err) raise_error(a.status, err, (unsigned long long)n);
   }
-  if (err) raise_error(a.status, err, (unsigned long long)n);
-  // Retained, held and newborn-carrier counts (one atomic per warp group).
-  count_lanes(&a.counters->held, !err && action == 0 && frozen1);
-  count_lanes(&a.counters->retained, action == 0);
-  count_lanes(&a.counters->born_kept, born_kept);
+  count_lanes(&a.counters->held, plain && frozen1);
   a.x1[n] = pos[0]; a.y1[n] = pos[1]; a.z1[n] = pos[2];
   a.ux1[n] = u[0]; a.uy1[n] = u[1]; a.uz1[n] = u[2];
   a.frozen1[n] = frozen1 ? 1 : 0;
@@ -1501,31 +1395,173 @@ __global__ void APRL_PUSH_BOUNDS push_deposit_kernel(const __grid_constant__ Pus
     a.slot.z0[n] = s.start[2];
     a.slot.dt[n] = s.dt;
   }
-  for (int d = 0; d < 3; ++d) {
-    a.used_e[3 * n + d] = used_e[d];
-    a.used_b[3 * n + d] = used_b[d];
-  }
   a.abs_grid_work[n] = abs_work;
-  a.action[n] = action;
-  if constexpr (S == 0) a.dep_mode[n] = deferred ? 1 : 0;
-  a.born_keep[n] = born_kept ? 1 : 0;
-  if (born_kept) {
-    a.born.px[n] = born.pos[0]; a.born.py[n] = born.pos[1]; a.born.pz[n] = born.pos[2];
-    a.born.vx[n] = born.vel[0]; a.born.vy[n] = born.vel[1]; a.born.vz[n] = born.vel[2];
-    a.born.q[n] = born.q;
-    a.born.w[n] = born.w;
-    a.born.key[n] = a.key_base | (a.p.order[n] & 0xffffffffull);
+  a.action[n] = 0;
+  a.plain[n] = plain ? 1 : 0;
+  a.born_keep[n] = 0;
+}
+
+// The deposit and boundary pass (src/simulation.cpp:5083-5368) of the listed
+// particles: upstream admission clip, the frozen part up to an activation
+// kink (4684-4756) and processActiveSegment (4760-4917) with
+// Simulation::firstMovingWindowEntry
+// (src/simulation_moving_window.cpp:380-395).  Runs beside the chord deposit.
+template <class F, int S, bool Q>
+__global__ void push_events_kernel(const __grid_constant__ PushArgs<F> a) {
+  if (trial_skipped(a.g)) return;
+  const unsigned listed = a.counters->events;
+  for (unsigned l = blockIdx.x * blockDim.x + threadIdx.x; l < listed;
+       l += gridDim.x * blockDim.x) {
+    const long long n = a.events[l];
+    const GridT<F>& g = a.g;
+    const double t = a.time, dt = g.dt;
+    double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
+    const double pos[3] = {a.x1[n], a.y1[n], a.z1[n]};
+    const double q = a.p.q[n];
+    const bool frozen0 = a.p.frozen[n] != 0;
+    const SlotPlan s = plan_slot(g, a.frame, a.activation_plane_lab_z, t, start, frozen0,
+                                 frozen0 ? a.p.beta[n] : 0.0);
+    unsigned err = s.err;
+    const bool frozen1 = frozen0 && !s.released;
+    if (!err && s.released) atomicAdd(&a.counters->activations, 1ull);
+    // An optional leading piece, then the main segment: the upstream part of
+    // an admitted held particle (deposited without validation), or the frozen
+    // part up to an activation kink (which may not cross a boundary).
+    double seg_frac = 0.0;
+    bool has_pre = false, pre_validate = false, has_main = true;
+    double pre_end[3] = {pos[0], pos[1], pos[2]};
+    const double pre_start[3] = {start[0], start[1], start[2]};
+    if (!err && start[2] < g.origin[2]) {
+      if (!frozen0 || !frozen1) {
+        err = kErrAdmission;
+      } else if (pos[2] < g.origin[2]) {
+        has_pre = true;
+        has_main = false;
+      } else {
+        const double fraction = (g.origin[2] - start[2]) / (pos[2] - start[2]);
+        if (!(fraction >= 0.0 && fraction <= 1.0) || !isfinite(fraction)) {
+          err = kErrAdmission;
+        } else {
+          for (int d = 0; d < 3; ++d) pre_end[d] = start[d] + fraction * (pos[d] - start[d]);
+          pre_end[2] = g.origin[2];
+          has_pre = true;
+          seg_frac = fraction;
+          for (int d = 0; d < 3; ++d) start[d] = pre_end[d];
+        }
+      }
+    } else if (!err && s.released && s.time > t && s.time < t + dt) {
+      Hit hc, ho;
+      bool enters = false, exits = false;
+      err = cpml_first_entry(a.region, start, s.start, hc, enters);
+      if (!err) err = outer_first_exit(a.region, start, s.start, ho, exits);
+      if (!err && (enters || exits)) err = kErrHeldBoundary;
+      for (int d = 0; d < 3; ++d) pre_end[d] = s.start[d];
+      has_pre = true;
+      pre_validate = true;
+      for (int d = 0; d < 3; ++d) start[d] = s.start[d];
+      seg_frac = (s.time - t) / dt;
+    }
+    unsigned char action = 0;
+    Hit selected;
+    for (int piece = has_pre ? 0 : 1; piece < (has_main ? 2 : 1) && !err; ++piece) {
+      double b[3], e[3];
+      bool validate = true;
+      if (piece == 0) {
+        for (int d = 0; d < 3; ++d) {
+          b[d] = pre_start[d];
+          e[d] = pre_end[d];
+        }
+        validate = pre_validate;
+      } else {
+        // firstMovingWindowEntry = CPML first entry + fixed-lab exit plane
+        Hit cpml_hit, outer_hit;
+        bool enters = false, exits = false;
+        err = cpml_first_entry(a.region, start, pos, cpml_hit, enters);
+        if (!err) {
+          const double za = lab_z_from_box_zt(a.frame, start[2], t + seg_frac * dt) - a.exit_lab_z;
+          const double zb = lab_z_from_box_zt(a.frame, pos[2], t + dt) - a.exit_lab_z;
+          if (za >= 0.) err = kErrBeyondExit;
+          else if (zb >= 0. && zb > za) {
+            const double fraction = -za / (zb - za);
+            if (!enters || fraction < cpml_hit.fraction) {
+              for (int d = 0; d < 3; ++d)
+                cpml_hit.position[d] = start[d] + fraction * (pos[d] - start[d]);
+              cpml_hit.fraction = fraction;
+              cpml_hit.face = 5;
+              enters = true;
+            }
+          }
+        }
+        if (!err) err = outer_first_exit(a.region, start, pos, outer_hit, exits);
+        if (err) break;
+        if (enters && (!exits || cpml_hit.fraction <= outer_hit.fraction + 64.0 * kEpsilon)) {
+          action = 1;
+          selected = cpml_hit;
+        } else if (exits) {
+          action = 2;
+          selected = outer_hit;
+        }
+        for (int d = 0; d < 3; ++d) {
+          b[d] = start[d];
+          e[d] = action ? selected.position[d] : pos[d];
+        }
+      }
+      err = validate ? deposit_segment<S, Q>(g, b, e, q) : deposit_current<S, Q>(g, b, e, q);
+    }
+    bool born_kept = false;
+    CarrierState born;
+    if (!err && has_main && action == 1) {
+      if (selected.face == 5) {
+        atomicAdd(&a.counters->exits, 1ull);
+        atomicAdd(&a.counters->exit_charge, q);
+      } else {
+        atomicAdd(&a.counters->cpml[selected.face], 1ull);
+        atomicAdd(&a.counters->cpml_charge[selected.face], q);
+      }
+      for (int d = 0; d < 3; ++d) born.pos[d] = pos[d];
+      const double u[3] = {a.ux1[n], a.uy1[n], a.uz1[n]};
+      const double gamma = gamma_u(u[0], u[1], u[2]);
+      const double sv = kC / gamma;
+      for (int d = 0; d < 3; ++d) born.vel[d] = u[d] * sv;
+      born.q = q;
+      born.w = 1.0;
+      const double global_end = seg_frac + selected.fraction * (1.0 - seg_frac);
+      err = carrier_segment<S, Q>(g, a.region, born, selected.position, global_end, a.counters,
+                                  born_kept);
+    } else if (!err && has_main && action == 2) {
+      atomicAdd(&a.counters->direct[selected.face], 1ull);
+      atomicAdd(&a.counters->direct_charge[selected.face], q);
+    }
+    if (err) raise_error(a.status, err, (unsigned long long)n);
+    if (born_kept && born.pos[2] >= a.crop_upper) {
+      born_kept = false;
+      atomicAdd(&a.counters->cropped, 1ull);
+      atomicAdd(&a.counters->cropped_charge, born.q * born.w);
+    }
+    // Held, lost and newborn-carrier counts (one atomic per warp group).
+    count_lanes(&a.counters->held, !err && action == 0 && frozen1);
+    count_lanes(&a.counters->lost, action != 0);
+    count_lanes(&a.counters->born_kept, born_kept);
+    a.action[n] = action;
+    if (born_kept) {
+      a.born_keep[n] = 1;
+      a.born.px[n] = born.pos[0]; a.born.py[n] = born.pos[1]; a.born.pz[n] = born.pos[2];
+      a.born.vx[n] = born.vel[0]; a.born.vy[n] = born.vel[1]; a.born.vz[n] = born.vel[2];
+      a.born.q[n] = born.q;
+      a.born.w[n] = born.w;
+      a.born.key[n] = a.key_base | (a.p.order[n] & 0xffffffffull);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// The deposit of the main chords of linear-binomial3 particles
-// (Current::deposit, src/longitudinal_shape.h:175-187, with the cut pieces of
-// weights() and binomialXZSegment, :61-117) into the raw current, one thread
-// per particle with the warp converged.  The warp walks the cut pieces of its
-// lanes' chords in step: at each step every lane holds at most one piece,
-// whose 12 narrow weights (binomial_linear_segment) fall on the 2x2 nodes of
-// each component around the piece's cell (i, j, k).  Particles are stored in
+// The deposit of the plain particles' chords (Current::deposit,
+// src/longitudinal_shape.h:175-187, with the cut pieces of weights(), :61-117)
+// into the raw current, one thread per particle with the warp converged.  The
+// warp walks the cut pieces of its lanes' chords in step: at each step every
+// lane holds at most one piece, whose narrow weights (binomial_linear_segment:
+// 12; quintic_linear_segment: 44) fall on nodes fixed by the piece's cell
+// (i, j, k).  Particles are stored in
 // cell order, so lanes holding pieces of the same cell sit side by side; such
 // a run of lanes adds its weights with a segmented shuffle scan, and the
 // run's last lane issues the reductions for all of them.  A lone lane adds
@@ -1552,20 +1588,32 @@ __device__ __forceinline__ void chord_add(const DGrid& g, int a, size_t at, doub
   }
 }
 
-// One cut piece's cell and narrow factors.
-struct PieceGeometry {
+// One cut piece's cell and narrow factors; piece_of is false for a quintic
+// piece whose Gauss points do not share a cell.
+template <int S>
+struct Piece;
+
+template <>
+struct Piece<0> {
   int i, j, k;
   double fx, fy, fz;
   double width, xy, xz, yz;
 };
 
-__device__ __forceinline__ void piece_geometry(const DGrid& g, const CutWalker& w, double first,
-                                               double last, PieceGeometry& p) {
+template <>
+struct Piece<1> {
+  int i, j, k;
+  double factor[4], fx[4], fy[4], fz[4];
+};
+
+// Cells by 32-bit conversion: the ends are inside the domain to roundoff
+// (validate_segment).
+__device__ __forceinline__ bool piece_of(const DGrid& g, const CutWalker& w, double first,
+                                         double last, Piece<0>& p) {
   p.width = last - first;
   const double mid = (first + last) * 0.5;
   const double px = w.a0.x + mid * w.a0.v, py = w.a1.x + mid * w.a1.v,
                pz = w.a2.x + mid * w.a2.v;
-  // the endpoints are inside the domain to roundoff (validate_segment)
   p.i = (int)floor(px);
   p.j = (int)floor(py);
   p.k = (int)floor(pz);
@@ -1578,6 +1626,37 @@ __device__ __forceinline__ void piece_geometry(const DGrid& g, const CutWalker& 
   p.xy = curvature * w.a0.v * w.a1.v;
   p.xz = curvature * w.a0.v * w.a2.v;
   p.yz = curvature * w.a1.v * w.a2.v;
+  return true;
+}
+
+__device__ __forceinline__ bool piece_of(const DGrid& g, const CutWalker& w, double first,
+                                         double last, Piece<1>& p) {
+  const double q[4] = {-.8611363115940525752, -.3399810435848562648,
+                       .3399810435848562648, .8611363115940525752};
+  const double qw[4] = {.3478548451374538574, .6521451548625461426,
+                        .6521451548625461426, .3478548451374538574};
+  const double width = last - first;
+  bool same = true;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const double u = .5 * (last + first + width * q[t]);
+    const double px = w.a0.x + u * w.a0.v, py = w.a1.x + u * w.a1.v, pz = w.a2.x + u * w.a2.v;
+    int i = (int)floor(px), j = (int)floor(py);
+    const int k = (int)floor(pz);
+    if (i == g.nx) --i;
+    if (j == g.ny) --j;
+    p.factor[t] = .5 * width * qw[t];
+    p.fx[t] = px - i;
+    p.fy[t] = py - j;
+    p.fz[t] = pz - k;
+    if (t == 0) {
+      p.i = i;
+      p.j = j;
+      p.k = k;
+    }
+    same = same && i == p.i && j == p.j && k == p.k;
+  }
+  return same;
 }
 
 // The 2x2 narrow weights of a piece over two directions, index 2 * second +
@@ -1591,10 +1670,9 @@ __device__ __forceinline__ void piece_weights(double width, double f, double h, 
   out[3] = s * (f * h + cross);
 }
 
-__device__ __forceinline__ unsigned long long piece_key(int i, int j, int k,
-                                                        unsigned long long kind) {
-  return (kind << 63) | ((unsigned long long)(k + 2) << 42) |
-         ((unsigned long long)(j + 2) << 21) | (unsigned long long)(i + 2);
+__device__ __forceinline__ unsigned long long piece_key(int i, int j, int k) {
+  return ((unsigned long long)(k + 2) << 42) | ((unsigned long long)(j + 2) << 21) |
+         (unsigned long long)(i + 2);
 }
 
 // Runs of neighbouring lanes holding the same key: this lane's run head,
@@ -1616,79 +1694,121 @@ __device__ __forceinline__ Runs lane_runs(unsigned long long key, int lane) {
   return r;
 }
 
-template <bool Q>
-__global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(ChordArgs a) {
+template <int S, bool Q>
+__global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ ChordArgs a) {
   if (trial_skipped(a.g)) return;
   const DGrid& g = a.g;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  bool alive = n < a.count && a.mode[n] != 0;
+  bool alive = n < a.count && a.plain[n] != 0;
   unsigned err = kErrNone;
   double scale[3] = {0., 0., 0.};
   CutWalker w;
   w.done = true;
   if (alive) {
-    double b[3], e[3];
-    for (int d = 0; d < 3; ++d) {
-      b[d] = a.b[d][n];
-      e[d] = a.e[d][n];
-    }
-    const double q = a.q[n];
-    for (int d = 0; d < 3; ++d) scale[d] = q * (e[d] - b[d]) / (g.dx * g.dy * g.dz * g.dt);
-    if (!w.init(g, b, e)) {
-      err = kErrCrossingBudget;
-      alive = false;
-    }
+    const double b[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
+    const double e[3] = {a.x1[n], a.y1[n], a.z1[n]};
+    const double q = a.p.q[n];
+    err = validate_segment(g, b, e, q);
+    if (!err && !w.init(g, b, e)) err = kErrCrossingBudget;
+    alive = !err;
+    if (alive)
+      for (int d = 0; d < 3; ++d) scale[d] = q * (e[d] - b[d]) / (g.dx * g.dy * g.dz * g.dt);
   }
   const long long p0 = g.nx + 2, p1 = g.nx + 3;  // row pitches of Jx and of Jy, Jz
-  const long long z0 = p0 * (g.ny + 1), z1 = p1 * g.ny;
+  const long long z0 = p0 * (g.ny + 1), z1 = p1 * g.ny, z2 = p1 * (g.ny + 1);
   // ---- one piece per lane per round; a chord of a beam that moves about a
   // cell per step along z has two, in z-neighbouring cells.
   while (__any_sync(0xffffffffu, alive)) {
     double first = 0., last = 0.;
-    const bool have = alive && w.advance(first, last);
+    bool have = alive && w.advance(first, last);
     if (!have) alive = false;
     // A lane without a piece takes a key no other lane has and adds nothing.
-    PieceGeometry p{};
     unsigned long long key = ~0ull - (unsigned long long)lane;
+    Piece<S> p;
     if (have) {
-      piece_geometry(g, w, first, last, p);
-      key = piece_key(p.i, p.j, p.k, 0);
+      if (piece_of(g, w, first, last, p)) {
+        key = piece_key(p.i, p.j, p.k);
+      } else {  // quintic Gauss points that straddle a cell
+        const double x[3] = {w.a0.x, w.a1.x, w.a2.x}, v[3] = {w.a0.v, w.a1.v, w.a2.v};
+        DepositVisitor<double, Q> visit{&g, {scale[0], scale[1], scale[2]}, S == 0, kErrNone};
+        quintic_linear_segment(g, x, v, first, last, last - first, visit);
+        if (visit.error) err = visit.error;
+        have = false;
+      }
     }
+    if (!have) p = Piece<S>{};
     const Runs runs = lane_runs(key, lane);
-    // The visitor's support rules: x outside is skipped (the F3 x support may
-    // leave the grid; the raw array holds the nodes one step outside, which
-    // still reach it), y outside is an error when the lane carries current on
-    // that axis, z outside the padding is skipped.
+    // The visitor's support rules: x outside is skipped by linear-binomial3
+    // (the F3 x support may leave the grid; the raw array holds the nodes one
+    // step outside, which still reach it) and an error for the quintic shape,
+    // y outside is an error when the lane carries current on that axis, z
+    // outside the padding is skipped.  The chord is inside the domain.
     const bool y_inside = p.j >= 0 && p.j < g.ny;
-    if (have && !y_inside && (scale[0] != 0. || scale[1] != 0. || scale[2] != 0.))
-      err = kErrSupportY;
-    const bool adds = have && runs.last && y_inside && p.i >= -1 && p.i <= g.nx && p.k >= -1 &&
-                      p.k <= g.nz;
-    const long long n0 = ((p.k + 1) * (long long)(g.ny + 1) + p.j) * p0 + (p.i + 1);
-    const long long n1 = ((p.k + 1) * (long long)g.ny + p.j) * p1 + (p.i + 1);
-    const long long n2 = ((p.k + 1) * (long long)(g.ny + 1) + p.j) * p1 + (p.i + 1);
-    double v[4];
-    piece_weights(p.width, p.fy, p.fz, p.yz, scale[0], v);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {  // Jx: y, z
-      const double total = run_sum(v[t], lane, runs.head, runs.span);
-      if (adds && total != 0.)
-        chord_add<Q>(g, 0, n0 + (t & 1 ? p0 : 0) + (t & 2 ? z0 : 0), total, err);
+    const bool x_inside = S == 0 ? p.i >= -1 && p.i <= g.nx : p.i >= 0 && p.i < g.nx;
+    if (have && (scale[0] != 0. || scale[1] != 0. || scale[2] != 0.)) {
+      if (!y_inside) err = kErrSupportY;
+      if (S != 0 && !x_inside) err = kErrSupportX;
     }
-    piece_weights(p.width, p.fx, p.fz, p.xz, scale[1], v);
+    const bool adds = have && runs.last && y_inside && x_inside && p.k >= -1 && p.k <= g.nz;
+    constexpr int kReach = S == 0 ? 0 : 2;  // nodes below the piece's cell in z
+    const long long kz = p.k + g.jpad - kReach;
+    const long long n0 = (kz * (g.ny + 1) + p.j) * p0 + (p.i + 1);
+    const long long n1 = (kz * g.ny + p.j) * p1 + (p.i + 1);
+    const long long n2 = (kz * (g.ny + 1) + p.j) * p1 + (p.i + 1);
+    auto add = [&](int c, long long at, double v) {
+      const double total = run_sum(v, lane, runs.head, runs.span);
+      if (adds && total != 0.) chord_add<Q>(g, c, (size_t)at, total, err);
+    };
+    if constexpr (S == 0) {
+      double v[4];
+      piece_weights(p.width, p.fy, p.fz, p.yz, scale[0], v);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {  // Jy: x, z
-      const double total = run_sum(v[t], lane, runs.head, runs.span);
-      if (adds && total != 0.)
-        chord_add<Q>(g, 1, n1 + (t & 1) + (t & 2 ? z1 : 0), total, err);
-    }
-    piece_weights(p.width, p.fx, p.fy, p.xy, scale[2], v);
+      for (int t = 0; t < 4; ++t) add(0, n0 + (t & 1 ? p0 : 0) + (t & 2 ? z0 : 0), v[t]);
+      piece_weights(p.width, p.fx, p.fz, p.xz, scale[1], v);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {  // Jz: x, y
-      const double total = run_sum(v[t], lane, runs.head, runs.span);
-      if (adds && total != 0.)
-        chord_add<Q>(g, 2, n2 + (t & 1) + (t & 2 ? p1 : 0), total, err);
+      for (int t = 0; t < 4; ++t) add(1, n1 + (t & 1) + (t & 2 ? z1 : 0), v[t]);
+      piece_weights(p.width, p.fx, p.fy, p.xy, scale[2], v);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) add(2, n2 + (t & 1) + (t & 2 ? p1 : 0), v[t]);
+    } else {
+      double m[4][6];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) spline_edge(p.fz[t], m[t]);
+#pragma unroll
+      for (int q = 0; q < 5; ++q) {  // Jz: edge basis
+        double v[4] = {0., 0., 0., 0.};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const double wt = p.factor[t] * m[t][q];
+          const double wx = wt * p.fx[t], wo = wt * (1. - p.fx[t]);
+          v[0] += wo * (1. - p.fy[t]);
+          v[1] += wx * (1. - p.fy[t]);
+          v[2] += wo * p.fy[t];
+          v[3] += wx * p.fy[t];
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          add(2, n2 + q * z2 + (t & 1) + (t & 2 ? p1 : 0), scale[2] * v[t]);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) quintic_spline_level(m[t], p.fz[t], 5);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {  // Jx, Jy: node basis
+        double v[4] = {0., 0., 0., 0.};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const double wt = p.factor[t] * m[t][q];
+          v[0] += wt * (1. - p.fy[t]);
+          v[1] += wt * p.fy[t];
+          v[2] += wt * (1. - p.fx[t]);
+          v[3] += wt * p.fx[t];
+        }
+        add(0, n0 + q * z0, scale[0] * v[0]);
+        add(0, n0 + q * z0 + p0, scale[0] * v[1]);
+        add(1, n1 + q * z1, scale[1] * v[2]);
+        add(1, n1 + q * z1 + 1, scale[1] * v[3]);
+      }
     }
   }
   if (err) raise_error(a.status, err, (unsigned long long)n);
@@ -1744,6 +1864,18 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
+}
+
+// solveConservativeSourceStep's stopping rule (src/simulation_source_coupling.cpp:50).
+__device__ __forceinline__ void trial_verdict(unsigned long long force_bits, double defect,
+                                              double scale, unsigned long long pushed,
+                                              unsigned iterations, double force_tolerance,
+                                              double work_tolerance, int* stop) {
+  const double force = __longlong_as_double((long long)force_bits);
+  const double calls = (double)pushed;
+  const double work = calls == 0. ? 0. : (scale > 0. ? defect / scale : defect);
+  if (iterations >= (calls > 0. ? 2u : 1u) && force < force_tolerance && work < work_tolerance)
+    *stop = (int)iterations;
 }
 
 template <class W, class F, int S, bool DB>
@@ -1862,16 +1994,20 @@ __global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ Res
     a.sums->defect = d;
     a.sums->scale = c;
     *a.ticket = 0u;
+    if (a.stop)
+      trial_verdict(__ldcg(&a.sums->force_bits), d, c, __ldcg(&a.sums->calls), a.iterations,
+                    a.force_tolerance, a.work_tolerance, a.stop);
   }
 }
 
 // ---------------------------------------------------------------------------
 // Stable compaction: the retained list keeps the reference's push_back
 // order (src/simulation.cpp:4916, 5581).
-__global__ void flag_count_kernel(const unsigned char* flag, unsigned char want, long long n,
-                                  unsigned* block_count) {
-  const long long i = (long long)blockIdx.x * kScanBlock + threadIdx.x;
-  const bool f = i < n && flag[i] == want;
+__global__ void flag_count_kernel(FlagLists a) {
+  const int l = blockIdx.x >= a.list[2].first ? 2 : (blockIdx.x >= a.list[1].first ? 1 : 0);
+  const FlagList& list = a.list[l];
+  const long long i = (long long)(blockIdx.x - list.first) * kScanBlock + threadIdx.x;
+  const bool f = i < list.n && list.flag[i] == list.want;
   const unsigned ballot = __ballot_sync(0xffffffffu, f);
   __shared__ unsigned warp_count[kScanBlock / 32];
   if ((threadIdx.x & 31) == 0) warp_count[threadIdx.x >> 5] = __popc(ballot);
@@ -1879,35 +2015,65 @@ __global__ void flag_count_kernel(const unsigned char* flag, unsigned char want,
   if (threadIdx.x == 0) {
     unsigned s = 0;
     for (int w = 0; w < kScanBlock / 32; ++w) s += warp_count[w];
-    block_count[blockIdx.x] = s;
+    a.block_count[blockIdx.x] = s;
   }
 }
 
-// Exclusive scan of the per-block counts by one block of 1024 threads.
-__global__ void block_offset_scan_kernel(const unsigned* block_count, int blocks,
-                                         unsigned* block_offset,
-                                         unsigned long long* total) {
-  __shared__ unsigned partial[1024];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
+// Exclusive scan by one block of 1024 threads, eight values a thread a round:
+// warps scan by shuffle, one warp scans their sums.  (With one value a thread
+// and a barrier per doubling it took 9 us for 4000 counts.)
+__device__ __forceinline__ void block_scan(const unsigned* in, int n, unsigned* out) {
+  constexpr int kItems = 8;
+  __shared__ unsigned warp_sum[32];
+  __shared__ unsigned carry;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry = 0u;
   __syncthreads();
-  for (int base = 0; base < blocks; base += 1024) {
-    const int i = base + threadIdx.x;
-    const unsigned v = i < blocks ? block_count[i] : 0u;
-    partial[threadIdx.x] = v;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      const unsigned add = threadIdx.x >= off ? partial[threadIdx.x - off] : 0u;
-      __syncthreads();
-      partial[threadIdx.x] += add;
-      __syncthreads();
+  for (int base = 0; base < n; base += 1024 * kItems) {
+    const int first = base + (int)threadIdx.x * kItems;
+    unsigned v[kItems], sum = 0u;
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+      v[t] = first + t < n ? in[first + t] : 0u;
+      sum += v[t];
     }
-    if (i < blocks) block_offset[i] = (unsigned)(carry + partial[threadIdx.x] - v);
+    unsigned below = sum;
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, below, d);
+      if (lane >= d) below += u;
+    }
+    if (lane == 31) warp_sum[warp] = below;
     __syncthreads();
-    if (threadIdx.x == 1023) carry += partial[1023];
+    if (warp == 0) {
+      const unsigned own = warp_sum[lane];
+      unsigned w = own;
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, w, d);
+        if (lane >= d) w += u;
+      }
+      warp_sum[lane] = w - own;
+    }
+    __syncthreads();
+    unsigned at = carry + warp_sum[warp] + below - sum;
+#pragma unroll
+    for (int t = 0; t < kItems; ++t) {
+      if (first + t < n) out[first + t] = at;
+      at += v[t];
+    }
+    __syncthreads();
+    if (threadIdx.x == 1023) carry = at;
     __syncthreads();
   }
-  if (threadIdx.x == 0) *total = carry;
+}
+
+__global__ void flag_scan_kernel(FlagLists a) {
+  const FlagList& list = a.list[blockIdx.x];
+  block_scan(a.block_count + list.first, (int)list.blocks, a.block_offset + list.first);
+}
+
+__global__ void block_offset_scan_kernel(const unsigned* block_count, int blocks,
+                                         unsigned* block_offset) {
+  block_scan(block_count, blocks, block_offset);
 }
 
 __device__ __forceinline__ long long compact_slot(const unsigned char* flag, unsigned char want,
@@ -2168,10 +2334,11 @@ __global__ void crop_flags_kernel(DCarriers c, long long n, double upper, double
 
 // migrateWindowObjects' inlet guard (src/simulation_moving_window.cpp:355-358).
 __global__ void inlet_check_kernel(const double* z, const unsigned char* frozen, long long n,
-                                   double origin, DeviceStatus* status) {
+                                   const double* cz, long long nc, double origin,
+                                   DeviceStatus* status) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && z[i] < origin && !frozen[i])
-    raise_error(status, kErrFellBehind, (unsigned long long)i);
+  if (i < n ? z[i] < origin && !frozen[i] : i < n + nc && cz[i - n] < origin)
+    raise_error(status, kErrFellBehind, (unsigned long long)(i < n ? i : i - n));
 }
 
 __global__ void inlet_charge_kernel(InletMatchArgs a) {
@@ -2241,8 +2408,8 @@ __global__ void inlet_charge_kernel(InletMatchArgs a) {
     }
 }
 
-__global__ void trial_clear_kernel(GridT<double> g, TrialCounters* counters, ResidualSums* sums,
-                                   int clear_current) {
+__global__ void trial_clear_kernel(GridT<double> g, TrialResult* result, int clear_current,
+                                   int* reset_stop) {
   if (trial_skipped(g)) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2256,8 +2423,8 @@ __global__ void trial_clear_kernel(GridT<double> g, TrialCounters* counters, Res
     }
   }
   if (first == 0) {
-    *counters = TrialCounters{};
-    *sums = ResidualSums{};
+    *result = TrialResult{};
+    if (reset_stop) *reset_stop = 0;
   }
 }
 
@@ -2286,12 +2453,8 @@ __global__ void fixed_convert_kernel(const unsigned long long* pairs, double* ou
 __global__ void trial_verdict_kernel(const ResidualSums* sums, unsigned iterations,
                                      double force_tolerance, double work_tolerance, int* stop) {
   if (*stop) return;
-  const double force = __longlong_as_double((long long)sums->force_bits);
-  const double calls = (double)sums->calls;
-  const double work =
-      calls == 0. ? 0. : (sums->scale > 0. ? sums->defect / sums->scale : sums->defect);
-  if (iterations >= (calls > 0. ? 2u : 1u) && force < force_tolerance && work < work_tolerance)
-    *stop = (int)iterations;
+  trial_verdict(sums->force_bits, sums->defect, sums->scale, sums->calls, iterations,
+                force_tolerance, work_tolerance, stop);
 }
 
 // The grid and J are binary64 in every mode; the gathers are built with
@@ -2300,8 +2463,10 @@ __global__ void trial_verdict_kernel(const ResidualSums* sums, unsigned iteratio
 // 1 quintic-compensated), so a kernel carries the registers and local
 // memory of its own shape's weights only.
 #define APRL_SHAPE_KERNELS(S)                                                        \
-  template __global__ void push_deposit_kernel<double, S, false>(const __grid_constant__ PushArgs<double>);  \
-  template __global__ void push_deposit_kernel<double, S, true>(const __grid_constant__ PushArgs<double>);   \
+  template __global__ void push_events_kernel<double, S, false>(const __grid_constant__ PushArgs<double>);  \
+  template __global__ void push_events_kernel<double, S, true>(const __grid_constant__ PushArgs<double>);   \
+  template __global__ void chord_deposit_kernel<S, false>(const __grid_constant__ ChordArgs); \
+  template __global__ void chord_deposit_kernel<S, true>(const __grid_constant__ ChordArgs);  \
   template __global__ void carrier_kernel<double, S, false>(const __grid_constant__ CarrierArgs<double>);    \
   template __global__ void carrier_kernel<double, S, true>(const __grid_constant__ CarrierArgs<double>);     \
   template __global__ void frozen_support_kernel<double, S, false>(const __grid_constant__ SupportArgs<double>); \
@@ -2317,8 +2482,7 @@ template __global__ void guess_gather_kernel<double, double, 0, true>(const __gr
 template __global__ void guess_gather_kernel<float, double, 0, true>(const __grid_constant__ PushArgs<double>);
 template __global__ void residual_kernel<double, double, 0, true>(const __grid_constant__ ResidualArgs<double>);
 template __global__ void residual_kernel<float, double, 0, true>(const __grid_constant__ ResidualArgs<double>);
-template __global__ void chord_deposit_kernel<false>(ChordArgs);
-template __global__ void chord_deposit_kernel<true>(ChordArgs);
+template __global__ void push_kernel<double>(const __grid_constant__ PushArgs<double>);
 #undef APRL_SHAPE_KERNELS
 
 }  // namespace aprl_gpu

@@ -58,9 +58,10 @@ struct TrialCounters {
   unsigned long long activations; // held particles crossing the activation plane
   unsigned long long held;        // held particles retained by the trial
   // Compaction sizes, so the commit needs no further host round trip.
-  unsigned long long retained;    // particles with action 0
+  unsigned long long lost;        // particles with action 1 or 2
   unsigned long long born_kept;   // newborn carriers kept
   unsigned long long carriers_kept;  // existing carriers kept
+  unsigned events;                // particles listed for push_events_kernel
 };
 
 struct ResidualSums {
@@ -68,6 +69,18 @@ struct ResidualSums {
   double defect;
   double scale;
   unsigned long long calls;       // pushed (seen) slots
+};
+
+// One trial's results, and a step's block of them: read back in one copy.
+struct TrialResult {
+  ResidualSums sums;
+  TrialCounters counters;
+};
+constexpr int kTrialSlots = 3;  // trials issued before the host reads any (run.cu)
+struct TrialBlock {
+  TrialResult trial[kTrialSlots];
+  int stop;             // verdict of the trials issued ahead
+  DeviceStatus status;
 };
 
 // Per-slot record of one trial push (ConservativeSourceCoupling::Impl::Slot,
@@ -108,18 +121,14 @@ struct PushArgs {
   double *x1, *y1, *z1, *ux1, *uy1, *uz1;  // state after the trial push
   unsigned char* frozen1;                  // held state after the trial
   DSlots slot;
-  double* used_e;        // 3*count, written
-  double* used_b;
-  const double* next_e;  // 3*count, from the previous residual
-  const double* next_b;
+  double* used_e;        // 3*count: the first-trial gather's or the previous
+  double* used_b;        // residual's fields (zeroed where there is no push)
   double* abs_grid_work; // sum over substeps of |grid work|
   unsigned char* action; // 0 retain, 1 CPML/exit carrier, 2 outer exit
   DCarriers born;        // carrier created by a CPML entry (when kept)
-  // linear-binomial3: the main chord, validated, for chord_deposit_kernel
-  // (dep_mode 1; 0 when the particle deposits no main chord this trial)
-  double* dep_b[3];
-  double* dep_e[3];
-  unsigned char* dep_mode;
+  unsigned char* plain;  // 1: chord_deposit_kernel deposits the chord start -> end
+  unsigned* events;      // the other particles, for push_events_kernel
+  double crop_upper;     // as in CarrierArgs, for newborn carriers
   unsigned long long key_base;  // (step + 1) << 32 for newborn carrier keys
   unsigned char* born_keep;
   TrialCounters* counters;
@@ -132,6 +141,7 @@ struct CarrierArgs {
   DRegion region;
   int shape;
   long long count;
+  double crop_upper;     // carriers at or above it are cropped by this step's shift
   DCarriers in;          // carriers at the start of the step
   DCarriers out;         // after this step's segment
   unsigned char* keep;
@@ -155,27 +165,23 @@ struct ResidualArgs {
   const double* abs_grid_work;
   ResidualSums* sums;
   // defect and scale per block; the last block to finish sums them in block
-  // order (ticket counts the finished blocks and is left at zero).
+  // order (ticket counts the finished blocks and is left at zero) and, for a
+  // trial issued ahead, applies the stopping rule.
   double* partial;
   unsigned* ticket;
+  unsigned iterations;      // this trial's number, from 1
+  double force_tolerance, work_tolerance;
+  int* stop;                // null: no verdict
   DeviceStatus* status;
 };
 
-// push_deposit_kernel leaves the main chords of linear-binomial3 particles
-// to chord_deposit_kernel, in both current-summation modes.  On the dipole
-// workload (1M particles, 128x128x512 cells) per trial: fused push and
-// deposit 0.49 ms; push 0.13 ms + merged deposit 0.30 ms with binary64
-// atomics; with the fixed-point sum, whose two integer reductions per
-// contribution bound it, 1.13 ms fused against 0.14 + 0.65 ms.
-
-// The deferred main chords of a linear-binomial3 trial.
+// The chords of a trial that chord_deposit_kernel deposits.
 struct ChordArgs {
   GridT<double> g;
   long long count;
-  const unsigned char* mode;
-  const double* b[3];
-  const double* e[3];
-  const double* q;
+  const unsigned char* plain;
+  DParticles p;                 // chord starts and charges
+  const double *x1, *y1, *z1;   // chord ends
   DeviceStatus* status;
 };
 
@@ -229,11 +235,13 @@ struct ChordArgs {
 // S: the particle shape, 0 linear-binomial3, 1 quintic-compensated.
 // D, DB: read the wide stencils directly (linear-binomial3, sparse runs).
 template <class W, class F, int S, bool D> __global__ void guess_gather_kernel(const __grid_constant__ PushArgs<F> a);
+template <class F> __global__ void APRL_PUSH_BOUNDS push_kernel(const __grid_constant__ PushArgs<F> a);
 // Q: the deterministic mode's fixed-point current sum.
 template <class F, int S, bool Q>
-__global__ void APRL_PUSH_BOUNDS push_deposit_kernel(const __grid_constant__ PushArgs<F> a);
+__global__ void push_events_kernel(const __grid_constant__ PushArgs<F> a);
 template <class F, int S, bool Q> __global__ void carrier_kernel(const __grid_constant__ CarrierArgs<F> a);
-template <bool Q> __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(ChordArgs a);
+template <int S, bool Q>
+__global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ ChordArgs a);
 template <class W, class F, int S, bool DB>
 __global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ ResidualArgs<F> a);
 
@@ -249,11 +257,25 @@ __global__ void boris_push_kernel(BorisArgs a);
 
 // Stable compaction helpers (warp ballot + block scan + block-offset scan).
 constexpr int kScanBlock = 256;
-__global__ void flag_count_kernel(const unsigned char* flag, unsigned char want,
-                                  long long n, unsigned* block_count);
+// Up to three flagged lists compacted together: one count launch, one scan
+// launch (a block per list), then a gather per kind.
+struct FlagList {
+  const unsigned char* flag;
+  long long n;
+  unsigned blocks;         // of kScanBlock
+  unsigned first;          // its first block in block_count and block_offset
+  unsigned char want;
+};
+struct FlagLists {
+  FlagList list[3];
+  unsigned* block_count;
+  unsigned* block_offset;
+};
+__global__ void flag_count_kernel(FlagLists a);
+__global__ void flag_scan_kernel(FlagLists a);
+// Exclusive scan of n counts by one block of 1024 threads.
 __global__ void block_offset_scan_kernel(const unsigned* block_count, int blocks,
-                                         unsigned* block_offset,
-                                         unsigned long long* total);
+                                         unsigned* block_offset);
 __global__ void gather_particles_kernel(DParticles out, DParticles src,
                                         const double* x1, const double* y1,
                                         const double* z1, const double* ux1,
@@ -307,8 +329,10 @@ __global__ void crop_flags_kernel(DCarriers c, long long n, double upper,
                                   TrialCounters* counters, DeviceStatus* status);
 // finishMovingWindowStep's guard (src/simulation_moving_window.cpp:358-359):
 // an active particle may not fall behind the inlet; held ones may.
+// Carriers may not either; `cz` counts on from n.
 __global__ void inlet_check_kernel(const double* z, const unsigned char* frozen, long long n,
-                                   double origin, DeviceStatus* status);
+                                   const double* cz, long long nc, double origin,
+                                   DeviceStatus* status);
 // The inlet-layer charge of the charge-matched inlet (ChargeMatchedInlet::particle,
 // src/charge_matched_inlet.h:31-53) from the stored particles and the
 // pending entries [pbegin, pbegin + pcount) at their held positions of step
@@ -336,8 +360,9 @@ __global__ void inlet_charge_kernel(InletMatchArgs a);
 // (skipped with the trial).
 // clear_current: 1 clears J; in the deterministic mode 2 clears the
 // fixed-point pairs of J instead (J is then written by current_convert).
-__global__ void trial_clear_kernel(GridT<double> g, TrialCounters* counters, ResidualSums* sums,
-                                   int clear_current);
+// reset_stop: a step's first trial, clearing the verdict of the step before.
+__global__ void trial_clear_kernel(GridT<double> g, TrialResult* result, int clear_current,
+                                   int* reset_stop);
 // Deterministic mode: J from its fixed-point pairs, every node.
 __global__ void current_convert_kernel(GridT<double> g, double unscale);
 // out[i] = value of pair i (fixed_value), for i < n.

@@ -63,7 +63,7 @@ enum Kernel : unsigned {
   kSfMoments, kSfFinish, kSfDeposit, kSfSource, kSfApply, kSfUpdate,
   kSfDirection, kSfSmooth, kSfElectric, kSfMagnetic, kSfClear, kSfGauss, kSfEnergy,
   kInletHalo, kInletCharge, kInletComplete, kRadixCount, kPermuteParticles,
-  kCurrentConvert, kFixedConvert, kChordDeposit, kSfModal, kSurfaceCurrent, kSfOpen, kKernelCount
+  kCurrentConvert, kFixedConvert, kChordDeposit, kSfModal, kSurfaceCurrent, kSfOpen, kPushEvents, kKernelCount
 };
 
 const char* kKernelNames[kKernelCount] = {
@@ -77,7 +77,7 @@ const char* kKernelNames[kKernelCount] = {
   "trial_verdict", "sf_moments", "sf_finish", "sf_deposit", "sf_source", "sf_apply",
   "sf_update", "sf_direction", "sf_smooth", "sf_electric", "sf_magnetic",
   "sf_clear", "sf_gauss", "sf_energy", "inlet_halo", "inlet_charge", "inlet_complete",
-  "radix_count", "permute_particles", "current_convert", "fixed_convert", "chord_deposit", "sf_modal", "surface_current", "sf_open"};
+  "radix_count", "permute_particles", "current_convert", "fixed_convert", "chord_deposit", "sf_modal", "surface_current", "sf_open", "push_events"};
 
 const char* device_error_text(unsigned code) {
   switch (code) {
@@ -231,9 +231,8 @@ struct Timing {
 
 }  // namespace
 
-// Fixed-point trials issued per step before the host reads any residual
-// (the usual count at FP64; FP32-mixed runs usually stop after two).
-constexpr unsigned kTrialSlots = 3;
+// kTrialSlots fixed-point trials are issued per step before the host reads any
+// residual (the usual count at FP64; FP32-mixed runs usually stop after two).
 
 // Steps between the cell sorts of the particle list (see do_commit).
 constexpr uint64_t kSortInterval = 4;
@@ -319,11 +318,13 @@ struct aprl_run {
          *uz1 = nullptr;
   double *used_e = nullptr, *used_b = nullptr, *next_e = nullptr, *next_b = nullptr;
   double* abs_work = nullptr;
-  // linear-binomial3: each particle's validated main chord of the trial,
-  // deposited by chord_deposit_kernel after the push
-  double* dep_b[3]{};
-  double* dep_e[3]{};
-  unsigned char* dep_mode = nullptr;
+  // The trial's particles whose chord chord_deposit_kernel deposits, and the
+  // list of the others for push_events_kernel.
+  unsigned char* plain = nullptr;
+  unsigned* events = nullptr;
+  // Whole steps fold the shift's crop of the carriers into the trials (the
+  // seams leave it to the shift).
+  bool crop_ahead = false;
   unsigned char* action = nullptr;
   DCarriers born{};
   unsigned char* born_keep = nullptr;
@@ -372,22 +373,16 @@ struct aprl_run {
   DCarriers c{}, c_alt{}, c_out{};
   unsigned char* c_keep = nullptr;
   // reductions, counters, status, scan scratch
-  TrialCounters* d_counters = nullptr;
-  ResidualSums* d_sums = nullptr;
-  DeviceStatus* d_status = nullptr;
+  TrialBlock* d_block = nullptr;      // trial results, verdict and status
+  DeviceStatus* d_status = nullptr;   // = &d_block->status
+  int* d_stop = nullptr;              // = &d_block->stop
   unsigned* scan_count = nullptr;
   unsigned* scan_offset = nullptr;
-  unsigned long long* scan_total = nullptr;
   size_t scan_cap = 0;
   // pinned host mirrors
-  ResidualSums* h_sums = nullptr;        // the slot of the last trial read
-  ResidualSums* h_sums_slots = nullptr;  // one slot per trial issued ahead of a read
-  TrialCounters* h_counters_slots = nullptr;
-  int* d_stop = nullptr;                 // device verdict of the trials issued ahead
-  int* h_stop = nullptr;
-  DeviceStatus* h_status = nullptr;
-  TrialCounters* h_counters = nullptr;
-  unsigned long long* h_total = nullptr;
+  TrialBlock* h_block = nullptr;
+  TrialCounters* h_counters = nullptr;  // of the last trial read
+  DeviceStatus* h_status = nullptr;     // = &h_block->status
   TrialCounters cumulative{};
   // window state
   uint64_t step = 0;
@@ -513,10 +508,7 @@ cudaError_t run_fill(aprl_run* r, void* dst, int value, size_t bytes) {
 // reuse (cudaMallocHost/cudaFreeHost per run cost milliseconds each).
 constexpr size_t kPinnedBlock = 4096;
 
-static_assert(kTrialSlots * sizeof(ResidualSums) + sizeof(DeviceStatus) +
-                      kTrialSlots * sizeof(TrialCounters) + sizeof(int) +
-                      sizeof(unsigned long long) + 5 * 64 <= kPinnedBlock,
-              "read-back areas exceed the pinned block");
+static_assert(sizeof(TrialBlock) <= kPinnedBlock, "the read-back block exceeds the pinned block");
 
 std::mutex& pinned_lock() {
   static std::mutex lock;
@@ -949,7 +941,9 @@ aprl_status validate(const aprl_run_config& g) {
 }
 
 aprl_status ensure_scan(aprl_run* r, size_t n) {
-  const size_t blocks = (n + kScanBlock - 1) / kScanBlock + 1;
+  // Blocks of up to three lists: particles and their newborn carriers (n each
+  // at most) and the existing carriers.
+  const size_t blocks = 3 * ((n + kScanBlock - 1) / kScanBlock + 1);
   if (blocks <= r->scan_cap) return APRL_OK;
   device_free(r, r->scan_count);
   device_free(r, r->scan_offset);
@@ -1017,8 +1011,7 @@ aprl_status reserve_particles(aprl_run* r, size_t n) {
   TRY(alloc_particles(r, r->p_alt, n));
   double** trial[] = {&r->x1,       &r->y1,       &r->z1,       &r->ux1,      &r->uy1,
                       &r->uz1,      &r->abs_work, &r->slots.x0, &r->slots.y0, &r->slots.z0,
-                      &r->slots.dt, &r->dep_b[0], &r->dep_b[1], &r->dep_b[2], &r->dep_e[0],
-                      &r->dep_e[1], &r->dep_e[2]};
+                      &r->slots.dt};
   for (double** t : trial) {
     device_free(r, *t);
     TRY(device_alloc(r, t, n));
@@ -1043,9 +1036,11 @@ aprl_status reserve_particles(aprl_run* r, size_t n) {
   device_free(r, r->slots.seen);
   TRY(device_alloc(r, &r->frozen1, n));
   TRY(device_alloc(r, &r->slots.seen, n));
-  device_free(r, r->dep_mode);
+  device_free(r, r->plain);
+  device_free(r, r->events);
   TRY(device_alloc(r, &r->action, n));
-  TRY(device_alloc(r, &r->dep_mode, n));
+  TRY(device_alloc(r, &r->plain, n));
+  TRY(device_alloc(r, &r->events, n));
   TRY(device_alloc(r, &r->born_keep, n));
   TRY(device_alloc(r, &r->slot_order, n));
   for (int k = 0; k < 2; ++k) {
@@ -1126,13 +1121,25 @@ aprl_status copy_ring(aprl_run* r, double* device, const double* host_in, double
   return APRL_OK;
 }
 
-aprl_status check_device(aprl_run* r) {
-  CUDA_TRY(cudaMemcpyAsync(r->h_status, r->d_status, sizeof(DeviceStatus),
-                           cudaMemcpyDeviceToHost, r->stream));
+// Waits for the stream; the device status as last read back.
+aprl_status wait_status(aprl_run* r) {
   CUDA_TRY(cudaStreamSynchronize(r->stream));
   if (r->h_status->code)
     return fail(device_error_status(r->h_status->code), "%s (element %llu)",
                 device_error_text(r->h_status->code), r->h_status->where);
+  return APRL_OK;
+}
+
+aprl_status check_device(aprl_run* r) {
+  CUDA_TRY(cudaMemcpyAsync(r->h_status, r->d_status, sizeof(DeviceStatus),
+                           cudaMemcpyDeviceToHost, r->stream));
+  return wait_status(r);
+}
+
+// The trials' results, the verdict and the status in one read-back.
+aprl_status read_block(aprl_run* r) {
+  CUDA_TRY(cudaMemcpyAsync(r->h_block, r->d_block, sizeof(TrialBlock), cudaMemcpyDeviceToHost,
+                           r->stream));
   return APRL_OK;
 }
 
@@ -1159,17 +1166,34 @@ void add_counters(TrialCounters& to, const TrialCounters& from) {
   to.activations += from.activations;
 }
 
-// Block offsets of a stable compaction of `n` flagged elements (the kept
-// count is known to the caller).
-aprl_status compact_offsets(aprl_run* r, const unsigned char* flag, unsigned char want,
-                            size_t n) {
-  if (n == 0) return APRL_OK;
-  TRY(ensure_scan(r, n));
-  const unsigned blocks = blocks_for(n, kScanBlock);
-  TRY(launch(r, kFlagCount, flag_count_kernel, dim3(blocks), dim3(kScanBlock), flag, want,
-             (long long)n, r->scan_count));
-  return launch(r, kBlockScan, block_offset_scan_kernel, dim3(1), dim3(1024),
-                (const unsigned*)r->scan_count, (int)blocks, r->scan_offset, r->scan_total);
+// Block offsets of the stable compactions of up to three flagged lists (the
+// kept counts are known to the caller).
+struct Compaction {
+  FlagLists lists{};
+  unsigned blocks = 0;
+  int count = 0;
+  // Returns the list's number, for offsets().
+  int add(const unsigned char* flag, unsigned char want, size_t n) {
+    FlagList& l = lists.list[count];
+    l.flag = flag;
+    l.want = want;
+    l.n = (long long)n;
+    l.blocks = blocks_for(n, kScanBlock);
+    l.first = blocks;
+    blocks += l.blocks;
+    for (int t = count + 1; t < 3; ++t) lists.list[t].first = blocks;
+    return count++;
+  }
+  const unsigned* offsets(int list) const { return lists.block_offset + lists.list[list].first; }
+};
+
+aprl_status compact_offsets(aprl_run* r, Compaction& c) {
+  if (!c.blocks) return APRL_OK;
+  TRY(ensure_scan(r, (size_t)(c.blocks / 3 + 1) * kScanBlock));
+  c.lists.block_count = r->scan_count;
+  c.lists.block_offset = r->scan_offset;
+  TRY(launch(r, kFlagCount, flag_count_kernel, dim3(c.blocks), dim3(kScanBlock), c.lists));
+  return launch(r, kBlockScan, flag_scan_kernel, dim3(c.count), dim3(1024), c.lists);
 }
 
 // Stable radix sort of the particle storage by cell index: the key pass,
@@ -1194,7 +1218,7 @@ aprl_status sort_particles(aprl_run* r) {
     TRY(launch(r, kChunkScan, chunk_scan_kernel, dim3(chunks), dim3(1024),
                (const unsigned*)r->radix_count, counts, r->radix_count, r->chunk_sum));
     TRY(launch(r, kBlockScan, block_offset_scan_kernel, dim3(1), dim3(1024),
-               (const unsigned*)r->chunk_sum, (int)chunks, r->chunk_offset, r->scan_total));
+               (const unsigned*)r->chunk_sum, (int)chunks, r->chunk_offset));
     TRY(launch(r, kChunkAdd, chunk_add_kernel, dim3(chunks), dim3(1024), r->radix_count,
                counts, (const unsigned*)r->chunk_offset));
     TRY(launch(r, kRadixScatter, radix_scatter_kernel, dim3(blocks), dim3(kRadixThreads),
@@ -1672,6 +1696,12 @@ aprl_status surface_current_add(aprl_run* r, const GridT<double>& g, double* jz)
                 dim3(blocks_for(r->surface_count * c.nz, 256)), dim3(256), a);
 }
 
+// The used and the re-gathered fields of the slots change places.
+void swap_slot_fields(aprl_run* r) {
+  std::swap(r->used_e, r->next_e);
+  std::swap(r->used_b, r->next_b);
+}
+
 // One coupling trial; W is the arithmetic of the gathers.
 template <class W>
 aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
@@ -1680,7 +1710,14 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     return fail(APRL_ERR_RUNTIME, "Coupling trial requires a previewed electric field");
   const aprl_run_config& c = r->cfg;
   GridT<F> g = make_grid<F>(r);
-  if (ahead) g.stop = r->d_stop;
+  // A step's first trial always runs (and clears the last step's verdict).
+  if (ahead && r->trials) g.stop = r->d_stop;
+  TrialResult* const result = &r->d_block->trial[slot];
+  const double next_origin =
+      std::fma(static_cast<double>(c.initial_offset - static_cast<int64_t>(r->step + 1)), c.dz,
+               c.reference_origin[2]);
+  const double crop_upper = r->crop_ahead ? std::fma(static_cast<double>(c.nz), c.dz, next_origin)
+                                          : static_cast<double>(INFINITY);
   // Frozen source support of the entries due within min(8, horizon) steps.
   size_t frozen_end = 0;
   if (r->queue.extracted) {
@@ -1701,8 +1738,8 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     // pairs instead when the conversion will write J).
     const int clear_current = convert ? 2 : (r->j_zero ? 0 : 1);
     const unsigned blocks = clear_current ? grid_blocks : 1u;
-    TRY(launch(r, kTrialClear, trial_clear_kernel, dim3(blocks), dim3(256), g, r->d_counters,
-               r->d_sums, clear_current));
+    TRY(launch(r, kTrialClear, trial_clear_kernel, dim3(blocks), dim3(256), g, result,
+               clear_current, ahead && r->trials == 0 ? r->d_stop : nullptr));
   }
   const bool surface = c.reference_surface_current != 0;
   r->j_zero = !deposits;
@@ -1750,10 +1787,11 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     ca.region = region;
     ca.shape = c.shape;
     ca.count = (long long)r->nc;
+    ca.crop_upper = crop_upper;
     ca.in = r->c;
     ca.out = r->c_out;
     ca.keep = r->c_keep;
-    ca.counters = r->d_counters;
+    ca.counters = &result->counters;
     ca.status = r->d_status;
     CUDA_TRY(cudaEventRecord(r->fork, r->stream));
     CUDA_TRY(cudaStreamWaitEvent(r->side, r->fork, 0));
@@ -1772,6 +1810,8 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     return APRL_OK;
   };
   if (r->np) {
+    // The last residual's fields are what this trial's push uses.
+    if (r->trials) swap_slot_fields(r);
     PushArgs<F> pa{};
     pa.g = g;
     pa.frame = make_frame(c);
@@ -1805,19 +1845,15 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     pa.slot = r->slots;
     pa.used_e = r->used_e;
     pa.used_b = r->used_b;
-    pa.next_e = r->next_e;
-    pa.next_b = r->next_b;
     pa.abs_grid_work = r->abs_work;
     pa.action = r->action;
     pa.born = r->born;
     pa.born_keep = r->born_keep;
-    for (int d = 0; d < 3; ++d) {
-      pa.dep_b[d] = r->dep_b[d];
-      pa.dep_e[d] = r->dep_e[d];
-    }
-    pa.dep_mode = r->dep_mode;
+    pa.plain = r->plain;
+    pa.events = r->events;
+    pa.crop_upper = crop_upper;
     pa.key_base = (unsigned long long)(r->step + 1) << 32;
-    pa.counters = r->d_counters;
+    pa.counters = &result->counters;
     pa.status = r->d_status;
     const bool direct = binomial && !r->dense;
     for (int a = 0; a < 3; ++a) {
@@ -1837,25 +1873,32 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
       // The step's surface current joins E* and S0 after the current-free gather.
       if (surface) TRY(surface_current_add(r, g, nullptr));
     }
-    TRY(launch(r, kPushDeposit,
-               r->deterministic
-                   ? (binomial ? push_deposit_kernel<F, 0, true> : push_deposit_kernel<F, 1, true>)
-                   : (binomial ? push_deposit_kernel<F, 0, false> : push_deposit_kernel<F, 1, false>),
-               dim3(blocks_for(r->np, 128)), dim3(128),
-               pa));
-    if (binomial) {
+    TRY(launch(r, kPushDeposit, push_kernel<F>, dim3(blocks_for(r->np, 128)), dim3(128), pa));
+    // The listed events share only J, the counters and the status word with
+    // the chord deposit, all through atomics, so they run beside it.
+    CUDA_TRY(cudaEventRecord(r->fork, r->stream));
+    CUDA_TRY(cudaStreamWaitEvent(r->side, r->fork, 0));
+    TRY(launch_on(r, r->side, kPushEvents,
+                  r->deterministic
+                      ? (binomial ? push_events_kernel<F, 0, true> : push_events_kernel<F, 1, true>)
+                      : (binomial ? push_events_kernel<F, 0, false> : push_events_kernel<F, 1, false>),
+                  dim3(std::min(blocks_for(r->np, 64), 148u * 4)), dim3(64), pa));
+    CUDA_TRY(cudaEventRecord(r->join, r->side));
+    joined = false;
+    {
       ChordArgs da{};
       da.g = g;
       da.count = (long long)r->np;
-      da.mode = r->dep_mode;
-      for (int d = 0; d < 3; ++d) {
-        da.b[d] = r->dep_b[d];
-        da.e[d] = r->dep_e[d];
-      }
-      da.q = r->p.q;
+      da.plain = r->plain;
+      da.p = r->p;
+      da.x1 = r->x1;
+      da.y1 = r->y1;
+      da.z1 = r->z1;
       da.status = r->d_status;
       TRY(launch(r, kChordDeposit,
-                 r->deterministic ? chord_deposit_kernel<true> : chord_deposit_kernel<false>,
+                 r->deterministic
+                     ? (binomial ? chord_deposit_kernel<0, true> : chord_deposit_kernel<1, true>)
+                     : (binomial ? chord_deposit_kernel<0, false> : chord_deposit_kernel<1, false>),
                  dim3(blocks_for(r->np, 128)), dim3(128), da));
     }
     TRY(join_carriers());
@@ -1886,7 +1929,11 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     ra.next_e = r->next_e;
     ra.next_b = r->next_b;
     ra.abs_grid_work = r->abs_work;
-    ra.sums = r->d_sums;
+    ra.sums = &result->sums;
+    ra.iterations = r->trials + 1;
+    ra.force_tolerance = c.force_tolerance;
+    ra.work_tolerance = c.work_tolerance;
+    ra.stop = ahead ? r->d_stop : nullptr;
     ra.partial = r->res_partial;
     ra.ticket = r->res_ticket;
     ra.status = r->d_status;
@@ -1899,31 +1946,27 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
   }
   TRY(join_carriers());
   TRY(convert_current());
-  if (ahead)
+  if (ahead && !r->np)
     TRY(launch(r, kTrialVerdict, trial_verdict_kernel, dim3(1), dim3(1),
-               (const ResidualSums*)r->d_sums, r->trials + 1, c.force_tolerance,
+               (const ResidualSums*)&result->sums, r->trials + 1, c.force_tolerance,
                c.work_tolerance, r->d_stop));
-  CUDA_TRY(cudaMemcpyAsync(&r->h_sums_slots[slot], r->d_sums, sizeof(ResidualSums),
-                           cudaMemcpyDeviceToHost, r->stream));
-  CUDA_TRY(cudaMemcpyAsync(&r->h_counters_slots[slot], r->d_counters, sizeof(TrialCounters),
-                           cudaMemcpyDeviceToHost, r->stream));
   ++r->trials;
   r->stage = 3;
   return APRL_OK;
 }
 
-// The residual of the trial copied to `slot` (after the stream has reached
-// it); the slot becomes the run's current trial counters.
+// The residual of the trial read back in `slot`, which becomes the run's
+// current trial counters.
 void trial_read(aprl_run* r, int slot, double residual[4]) {
-  r->h_sums = &r->h_sums_slots[slot];
-  r->h_counters = &r->h_counters_slots[slot];
+  const ResidualSums& sums = r->h_block->trial[slot].sums;
+  r->h_counters = &r->h_block->trial[slot].counters;
   double force;
-  const unsigned long long bits = r->h_sums->force_bits;
+  const unsigned long long bits = sums.force_bits;
   std::memcpy(&force, &bits, sizeof force);
   residual[0] = force;
-  residual[1] = r->h_sums->defect;
-  residual[2] = r->h_sums->scale;
-  residual[3] = static_cast<double>(r->h_sums->calls);
+  residual[1] = sums.defect;
+  residual[2] = sums.scale;
+  residual[3] = static_cast<double>(sums.calls);
 }
 
 aprl_status enqueue_trial(aprl_run* r, int slot, bool ahead) {
@@ -1941,7 +1984,8 @@ bool trial_converged(const aprl_run_config& c, unsigned iterations, const double
 
 aprl_status do_trial(aprl_run* r, double residual[4]) {
   TRY(enqueue_trial(r, 0, false));
-  TRY(check_device(r));
+  TRY(read_block(r));
+  TRY(wait_status(r));
   trial_read(r, 0, residual);
   return APRL_OK;
 }
@@ -1966,33 +2010,49 @@ aprl_status do_commit(aprl_run* r) {
   const unsigned long long kept_born = r->np ? tc.born_kept : 0;
   // Carriers: surviving old carriers, then carriers born this step, in
   // particle order (retainedCarriers, src/simulation.cpp:4401-4405).
-  TRY(reserve_carriers(r, kept_old + kept_born));
-  if (r->nc) {
-    TRY(compact_offsets(r, r->c_keep, 1, r->nc));
-    TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->nc, kScanBlock)),
-               dim3(kScanBlock), r->c_alt, r->c_out, (const unsigned char*)r->c_keep,
-               (unsigned char)1, (long long)r->nc, (const unsigned*)r->scan_offset, 0ull));
-  }
-  if (r->np && kept_born) {
-    TRY(compact_offsets(r, r->born_keep, 1, r->np));
-    TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->np, kScanBlock)),
-               dim3(kScanBlock), r->c_alt, r->born, (const unsigned char*)r->born_keep,
-               (unsigned char)1, (long long)r->np, (const unsigned*)r->scan_offset,
-               (unsigned long long)kept_old));
-  }
-  std::swap(r->c, r->c_alt);
-  r->nc = kept_old + kept_born;
   // Particles: the retained list in order (src/simulation.cpp:4916, 5581).
+  // A list that keeps every element takes its new state by exchanging arrays.
+  TRY(reserve_carriers(r, kept_old + kept_born));
+  const bool gather_old = r->nc && kept_old != r->nc;
+  const bool gather_born = r->np && kept_born;
+  const bool gather_p = r->np && tc.lost;
+  Compaction lists;
+  const int old_list = gather_old ? lists.add(r->c_keep, 1, r->nc) : 0;
+  const int born_list = gather_born ? lists.add(r->born_keep, 1, r->np) : 0;
+  const int p_list = gather_p ? lists.add(r->action, 0, r->np) : 0;
+  TRY(compact_offsets(r, lists));
+  if (gather_old) {
+    TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->nc, kScanBlock)),
+               dim3(kScanBlock), r->c, r->c_out, (const unsigned char*)r->c_keep,
+               (unsigned char)1, (long long)r->nc, lists.offsets(old_list), 0ull));
+  } else if (r->nc) {
+    std::swap(r->c, r->c_out);
+  }
+  if (gather_born)
+    TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->np, kScanBlock)),
+               dim3(kScanBlock), r->c, r->born, (const unsigned char*)r->born_keep,
+               (unsigned char)1, (long long)r->np, lists.offsets(born_list),
+               (unsigned long long)kept_old));
+  r->nc = kept_old + kept_born;
   if (r->np) {
-    const unsigned long long kept = tc.retained;
-    TRY(compact_offsets(r, r->action, 0, r->np));
-    TRY(launch(r, kGatherParticles, gather_particles_kernel, dim3(blocks_for(r->np, kScanBlock)),
-               dim3(kScanBlock), r->p_alt, r->p, (const double*)r->x1, (const double*)r->y1,
-               (const double*)r->z1, (const double*)r->ux1, (const double*)r->uy1,
-               (const double*)r->uz1, (const unsigned char*)r->frozen1,
-               (const unsigned char*)r->action, (unsigned char)0, (long long)r->np,
-               (const unsigned*)r->scan_offset));
-    std::swap(r->p, r->p_alt);
+    const unsigned long long kept = r->np - tc.lost;
+    if (gather_p) {
+      TRY(launch(r, kGatherParticles, gather_particles_kernel,
+                 dim3(blocks_for(r->np, kScanBlock)), dim3(kScanBlock), r->p_alt, r->p,
+                 (const double*)r->x1, (const double*)r->y1, (const double*)r->z1,
+                 (const double*)r->ux1, (const double*)r->uy1, (const double*)r->uz1,
+                 (const unsigned char*)r->frozen1, (const unsigned char*)r->action,
+                 (unsigned char)0, (long long)r->np, lists.offsets(p_list)));
+      std::swap(r->p, r->p_alt);
+    } else {
+      std::swap(r->p.x, r->x1);
+      std::swap(r->p.y, r->y1);
+      std::swap(r->p.z, r->z1);
+      std::swap(r->p.ux, r->ux1);
+      std::swap(r->p.uy, r->uy1);
+      std::swap(r->p.uz, r->uz1);
+      std::swap(r->p.frozen, r->frozen1);
+    }
     r->np = kept;
     // Particles move about one cell per step, so the cell order survives a
     // few steps: re-sorting every kSortInterval steps kept push_deposit and
@@ -2106,28 +2166,33 @@ aprl_status do_shift(aprl_run* r, bool defer_check = false) {
   if (c.inlet_charge_match) TRY(inlet_charge_match(r));
   if (r->ledger_on) TRY(ledger_shift(r));
   r->origin[2] = std::fma(static_cast<double>(r->offset), c.dz, c.reference_origin[2]);
-  if (r->np)
-    TRY(launch(r, kInletCheck, inlet_check_kernel, dim3(blocks_for(r->np, 256)), dim3(256),
-               (const double*)r->p.z, (const unsigned char*)r->p.frozen, (long long)r->np,
-               r->origin[2], r->d_status));
-  if (r->nc) {
+  if (r->np || r->nc)
+    TRY(launch(r, kInletCheck, inlet_check_kernel, dim3(blocks_for(r->np + r->nc, 256)),
+               dim3(256), (const double*)r->p.z, (const unsigned char*)r->p.frozen,
+               (long long)r->np, (const double*)r->c.pz, (long long)r->nc, r->origin[2],
+               r->d_status));
+  if (r->nc && !r->crop_ahead) {
     // Crop flags and counts in one round trip (with the device status).
     const double upper = std::fma(static_cast<double>(c.nz), c.dz, r->origin[2]);
-    CUDA_TRY(cudaMemsetAsync(r->d_counters, 0, sizeof(TrialCounters), r->stream));
+    TrialCounters* const counters = &r->d_block->trial[0].counters;
+    CUDA_TRY(cudaMemsetAsync(counters, 0, sizeof(TrialCounters), r->stream));
     TRY(launch(r, kCropFlags, crop_flags_kernel, dim3(blocks_for(r->nc, 256)), dim3(256), r->c,
-               (long long)r->nc, upper, r->origin[2], r->c_keep, r->d_counters, r->d_status));
-    CUDA_TRY(cudaMemcpyAsync(r->h_counters, r->d_counters, sizeof(TrialCounters),
-                             cudaMemcpyDeviceToHost, r->stream));
-    TRY(check_device(r));
-    const unsigned long long kept = r->nc - r->h_counters->cropped;
-    TRY(compact_offsets(r, r->c_keep, 1, r->nc));
-    TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->nc, kScanBlock)),
-               dim3(kScanBlock), r->c_alt, r->c, (const unsigned char*)r->c_keep,
-               (unsigned char)1, (long long)r->nc, (const unsigned*)r->scan_offset, 0ull));
-    std::swap(r->c, r->c_alt);
-    r->nc = kept;
-    r->cumulative.cropped += r->h_counters->cropped;
-    r->cumulative.cropped_charge += r->h_counters->cropped_charge;
+               (long long)r->nc, upper, r->origin[2], r->c_keep, counters, r->d_status));
+    TRY(read_block(r));
+    TRY(wait_status(r));
+    const TrialCounters& tc = r->h_block->trial[0].counters;
+    if (tc.cropped) {
+      Compaction lists;
+      lists.add(r->c_keep, 1, r->nc);
+      TRY(compact_offsets(r, lists));
+      TRY(launch(r, kGatherCarriers, gather_carriers_kernel, dim3(blocks_for(r->nc, kScanBlock)),
+                 dim3(kScanBlock), r->c_alt, r->c, (const unsigned char*)r->c_keep,
+                 (unsigned char)1, (long long)r->nc, lists.offsets(0), 0ull));
+      std::swap(r->c, r->c_alt);
+      r->nc -= tc.cropped;
+      r->cumulative.cropped += tc.cropped;
+      r->cumulative.cropped_charge += tc.cropped_charge;
+    }
   } else if (!defer_check) {
     TRY(check_device(r));
   }
@@ -2334,32 +2399,19 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
         (s = device_alloc(r, &r->inlet_rho_pairs, 2 * (size_t)(c.nx + 1) * (c.ny + 1))) != APRL_OK)
       return cleanup(s);
   }
-  if ((s = device_alloc(r, &r->d_counters, 1)) != APRL_OK) return cleanup(s);
-  if ((s = device_alloc(r, &r->d_sums, 1)) != APRL_OK) return cleanup(s);
-  if ((s = device_alloc(r, &r->d_status, 1)) != APRL_OK) return cleanup(s);
-  if ((s = device_alloc(r, &r->scan_total, 1)) != APRL_OK) return cleanup(s);
-  cudaMemsetAsync(r->d_status, 0, sizeof(DeviceStatus), r->stream);
-  if ((s = device_alloc(r, &r->d_stop, 1)) != APRL_OK) return cleanup(s);
+  if ((s = device_alloc(r, &r->d_block, 1)) != APRL_OK) return cleanup(s);
+  r->d_status = &r->d_block->status;
+  r->d_stop = &r->d_block->stop;
+  cudaMemsetAsync(r->d_block, 0, sizeof(TrialBlock), r->stream);
   if (c.inlet_charge_match &&
       (s = device_alloc(r, &r->inlet_rho, (size_t)(c.nx + 1) * (c.ny + 1))) != APRL_OK)
     return cleanup(s);
-  // The read-back areas, 64-byte aligned inside one reused page-locked block.
+  // The read-back block, in a reused page-locked block.
   if (!(r->pinned = pinned_take()))
     return cleanup(fail(APRL_ERR_CUDA, "cudaMallocHost failed"));
-  {
-    char* at = static_cast<char*>(r->pinned);
-    auto carve = [&](size_t bytes) {
-      char* p = at;
-      at += (bytes + 63) / 64 * 64;
-      return static_cast<void*>(p);
-    };
-    r->h_sums_slots = static_cast<ResidualSums*>(carve(kTrialSlots * sizeof(ResidualSums)));
-    r->h_status = static_cast<DeviceStatus*>(carve(sizeof(DeviceStatus)));
-    r->h_counters_slots = static_cast<TrialCounters*>(carve(kTrialSlots * sizeof(TrialCounters)));
-    r->h_stop = static_cast<int*>(carve(sizeof(int)));
-    r->h_total = static_cast<unsigned long long*>(carve(sizeof(unsigned long long)));
-    std::memset(r->pinned, 0, kPinnedBlock);
-  }
+  std::memset(r->pinned, 0, kPinnedBlock);
+  r->h_block = static_cast<TrialBlock*>(r->pinned);
+  r->h_status = &r->h_block->status;
   if (cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming) != cudaSuccess)
@@ -2371,8 +2423,7 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
       if (cudaEventCreateWithFlags(&st.staged, cudaEventDisableTiming) != cudaSuccess ||
           cudaEventCreateWithFlags(&st.drained, cudaEventDisableTiming) != cudaSuccess)
         return cleanup(fail(APRL_ERR_CUDA, "upload event creation failed"));
-  r->h_sums = r->h_sums_slots;
-  r->h_counters = r->h_counters_slots;
+  r->h_counters = &r->h_block->trial[0].counters;
   r->offset = c.initial_offset;
   r->origin[0] = c.reference_origin[0];
   r->origin[1] = c.reference_origin[1];
@@ -2431,14 +2482,14 @@ aprl_status aprl_run_destroy(aprl_run* r) {
   double* singles[] = {r->x1,       r->y1,       r->z1,       r->ux1,        r->uy1,
                        r->uz1,      r->used_e,   r->used_b,   r->next_e,     r->next_b,
                        r->abs_work, r->slots.x0, r->slots.y0, r->slots.z0,   r->slots.dt,
-                       r->d_detector, r->dep_b[0], r->dep_b[1], r->dep_b[2], r->dep_e[0],
-                       r->dep_e[1], r->dep_e[2]};
+                       r->d_detector};
   for (double* d : singles) device_free(r, d);
   device_free(r, r->slots.seen);
   device_free(r, r->frozen1);
   free_pending(r, r->queue.d);
   device_free(r, r->action);
-  device_free(r, r->dep_mode);
+  device_free(r, r->plain);
+  device_free(r, r->events);
   device_free(r, r->born_keep);
   device_free(r, r->slot_order);
   for (int k = 0; k < 2; ++k) {
@@ -2465,19 +2516,11 @@ aprl_status aprl_run_destroy(aprl_run* r) {
   device_free(r, r->d_ledger_partial);
   device_free(r, r->ledger_pre[0]);
   device_free(r, r->ledger_pre[1]);
-  device_free(r, r->d_counters);
-  device_free(r, r->d_sums);
-  device_free(r, r->d_status);
+  device_free(r, r->d_block);
   device_free(r, r->scan_count);
   device_free(r, r->scan_offset);
-  device_free(r, r->scan_total);
-  r->h_sums_slots = nullptr;
-  r->h_stop = nullptr;
-  device_free(r, r->d_stop);
   device_free(r, r->inlet_rho);
   r->h_status = nullptr;
-  r->h_counters_slots = nullptr;
-  r->h_total = nullptr;
   pinned_give(r->pinned);
   delete r;
   return APRL_OK;
@@ -2923,6 +2966,7 @@ aprl_status aprl_run_preview_electric(aprl_run* r) {
 aprl_status aprl_run_coupling_trial(aprl_run* r, double residual[4]) {
   if (!r || !residual) return fail(APRL_ERR_INVALID_ARGUMENT, "null argument");
   TRY(no_open_step(r));
+  r->crop_ahead = false;
   return do_trial(r, residual);
 }
 
@@ -2963,11 +3007,9 @@ aprl_status step_enqueue(aprl_run* r) {
   // verdict applies the stopping rule, and the kernels of the trials after
   // a converged one return at once.  One round trip then reads them all.
   const unsigned ahead = trials_ahead(r);
-  CUDA_TRY(cudaMemsetAsync(r->d_stop, 0, sizeof(int), r->stream));
+  r->crop_ahead = true;
   for (unsigned t = 0; t < ahead; ++t) TRY(enqueue_trial(r, (int)t, true));
-  CUDA_TRY(cudaMemcpyAsync(r->h_stop, r->d_stop, sizeof(int), cudaMemcpyDeviceToHost,
-                           r->stream));
-  return APRL_OK;
+  return read_block(r);
 }
 
 aprl_status step_finish(aprl_run* r) {
@@ -2975,7 +3017,7 @@ aprl_status step_finish(aprl_run* r) {
   unsigned iterations = 0;
   double force = 0.0, work = 0.0;
   const unsigned ahead = trials_ahead(r);
-  TRY(check_device(r));
+  TRY(wait_status(r));
   tune_harvest(r);
   unsigned t = 0;
   // forceHistory / workHistory of the reference's failure message.
@@ -2988,8 +3030,11 @@ aprl_status step_finish(aprl_run* r) {
     history.push_back(force);
     history.push_back(work);
   }
-  if ((converged ? (int)iterations : 0) != *r->h_stop)
+  if ((converged ? (int)iterations : 0) != r->h_block->stop)
     return fail(APRL_ERR_RUNTIME, "Device and host verdicts on the coupling trials differ");
+  // Trials issued beyond the converged one did nothing: the slot fields are
+  // where that one left them.
+  if (r->np && (ahead - t) % 2) swap_slot_fields(r);
   for (; !converged && t < r->cfg.max_trials; ++t) {
     double res[4];
     TRY(do_trial(r, res));
