@@ -2166,6 +2166,20 @@ __global__ void sort_key_kernel(DParticles p, long long n, DGrid g, int tiles_x,
   index[i] = (unsigned)i;
 }
 
+__global__ void order_key_kernel(const unsigned long long* order, const unsigned* index_in,
+                                 long long n, int shift, unsigned* key, unsigned* index) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned at = index_in ? index_in[i] : (unsigned)i;
+  key[i] = (unsigned)(order[at] >> shift);
+  index[i] = at;
+}
+
+__global__ void iota_kernel(unsigned long long* out, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (unsigned long long)i;
+}
+
 // Digit counts of each block's kRadixTile keys: count[digit * blocks + block].
 __global__ void __launch_bounds__(kRadixThreads) radix_count_kernel(const unsigned* key,
                                                                     long long n, int shift,

@@ -295,6 +295,11 @@ constexpr int kRadixTile = kRadixThreads * kRadixItems;
 static_assert(kRadixThreads == kRadixBins, "radix_scatter_kernel: one thread per digit");
 __global__ void sort_key_kernel(DParticles p, long long n, DGrid g, int tiles_x, int tiles_y,
                                 unsigned* key, unsigned* index);
+// Keys of a sort by list order: bits [shift, shift + 32) of order[index[i]]
+// (of order[i], with index filled by i, when index_in is null).
+__global__ void order_key_kernel(const unsigned long long* order, const unsigned* index_in,
+                                 long long n, int shift, unsigned* key, unsigned* index);
+__global__ void iota_kernel(unsigned long long* out, long long n);
 __global__ void radix_count_kernel(const unsigned* key, long long n, int shift, unsigned* count);
 __global__ void radix_scatter_kernel(const unsigned* key_in, const unsigned* index_in,
                                      unsigned* key_out, unsigned* index_out, long long n,

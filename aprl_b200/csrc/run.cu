@@ -21,6 +21,8 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/aprl_gpu.h"
@@ -459,14 +461,12 @@ cudaMemPool_t device_pool(int device) {
   return pools[device];
 }
 
-// The allocation is waited for on the run's stream, so the block is valid for
-// every stream and for the synchronous copies that fill it (allocations are
-// made outside the step loop, or on a stream that is idle anyway).
+// Ordered on the run's stream, like every use of the block: kernels, copies
+// and fills go through that stream, and the side stream follows it by event.
 aprl_status device_alloc_bytes(aprl_run* r, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) bytes = 8;
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, r->pool, r->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
+  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, r->pool, r->stream);
   if (e != cudaSuccess) {
     *p = nullptr;
     return fail(APRL_ERR_CUDA, "device allocation of %zu bytes failed: %s", bytes,
@@ -502,6 +502,192 @@ cudaError_t run_copy(aprl_run* r, void* dst, const void* src, size_t bytes, cuda
 }
 cudaError_t run_fill(aprl_run* r, void* dst, int value, size_t bytes) {
   return cudaMemsetAsync(dst, value, bytes, r->stream);
+}
+
+// fn(item) for every item < items, on up to kHostThreads threads (the caller's
+// among them).  A thread that cannot be started is done without.
+constexpr int kHostThreads = 6;
+
+template <class Fn>
+void host_parallel(size_t items, Fn fn) {
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t i; (i = next.fetch_add(1)) < items;) fn(i);
+  };
+  std::vector<std::thread> threads;
+  try {
+    threads.reserve(kHostThreads);
+    while (threads.size() + 1 < std::min<size_t>(kHostThreads, items)) threads.emplace_back(work);
+  } catch (const std::exception&) {
+  }
+  work();
+  for (auto& t : threads) t.join();
+}
+
+// Large copies between pageable host memory and the device.  The driver
+// stages such a copy through page-locked memory on one thread, about 4 GB/s
+// here once the host pages are touched for the first time; several threads,
+// each with a page-locked lane and a stream of its own, keep the link busy
+// instead.  Lanes are made on demand, at most kHostThreads for all callers,
+// and kept for reuse; a caller that finds none copies plainly.
+constexpr size_t kLaneBytes = 2u << 20;
+constexpr size_t kStagedFrom = 4u << 20;  // smaller copies go plainly
+
+struct CopyLane {
+  int device = -1;
+  void* buffer[2] = {nullptr, nullptr};
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+};
+
+struct CopyLanes {
+  std::mutex lock;
+  std::vector<CopyLane*> free;
+  int made = 0;
+};
+CopyLanes& copy_lanes() {
+  static CopyLanes* lanes = new CopyLanes;  // outlives every thread's use
+  return *lanes;
+}
+
+void lane_destroy(CopyLane* l) {
+  for (int b = 0; b < 2; ++b) {
+    if (l->buffer[b]) cudaFreeHost(l->buffer[b]);
+    if (l->done[b]) cudaEventDestroy(l->done[b]);
+  }
+  if (l->stream) cudaStreamDestroy(l->stream);
+  delete l;
+}
+
+// A lane of the current device, or null.
+CopyLane* lane_take(int device) {
+  CopyLanes& pool = copy_lanes();
+  CopyLane* other = nullptr;
+  {
+    std::lock_guard<std::mutex> hold(pool.lock);
+    for (size_t i = 0; i < pool.free.size(); ++i)
+      if (pool.free[i]->device == device) {
+        CopyLane* l = pool.free[i];
+        pool.free.erase(pool.free.begin() + (long)i);
+        return l;
+      }
+    if (pool.made >= kHostThreads) {  // make room from another device's lane
+      if (pool.free.empty()) return nullptr;
+      other = pool.free.back();
+      pool.free.pop_back();
+    } else {
+      ++pool.made;
+    }
+  }
+  if (other) lane_destroy(other);
+  CopyLane* l = new (std::nothrow) CopyLane;
+  bool ok = l != nullptr;
+  if (ok) {
+    l->device = device;
+    ok = cudaStreamCreateWithFlags(&l->stream, cudaStreamNonBlocking) == cudaSuccess;
+    for (int b = 0; b < 2 && ok; ++b)
+      ok = cudaMallocHost(&l->buffer[b], kLaneBytes) == cudaSuccess &&
+           cudaEventCreateWithFlags(&l->done[b], cudaEventDisableTiming) == cudaSuccess;
+  }
+  if (ok) return l;
+  if (l) lane_destroy(l);
+  (void)cudaGetLastError();
+  std::lock_guard<std::mutex> hold(pool.lock);
+  --pool.made;
+  return nullptr;
+}
+
+void lane_give(CopyLane* l) {
+  CopyLanes& pool = copy_lanes();
+  std::lock_guard<std::mutex> hold(pool.lock);
+  pool.free.push_back(l);
+}
+
+struct HostCopy {
+  char* device;
+  char* host;
+  size_t bytes;
+};
+
+// Copies `list` after the work queued on the run's stream, and returns once
+// everything has landed.
+cudaError_t run_copies(aprl_run* r, const HostCopy* list, size_t count, bool to_host) {
+  std::vector<HostCopy> items;
+  size_t total = 0;
+  for (size_t i = 0; i < count; ++i) total += list[i].bytes;
+  std::vector<CopyLane*> lanes;
+  cudaEvent_t ready = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (total >= kStagedFrom) {
+    const size_t want = std::min<size_t>(kHostThreads, total / kLaneBytes);
+    while (lanes.size() < want) {
+      CopyLane* l = lane_take(r->device);
+      if (!l) break;
+      lanes.push_back(l);
+    }
+  }
+  if (lanes.size() >= 2) {
+    for (size_t i = 0; i < count; ++i)
+      for (size_t at = 0; at < list[i].bytes; at += kLaneBytes)
+        items.push_back(HostCopy{list[i].device + at, list[i].host + at,
+                                 std::min(kLaneBytes, list[i].bytes - at)});
+    e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ready, r->stream);
+    std::atomic<size_t> next{0};
+    std::vector<cudaError_t> status(lanes.size(), cudaSuccess);
+    auto drive = [&](size_t n) {
+      CopyLane& l = *lanes[n];
+      int previous = r->device;  // the caller's own thread drives a lane too
+      (void)cudaGetDevice(&previous);
+      cudaError_t x = cudaSetDevice(r->device);
+      if (x == cudaSuccess) x = cudaStreamWaitEvent(l.stream, ready, 0);
+      const HostCopy* in_flight[2] = {nullptr, nullptr};
+      auto land = [&](int b) {  // the copy out of (or the use of) buffer b is over
+        if (!in_flight[b]) return;
+        const cudaError_t w = cudaEventSynchronize(l.done[b]);
+        if (x == cudaSuccess) x = w;
+        if (to_host && x == cudaSuccess)
+          std::memcpy(in_flight[b]->host, l.buffer[b], in_flight[b]->bytes);
+        in_flight[b] = nullptr;
+      };
+      int b = 0;
+      for (size_t i; x == cudaSuccess && (i = next.fetch_add(1)) < items.size(); b ^= 1) {
+        const HostCopy& c = items[i];
+        land(b);
+        if (x != cudaSuccess) break;
+        if (!to_host) std::memcpy(l.buffer[b], c.host, c.bytes);
+        x = to_host ? cudaMemcpyAsync(l.buffer[b], c.device, c.bytes, cudaMemcpyDeviceToHost,
+                                      l.stream)
+                    : cudaMemcpyAsync(c.device, l.buffer[b], c.bytes, cudaMemcpyHostToDevice,
+                                      l.stream);
+        if (x == cudaSuccess) x = cudaEventRecord(l.done[b], l.stream);
+        if (x == cudaSuccess) in_flight[b] = &c;
+      }
+      land(b);
+      land(b ^ 1);
+      const cudaError_t w = cudaStreamSynchronize(l.stream);
+      status[n] = x == cudaSuccess ? w : x;
+      if (previous != r->device) (void)cudaSetDevice(previous);
+    };
+    if (e == cudaSuccess) {
+      // one driver per lane; drivers that got no thread of their own find the
+      // items already taken
+      host_parallel(lanes.size(), drive);
+      for (const cudaError_t x : status)
+        if (e == cudaSuccess) e = x;
+    }
+    if (ready) cudaEventDestroy(ready);
+  } else {
+    for (size_t i = 0; i < count && e == cudaSuccess; ++i)
+      if (list[i].bytes)
+        e = to_host ? cudaMemcpyAsync(list[i].host, list[i].device, list[i].bytes,
+                                      cudaMemcpyDeviceToHost, r->stream)
+                    : cudaMemcpyAsync(list[i].device, list[i].host, list[i].bytes,
+                                      cudaMemcpyHostToDevice, r->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(r->stream);
+  }
+  for (CopyLane* l : lanes) lane_give(l);
+  return e;
 }
 
 // Page-locked 4 KiB blocks for the runs' small read-back areas, kept for
@@ -579,6 +765,19 @@ bool all_finite(const double* v, size_t n) {
     if (bad) return false;
   }
   return true;
+}
+
+// all_finite over large host arrays, a share per thread.
+bool all_finite_parallel(const double* v, size_t n) {
+  constexpr size_t kShare = 1u << 18;
+  if (n < 4 * kShare) return all_finite(v, n);
+  std::atomic<bool> ok{true};
+  host_parallel((n + kShare - 1) / kShare, [&](size_t i) {
+    if (ok.load(std::memory_order_relaxed) &&
+        !all_finite(v + i * kShare, std::min(kShare, n - i * kShare)))
+      ok.store(false, std::memory_order_relaxed);
+  });
+  return ok.load();
 }
 
 cudaEvent_t take_event(aprl_run* r) {
@@ -1101,23 +1300,21 @@ aprl_status reserve_carriers(aprl_run* r, size_t n) {
   return ensure_scan(r, n);
 }
 
-// Rotate between logical (window) and physical (ring) plane order.
+// Between logical (window) and physical (ring) plane order: the ring is two
+// contiguous runs of planes, the same two in every slot.
 aprl_status copy_ring(aprl_run* r, double* device, const double* host_in, double* host_out,
                       size_t plane, size_t layers, int base, size_t slots = 1) {
-  for (size_t s = 0; s < slots; ++s) {
-    const size_t slot_offset = s * layers * plane;
-    for (size_t k = 0; k < layers; ++k) {
-      const size_t pk = (k + base) % layers;
-      double* d = device + slot_offset + pk * plane;
-      if (host_in)
-        CUDA_TRY(cudaMemcpyAsync(d, host_in + slot_offset + k * plane, plane * 8,
-                                 cudaMemcpyHostToDevice, r->stream));
-      else
-        CUDA_TRY(cudaMemcpyAsync(host_out + slot_offset + k * plane, d, plane * 8,
-                                 cudaMemcpyDeviceToHost, r->stream));
-    }
-  }
-  CUDA_TRY(cudaStreamSynchronize(r->stream));
+  const size_t pitch = layers * plane * 8;
+  char* const host = reinterpret_cast<char*>(host_in ? const_cast<double*>(host_in) : host_out);
+  const size_t cut = layers - (size_t)base;  // logical planes before the wrap
+  const size_t at[2][3] = {{0, (size_t)base, cut}, {cut, 0, (size_t)base}};
+  std::vector<HostCopy> list;
+  for (size_t slot = 0; slot < slots; ++slot)
+    for (const auto& run : at)  // logical first, physical first, planes
+      if (run[2])
+        list.push_back(HostCopy{reinterpret_cast<char*>(device) + slot * pitch + run[1] * plane * 8,
+                                host + slot * pitch + run[0] * plane * 8, run[2] * plane * 8});
+  CUDA_TRY(run_copies(r, list.data(), list.size(), !host_in));
   return APRL_OK;
 }
 
@@ -1196,23 +1393,14 @@ aprl_status compact_offsets(aprl_run* r, Compaction& c) {
   return launch(r, kBlockScan, flag_scan_kernel, dim3(c.count), dim3(1024), c.lists);
 }
 
-// Stable radix sort of the particle storage by cell index: the key pass,
-// then per 8-bit digit the block digit counts, their exclusive scan in
-// digit-major order (chunk scan, chunk-sum scan, chunk add) and the stable
-// scatter of keys and storage indices; finally the particle arrays are
-// permuted.  No atomic ticket decides an order, so the storage order after
-// a sort is a function of the storage order before it.
-aprl_status sort_particles(aprl_run* r) {
-  if (r->np < 2 || r->sort_bits == 0) return APRL_OK;
-  const long long n = (long long)r->np;
-  const DGrid g = make_geometry(r);
-  TRY(launch(r, kSortKey, sort_key_kernel, dim3(blocks_for(r->np, 256)), dim3(256), r->p, n, g,
-             r->tiles[0], r->tiles[1], r->sort_key[0], r->sort_index[0]));
-  const unsigned blocks = blocks_for(r->np, kRadixTile);
+// The digit passes of a stable radix sort of n (key, index) pairs in
+// sort_key/sort_index[from], which is where they end.
+aprl_status radix_passes(aprl_run* r, size_t count, int bits, int& from) {
+  const long long n = (long long)count;
+  const unsigned blocks = blocks_for(count, kRadixTile);
   const long long counts = (long long)kRadixBins * blocks;
   const unsigned chunks = blocks_for((size_t)counts, 1024);
-  int from = 0;
-  for (int shift = 0; shift < r->sort_bits; shift += 8) {
+  for (int shift = 0; shift < bits; shift += 8) {
     TRY(launch(r, kRadixCount, radix_count_kernel, dim3(blocks), dim3(kRadixThreads),
                (const unsigned*)r->sort_key[from], n, shift, r->radix_count));
     TRY(launch(r, kChunkScan, chunk_scan_kernel, dim3(chunks), dim3(1024),
@@ -1227,10 +1415,51 @@ aprl_status sort_particles(aprl_run* r) {
                (const unsigned*)r->radix_count));
     from = 1 - from;
   }
+  return APRL_OK;
+}
+
+// Stable radix sort of the particle storage by cell index: the key pass,
+// then per 8-bit digit the block digit counts, their exclusive scan in
+// digit-major order (chunk scan, chunk-sum scan, chunk add) and the stable
+// scatter of keys and storage indices; finally the particle arrays are
+// permuted.  No atomic ticket decides an order, so the storage order after
+// a sort is a function of the storage order before it.
+aprl_status sort_particles(aprl_run* r) {
+  if (r->np < 2 || r->sort_bits == 0) return APRL_OK;
+  const long long n = (long long)r->np;
+  const DGrid g = make_geometry(r);
+  TRY(launch(r, kSortKey, sort_key_kernel, dim3(blocks_for(r->np, 256)), dim3(256), r->p, n, g,
+             r->tiles[0], r->tiles[1], r->sort_key[0], r->sort_index[0]));
+  int from = 0;
+  TRY(radix_passes(r, r->np, r->sort_bits, from));
   TRY(launch(r, kPermuteParticles, permute_particles_kernel, dim3(blocks_for(r->np, 256)),
              dim3(256), r->p_alt, r->p, n, (const unsigned*)r->sort_index[from]));
   std::swap(r->p, r->p_alt);
   return APRL_OK;
+}
+
+// The particle list in reference order, in p_alt (which the next sort or
+// commit overwrites): sorted on the device by each particle's rank, so a
+// read-out copies contiguous arrays instead of permuting them on the host.
+aprl_status ordered_particles(aprl_run* r) {
+  if (!r->np) return APRL_OK;
+  const long long n = (long long)r->np;
+  const dim3 grid(blocks_for(r->np, 256)), block(256);
+  int from = 0;
+  TRY(launch(r, kSortKey, order_key_kernel, grid, block, (const unsigned long long*)r->p.order,
+             (const unsigned*)nullptr, n, 0, r->sort_key[0], r->sort_index[0]));
+  int bits = 0;
+  while (bits < 64 && (r->next_order >> bits)) ++bits;
+  TRY(radix_passes(r, r->np, std::min(bits, 32), from));
+  if (bits > 32) {
+    TRY(launch(r, kSortKey, order_key_kernel, grid, block, (const unsigned long long*)r->p.order,
+               (const unsigned*)r->sort_index[from], n, 32, r->sort_key[1 - from],
+               r->sort_index[1 - from]));
+    from = 1 - from;
+    TRY(radix_passes(r, r->np, bits - 32, from));
+  }
+  return launch(r, kPermuteParticles, permute_particles_kernel, grid, block, r->p_alt, r->p, n,
+                (const unsigned*)r->sort_index[from]);
 }
 
 // ---- held lab-plane injection: PendingParticleQueue at one rank
@@ -2532,13 +2761,16 @@ aprl_status aprl_run_set_reference(aprl_run* r, unsigned a, const double* host, 
   comp_shape(r->cfg, a, s);
   const size_t n = s[0] * s[1] * (r->cfg.reference_nz + ((a == 0 || a == 1 || a == 5) ? 1 : 0));
   if (count != n) return fail(APRL_ERR_INVALID_ARGUMENT, "Reference component size mismatch");
-  if (host && !all_finite(host, n)) return fail(APRL_ERR_RUNTIME, "Non-finite moving-window inlet");
+  if (host && !all_finite_parallel(host, n))
+    return fail(APRL_ERR_RUNTIME, "Non-finite moving-window inlet");
   CUDA_TRY(cudaStreamSynchronize(r->stream));
   device_free(r, r->ref[a]);
   r->ref[a] = nullptr;
   TRY(device_alloc(r, &r->ref[a], n));
+  const HostCopy table{reinterpret_cast<char*>(r->ref[a]),
+                       reinterpret_cast<char*>(const_cast<double*>(host)), n * 8};
   if (host)
-    CUDA_TRY(run_copy(r, r->ref[a], host, n * 8, cudaMemcpyHostToDevice));
+    CUDA_TRY(run_copies(r, &table, 1, false));
   else
     CUDA_TRY(run_fill(r, r->ref[a], 0, n * 8));
   r->ref_set[a] = true;
@@ -2681,7 +2913,12 @@ aprl_status aprl_run_set_particles(aprl_run* r, size_t n, const double* x, const
   if (r->stage != 0) return fail(APRL_ERR_RUNTIME, "Particles can only be replaced between steps");
   if (n && (!x || !y || !z || !ux || !uy || !uz || !q || !m || !id))
     return fail(APRL_ERR_INVALID_ARGUMENT, "null particle array");
-  for (size_t i = 0; i < n; ++i)
+  bool valid = true;
+  for (const double* v : {x, y, z, ux, uy, uz, q}) valid = valid && all_finite_parallel(v, n);
+  size_t positive = 0;
+  for (size_t i = 0; i < n; ++i) positive += m[i] > 0.0;
+  valid = valid && positive == n;
+  for (size_t i = 0; !valid && i < n; ++i)
     if (!std::isfinite(x[i]) || !std::isfinite(y[i]) || !std::isfinite(z[i]) ||
         !std::isfinite(ux[i]) || !std::isfinite(uy[i]) || !std::isfinite(uz[i]) ||
         !std::isfinite(q[i]) || !(m[i] > 0.0))
@@ -2692,13 +2929,16 @@ aprl_status aprl_run_set_particles(aprl_run* r, size_t n, const double* x, const
   r->np = 0;
   const double* src[] = {x, y, z, ux, uy, uz, q, m};
   double* dst[] = {r->p.x, r->p.y, r->p.z, r->p.ux, r->p.uy, r->p.uz, r->p.q, r->p.m};
-  for (int k = 0; k < 8; ++k)
-    CUDA_TRY(run_copy(r, dst[k], src[k], n * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(run_copy(r, r->p.id, id, n * 8, cudaMemcpyHostToDevice));
-  std::vector<unsigned long long> order(n);
-  for (size_t i = 0; i < n; ++i) order[i] = i;
-  if (n) CUDA_TRY(run_copy(r, r->p.order, order.data(), n * 8, cudaMemcpyHostToDevice));
   if (n) {
+    HostCopy list[9];
+    for (int k = 0; k < 8; ++k)
+      list[k] = HostCopy{reinterpret_cast<char*>(dst[k]),
+                         reinterpret_cast<char*>(const_cast<double*>(src[k])), n * 8};
+    list[8] = HostCopy{reinterpret_cast<char*>(r->p.id),
+                       reinterpret_cast<char*>(const_cast<uint64_t*>(id)), n * 8};
+    CUDA_TRY(run_copies(r, list, 9, false));
+    TRY(launch(r, kSortKey, iota_kernel, dim3(blocks_for(n, 256)), dim3(256), r->p.order,
+               (long long)n));
     CUDA_TRY(run_fill(r, r->p.frozen, 0, n));
     CUDA_TRY(run_fill(r, r->p.beta, 0, n * 8));
   }
@@ -2733,23 +2973,19 @@ aprl_status aprl_run_get_particles(aprl_run* r, size_t capacity, double* x, doub
                                    uint64_t* id, size_t* count) {
   if (!r || !count) return fail(APRL_ERR_INVALID_ARGUMENT, "null argument");
   if (capacity < r->np) return fail(APRL_ERR_INVALID_ARGUMENT, "Particle buffer too small");
-  CUDA_TRY(cudaStreamSynchronize(r->stream));
   const size_t n = r->np;
-  std::vector<size_t> perm;
-  TRY(storage_permutation(r, r->p.order, n, perm));
-  std::vector<double> t(n);
+  TRY(ordered_particles(r));
+  const DParticles& o = r->p_alt;
   double* dst[] = {x, y, z, ux, uy, uz, q, m};
-  const double* src[] = {r->p.x, r->p.y, r->p.z, r->p.ux, r->p.uy, r->p.uz, r->p.q, r->p.m};
-  for (int k = 0; k < 8; ++k) {
-    if (!dst[k] || !n) continue;
-    CUDA_TRY(run_copy(r, t.data(), src[k], n * 8, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) dst[k][i] = t[perm[i]];
-  }
-  if (id && n) {
-    std::vector<uint64_t> ids(n);
-    CUDA_TRY(run_copy(r, ids.data(), r->p.id, n * 8, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) id[i] = ids[perm[i]];
-  }
+  double* const src[] = {o.x, o.y, o.z, o.ux, o.uy, o.uz, o.q, o.m};
+  std::vector<HostCopy> list;
+  for (int k = 0; k < 8; ++k)
+    if (dst[k] && n)
+      list.push_back(HostCopy{reinterpret_cast<char*>(src[k]), reinterpret_cast<char*>(dst[k]),
+                              n * 8});
+  if (id && n)
+    list.push_back(HostCopy{reinterpret_cast<char*>(o.id), reinterpret_cast<char*>(id), n * 8});
+  CUDA_TRY(run_copies(r, list.data(), list.size(), true));
   *count = n;
   return APRL_OK;
 }
@@ -2769,20 +3005,16 @@ aprl_status aprl_run_set_held(aprl_run* r, size_t n, const uint8_t* frozen, cons
   if (!(c.dz > 0.) || q.initial_step > q.maximum_step)
     return fail(APRL_ERR_INVALID_ARGUMENT, "Invalid pending-window geometry/horizon");
   // The list in reference order.
-  CUDA_TRY(cudaStreamSynchronize(r->stream));
-  std::vector<size_t> perm;
-  TRY(storage_permutation(r, r->p.order, n, perm));
+  TRY(ordered_particles(r));
+  const DParticles& o = r->p_alt;
   std::vector<double> v[8];
-  const double* dsrc[] = {r->p.x, r->p.y, r->p.z, r->p.ux, r->p.uy, r->p.uz, r->p.q, r->p.m};
+  const double* dsrc[] = {o.x, o.y, o.z, o.ux, o.uy, o.uz, o.q, o.m};
   for (int k = 0; k < 8; ++k) {
-    std::vector<double> t(n);
-    if (n) CUDA_TRY(run_copy(r, t.data(), dsrc[k], n * 8, cudaMemcpyDeviceToHost));
     v[k].resize(n);
-    for (size_t i = 0; i < n; ++i) v[k][i] = t[perm[i]];
+    if (n) CUDA_TRY(run_copy(r, v[k].data(), dsrc[k], n * 8, cudaMemcpyDeviceToHost));
   }
-  std::vector<unsigned long long> ids(n), id(n);
-  if (n) CUDA_TRY(run_copy(r, ids.data(), r->p.id, n * 8, cudaMemcpyDeviceToHost));
-  for (size_t i = 0; i < n; ++i) id[i] = ids[perm[i]];
+  std::vector<unsigned long long> id(n);
+  if (n) CUDA_TRY(run_copy(r, id.data(), o.id, n * 8, cudaMemcpyDeviceToHost));
   // PendingParticleQueue::extract (src/pending_particle_queue.cpp:128-154).
   const size_t buckets = static_cast<size_t>(q.maximum_step - q.initial_step + 2);
   q.offsets.assign(buckets + 1, 0);
@@ -2866,20 +3098,10 @@ aprl_status aprl_run_get_held(aprl_run* r, size_t capacity, uint8_t* frozen, dou
                               size_t* count) {
   if (!r || !count) return fail(APRL_ERR_INVALID_ARGUMENT, "null argument");
   if (capacity < r->np) return fail(APRL_ERR_INVALID_ARGUMENT, "Particle buffer too small");
-  CUDA_TRY(cudaStreamSynchronize(r->stream));
   const size_t n = r->np;
-  std::vector<size_t> perm;
-  TRY(storage_permutation(r, r->p.order, n, perm));
-  if (frozen && n) {
-    std::vector<unsigned char> f(n);
-    CUDA_TRY(run_copy(r, f.data(), r->p.frozen, n, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) frozen[i] = f[perm[i]];
-  }
-  if (beta && n) {
-    std::vector<double> b(n);
-    CUDA_TRY(run_copy(r, b.data(), r->p.beta, n * 8, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) beta[i] = b[perm[i]];
-  }
+  TRY(ordered_particles(r));
+  if (frozen && n) CUDA_TRY(run_copy(r, frozen, r->p_alt.frozen, n, cudaMemcpyDeviceToHost));
+  if (beta && n) CUDA_TRY(run_copy(r, beta, r->p_alt.beta, n * 8, cudaMemcpyDeviceToHost));
   *count = n;
   return APRL_OK;
 }
