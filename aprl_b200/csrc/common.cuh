@@ -131,6 +131,12 @@ struct GridT {
   double* b[3];          // B    (ring)
   F* j[3];               // raw current (plain, padded)
   int jpad;              // its z padding: 1 (linear-binomial3) or 3 (quintic)
+  // Columns of the raw current that hold deposits of this step: one byte per
+  // row j and eight x nodes (mark_column).  Unmarked columns are zero, so the
+  // clears and the filter passes skip them: a bunch reaches about half of a
+  // window's columns (and all of their z), and the marks fit in one SM's L1.
+  unsigned char* mark;
+  int mark_pitch;
   double inv_h[3];       // 1/dx, 1/dy, 1/dz, each rounded once
   int zb_e[3];           // ring bases of Ex Ey Ez
   int zb_b[3];           // ring bases of Bx By Bz
@@ -214,6 +220,20 @@ __device__ __forceinline__ size_t j_index(const GridT<F>& g, int c, int i, int j
 template <class F>
 __device__ __forceinline__ size_t j_count(const GridT<F>& g, int c) {
   return (size_t)(e_nx(g, c) + 2) * e_ny(g, c) * (e_nz(g, c) + 2 * g.jpad);
+}
+
+// Marks raw column (i, j), -1 <= i <= nx + 1, 0 <= j <= ny.  The read spares
+// the store of a byte that is already set; a stale read only repeats it.
+constexpr int kMarkNodes = 8;
+__host__ __device__ __forceinline__ int mark_block(int i) { return (i + 1) / kMarkNodes; }
+template <class F>
+__device__ __forceinline__ void mark_column(const GridT<F>& g, int i, int j) {
+  unsigned char* const m = g.mark + (size_t)j * g.mark_pitch + mark_block(i);
+  if (!*m) *m = 1;
+}
+template <class F>
+__device__ __forceinline__ bool column_marked(const GridT<F>& g, int i, int j) {
+  return g.mark[(size_t)j * g.mark_pitch + mark_block(i)] != 0;
 }
 
 // The filtered B of component c: nodes -1 <= i <= b_nx, 0 <= j < b_ny,

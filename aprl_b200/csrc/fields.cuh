@@ -133,6 +133,7 @@ struct FilterArgs {
   GridT<double> g;
   const double* sum[3];   // S0 = E* + E^n (ring layout of E)
   void* out[3];           // kFilterOrbit*: W, layout of j_index; kFilterCurrent: J, native layout
+  int full;               // kFilterOrbit: every column, not only those marks reach
   int planes;             // output planes marched by one warp
   int chunks;             // z chunks (blockIdx.z = component * chunks + chunk)
 };

@@ -831,6 +831,7 @@ struct DepositVisitor {
     }
     if (k < -G.jpad || k >= e_nz(G, a) + G.jpad) return;
     const size_t at = j_index(G, a, (int)i, (int)j, (int)k);
+    mark_column(G, (int)i, (int)j);
     if constexpr (Q) {
       // Order-free integer sum, converted to J once per trial.
       if (!fixed_add(G.jq[a] + 2 * at, double(scale[a] * w), G.jq_scale)) error = kErrFixedRange;
@@ -1119,7 +1120,9 @@ __device__ double conductivity_rate(const DRegion& r, const double p[3]) {
     else if (p[axis] > r.physical_upper[axis])
       depth = (p[axis] - r.physical_upper[axis]) / r.thickness[axis];
     depth = fmax(0.0, fmin(1.0, depth));
-    rate += r.max_rate[axis] * pow(depth, r.order);
+    // pow(0, order) is 0 (order > 0): outside the layers, where most carriers
+    // are, nothing is left of the rate.
+    if (depth > 0.0) rate += r.max_rate[axis] * pow(depth, r.order);
   }
   return rate;
 }
@@ -1136,6 +1139,7 @@ __device__ double damping_factor(const DRegion& r, const double s[3], const doub
     for (int a = 0; a < 3; ++a) p[a] = s[a] + node[k] * (e[a] - s[a]);
     average += weight[k] * conductivity_rate(r, p);
   }
+  if (average == 0.0) return 1.0;
   const double exponent = -duration * average;
   return exponent < log(kDblMin) ? 0.0 : exp(exponent);
 }
@@ -1751,6 +1755,14 @@ __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ C
       if (S != 0 && !x_inside) err = kErrSupportX;
     }
     const bool adds = have && runs.last && y_inside && x_inside && p.k >= -1 && p.k <= g.nz;
+    if (adds) {
+      mark_column(g, p.i, p.j);
+      mark_column(g, p.i, p.j + 1);
+      if (mark_block(p.i + 1) != mark_block(p.i)) {
+        mark_column(g, p.i + 1, p.j);
+        mark_column(g, p.i + 1, p.j + 1);
+      }
+    }
     constexpr int kReach = S == 0 ? 0 : 2;  // nodes below the piece's cell in z
     const long long kz = p.k + g.jpad - kReach;
     const long long n0 = (kz * (g.ny + 1) + p.j) * p0 + (p.i + 1);
@@ -2422,21 +2434,40 @@ __global__ void inlet_charge_kernel(InletMatchArgs a) {
     }
 }
 
+// fn(c, offset) for every node of the raw current's marked columns; a warp
+// takes 32 x nodes of one row and `kMarkPlanes` planes at a time.
+constexpr int kMarkPlanes = 32;
+template <class Fn>
+__device__ __forceinline__ void marked_nodes(const GridT<double>& g, Fn fn) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  const int tiles = (g.nx + 3 + 31) / 32, rows = g.ny + 1;
+  const int chunks = (g.nz + 1 + 2 * g.jpad + kMarkPlanes - 1) / kMarkPlanes;
+  const long long tasks = (long long)tiles * rows * chunks * 3;
+  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < tasks;
+       t += warps) {
+    const int tile = (int)(t % tiles), j = (int)(t / tiles % rows);
+    const int chunk = (int)(t / tiles / rows % chunks), c = (int)(t / tiles / rows / chunks);
+    const int i = tile * 32 + lane - 1;
+    if (i > e_nx(g, c) || j >= e_ny(g, c) || !column_marked(g, i, j)) continue;
+    const int last = min((chunk + 1) * kMarkPlanes, e_nz(g, c) + 2 * g.jpad);
+    const size_t plane = (size_t)e_ny(g, c) * (e_nx(g, c) + 2);
+    size_t at = (size_t)(chunk * kMarkPlanes) * plane + (size_t)j * (e_nx(g, c) + 2) + (i + 1);
+    for (int k = chunk * kMarkPlanes; k < last; ++k, at += plane) fn(c, at);
+  }
+}
+
 __global__ void trial_clear_kernel(GridT<double> g, TrialResult* result, int clear_current,
                                    int* reset_stop) {
   if (trial_skipped(g)) return;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int c = 0; c < 3 && clear_current; ++c) {
-    const long long count = (long long)j_count(g, c);
-    if (clear_current == 2) {
-      ulonglong2* pairs = reinterpret_cast<ulonglong2*>(g.jq[c]);
-      for (long long n = first; n < count; n += stride) pairs[n] = make_ulonglong2(0ull, 0ull);
-    } else {
-      for (long long n = first; n < count; n += stride) g.j[c][n] = 0.;
-    }
-  }
-  if (first == 0) {
+  if (clear_current == 2)
+    marked_nodes(g, [&](int c, size_t n) {
+      reinterpret_cast<ulonglong2*>(c == 0 ? g.jq[0] : (c == 1 ? g.jq[1] : g.jq[2]))[n] =
+          make_ulonglong2(0ull, 0ull);
+    });
+  else if (clear_current)
+    marked_nodes(g, [&](int c, size_t n) { (c == 0 ? g.j[0] : (c == 1 ? g.j[1] : g.j[2]))[n] = 0.; });
+  if (result && blockIdx.x == 0 && threadIdx.x == 0) {
     *result = TrialResult{};
     if (reset_stop) *reset_stop = 0;
   }
@@ -2444,16 +2475,12 @@ __global__ void trial_clear_kernel(GridT<double> g, TrialResult* result, int cle
 
 __global__ void current_convert_kernel(GridT<double> g, double unscale) {
   if (trial_skipped(g)) return;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int c = 0; c < 3; ++c) {
-    const long long count = (long long)j_count(g, c);
-    const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(g.jq[c]);
-    for (long long n = first; n < count; n += stride) {
-      const ulonglong2 v = pairs[n];
-      g.j[c][n] = (v.x | v.y) ? fixed_value(v.x, v.y, unscale) : 0.;
-    }
-  }
+  marked_nodes(g, [&](int c, size_t n) {
+    const ulonglong2 v =
+        reinterpret_cast<const ulonglong2*>(c == 0 ? g.jq[0] : (c == 1 ? g.jq[1] : g.jq[2]))[n];
+    (c == 0 ? g.j[0] : (c == 1 ? g.j[1] : g.j[2]))[n] =
+        (v.x | v.y) ? fixed_value(v.x, v.y, unscale) : 0.;
+  });
 }
 
 __global__ void fixed_convert_kernel(const unsigned long long* pairs, double* out, long long n,

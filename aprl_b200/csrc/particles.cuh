@@ -361,14 +361,15 @@ struct InletMatchArgs {
 };
 __global__ void inlet_charge_kernel(InletMatchArgs a);
 
-// A trial's start: J, the trial counters and the residual sums cleared
-// (skipped with the trial).
-// clear_current: 1 clears J; in the deterministic mode 2 clears the
-// fixed-point pairs of J instead (J is then written by current_convert).
+// A trial's start: the raw current's marked columns, the trial counters and
+// the residual sums cleared (skipped with the trial).
+// clear_current: 1 clears the current; in the deterministic mode 2 clears its
+// fixed-point pairs instead (it is then written by current_convert_kernel).
 // reset_stop: a step's first trial, clearing the verdict of the step before.
 __global__ void trial_clear_kernel(GridT<double> g, TrialResult* result, int clear_current,
                                    int* reset_stop);
-// Deterministic mode: J from its fixed-point pairs, every node.
+// Deterministic mode: the raw current from its fixed-point pairs, in the
+// marked columns.
 __global__ void current_convert_kernel(GridT<double> g, double unscale);
 // out[i] = value of pair i (fixed_value), for i < n.
 __global__ void fixed_convert_kernel(const unsigned long long* pairs, double* out, long long n,

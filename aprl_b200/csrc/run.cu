@@ -290,6 +290,7 @@ struct aprl_run {
   // over it are skipped, which is most of a field-only step's work besides
   // the field updates.
   bool j_zero = true;
+  unsigned char* mark = nullptr;  // the raw current's marked columns (GridT)
   // J as set by aprl_run_set_field, until the next step clears it.
   double* j_set[3]{};
   // The equivalent surface current that the current step's E* holds, for a
@@ -737,6 +738,7 @@ int raw_pad(const aprl_run_config& g) { return g.shape == APRL_SHAPE_LINEAR_BINO
 size_t raw_count(const aprl_run_config& g, int c) {
   return (size_t)(g.nx + (c != 0) + 2) * (g.ny + (c != 1)) * (g.nz + (c != 2) + 2 * raw_pad(g));
 }
+int mark_pitch(const aprl_run_config& g) { return mark_block((int)g.nx + 1) + 1; }
 size_t bfilter_count(const aprl_run_config& g, int c) {
   return (size_t)(g.nx + (c == 0) + 2) * (g.ny + (c == 1)) * (g.nz + (c == 2) + 2);
 }
@@ -989,6 +991,8 @@ GridT<F> make_grid(const aprl_run* r) {
     g.zb_b[a] = r->zb_b[a];
   }
   g.jpad = raw_pad(r->cfg);
+  g.mark = r->mark;
+  g.mark_pitch = mark_pitch(r->cfg);
   g.inv_h[0] = 1. / g.dx;
   g.inv_h[1] = 1. / g.dy;
   g.inv_h[2] = 1. / g.dz;
@@ -1676,9 +1680,12 @@ aprl_status advance_magnetic_t(aprl_run* r) {
   if (r->ledger_on && !r->ledger_start_ready) TRY(ledger_begin(r));
   r->ledger_start_ready = false;
   const aprl_run_config& c = r->cfg;
-  if (!r->j_zero)
-    for (int a = 0; a < 3; ++a)
-      CUDA_TRY(cudaMemsetAsync(r->jc[a], 0, raw_count(c, a) * sizeof(F), r->stream));
+  if (!r->j_zero) {
+    for (int kind = 1; kind <= (r->deterministic ? 2 : 1); ++kind)
+      TRY(launch(r, kTrialClear, trial_clear_kernel, dim3(148 * 8), dim3(256),
+                 make_grid<double>(r), (TrialResult*)nullptr, kind, (int*)nullptr));
+    CUDA_TRY(cudaMemsetAsync(r->mark, 0, (c.ny + 1) * mark_pitch(c), r->stream));
+  }
   r->j_zero = true;
   r->surface_in_j = false;
   for (int a = 0; a < 3; ++a) {
@@ -1781,8 +1788,9 @@ dim3 filter_grid(const aprl_run_config& c, dim3 block, unsigned written, int pad
 // thread block `block` (a multiple of 32 wide).
 template <int MODE, class W>
 aprl_status filter_pass(aprl_run* r, unsigned id, const GridT<double>& g, dim3 block,
-                        void* const out[3]) {
+                        void* const out[3], bool full = false) {
   FilterArgs a{};
+  a.full = full ? 1 : 0;
   a.g = g;
   for (int d = 0; d < 3; ++d) {
     a.sum[d] = r->sum[d];
@@ -1956,9 +1964,7 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     frozen_end = q.offsets[until - q.initial_step + 1];
   }
   const bool deposits = r->np || r->nc || (r->queue.extracted && frozen_end > r->queue.cursor);
-  size_t most = 0;
-  for (int a = 0; a < 3; ++a) most = std::max(most, raw_count(c, a));
-  const unsigned grid_blocks = std::min<unsigned>(blocks_for(most, 256), 148 * 8);
+  const unsigned grid_blocks = 148 * 8;
   // Deterministic mode: the deposits of the trial go into J's fixed-point
   // pairs, and J is written from them once they are all done.
   const bool convert = r->deterministic && deposits;
@@ -2141,8 +2147,9 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
       } else {
         tl.candidate = std::max(0, r->tune_choice[kTuneOrbit]);
       }
+      // Without a guess pass the step's first sum is formed everywhere.
       TRY((filter_pass<kFilterOrbit, W>(r, kOrbitSum, g, kGridBlocks[tl.candidate],
-                                        r->filtered)));
+                                        r->filtered, direct && r->trials == 0)));
       TRY(tune_end(r, tl));
     }
     ResidualArgs<F> ra{};
@@ -2628,6 +2635,8 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
         (s = device_alloc(r, &r->inlet_rho_pairs, 2 * (size_t)(c.nx + 1) * (c.ny + 1))) != APRL_OK)
       return cleanup(s);
   }
+  if ((s = device_alloc(r, &r->mark, (c.ny + 1) * mark_pitch(c))) != APRL_OK) return cleanup(s);
+  cudaMemsetAsync(r->mark, 0, (c.ny + 1) * mark_pitch(c), r->stream);
   if ((s = device_alloc(r, &r->d_block, 1)) != APRL_OK) return cleanup(s);
   r->d_status = &r->d_block->status;
   r->d_stop = &r->d_block->stop;
@@ -2746,6 +2755,7 @@ aprl_status aprl_run_destroy(aprl_run* r) {
   device_free(r, r->ledger_pre[0]);
   device_free(r, r->ledger_pre[1]);
   device_free(r, r->d_block);
+  device_free(r, r->mark);
   device_free(r, r->scan_count);
   device_free(r, r->scan_offset);
   device_free(r, r->inlet_rho);
