@@ -99,7 +99,7 @@ __device__ __forceinline__ size_t bounded(DeviceStatus* s, size_t index, size_t 
 #define APRL_BOUNDED(status, index, extent, site) \
   ::aprl_gpu::bounded((status), (size_t)(index), (size_t)(extent), (site))
 #else
-#define APRL_BOUNDED(status, index, extent, site) ((size_t)(index))
+#define APRL_BOUNDED(status, index, extent, site) (index)
 #endif
 
 // One magnet of SIFieldSourceSet (src/eb_sources.h:103-140).
@@ -195,27 +195,31 @@ __device__ __forceinline__ bool node_inside(DeviceStatus* s, int i, int j, int k
 #define APRL_NODE_CHECK(g, i, j, k, nx, ny, nz, site)
 #endif
 
+// Array offsets are formed in 32 bits: a run holds more than fifteen arrays of
+// a component's size, so no component that fits a GPU has 2^32 elements.  In
+// 64 bits the index arithmetic was over half of the grid kernels'
+// instructions.
 template <class F>
-__device__ __forceinline__ size_t e_index(const GridT<F>& g, int c, int i, int j, int k) {
+__device__ __forceinline__ unsigned e_index(const GridT<F>& g, int c, int i, int j, int k) {
   const int nzc = e_nz(g, c);
   APRL_NODE_CHECK(g, i, j, k, e_nx(g, c), e_ny(g, c), nzc, 1 + c);
-  return ((size_t)ring(k, g.zb_e[c], nzc) * e_ny(g, c) + j) * e_nx(g, c) + i;
+  return (unsigned)((ring(k, g.zb_e[c], nzc) * e_ny(g, c) + j) * (unsigned)e_nx(g, c) + i);
 }
 
 template <class F>
-__device__ __forceinline__ size_t b_index(const GridT<F>& g, int c, int i, int j, int k) {
+__device__ __forceinline__ unsigned b_index(const GridT<F>& g, int c, int i, int j, int k) {
   const int nzc = b_nz(g, c);
   APRL_NODE_CHECK(g, i, j, k, b_nx(g, c), b_ny(g, c), nzc, 4 + c);
-  return ((size_t)ring(k, g.zb_b[c], nzc) * b_ny(g, c) + j) * b_nx(g, c) + i;
+  return (unsigned)((ring(k, g.zb_b[c], nzc) * b_ny(g, c) + j) * (unsigned)b_nx(g, c) + i);
 }
 
 // The raw current and the filtered orbit sum of E component c: nodes
 // -1 <= i <= e_nx, 0 <= j < e_ny, -jpad <= k < e_nz + jpad.
 template <class F>
-__device__ __forceinline__ size_t j_index(const GridT<F>& g, int c, int i, int j, int k) {
+__device__ __forceinline__ unsigned j_index(const GridT<F>& g, int c, int i, int j, int k) {
   APRL_NODE_CHECK(g, i + 1, j, k + g.jpad, e_nx(g, c) + 2, e_ny(g, c), e_nz(g, c) + 2 * g.jpad,
                   7 + c);
-  return ((size_t)(k + g.jpad) * e_ny(g, c) + j) * (e_nx(g, c) + 2) + (i + 1);
+  return (unsigned)(((k + g.jpad) * e_ny(g, c) + j) * (unsigned)(e_nx(g, c) + 2) + (i + 1));
 }
 template <class F>
 __device__ __forceinline__ size_t j_count(const GridT<F>& g, int c) {
@@ -239,9 +243,9 @@ __device__ __forceinline__ bool column_marked(const GridT<F>& g, int i, int j) {
 // The filtered B of component c: nodes -1 <= i <= b_nx, 0 <= j < b_ny,
 // -1 <= k <= b_nz.
 template <class F>
-__device__ __forceinline__ size_t bf_index(const GridT<F>& g, int c, int i, int j, int k) {
+__device__ __forceinline__ unsigned bf_index(const GridT<F>& g, int c, int i, int j, int k) {
   APRL_NODE_CHECK(g, i + 1, j, k + 1, b_nx(g, c) + 2, b_ny(g, c), b_nz(g, c) + 2, 27 + c);
-  return ((size_t)(k + 1) * b_ny(g, c) + j) * (b_nx(g, c) + 2) + (i + 1);
+  return (unsigned)(((k + 1) * b_ny(g, c) + j) * (unsigned)(b_nx(g, c) + 2) + (i + 1));
 }
 
 // Elements of E component c and of B component c.

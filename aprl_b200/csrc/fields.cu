@@ -14,32 +14,6 @@
 
 namespace aprl_gpu {
 
-// electricValue (src/eb_field.cpp:350-417) under the moving window: x/y
-// PEC parity extension, z halo planes (lower = inlet reference plane,
-// upper = the last rank's zero plane).
-template <class F>
-__device__ __forceinline__ double electric_value(const CowanArgs<F>& a, int c, int i, int j,
-                                                 int k) {
-  const int nxc = a.g.nx + (c != 0), nyc = a.g.ny + (c != 1), nzc = a.g.nz + (c != 2);
-  double sign = 1.0;
-  if (i < 0) {
-    if (c == 0) i = 0; else { i = -i; sign = -sign; }
-  } else if (i >= nxc) {
-    if (c == 0) i = nxc - 1; else { i = 2 * (nxc - 1) - i; sign = -sign; }
-  }
-  if (j < 0) {
-    if (c == 1) j = 0; else { j = -j; sign = -sign; }
-  } else if (j >= nyc) {
-    if (c == 1) j = nyc - 1; else { j = 2 * (nyc - 1) - j; sign = -sign; }
-  }
-  if (k < 0)
-    return sign * a.lower[c][APRL_BOUNDED(a.g.status, (size_t)j * nxc + i, (size_t)nxc * nyc, 10 + c)];
-  if (k >= nzc) return sign * 0.0;
-  return sign * a.e[c][APRL_BOUNDED(a.g.status,
-                                    ((size_t)ring(k, a.g.zb_e[c], nzc) * nyc + j) * nxc + i,
-                                    (size_t)nxc * nyc * nzc, 13 + c)];
-}
-
 // transformedCorrection (src/eb_cpml.cpp:131-138).
 __device__ __forceinline__ double cpml_correction(const CpmlAxis& ax, int index,
                                                   double difference, double* history) {
@@ -52,8 +26,9 @@ __device__ __forceinline__ double* history_at(const CpmlHistory& h, int slot, in
                                               int row_index, DeviceStatus* status) {
   (void)status;
   return h.data + APRL_BOUNDED(status,
-                               ((size_t)slot * h.layers + ring(k, zbase, h.layers)) * h.row +
-                                   row_index,
+                               (unsigned)((slot * h.layers + ring(k, zbase, h.layers)) *
+                                              (unsigned)h.row +
+                                          row_index),
                                (size_t)h.slots * h.layers * h.row, 16);
 }
 
@@ -63,8 +38,8 @@ __device__ __forceinline__ double* history_at(const CpmlHistory& h, int slot, in
 // A block owns a TX x TY tile of (i, j) columns and marches a chunk of z
 // planes.  The three E components of planes k-1, k, k+1 live in a shared
 // memory ring, one (TX+2) x (TY+2) tile each, loaded once per plane through
-// electricValue's parity/halo rules.  Every smoothed difference (the
-// 9-point smoothedElectric of src/eb_field.cpp:419-486: alpha*centre, the
+// the reference electricValue's parity/halo rules (map_tile).  Every smoothed
+// difference (the 9-point smoothedElectric of src/eb_field.cpp:419-486: alpha*centre, the
 // four beta edge samples, the four delta corners) is then evaluated from
 // shared memory in the reference's order, so the FP64 update is
 // bit-identical to the reference.  Each B node is updated by the
@@ -118,49 +93,79 @@ __device__ __forceinline__ double tile_smoothed(const ETile& t, const CowanArgs<
   return result;
 }
 
-// Fills one plane of the tile.  Only coordinates within one cell of a
-// component's index range are ever read by the smoothing (the reference's
-// own reach); tile points farther out, which exist only where a small grid
-// ends inside a tile, are stored as zero and never used.
+// A thread's share of a tile plane: which E value each of its entries holds
+// under electricValue's x and y rules (parity extension at the PEC walls).
+// The rules do not depend on the plane, so they are evaluated once a march;
+// evaluated for every value of every plane they were most of the kernel's
+// instructions, in the boundary tiles that are over half of a 129-node row's.
+// Only coordinates within one cell of a component's index range are ever used
+// by the smoothing (the reference's own reach); tile points farther out, which
+// exist only where a small grid ends inside a tile, hold zero.
+constexpr int kTileW = kTX + 2, kTileN = (kTX + 2) * (kTY + 2), kTileT = kTX * kTY,
+              kTileR = (kTileN + kTileT - 1) / kTileT;
+
+struct TileMap {
+  int at[3][kTileR];  // offset in the component's plane, -1: none
+  unsigned odd;       // bit kTileR * c + r: the entry is a sign-reversed mirror image
+};
+
 template <class F>
-__device__ __forceinline__ void load_plane(ETile& t, const CowanArgs<F>& a, int k, int slot,
-                                           int i0, int j0) {
-  constexpr int W = kTX + 2, H = kTY + 2, N = W * H, T = kTX * kTY, R = (N + T - 1) / T;
+__device__ __forceinline__ void map_tile(TileMap& m, const CowanArgs<F>& a, int i0, int j0) {
   const int tid = threadIdx.y * kTX + threadIdx.x;
-  // A tile whose rim lies inside every component's index range, on a plane
-  // inside every component's z range, needs none of electricValue's parity
-  // and halo rules: its values are read straight from E.
-  const bool interior = i0 >= 1 && i0 + kTX <= a.g.nx - 1 && j0 >= 1 &&
-                        j0 + kTY <= a.g.ny - 1 && k >= 0 && k < a.g.nz;
+  m.odd = 0u;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int nxc = a.g.nx + (c != 0), nyc = a.g.ny + (c != 1);
+#pragma unroll
+    for (int r = 0; r < kTileR; ++r) {
+      const int n = tid + r * kTileT;
+      const int jj = n / kTileW;
+      int i = i0 - 1 + (n - jj * kTileW), j = j0 - 1 + jj;
+      m.at[c][r] = -1;
+      if (n >= kTileN || i > nxc || j > nyc) continue;
+      bool odd = false;
+      if (i < 0 || i >= nxc) {
+        if (c != 0) odd = !odd;
+        i = i < 0 ? (c == 0 ? 0 : -i) : (c == 0 ? nxc - 1 : 2 * (nxc - 1) - i);
+      }
+      if (j < 0 || j >= nyc) {
+        if (c != 1) odd = !odd;
+        j = j < 0 ? (c == 1 ? 0 : -j) : (c == 1 ? nyc - 1 : 2 * (nyc - 1) - j);
+      }
+      m.at[c][r] = j * nxc + i;
+      if (odd) m.odd |= 1u << (kTileR * c + r);
+    }
+  }
+}
+
+// Fills one plane of the tile: the inlet's halo plane below the grid, zero
+// above it.
+template <class F>
+__device__ __forceinline__ void load_plane(ETile& t, const TileMap& m, const CowanArgs<F>& a,
+                                           int k, int slot) {
+  const int tid = threadIdx.y * kTX + threadIdx.x;
   // All of a thread's loads are issued before any shared-memory store, so
   // their latencies overlap instead of adding up.
-  double v[3][R];
+  double v[3][kTileR];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const int nxc = a.g.nx + (c != 0), nyc = a.g.ny + (c != 1), nzc = a.g.nz + (c != 2);
-    const double* plane =
-        interior ? a.e[c] + (size_t)ring(k, a.g.zb_e[c], nzc) * nyc * nxc : nullptr;
+    const unsigned plane = nxc * nyc;
+    const double* from =
+        k < 0 ? a.lower[c] : a.e[c] + (k < nzc ? ring(k, a.g.zb_e[c], nzc) * plane : 0u);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int n = tid + r * T;
-      double x = 0.0;
-      if (n < N) {
-        const int ii = n % W, jj = n / W;
-        const int i = i0 - 1 + ii, j = j0 - 1 + jj;
-        if (interior)
-          x = plane[APRL_BOUNDED(a.g.status, (size_t)j * nxc + i, (size_t)nxc * nyc, 19 + c)];
-        else if (!(i < -1 || i > nxc || j < -1 || j > nyc))
-          x = electric_value(a, c, i, j, k);
-      }
-      v[c][r] = x;
-    }
+    for (int r = 0; r < kTileR; ++r)
+      v[c][r] = m.at[c][r] >= 0 && k < nzc
+                    ? from[APRL_BOUNDED(a.g.status, m.at[c][r], plane, 10 + c)]
+                    : 0.0;
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int n = tid + r * T;
-      if (n < N) t.v[c][slot][n / W][n % W] = v[c][r];
+    for (int r = 0; r < kTileR; ++r) {
+      const int n = tid + r * kTileT;
+      if (n < kTileN)
+        (&t.v[c][slot][0][0])[n] = (m.odd >> (kTileR * c + r)) & 1u ? -v[c][r] : v[c][r];
     }
 }
 
@@ -173,11 +178,13 @@ __global__ void __launch_bounds__(kTX * kTY, APRL_COWAN_MIN_BLOCKS)
   const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
   const int k0 = blockIdx.z * a.chunk;
   const int k1 = min(k0 + a.chunk, g.nz + 1);
-  const double dtdx = g.dt / g.dx, dtdy = g.dt / g.dy, dtdz = g.dt / g.dz;
+  const double dtdx = a.dtdx, dtdy = a.dtdy, dtdz = a.dtdz;
   const int li = threadIdx.x + 1, lj = threadIdx.y + 1;
   PlaneSlots ps = {{0, 1, 2}};
-  load_plane(t, a, k0 - 1, ps.s[0], i0, j0);
-  load_plane(t, a, k0, ps.s[1], i0, j0);
+  TileMap map;
+  map_tile(map, a, i0, j0);
+  load_plane(t, map, a, k0 - 1, ps.s[0]);
+  load_plane(t, map, a, k0, ps.s[1]);
   // The column's CPML slots are the same on every plane of the march.
   const bool column = i <= g.nx && j <= g.ny;
   const int slot_x = column && i < g.nx ? a.mx.ordinal[i] : -1;
@@ -187,7 +194,7 @@ __global__ void __launch_bounds__(kTX * kTY, APRL_COWAN_MIN_BLOCKS)
   // of the next step: carried in registers instead of evaluated again.
   double ey_above = 0.0, ex_above = 0.0;
   for (int k = k0; k < k1; ++k) {
-    load_plane(t, a, k + 1, ps.s[2], i0, j0);
+    load_plane(t, map, a, k + 1, ps.s[2]);
     // The node's three B values are read before the first B store (which
     // may alias them as far as the compiler knows).
     const bool has_bx = column && j < g.ny && k < g.nz;
@@ -249,112 +256,128 @@ __global__ void __launch_bounds__(kTX * kTY, APRL_COWAN_MIN_BLOCKS)
   }
 }
 
-template <class F>
-__device__ __forceinline__ double bval(const GridT<F>& g, int c, int i, int j, int k) {
-  return g.b[c][b_index(g, c, i, j, k)];
-}
-
 // advanceElectric with J = 0 (src/eb_field.cpp:582-627) followed by the
 // moving-window boundary (src/moving_window_fields.cpp:254-293): the CPML
 // electric terms (src/eb_cpml.cpp:470-539; the convolution histories are
 // advanced here once, exactly as the later commit would advance them from
 // the same B), PEC on the x/y faces, and the inlet Ex/Ey overwrite at k=0.
 // Reads E^n from e_old, writes E* to e_star.
+//
+// One thread per (i, j) column, marching `chunk` planes: the column's
+// predicates, offsets and CPML slots are formed once, a plane's base pointers
+// are the same for the whole block, and Bx and By of the plane below stay in
+// registers.  One thread per node spent 740 instructions on a node's twelve
+// reads, four divisions and some 60 floating-point operations.  On the
+// 128x128x512 grid, with the orbit sum written: 0.234 -> 0.225 ms at 2 planes
+// (1 plane 0.235, 4 planes 0.226, 16 planes 0.25-0.26: a plane's latency is
+// then serial); the 805 MB it moves take 0.123 ms at the copy rate.
 template <class F>
-__global__ void electric_preview_kernel(PreviewArgs<F> a) {
+__global__ void __launch_bounds__(256, 4) electric_preview_kernel(PreviewArgs<F> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
   const GridT<F>& g = a.g;
-  if (i > g.nx || j > g.ny || k > g.nz) return;
-  const double curl = g.dt / (kMu0 * kEpsilon0);
-  const double cx = curl / g.dx, cy = curl / g.dy, cz = curl / g.dz;
-  // Every E and B read of the node is issued before its first store (the
-  // stores may alias them as far as the compiler knows), so their latencies
-  // overlap; each difference below is formed from the same two values as
-  // before, in the same order.
-  const bool has_x = i < g.nx, has_y = j < g.ny, has_z = k < g.nz;
-  const bool x_row = has_x && j >= 1 && j < g.ny;     // Ex: y difference of Bz
-  const bool x_curl = x_row && k >= 1 && k < g.nz;    // Ex: the whole curl
-  const bool y_row = has_y && i >= 1 && i < g.nx;     // Ey: x difference of Bz
-  const bool y_curl = y_row && k >= 1 && k < g.nz;    // Ey: the whole curl
-  const bool z_inner = has_z && i >= 1 && i < g.nx && j >= 1 && j < g.ny;
-  const size_t n0 = has_x ? e_index(g, 0, i, j, k) : 0;
-  const size_t n1 = has_y ? e_index(g, 1, i, j, k) : 0;
-  const size_t n2 = has_z ? e_index(g, 2, i, j, k) : 0;
-  const double old0 = has_x ? g.e_old[0][n0] : 0.0;
-  const double old1 = has_y ? g.e_old[1][n1] : 0.0;
-  const double old2 = has_z ? g.e_old[2][n2] : 0.0;
-  const double bz = x_row || y_row ? bval(g, 2, i, j, k) : 0.0;
-  const double bz_j = x_row ? bval(g, 2, i, j - 1, k) : 0.0;
-  const double bz_i = y_row ? bval(g, 2, i - 1, j, k) : 0.0;
-  const double by = x_curl || z_inner ? bval(g, 1, i, j, k) : 0.0;
-  const double by_k = x_curl ? bval(g, 1, i, j, k - 1) : 0.0;
-  const double by_i = z_inner ? bval(g, 1, i - 1, j, k) : 0.0;
-  const double bx = y_curl || z_inner ? bval(g, 0, i, j, k) : 0.0;
-  const double bx_k = y_curl ? bval(g, 0, i, j, k - 1) : 0.0;
-  const double bx_j = z_inner ? bval(g, 0, i, j - 1, k) : 0.0;
-  if (has_x) {  // Ex (nx, ny+1, nz+1)
-    double v = old0;
-    if (x_curl) v += cy * (bz - bz_j) - cz * (by - by_k);
-    if (x_row) {
-      const int s = a.ey_prof.ordinal[j];
-      if (s >= 0) {
+  if (i > g.nx || j > g.ny) return;
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const int k0 = blockIdx.z * a.chunk, k1 = min(k0 + a.chunk, nz + 1);
+  const double cx = a.cx, cy = a.cy, cz = a.cz;
+  const bool has_x = i < nx, has_y = j < ny;
+  const bool x_row = has_x && j >= 1 && j < ny;  // Ex: y difference of Bz
+  const bool y_row = has_y && i >= 1 && i < nx;  // Ey: x difference of Bz
+  const bool z_col = i >= 1 && i < nx && j >= 1 && j < ny;
+  const int slot_x = has_x ? a.ex_prof.ordinal[i] : -1;
+  const int slot_y = has_y ? a.ey_prof.ordinal[j] : -1;
+  // Offsets in a plane of rows nx and nx + 1 wide, and the planes' sizes.
+  const int on = j * nx + i, ow = j * (nx + 1) + i;
+  const unsigned pe0 = nx * (ny + 1), pe1 = (nx + 1) * ny, pe2 = (nx + 1) * (ny + 1),
+                 pbz = nx * ny;
+  auto plane = [&](const double* v, int k, int zb, int n, unsigned size) {
+    return v + ring(k, zb, n) * size;
+  };
+  auto at = [&](const double* v, unsigned offset, unsigned size, unsigned site) {
+    (void)size;
+    (void)site;
+    return v[APRL_BOUNDED(g.status, offset, size, site)];
+  };
+  // The plane below: By for Ex and Bx for Ey.
+  double by_k = 0.0, bx_k = 0.0;
+  if (k0 >= 1 && k0 <= nz) {
+    if (x_row) by_k = at(plane(g.b[1], k0 - 1, g.zb_b[1], nz, pe0), on, pe0, 5);
+    if (y_row) bx_k = at(plane(g.b[0], k0 - 1, g.zb_b[0], nz, pe1), ow, pe1, 4);
+  }
+  for (int k = k0; k < k1; ++k) {
+    // Every E and B read of the node is issued before its first store (the
+    // stores may alias them as far as the compiler knows).
+    const bool has_z = k < nz, inner_k = k >= 1 && k < nz;
+    const unsigned b0 = ring(k, g.zb_e[0], nz + 1) * pe0, b1 = ring(k, g.zb_e[1], nz + 1) * pe1,
+                   b2 = has_z ? ring(k, g.zb_e[2], nz) * pe2 : 0u;
+    const double* const pz = plane(g.b[2], k, g.zb_b[2], nz + 1, pbz);
+    const double old0 = has_x ? at(g.e_old[0] + b0, on, pe0, 1) : 0.0;
+    const double old1 = has_y ? at(g.e_old[1] + b1, ow, pe1, 2) : 0.0;
+    const double old2 = has_z ? at(g.e_old[2] + b2, ow, pe2, 3) : 0.0;
+    const double bz = x_row || y_row ? (has_x && has_y ? at(pz, on, pbz, 6) : 0.0) : 0.0;
+    const double bz_j = x_row ? at(pz, on - nx, pbz, 6) : 0.0;
+    const double bz_i = y_row ? at(pz, on - 1, pbz, 6) : 0.0;
+    double by = 0.0, by_i = 0.0, bx = 0.0, bx_j = 0.0;
+    if (has_z) {
+      const double* const py = plane(g.b[1], k, g.zb_b[1], nz, pe0);
+      const double* const px = plane(g.b[0], k, g.zb_b[0], nz, pe1);
+      if (x_row) by = at(py, on, pe0, 5);
+      if (y_row) bx = at(px, ow, pe1, 4);
+      if (z_col) {
+        by_i = at(py, on - 1, pe0, 5);
+        bx_j = at(px, ow - (nx + 1), pe1, 4);
+      }
+    }
+    if (has_x) {  // Ex (nx, ny+1, nz+1)
+      double v = old0;
+      if (x_row && inner_k) v += cy * (bz - bz_j) - cz * (by - by_k);
+      if (x_row && slot_y >= 0) {
         const double diff = bz - bz_j;
         v += 1.0 * cy * cpml_correction(a.ey_prof, j, diff,
-                                        history_at(a.h[0], s, k, g.zb_e[0], i, g.status));
+                                        history_at(a.h[0], slot_y, k, g.zb_e[0], i, g.status));
       }
+      if (j == 0 || j == ny) v = 0.0;
+      if (k == 0) {
+        if (a.pre_inlet[0]) a.pre_inlet[0][APRL_BOUNDED(g.status, on, pe0, 22)] = v;
+        v = inlet_value(a.inlet, 0, i, j);
+      }
+      g.e_star[0][b0 + on] = v;
+      if (a.sum[0]) a.sum[0][b0 + on] = v + old0;
     }
-    if (j == 0 || j == g.ny) v = 0.0;
-    if (k == 0) {
-      if (a.pre_inlet[0])
-        a.pre_inlet[0][APRL_BOUNDED(g.status, (size_t)j * g.nx + i, (size_t)g.nx * (g.ny + 1), 22)] = v;
-      v = inlet_value(a.inlet, 0, i, j);
-    }
-    g.e_star[0][n0] = v;
-    if (a.sum[0]) a.sum[0][n0] = v + old0;
-  }
-  if (has_y) {  // Ey (nx+1, ny, nz+1)
-    double v = old1;
-    if (y_curl) v += cz * (bx - bx_k) - cx * (bz - bz_i);
-    if (y_row) {
-      const int s = a.ex_prof.ordinal[i];
-      if (s >= 0) {
+    if (has_y) {  // Ey (nx+1, ny, nz+1)
+      double v = old1;
+      if (y_row && inner_k) v += cz * (bx - bx_k) - cx * (bz - bz_i);
+      if (y_row && slot_x >= 0) {
         const double diff = bz - bz_i;
         v += -1.0 * cx * cpml_correction(a.ex_prof, i, diff,
-                                         history_at(a.h[1], s, k, g.zb_e[1], j, g.status));
+                                         history_at(a.h[1], slot_x, k, g.zb_e[1], j, g.status));
       }
-    }
-    if (i == 0 || i == g.nx) v = 0.0;
-    if (k == 0) {
-      if (a.pre_inlet[1])
-        a.pre_inlet[1][APRL_BOUNDED(g.status, (size_t)j * (g.nx + 1) + i,
-                                    (size_t)(g.nx + 1) * g.ny, 23)] = v;
-      v = inlet_value(a.inlet, 1, i, j);
-    }
-    g.e_star[1][n1] = v;
-    if (a.sum[0]) a.sum[1][n1] = v + old1;
-  }
-  if (has_z) {  // Ez (nx+1, ny+1, nz)
-    double v = old2;
-    if (z_inner) v += cx * (by - by_i) - cy * (bx - bx_j);
-    if (z_inner) {
-      const int sx = a.ex_prof.ordinal[i];
-      if (sx >= 0) {
-        const double diff = by - by_i;
-        v += 1.0 * cx * cpml_correction(a.ex_prof, i, diff,
-                                        history_at(a.h[2], sx, k, g.zb_e[2], j, g.status));
+      if (i == 0 || i == nx) v = 0.0;
+      if (k == 0) {
+        if (a.pre_inlet[1]) a.pre_inlet[1][APRL_BOUNDED(g.status, ow, pe1, 23)] = v;
+        v = inlet_value(a.inlet, 1, i, j);
       }
-      const int sy = a.ey_prof.ordinal[j];
-      if (sy >= 0) {
-        const double diff = bx - bx_j;
-        v += -1.0 * cy * cpml_correction(a.ey_prof, j, diff,
-                                         history_at(a.h[3], sy, k, g.zb_e[2], i, g.status));
-      }
+      g.e_star[1][b1 + ow] = v;
+      if (a.sum[0]) a.sum[1][b1 + ow] = v + old1;
     }
-    if (i == 0 || i == g.nx || j == 0 || j == g.ny) v = 0.0;
-    g.e_star[2][n2] = v;
-    if (a.sum[0]) a.sum[2][n2] = v + old2;
+    if (has_z) {  // Ez (nx+1, ny+1, nz)
+      double v = old2;
+      if (z_col) {
+        const double dby = by - by_i, dbx = bx - bx_j;
+        v += cx * dby - cy * dbx;
+        if (slot_x >= 0)
+          v += 1.0 * cx * cpml_correction(a.ex_prof, i, dby,
+                                          history_at(a.h[2], slot_x, k, g.zb_e[2], j, g.status));
+        if (slot_y >= 0)
+          v += -1.0 * cy * cpml_correction(a.ey_prof, j, dbx,
+                                           history_at(a.h[3], slot_y, k, g.zb_e[2], i, g.status));
+      }
+      if (i == 0 || i == nx || j == 0 || j == ny) v = 0.0;
+      g.e_star[2][b2 + ow] = v;
+      if (a.sum[0]) a.sum[2][b2 + ow] = v + old2;
+    }
+    by_k = by;
+    bx_k = bx;
   }
 }
 
@@ -469,13 +492,119 @@ struct ZWindow {
   }
 };
 
+// One lane's column of a filter pass.
+struct FilterMarch {
+  unsigned plane, nplane;  // plane sizes of the padded arrays and of E
+  int row, node;           // the lane's offsets in a plane of either
+  int nzc, zb, zlo, zhi;   // planes, ring base, the mask's planes
+  bool inside, raw_in, writes, column;
+  const double *raw, *sum;
+  double* star;
+  void* out;
+};
+
+// Output planes from k0 on, the candidate sum's planes [s0, s1).  A plane costs
+// few arithmetic operations, so the loop is kept to them: 32-bit offsets that
+// step by a plane, the ring's wrap a uniform test, two planes' reads together
+// (with the tests and 64-bit offsets of every plane the guess pass took 85
+// instructions a plane, of which 12 were arithmetic and memory).
+template <int S, int MODE, class W, bool WHOLE>
+__device__ __forceinline__ void filter_march(const GridT<double>& g, const FilterMarch& m, int c,
+                                             int k0, int s0, int s1) {
+  constexpr int R = ZWindow<S>::R;
+  constexpr bool kOrbit = MODE == kFilterGuess || MODE == kFilterOrbit;
+  constexpr bool kRaw = MODE != kFilterGuess;
+  ZWindow<S> wj, ws;
+  wj.clear();
+  ws.clear();
+  // Offsets of plane k of the raw current (modulo 2^32 below the array, where
+  // nothing is read), and of the ring's plane p.
+  unsigned raw_off = (unsigned)(s0 - R + g.jpad) * m.plane + m.row;
+  auto raw_at = [&](int k) -> double {
+    if (!m.raw_in || (!WHOLE && (k < -g.jpad || k >= m.nzc + g.jpad))) return 0.;
+    return m.raw[APRL_BOUNDED(g.status, raw_off, j_count(g, c), 33 + c)];
+  };
+  int p = ring(max(s0, 0) < m.nzc ? max(s0, 0) : 0, m.zb, m.nzc);
+  unsigned ring_off = p * m.nplane + m.node;
+  auto next_ring = [&](int k) {  // from plane k on to the next
+    if (!WHOLE && k < 0) return;
+    ring_off += m.nplane;
+    if (++p == m.nzc) {
+      p = 0;
+      ring_off = m.node;
+    }
+  };
+  auto sum_at = [&](int k) -> double {
+    if (!m.inside || (!WHOLE && (k < 0 || k >= m.nzc))) return 0.;
+    return m.sum[APRL_BOUNDED(g.status, ring_off, e_count(g, c), 36 + c)];
+  };
+  if constexpr (kRaw) {
+#pragma unroll
+    for (int t = -R; t < R; ++t) {
+      double v = raw_at(s0 + t);
+      raw_off += m.plane;
+      if constexpr (S == 0) v = lane_filter(v);
+      wj.push(v);
+    }
+  }
+  unsigned out_off = kOrbit ? (unsigned)(k0 + g.jpad) * m.plane + m.row
+                            : (unsigned)k0 * m.nplane + m.node;
+  constexpr int U = MODE == kFilterCommit ? 4 : 2;
+  for (int kb = s0; kb < s1; kb += U) {
+    double raw_v[U], sum_v[U];
+    unsigned star_off[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      raw_v[u] = sum_v[u] = 0.;
+      star_off[u] = ring_off;
+      if (kb + u >= s1) break;
+      if constexpr (kRaw) {
+        raw_v[u] = raw_at(kb + u + R);
+        raw_off += m.plane;
+      }
+      if constexpr (kOrbit) sum_v[u] = sum_at(kb + u);
+      if constexpr (kOrbit || MODE == kFilterCommit) next_ring(kb + u);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = kb + u;
+      if (k >= s1) break;
+      double current = 0.;
+      if constexpr (kRaw) {
+        double v = raw_v[u];
+        if constexpr (S == 0) v = lane_filter(v);
+        wj.push(v);
+        current = wj.value();
+      }
+      const bool masked = m.column && (WHOLE || (k >= m.zlo && k <= m.zhi));
+      if constexpr (MODE == kFilterCommit) {
+        if (m.writes && masked && current != 0.)
+          m.star[APRL_BOUNDED(g.status, star_off[u], e_count(g, c), 39 + c)] += g.jcoef * current;
+      } else if constexpr (MODE == kFilterCurrent) {
+        if (m.writes) static_cast<double*>(m.out)[out_off] = current;
+        out_off += m.nplane;
+      } else {
+        double s = sum_v[u];
+        if (masked && current != 0.) s += g.jcoef * current;
+        if constexpr (S == 0) s = lane_filter(s);
+        ws.push(s);
+        if (k - R >= k0) {
+          if (m.writes)
+            static_cast<W*>(m.out)[APRL_BOUNDED(g.status, out_off, j_count(g, c), 42 + c)] =
+                W(ws.value());
+          out_off += m.plane;
+        }
+      }
+    }
+  }
+}
+
 template <int S, int MODE, class W>
 __global__ void current_filter_kernel(FilterArgs a) {
   const GridT<double>& g = a.g;
   if (trial_skipped(g)) return;
   constexpr int R = ZWindow<S>::R;
   constexpr bool kOrbit = MODE == kFilterGuess || MODE == kFilterOrbit;
-  constexpr bool kRaw = MODE != kFilterGuess;
   const int lane = threadIdx.x & 31;
   const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -511,88 +640,30 @@ __global__ void current_filter_kernel(FilterArgs a) {
   const int k0 = first + (int)(blockIdx.z % a.chunks) * a.planes;
   const int k1 = min(k0 + a.planes, last);
   if (k0 >= k1) return;
-  const size_t plane = (size_t)nyc * (nxc + 2), nplane = (size_t)nyc * nxc;
-  ZWindow<S> wj, ws;
-  wj.clear();
-  ws.clear();
   const int s0 = kOrbit ? k0 - R : k0;  // first plane of the (candidate) sum
   const int s1 = kOrbit ? k1 + R : k1;
-  // The warp walks its columns by adding a plane's size: offsets of the next
-  // plane of the padded arrays, of J, and of the ring (and its next plane).
-  const int row = j * (nxc + 2) + (i + 1), node = j * nxc + i;
-  size_t raw_off = (size_t)(s0 - R + g.jpad) * plane;  // unsigned: wraps below the array,
-  int raw_k = s0 - R;                                  // where nothing is read
-  int ring_k = s0;
-  size_t ring_off = (size_t)ring(max(s0, 0), zb, nzc) * nplane;
-  int to_wrap = nzc - (zb + max(s0, 0)) % nzc;
-  auto next_raw = [&]() -> double {
-    double v = 0.;
-    if (raw_in && raw_k >= -g.jpad && raw_k < nzc + g.jpad)
-      v = raw[APRL_BOUNDED(g.status, raw_off + row, j_count(g, c), 33 + c)];
-    raw_off += plane;
-    ++raw_k;
-    return v;
-  };
-  auto next_ring = [&]() {  // on to the ring's next plane
-    if (ring_k++ < 0) return;
-    ring_off += nplane;
-    if (--to_wrap == 0) {
-      ring_off -= (size_t)nzc * nplane;
-      to_wrap = nzc;
-    }
-  };
-  auto next_sum = [&]() -> double {
-    double v = 0.;
-    if (inside && ring_k >= 0 && ring_k < nzc)
-      v = sum[APRL_BOUNDED(g.status, ring_off + node, e_count(g, c), 36 + c)];
-    next_ring();
-    return v;
-  };
-  if constexpr (kRaw) {
-#pragma unroll
-    for (int t = -R; t < R; ++t) {
-      double v = next_raw();
-      if constexpr (S == 0) v = lane_filter(v);
-      wj.push(v);
-    }
-  }
-  size_t out_off = kOrbit ? (size_t)(k0 + g.jpad) * plane : (size_t)k0 * nplane;
-  // The next plane's reads are issued before this plane's arithmetic.
-  double raw_ahead = kRaw ? next_raw() : 0.;
-  double sum_ahead = kOrbit ? next_sum() : 0.;
-  for (int k = s0; k < s1; ++k) {
-    double v = raw_ahead;
-    double s = sum_ahead;
-    if (k + 1 < s1) {
-      if constexpr (kRaw) raw_ahead = next_raw();
-      if constexpr (kOrbit) sum_ahead = next_sum();
-    }
-    double current = 0.;
-    if constexpr (kRaw) {
-      if constexpr (S == 0) v = lane_filter(v);
-      wj.push(v);
-      current = wj.value();
-    }
-    const bool masked = column && k >= zlo && k <= zhi;
-    if constexpr (MODE == kFilterCommit) {
-      if (writes && masked && current != 0.)
-        star[APRL_BOUNDED(g.status, ring_off + node, e_count(g, c), 39 + c)] += g.jcoef * current;
-      next_ring();
-    } else if constexpr (MODE == kFilterCurrent) {
-      if (writes) static_cast<double*>(out)[out_off + node] = current;
-      out_off += nplane;
-    } else {
-      if (masked && current != 0.) s += g.jcoef * current;
-      if constexpr (S == 0) s = lane_filter(s);
-      ws.push(s);
-      if (k - R >= k0) {
-        if (writes)
-          static_cast<W*>(out)[APRL_BOUNDED(g.status, out_off + row, j_count(g, c), 42 + c)] =
-              W(ws.value());
-        out_off += plane;
-      }
-    }
-  }
+  FilterMarch m;
+  m.plane = nyc * (nxc + 2);
+  m.nplane = nyc * nxc;
+  m.row = j * (nxc + 2) + (i + 1);
+  m.node = j * nxc + i;
+  m.nzc = nzc;
+  m.zb = zb;
+  m.zlo = zlo;
+  m.zhi = zhi;
+  m.inside = inside;
+  m.raw_in = raw_in;
+  m.writes = writes;
+  m.column = column;
+  m.raw = raw;
+  m.sum = sum;
+  m.star = star;
+  m.out = out;
+  // A march whose planes are all inside every array tests no plane number.
+  if (s0 - R >= 0 && s1 + R <= nzc && s0 >= zlo && s1 - 1 <= zhi)
+    filter_march<S, MODE, W, true>(g, m, c, k0, s0, s1);
+  else
+    filter_march<S, MODE, W, false>(g, m, c, k0, s0, s1);
 }
 
 // The x-z filtered B of the linear-binomial3 gathers, one pass per step:
@@ -616,18 +687,17 @@ __global__ void magnetic_filter_kernel(BFilterArgs a) {
   const int k0 = -1 + (int)(blockIdx.z % a.chunks) * a.planes;
   const int k1 = min(k0 + a.planes, nzc + 1);
   if (k0 >= k1) return;
-  const size_t nplane = (size_t)nyc * nxc, plane = (size_t)nyc * (nxc + 2);
+  const unsigned nplane = nyc * nxc, plane = nyc * (nxc + 2);
   const int node = j * nxc + ic, row = j * (nxc + 2) + (i + 1);
   auto at = [&](int k) -> double {
     const int kc = min(max(k, 0), nzc - 1);
-    return b[APRL_BOUNDED(g.status, (size_t)ring(kc, zb, nzc) * nplane + node, b_count(g, c),
-                          45 + c)];
+    return b[APRL_BOUNDED(g.status, ring(kc, zb, nzc) * nplane + node, b_count(g, c), 45 + c)];
   };
   ZWindow<0> w;
   w.clear();
   w.push(lane_filter(at(k0 - 1)));
   w.push(lane_filter(at(k0)));
-  W* to = out + (size_t)(k0 + 1) * plane + row;
+  W* to = out + (unsigned)((k0 + 1) * plane + row);
   // Four planes' reads are issued together (one at a time left too few bytes
   // in flight: 0.117 against 0.100 ms on the 128x128x512 grid).
   constexpr int U = 4;

@@ -48,6 +48,7 @@ struct CowanArgs {
   const double* e[3];    // E^n (ring)
   const double* lower[3];  // inlet lower halo planes
   double alpha[3], beta[3], delta_xy, delta_yz, delta_zx;
+  double dtdx, dtdy, dtdz;
   CpmlAxis mx, my;       // magnetic profiles (half-integer positions)
   CpmlHistory h[4];      // magnetic histories 0 (Bx,y) 3 (By,x) 4 (Bz,x) 5 (Bz,y)
   int chunk;             // z planes marched by one block
@@ -63,6 +64,8 @@ struct PreviewArgs {
   // When set: the current-free orbit sum S0 = E* + E^n (ring layout of E),
   // written here from the values already in hand.
   double* sum[3];
+  double cx, cy, cz;     // dt/(mu0 eps0) over dx, dy, dz
+  int chunk;             // z planes marched by one thread
 };
 
 // ChargeMatchedInlet::complete (src/charge_matched_inlet.h:55-71): Ez of the
@@ -112,10 +115,13 @@ struct DetectorArgs {
 // Cowan kernel geometry: 32x8 column tiles, each block marching up to
 // kCowanChunk z planes (fewer on small grids, so that there are enough
 // blocks); APRL_COWAN_MIN_BLOCKS resident blocks per SM bound its registers.
-// Measured on the 128x128x512 dipole grid: 8 planes at 6 blocks per SM,
-// 0.47 ms, against 0.50 (16 at 5), 0.49 (16 at 6), 0.56-0.58 (32) and 0.47
-// (4 at 6): more, shorter marches hide the plane loads better than the two
-// halo planes per chunk cost.
+// Bound by instruction issue and the shared-memory reads of the smoothing, not
+// by memory (604 MB, 0.09 ms at the copy rate).  On the 128x128x512 dipole grid
+// a launch took 0.430 ms while every tile value went through the parity rules
+// and 64-bit offsets; with the rules mapped once a march (TileMap) 0.331 ms at
+// 6 blocks per SM, 0.336 at 5, 0.355 at 4.  8 planes a march: 16, 32 and 4
+// were slower or equal (more, shorter marches hide the plane loads better
+// than the two halo planes per chunk cost).
 #ifndef APRL_COWAN_CHUNK
 #define APRL_COWAN_CHUNK 8
 #endif

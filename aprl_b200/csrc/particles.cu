@@ -80,6 +80,41 @@ __device__ __forceinline__ void binomial_xz_segment(const GridT<G>& g, const dou
     }
 }
 
+// A visitor's unchecked view of the nodes around a cell whose whole narrow
+// stencil lies inside the padded arrays: the range tests and the index of
+// every visit, which were most of a walk's instructions, become one test and
+// one base offset per component.
+template <class V>
+struct Near {
+  using Weight = typename V::Weight;
+  V* v;
+  unsigned base[3], plane[3], pitch[3];
+  long long i0, j0, k0;
+  __device__ __forceinline__ Near(V& visit, long long i, long long j, long long k)
+      : v(&visit), i0(i), j0(j), k0(k) {
+    const auto& g = *visit.g;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      pitch[d] = g.nx + (d != 0) + 2;
+      plane[d] = (g.ny + (d != 1)) * pitch[d];
+      base[d] = (unsigned)(k + g.jpad) * plane[d] + (unsigned)j * pitch[d] + (unsigned)(i + 1);
+    }
+  }
+  __device__ __forceinline__ void operator()(int d, long long i, long long j, long long k,
+                                             Weight w) {
+    v->at(d, base[d] + (unsigned)(k - k0) * plane[d] + (unsigned)(j - j0) * pitch[d] +
+                 (unsigned)(i - i0), w);
+  }
+};
+
+// Whether the nodes i .. i+1, j .. j+1, k .. k+above are inside every
+// component's padded array.
+template <class G>
+__device__ __forceinline__ bool near_inside(const GridT<G>& g, long long i, long long j,
+                                            long long k, int above) {
+  return i >= 0 && i < g.nx && j >= 0 && j < g.ny && k >= -g.jpad && k + above < g.nz + g.jpad;
+}
+
 // The narrow weights of binomialXZSegment: with wx = lx * [1/4, 1/2, 1/4] and
 // slope = (-1, 1) * [1/4, 1/2, 1/4] (convolutions), the 4x2x4 stencil's
 // weights are those of this 12-node one -- linear along the two axes across
@@ -102,14 +137,25 @@ __device__ __forceinline__ void binomial_linear_segment(const GridT<G>& g, const
   const F xy = curvature * F(d[0]) * F(d[1]);
   const F xz = curvature * F(d[0]) * F(d[2]);
   const F yz = curvature * F(d[1]) * F(d[2]);
+  auto walk = [&](auto& to) {
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      visit(0, i, j + b, k + c, width * (ly[b] * lz[c] + (b == c ? yz : -yz)));
-      visit(1, i + b, j, k + c, width * (lx[b] * lz[c] + (b == c ? xz : -xz)));
-      visit(2, i + b, j + c, k, width * (lx[b] * ly[c] + (b == c ? xy : -xy)));
+      for (int b = 0; b < 2; ++b) {
+        to(0, i, j + b, k + c, width * (ly[b] * lz[c] + (b == c ? yz : -yz)));
+        to(1, i + b, j, k + c, width * (lx[b] * lz[c] + (b == c ? xz : -xz)));
+        to(2, i + b, j + c, k, width * (lx[b] * ly[c] + (b == c ? xy : -xy)));
+      }
+  };
+  if constexpr (!V::kOwnSegment) {
+    if (near_inside(g, i, j, k, 1)) {
+      visit.touch((int)i, (int)j);
+      Near<V> near(visit, i, j, k);
+      walk(near);
+      return;
     }
+  }
+  walk(visit);
 }
 
 // B-spline values on f = z - floor(z): degree 4 (the edge basis, n[0..4]) and
@@ -123,8 +169,19 @@ __device__ __forceinline__ void spline_edge(F f, F n[6]) {
   for (unsigned j = 1; j <= 4; ++j) quintic_spline_level(n, f, j);
 }
 
+// The four-point Gauss rule on a piece [lower, upper]: parameter and weight of
+// point t.
+__device__ __forceinline__ double quintic_point(double lower, double upper, int t) {
+  const double q[4] = {-.8611363115940525752, -.3399810435848562648,
+                       .3399810435848562648, .8611363115940525752};
+  return .5 * (upper + lower + (upper - lower) * q[t]);
+}
+__device__ __forceinline__ double quintic_factor(double width, int t) {
+  return .5 * width * (t == 0 || t == 3 ? .3478548451374538574 : .6521451548625461426);
+}
+
 // One Gauss point at parameter u of the chord, weighted by `factor`, visited
-// on its own (the rare piece whose points straddle a cell).
+// on its own.
 template <class G, class V>
 __device__ __noinline__ void quintic_linear_point(const GridT<G>& g, const double x[3],
                                                   const double v[3], double u,
@@ -161,7 +218,8 @@ __device__ __noinline__ void quintic_linear_point(const GridT<G>& g, const doubl
 // piece reaches 6 z nodes of Jx and Jy and 5 of Jz.  Every Gauss point of a
 // cut piece lies in the same cell, so the four points' weights are summed per
 // node first and each node visited once.  A piece whose Gauss points straddle
-// a cell (only possible through rounding at a cut) is visited point by point.
+// a cell (only possible through rounding at a cut), or whose nodes leave the
+// padded arrays, is visited point by point.
 template <class G, class V>
 __device__ __forceinline__ void quintic_linear_segment(const GridT<G>& g, const double x[3],
                                                        const double v[3], double lower,
@@ -193,7 +251,7 @@ __device__ __forceinline__ void quintic_linear_segment(const GridT<G>& g, const 
     }
     same = same && it == i && jt == j && kt == k;
   }
-  if (!same) {
+  if (!same || !near_inside(g, i, j, k - 2, 5)) {
     V copy = visit;  // the call takes an address; the visitor itself stays in registers
 #pragma unroll 1
     for (int t = 0; t < 4; ++t)
@@ -202,47 +260,52 @@ __device__ __forceinline__ void quintic_linear_segment(const GridT<G>& g, const 
     visit = copy;
     return;
   }
-  F n[4][6];
+  auto walk = [&](auto& to) {
+    F n[4][6];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) spline_edge(fz[t], n[t]);
-  // Jz at (i + a, j + c): edge basis, 5 nodes.
+    for (int t = 0; t < 4; ++t) spline_edge(fz[t], n[t]);
+    // Jz at (i + a, j + c): edge basis, 5 nodes.
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
+    for (int m = 0; m < 5; ++m) {
+      F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const F w = factor[t] * n[t][m];
-      const F wx = w * fx[t], wo = w * (F(1.) - fx[t]);
-      acc[0] += wo * (F(1.) - fy[t]);
-      acc[1] += wx * (F(1.) - fy[t]);
-      acc[2] += wo * fy[t];
-      acc[3] += wx * fy[t];
+      for (int t = 0; t < 4; ++t) {
+        const F w = factor[t] * n[t][m];
+        const F wx = w * fx[t], wo = w * (F(1.) - fx[t]);
+        acc[0] += wo * (F(1.) - fy[t]);
+        acc[1] += wx * (F(1.) - fy[t]);
+        acc[2] += wo * fy[t];
+        acc[3] += wx * fy[t];
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int a = 0; a < 2; ++a) to(2, i + a, j + c, k - 2 + m, acc[2 * c + a]);
     }
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
+    for (int t = 0; t < 4; ++t) quintic_spline_level(n[t], fz[t], 5);
+    // Jx at (i, j + c) and Jy at (i + c, j): node basis, 6 nodes.
 #pragma unroll
-      for (int a = 0; a < 2; ++a) visit(2, i + a, j + c, k - 2 + m, acc[2 * c + a]);
-  }
+    for (int m = 0; m < 6; ++m) {
+      F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
 #pragma unroll
-  for (int t = 0; t < 4; ++t) quintic_spline_level(n[t], fz[t], 5);
-  // Jx at (i, j + c) and Jy at (i + c, j): node basis, 6 nodes.
+      for (int t = 0; t < 4; ++t) {
+        const F w = factor[t] * n[t][m];
+        acc[0] += w * (F(1.) - fy[t]);
+        acc[1] += w * fy[t];
+        acc[2] += w * (F(1.) - fx[t]);
+        acc[3] += w * fx[t];
+      }
 #pragma unroll
-  for (int m = 0; m < 6; ++m) {
-    F acc[4] = {F(0.), F(0.), F(0.), F(0.)};
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const F w = factor[t] * n[t][m];
-      acc[0] += w * (F(1.) - fy[t]);
-      acc[1] += w * fy[t];
-      acc[2] += w * (F(1.) - fx[t]);
-      acc[3] += w * fx[t];
+      for (int c = 0; c < 2; ++c) {
+        to(0, i, j + c, k - 2 + m, acc[c]);
+        to(1, i + c, j, k - 2 + m, acc[2 + c]);
+      }
     }
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      visit(0, i, j + c, k - 2 + m, acc[c]);
-      visit(1, i + c, j, k - 2 + m, acc[2 + c]);
-    }
-  }
+  };
+  visit.touch((int)i, (int)j);
+  Near<V> near(visit, i, j, k - 2);
+  walk(near);
 }
 
 // longitudinal_shape::weights (src/longitudinal_shape.h:97-117) with
@@ -390,7 +453,7 @@ __device__ __forceinline__ bool clip_open_orbit(const GridT<F>& g, const double 
 }
 
 // Orbit average of 1/2 (E_new + E^n) with the shape weights, read from the
-// orbit sum S = E_new + E^n that orbit_sum_kernel forms once per trial
+// orbit sum S = E_new + E^n that the orbit filter forms once per trial
 // (E_new = E* - dt/eps0 J for the residual, E* for the first-trial guess).
 // Three component arrays passed by value, so that constant component
 // indices keep the pointers in registers.
@@ -451,9 +514,11 @@ struct FilteredVisitor {
     if (k < -G.jpad || k >= e_nz(G, d) + G.jpad) return;
     r[d] += W(.5) * w * s.p[d][j_index(G, d, (int)i, (int)j, (int)k)];
   }
-  __device__ __forceinline__ W at(int d, size_t n) const {
+  __device__ __forceinline__ W at(int d, unsigned n) const {
     return s.p[d][APRL_BOUNDED(g->status, n, j_count(*g, d), 24 + d)];
   }
+  __device__ __forceinline__ void at(int d, unsigned n, W w) { r[d] = fma(W(.5) * w, at(d, n), r[d]); }
+  __device__ __forceinline__ void touch(int, int) const {}
   // One linear-binomial3 piece.  12 reads; in the 4x2x4 form it was 64 and
   // the reads' latency bound the kernel.
   __device__ __forceinline__ void segment(const GridT<F>& G, const double s0[3],
@@ -474,11 +539,11 @@ struct FilteredVisitor {
     const W xy = curvature * W(d[0]) * W(d[1]);
     const W xz = curvature * W(d[0]) * W(d[2]);
     const W yz = curvature * W(d[1]) * W(d[2]);
-    const size_t p0 = (size_t)G.nx + 2, p1 = p0 + 1;  // row pitches of Ex and of Ey, Ez
-    const size_t n0 = ((size_t)(k + G.jpad) * (G.ny + 1) + j) * p0 + (i + 1);
-    const size_t n1 = ((size_t)(k + G.jpad) * G.ny + j) * p1 + (i + 1);
-    const size_t n2 = ((size_t)(k + G.jpad) * (G.ny + 1) + j) * p1 + (i + 1);
-    const size_t z0 = p0 * (G.ny + 1), z1 = p1 * G.ny;
+    const unsigned p0 = G.nx + 2, p1 = p0 + 1;  // row pitches of Ex and of Ey, Ez
+    const unsigned n0 = ((k + G.jpad) * (G.ny + 1) + j) * p0 + (i + 1);
+    const unsigned n1 = ((k + G.jpad) * G.ny + j) * p1 + (i + 1);
+    const unsigned n2 = ((k + G.jpad) * (G.ny + 1) + j) * p1 + (i + 1);
+    const unsigned z0 = p0 * (G.ny + 1), z1 = p1 * G.ny;
     W e0[4], e1[4], e2[4];
 #pragma unroll
     for (int c = 0; c < 2; ++c)
@@ -521,7 +586,7 @@ struct DirectVisitor {
   }
 
   // One accumulation .5*w*(E_new + E^n) at the ring offset n of a node.
-  __device__ __forceinline__ W term(int d, size_t n, W w) const {
+  __device__ __forceinline__ W term(int d, unsigned n, W w) const {
     return W(.5) * w * W(s.p[d][APRL_BOUNDED(g->status, n, e_count(*g, d), 24 + d)]);
   }
 
@@ -561,11 +626,11 @@ struct DirectVisitor {
       const int nxc = G.nx, nyc = G.ny + 1, nzc = G.nz + 1;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const size_t plane = (size_t)ring(K - 1 + c, G.zb_e[0], nzc) * nyc;
+        const unsigned plane = ring(K - 1 + c, G.zb_e[0], nzc) * nyc;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
           const W weight = width * (wy[b] * wz[c] + yz * sy[b] * slope[c]);
-          const size_t n0 = (plane + J + b) * nxc + (I - 1);
+          const unsigned n0 = (plane + J + b) * nxc + (I - 1);
 #pragma unroll
           for (int a = 0; a < 3; ++a) r[0] += term(0, n0 + a, weight * edge[a]);
         }
@@ -576,7 +641,7 @@ struct DirectVisitor {
       const int nxc = G.nx + 1, nyc = G.ny, nzc = G.nz + 1;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const size_t n0 = ((size_t)ring(K - 1 + c, G.zb_e[1], nzc) * nyc + J) * nxc + (I - 1);
+        const unsigned n0 = (ring(K - 1 + c, G.zb_e[1], nzc) * nyc + J) * (unsigned)nxc + (I - 1);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
           r[1] += term(1, n0 + a, width * (wx[a] * wz[c] + xz * slope[a] * slope[c]));
@@ -585,9 +650,9 @@ struct DirectVisitor {
     // Ez (nx+1, ny+1, nz): nodes x I-1..I+2, y J..J+1, z K-1..K+1
     {
       const int nxc = G.nx + 1, nyc = G.ny + 1, nzc = G.nz;
-      size_t plane[3];
+      unsigned plane[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) plane[c] = (size_t)ring(K - 1 + c, G.zb_e[2], nzc) * nyc;
+      for (int c = 0; c < 3; ++c) plane[c] = ring(K - 1 + c, G.zb_e[2], nzc) * nyc;
 #pragma unroll
       for (int b = 0; b < 2; ++b)
 #pragma unroll
@@ -640,10 +705,10 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const do
       const double* base = g.b[a];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const size_t plane = (size_t)ring((int)cell[2] - 1 + k, g.zb_b[a], (int)nzc) * nyc;
+        const unsigned plane = ring((int)cell[2] - 1 + k, g.zb_b[a], (int)nzc) * (int)nyc;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const size_t row = (plane + cell[1] + j) * nxc + (cell[0] - 1);
+          const unsigned row = (plane + (int)cell[1] + j) * (int)nxc + ((int)cell[0] - 1);
           W r = W(0.);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -816,6 +881,23 @@ struct DepositVisitor {
   F scale[3];
   bool smooth_x;
   unsigned error;
+  __device__ __forceinline__ void at(int a, unsigned n, F w) {
+    if (scale[a] == F(0.)) return;
+    n = APRL_BOUNDED(g->status, n, j_count(*g, a), 48 + a);
+    if constexpr (Q) {
+      // Order-free integer sum, converted to J once per trial.
+      if (!fixed_add(g->jq[a] + 2 * (size_t)n, double(scale[a] * w), g->jq_scale))
+        error = kErrFixedRange;
+    } else {
+      atomicAdd(&g->j[a][n], scale[a] * w);
+    }
+  }
+  __device__ __forceinline__ void touch(int i, int j) const {
+    mark_column(*g, i, j);
+    mark_column(*g, i, j + 1);
+    mark_column(*g, i + 1, j);
+    mark_column(*g, i + 1, j + 1);
+  }
   __device__ __forceinline__ void operator()(int a, long long i, long long j, long long k, F w) {
     if (scale[a] == F(0.)) return;
     const GridT<F>& G = *g;
@@ -830,14 +912,8 @@ struct DepositVisitor {
       return;
     }
     if (k < -G.jpad || k >= e_nz(G, a) + G.jpad) return;
-    const size_t at = j_index(G, a, (int)i, (int)j, (int)k);
     mark_column(G, (int)i, (int)j);
-    if constexpr (Q) {
-      // Order-free integer sum, converted to J once per trial.
-      if (!fixed_add(G.jq[a] + 2 * at, double(scale[a] * w), G.jq_scale)) error = kErrFixedRange;
-    } else {
-      atomicAdd(&G.j[a][at], scale[a] * w);
-    }
+    at(a, j_index(G, a, (int)i, (int)j, (int)k), w);
   }
 };
 
@@ -1321,7 +1397,7 @@ __device__ __forceinline__ SlotPlan plan_slot(const GridT<F>& g, const DFrame& f
 // before any current of the trial is deposited; the push reads them as the
 // previous residual's fields.
 template <class W, class F, int S, bool D>
-__global__ void APRL_GATHER_BOUNDS guess_gather_kernel(const __grid_constant__ PushArgs<F> a) {
+__global__ void APRL_GATHER_BOUNDS(S) guess_gather_kernel(const __grid_constant__ PushArgs<F> a) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
   const double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
@@ -1582,11 +1658,11 @@ __device__ __forceinline__ double run_sum(double v, int lane, int head, unsigned
 }
 
 template <bool Q>
-__device__ __forceinline__ void chord_add(const DGrid& g, int a, size_t at, double v,
+__device__ __forceinline__ void chord_add(const DGrid& g, int a, unsigned at, double v,
                                           unsigned& err) {
   at = APRL_BOUNDED(g.status, at, j_count(g, a), 30 + a);
   if constexpr (Q) {
-    if (!fixed_add(g.jq[a] + 2 * at, v, g.jq_scale)) err = kErrFixedRange;
+    if (!fixed_add(g.jq[a] + 2 * (size_t)at, v, g.jq_scale)) err = kErrFixedRange;
   } else {
     atomicAdd(&g.j[a][at], v);
   }
@@ -1719,8 +1795,8 @@ __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ C
     if (alive)
       for (int d = 0; d < 3; ++d) scale[d] = q * (e[d] - b[d]) / (g.dx * g.dy * g.dz * g.dt);
   }
-  const long long p0 = g.nx + 2, p1 = g.nx + 3;  // row pitches of Jx and of Jy, Jz
-  const long long z0 = p0 * (g.ny + 1), z1 = p1 * g.ny, z2 = p1 * (g.ny + 1);
+  const unsigned p0 = g.nx + 2, p1 = g.nx + 3;  // row pitches of Jx and of Jy, Jz
+  const unsigned z0 = p0 * (g.ny + 1), z1 = p1 * g.ny, z2 = p1 * (g.ny + 1);
   // ---- one piece per lane per round; a chord of a beam that moves about a
   // cell per step along z has two, in z-neighbouring cells.
   while (__any_sync(0xffffffffu, alive)) {
@@ -1736,7 +1812,11 @@ __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ C
       } else {  // quintic Gauss points that straddle a cell
         const double x[3] = {w.a0.x, w.a1.x, w.a2.x}, v[3] = {w.a0.v, w.a1.v, w.a2.v};
         DepositVisitor<double, Q> visit{&g, {scale[0], scale[1], scale[2]}, S == 0, kErrNone};
-        quintic_linear_segment(g, x, v, first, last, last - first, visit);
+        if constexpr (S != 0)
+#pragma unroll 1
+          for (int t = 0; t < 4; ++t)
+            quintic_linear_point(g, x, v, quintic_point(first, last, t),
+                                 quintic_factor(last - first, t), visit);
         if (visit.error) err = visit.error;
         have = false;
       }
@@ -1764,13 +1844,13 @@ __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ C
       }
     }
     constexpr int kReach = S == 0 ? 0 : 2;  // nodes below the piece's cell in z
-    const long long kz = p.k + g.jpad - kReach;
-    const long long n0 = (kz * (g.ny + 1) + p.j) * p0 + (p.i + 1);
-    const long long n1 = (kz * g.ny + p.j) * p1 + (p.i + 1);
-    const long long n2 = (kz * (g.ny + 1) + p.j) * p1 + (p.i + 1);
-    auto add = [&](int c, long long at, double v) {
+    const int kz = p.k + g.jpad - kReach;
+    const unsigned n0 = (kz * (g.ny + 1) + p.j) * p0 + (p.i + 1);
+    const unsigned n1 = (kz * g.ny + p.j) * p1 + (p.i + 1);
+    const unsigned n2 = (kz * (g.ny + 1) + p.j) * p1 + (p.i + 1);
+    auto add = [&](int c, unsigned at, double v) {
       const double total = run_sum(v, lane, runs.head, runs.span);
-      if (adds && total != 0.) chord_add<Q>(g, c, (size_t)at, total, err);
+      if (adds && total != 0.) chord_add<Q>(g, c, at, total, err);
     };
     if constexpr (S == 0) {
       double v[4];
@@ -1891,7 +1971,7 @@ __device__ __forceinline__ void trial_verdict(unsigned long long force_bits, dou
 }
 
 template <class W, class F, int S, bool DB>
-__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ ResidualArgs<F> a) {
+__global__ void APRL_RESIDUAL_BOUNDS(S) residual_kernel(const __grid_constant__ ResidualArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double force = 0.0, defect = 0.0, scale = 0.0;
@@ -2436,7 +2516,7 @@ __global__ void inlet_charge_kernel(InletMatchArgs a) {
 
 // fn(c, offset) for every node of the raw current's marked columns; a warp
 // takes 32 x nodes of one row and `kMarkPlanes` planes at a time.
-constexpr int kMarkPlanes = 32;
+constexpr int kMarkPlanes = 16;
 template <class Fn>
 __device__ __forceinline__ void marked_nodes(const GridT<double>& g, Fn fn) {
   const int lane = threadIdx.x & 31;
@@ -2453,7 +2533,9 @@ __device__ __forceinline__ void marked_nodes(const GridT<double>& g, Fn fn) {
     const int last = min((chunk + 1) * kMarkPlanes, e_nz(g, c) + 2 * g.jpad);
     const size_t plane = (size_t)e_ny(g, c) * (e_nx(g, c) + 2);
     size_t at = (size_t)(chunk * kMarkPlanes) * plane + (size_t)j * (e_nx(g, c) + 2) + (i + 1);
-    for (int k = chunk * kMarkPlanes; k < last; ++k, at += plane) fn(c, at);
+#pragma unroll
+    for (int k = 0; k < kMarkPlanes; ++k)
+      if (chunk * kMarkPlanes + k < last) fn(c, at + k * plane);
   }
 }
 

@@ -187,14 +187,12 @@ struct ChordArgs {
 
 // Occupancy knobs of the hot particle kernels (blocks of 128 threads
 // that must fit one SM; 0 leaves the register count to the compiler).
-// Measured on the 128x128x512 dipole grid with 1M particles, with the
-// kernels built per shape: push_deposit at 6 blocks (80 registers) beats 5,
-// 7 and 8 on the binomial3, FP32-mixed and drift workloads and ties on
-// quintic (binomial3 launch 0.133 -> 0.120 ms against 8 blocks, whose
-// 64 registers spilled; with the main chords still deposited inside it, 8
-// had been best); the residual and the guess gather at 6 blocks (80
-// registers) beat 4, 5, 7 and 8 (dipole step 4.47 -> 4.44 ms, FP32-mixed
-// 3.44 -> 3.35 ms, quintic 15.99 -> 15.62 ms).
+// 6 blocks (80 registers) were best for push_deposit, the residual and the
+// guess gather among 4, 5, 6, 7 and 8 on the 128x128x512 dipole grid with 1M
+// particles while they read the wide stencils (8 blocks' 64 registers spill).
+// With the narrow stencils a launch takes there: push_deposit 0.078 ms (0.120
+// while it deposited the boundary events' pieces itself), residual 0.104
+// (0.296 with the wide stencils), guess gather 0.068 (0.231).
 #ifndef APRL_PUSH_MIN_BLOCKS
 #define APRL_PUSH_MIN_BLOCKS 6
 #endif
@@ -204,9 +202,9 @@ struct ChordArgs {
 #ifndef APRL_GATHER_MIN_BLOCKS
 #define APRL_GATHER_MIN_BLOCKS 6
 #endif
-// chord_deposit is left to the compiler (96 registers, 5 blocks): at 6 or 8
-// blocks it was unchanged; at 4 (118 registers) the dipole launch went
-// 0.307 -> 0.302 ms but the drift one 0.048 -> 0.049 ms.
+// chord_deposit is left to the compiler.  It is bound by the L2's reductions:
+// the wide stencils' 64 a piece took 0.307 ms a launch on the dipole grid,
+// the narrow 12 take 0.114.
 #ifndef APRL_CHORD_MIN_BLOCKS
 #define APRL_CHORD_MIN_BLOCKS 0
 #endif
@@ -215,22 +213,22 @@ struct ChordArgs {
 #else
 #define APRL_CHORD_BOUNDS __launch_bounds__(128)
 #endif
-#if APRL_GATHER_MIN_BLOCKS > 0
-#define APRL_GATHER_BOUNDS __launch_bounds__(128, APRL_GATHER_MIN_BLOCKS)
-#else
-#define APRL_GATHER_BOUNDS
+// The quintic gathers keep 24 spline values: 4 blocks (128 registers).  With
+// that, and with the visits' range tests made once a particle (Near), the
+// residual of 265k particles takes 0.106 ms (0.269 before), the guess gather
+// 0.091 (0.260).
+#ifndef APRL_QUINTIC_MIN_BLOCKS
+#define APRL_QUINTIC_MIN_BLOCKS 4
 #endif
+#define APRL_GATHER_BOUNDS(S) \
+  __launch_bounds__(128, (S) == 0 ? APRL_GATHER_MIN_BLOCKS : APRL_QUINTIC_MIN_BLOCKS)
+#define APRL_RESIDUAL_BOUNDS(S) \
+  __launch_bounds__(128, (S) == 0 ? APRL_RESIDUAL_MIN_BLOCKS : APRL_QUINTIC_MIN_BLOCKS)
 #if APRL_PUSH_MIN_BLOCKS > 0
 #define APRL_PUSH_BOUNDS __launch_bounds__(128, APRL_PUSH_MIN_BLOCKS)
 #else
 #define APRL_PUSH_BOUNDS
 #endif
-#if APRL_RESIDUAL_MIN_BLOCKS > 0
-#define APRL_RESIDUAL_BOUNDS __launch_bounds__(128, APRL_RESIDUAL_MIN_BLOCKS)
-#else
-#define APRL_RESIDUAL_BOUNDS
-#endif
-
 // W: arithmetic of the gathers (double, or float in the FP32-mixed mode).
 // S: the particle shape, 0 linear-binomial3, 1 quintic-compensated.
 // D, DB: read the wide stencils directly (linear-binomial3, sparse runs).
@@ -243,7 +241,7 @@ template <class F, int S, bool Q> __global__ void carrier_kernel(const __grid_co
 template <int S, bool Q>
 __global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ ChordArgs a);
 template <class W, class F, int S, bool DB>
-__global__ void APRL_RESIDUAL_BOUNDS residual_kernel(const __grid_constant__ ResidualArgs<F> a);
+__global__ void APRL_RESIDUAL_BOUNDS(S) residual_kernel(const __grid_constant__ ResidualArgs<F> a);
 
 // RelativisticBorisPusher::push of `count` particles (SoA, in place) with
 // per-particle E and B (3 values each).

@@ -1723,12 +1723,11 @@ aprl_status advance_magnetic_t(aprl_run* r) {
   ca.mx = r->mprof[0].view();
   ca.my = r->mprof[1].view();
   for (int h = 0; h < 4; ++h) ca.h[h] = r->hist[h].view();
-  // Column tiles marching z chunks (fields.cuh: kCowanTileX/Y, kCowanChunk):
-  // at most kCowanChunk planes per block, fewer when that leaves fewer than
-  // about four blocks per SM.
+  ca.dtdx = c.dt / c.dx;
+  ca.dtdy = c.dt / c.dy;
+  ca.dtdz = c.dt / c.dz;
+  // Column tiles marching z chunks (fields.cuh: kCowanTileX/Y).
   const dim3 cblock(kCowanTileX, kCowanTileY);
-  const unsigned columns = blocks_for(c.nx + 1, kCowanTileX) * blocks_for(c.ny + 1, kCowanTileY);
-  (void)columns;
   const size_t planes = c.nz + 1;
   TuneLaunch tl;
   TRY(tune_begin(r, kTuneCowan, tl));
@@ -1746,11 +1745,15 @@ aprl_status do_advance_magnetic(aprl_run* r) {
 }
 
 // Whether this step's linear-binomial3 gathers read the filtered B and, in
-// the first trial, the filtered current-free sum.  The two grid passes cost
-// about 28 B of traffic a cell; the wide stencils cost a particle some 220
-// reads more.  Below one particle per 16 cells the direct reads are the
-// cheaper side.  The quintic shape always gathers from the filtered sum.  A run that cannot have
-// the filtered B's memory reads the wide stencils.
+// the first trial, the filtered current-free sum.  The two grid passes move
+// 96 B a cell: 0.165 ms a step on the 128x128x512 grid.  There the first-trial
+// gather takes 0.088 ms for 289k particles with the wide stencils and 0.068 ms
+// for 962k with the narrow ones, and the residual 0.22 ns a particle and trial
+// against 0.11, so the sides cross at one particle per 20 to 30 cells,
+// depending on the trials.  16 keeps what is near the crossing on the direct
+// reads, which need no memory of their own.  The quintic shape always gathers
+// from the filtered sum.  A run that cannot have the filtered B's memory reads
+// the wide stencils.
 constexpr size_t kDenseCells = 16;
 
 bool dense_gathers(aprl_run* r) {
@@ -1822,7 +1825,17 @@ aprl_status preview_electric_t(aprl_run* r) {
   TuneLaunch tl;
   TRY(tune_begin(r, kTunePreview, tl));
   const dim3 block = kGridBlocks[tl.candidate];
-  TRY(launch(r, kElectricPreview, electric_preview_kernel<F>, grid3(c, block), block, pa));
+  const double curl = c.dt / (kMu0 * kEpsilon0);
+  pa.cx = curl / c.dx;
+  pa.cy = curl / c.dy;
+  pa.cz = curl / c.dz;
+  // Planes per thread: two, one when that leaves fewer than about eight
+  // blocks an SM.
+  dim3 pgrid = grid3(c, block);
+  pa.chunk = 2;
+  while (pa.chunk > 1 && (size_t)pgrid.x * pgrid.y * (c.nz / pa.chunk) < 148 * 8) pa.chunk /= 2;
+  pgrid.z = blocks_for(c.nz + 1, (unsigned)pa.chunk);
+  TRY(launch(r, kElectricPreview, electric_preview_kernel<F>, pgrid, block, pa));
   TRY(tune_end(r, tl));
   r->dense = dense_gathers(r);
   if (r->dense && c.shape == APRL_SHAPE_LINEAR_BINOMIAL3) {  // B is final for the step
@@ -2650,7 +2663,11 @@ aprl_status aprl_run_create(const aprl_run_config* config, void* stream, aprl_ru
   std::memset(r->pinned, 0, kPinnedBlock);
   r->h_block = static_cast<TrialBlock*>(r->pinned);
   r->h_status = &r->h_block->status;
-  if (cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking) != cudaSuccess ||
+  // The side stream's kernels are short and few: let them start ahead of the
+  // blocks of the kernel they run beside, or they end long after it.
+  int low = 0, high = 0;
+  if (cudaDeviceGetStreamPriorityRange(&low, &high) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&r->side, cudaStreamNonBlocking, high) != cudaSuccess ||
       cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming) != cudaSuccess)
     return cleanup(fail(APRL_ERR_CUDA, "side stream creation failed"));
