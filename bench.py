@@ -196,18 +196,20 @@ def algorithmic_bytes(kernel, cfg, particles, carriers):
         return 9 * 8 * n_cells
     if kernel == "electric_preview":    # read 3 E^n and 3 B, write 3 E* and, with particles
         return (12 if particles else 9) * 8 * n_cells   # in the window, the orbit sum E* + E^n
-    if kernel == "electric_commit":     # read J; E* += -dt/eps0 J only where J != 0
+    if kernel == "electric_commit":     # read the raw current; E* += -dt/eps0 J only where J != 0
         return 3 * 8 * n_cells          # (that part depends on the bunch; not counted)
-    if kernel == "push_deposit":        # read x,u,q,m,nextE/B; write x1,u1,usedE/B,work,flags,
-        return particles * (64 + 48 + 48 + 48 + 8 + 2 + 49)   # and the chord (b, e, mode)
-    if kernel == "chord_deposit":       # read the chord (b, e), q, mode; J updates are L2 reductions
+    if kernel == "push_deposit":        # read x,u,q,m,frozen,usedE/B; write x1,u1,work,flags
+        return particles * (64 + 1 + 48 + 48 + 8 + 5)
+    if kernel == "chord_deposit":       # read the chord (x0, x1), q, flag; J updates are L2 reductions
         return particles * (48 + 8 + 1)
     if kernel == "residual":            # read x0,x1,q,m,usedE/B,work; write nextE/B
         return particles * (48 + 16 + 48 + 8 + 48)
     if kernel == "guess_gather":        # read x,u,flags; write nextE/B
         return particles * (48 + 1 + 48)
-    if kernel == "orbit_sum":           # read E*, J, E^n; write S, per E node
-        return 4 * 8 * 3 * n_cells
+    if kernel == "orbit_filter":        # the columns the bunch's deposits marked: their share of
+        return None                     # the grid is not known here
+    if kernel == "magnetic_filter":     # read B, write the filtered B
+        return 2 * 8 * 3 * n_cells
     if kernel == "carrier":             # read + write 8 words
         return carriers * 128
     return None
@@ -219,19 +221,19 @@ def algorithmic_bytes(kernel, cfg, particles, carriers):
 # passes move the same bytes for any bunch on this grid; the particle
 # kernels' traffic is mostly the fields over the bunch's region, which does
 # not grow with the particle count, so they have a figure only at 1M.
-GRID_TRAFFIC = {"cowan_magnetic": 669_778_944, "orbit_sum": 791_749_632,
-                "electric_preview": 845_800_448, "electric_commit": 280_096_512}
-PARTICLE_TRAFFIC = {"chord_deposit": 118_682_624, "push_deposit": 252_511_232,
-                    "residual": 287_908_096, "guess_gather": 191_039_744}
+GRID_TRAFFIC = {"cowan_magnetic": 682_828_544, "electric_preview": 842_188_288,
+                "magnetic_filter": 370_274_816}
+PARTICLE_TRAFFIC = {"chord_deposit": 100_710_656, "push_deposit": 148_692_992,
+                    "residual": 246_043_136, "guess_gather": 169_076_992,
+                    "orbit_filter": 203_790_848}
 PARTICLE_TRAFFIC_CONFIG = {"workload": "dipole", "shape": "linear-binomial3",
                            "precision": "fp64", "particles": 1_000_000,
                            "deterministic": False}
 
 
 # L2 reduction sectors per particle of one chord_deposit launch: ncu
-# lts__t_sectors_srcunit_tex_op_red on the dipole workload (the unmerged
-# one-reduction-per-visit deposit of the same chords took 90.4 at 250k).
-RED_SECTORS_PER_PARTICLE = {250_000: 45.5, 1_000_000: 21.3}
+# lts__t_sectors_srcunit_tex_op_red on the dipole workload with 1M particles.
+RED_SECTORS_PER_PARTICLE = {1_000_000: 6.47}
 
 
 PROBE_SOURCE = os.path.join(REPO, "bench_probe.cu")
