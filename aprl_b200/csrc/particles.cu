@@ -1397,7 +1397,7 @@ __device__ __forceinline__ SlotPlan plan_slot(const GridT<F>& g, const DFrame& f
 // before any current of the trial is deposited; the push reads them as the
 // previous residual's fields.
 template <class W, class F, int S, bool D>
-__global__ void APRL_GATHER_BOUNDS(S) guess_gather_kernel(const __grid_constant__ PushArgs<F> a) {
+__global__ void APRL_GATHER_BOUNDS(W, S, D) guess_gather_kernel(const __grid_constant__ PushArgs<F> a) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.count) return;
   const double start[3] = {a.p.x[n], a.p.y[n], a.p.z[n]};
@@ -1775,7 +1775,7 @@ __device__ __forceinline__ Runs lane_runs(unsigned long long key, int lane) {
 }
 
 template <int S, bool Q>
-__global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ ChordArgs a) {
+__global__ void APRL_CHORD_BOUNDS(S) chord_deposit_kernel(const __grid_constant__ ChordArgs a) {
   if (trial_skipped(a.g)) return;
   const DGrid& g = a.g;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1971,7 +1971,7 @@ __device__ __forceinline__ void trial_verdict(unsigned long long force_bits, dou
 }
 
 template <class W, class F, int S, bool DB>
-__global__ void APRL_RESIDUAL_BOUNDS(S) residual_kernel(const __grid_constant__ ResidualArgs<F> a) {
+__global__ void APRL_RESIDUAL_BOUNDS(W, S, DB) residual_kernel(const __grid_constant__ ResidualArgs<F> a) {
   if (trial_skipped(a.g)) return;
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double force = 0.0, defect = 0.0, scale = 0.0;

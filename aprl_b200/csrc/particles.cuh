@@ -185,50 +185,57 @@ struct ChordArgs {
   DeviceStatus* status;
 };
 
-// Occupancy knobs of the hot particle kernels (blocks of 128 threads
-// that must fit one SM; 0 leaves the register count to the compiler).
-// 6 blocks (80 registers) were best for push_deposit, the residual and the
-// guess gather among 4, 5, 6, 7 and 8 on the 128x128x512 dipole grid with 1M
-// particles while they read the wide stencils (8 blocks' 64 registers spill).
-// With the narrow stencils a launch takes there: push_deposit 0.078 ms (0.120
-// while it deposited the boundary events' pieces itself), residual 0.104
-// (0.296 with the wide stencils), guess gather 0.068 (0.231).
+// Occupancy of the hot particle kernels (blocks of 128 threads that must fit
+// one SM), measured on the 128x128x512 dipole grid with 1M particles (FP64),
+// on the 128x128x2048 undulator grid with 4M (FP32-mixed) and on smaller runs.
+//
+// push_deposit is bound by FP64 issue (Newton, divisions) with long serial
+// chains: 8 blocks (64 registers) 0.074 and 0.295 ms against 0.075 and 0.297
+// at 7, 0.078 and 0.323 at 6.  (While the kernel carried the boundary events'
+// pieces, 6 were best.)
 #ifndef APRL_PUSH_MIN_BLOCKS
-#define APRL_PUSH_MIN_BLOCKS 6
+#define APRL_PUSH_MIN_BLOCKS 8
 #endif
+// The gathers are bound by load latency.  The binary32 narrow stencils fit 64
+// registers: residual 0.308 ms at 8 blocks against 0.325 at 7 and 0.360 at 6,
+// guess gather 0.209, 0.214 and 0.265.  The binary64 ones and the wide stencils
+// of sparse runs spill there: residual 0.107 ms (FP64) at 8, 0.101 at 7, 0.104
+// at 6, but 0.0212, 0.0198 and 0.0189 with 84k particles; guess gather 0.072,
+// 0.069 and 0.068; wide binary32 residual 0.073, 0.070 and 0.064: 6 blocks.
+// (With the wide stencils these launches took 0.296 and 0.231 ms.)
 #ifndef APRL_RESIDUAL_MIN_BLOCKS
 #define APRL_RESIDUAL_MIN_BLOCKS 6
 #endif
 #ifndef APRL_GATHER_MIN_BLOCKS
 #define APRL_GATHER_MIN_BLOCKS 6
 #endif
-// chord_deposit is left to the compiler.  It is bound by the L2's reductions:
-// the wide stencils' 64 a piece took 0.307 ms a launch on the dipole grid,
-// the narrow 12 take 0.114.
-#ifndef APRL_CHORD_MIN_BLOCKS
-#define APRL_CHORD_MIN_BLOCKS 0
-#endif
-#if APRL_CHORD_MIN_BLOCKS > 0
-#define APRL_CHORD_BOUNDS __launch_bounds__(128, APRL_CHORD_MIN_BLOCKS)
-#else
-#define APRL_CHORD_BOUNDS __launch_bounds__(128)
+#ifndef APRL_NARROW32_MIN_BLOCKS
+#define APRL_NARROW32_MIN_BLOCKS 8
 #endif
 // The quintic gathers keep 24 spline values: 4 blocks (128 registers).  With
 // that, and with the visits' range tests made once a particle (Near), the
-// residual of 265k particles takes 0.106 ms (0.269 before), the guess gather
-// 0.091 (0.260).
+// residual of 265k particles takes 0.106 ms (0.269 before; 0.110 at 3 blocks,
+// 0.152 at 5, 0.191 at 6), the guess gather 0.091 (0.260).
 #ifndef APRL_QUINTIC_MIN_BLOCKS
 #define APRL_QUINTIC_MIN_BLOCKS 4
 #endif
-#define APRL_GATHER_BOUNDS(S) \
-  __launch_bounds__(128, (S) == 0 ? APRL_GATHER_MIN_BLOCKS : APRL_QUINTIC_MIN_BLOCKS)
-#define APRL_RESIDUAL_BOUNDS(S) \
-  __launch_bounds__(128, (S) == 0 ? APRL_RESIDUAL_MIN_BLOCKS : APRL_QUINTIC_MIN_BLOCKS)
-#if APRL_PUSH_MIN_BLOCKS > 0
-#define APRL_PUSH_BOUNDS __launch_bounds__(128, APRL_PUSH_MIN_BLOCKS)
-#else
-#define APRL_PUSH_BOUNDS
+// chord_deposit is bound by issue and the scan's shuffles (6.5 L2 reductions a
+// particle, a quarter of their ceiling rate): 0.101 and 0.375 ms at 8 blocks
+// against 0.105 and 0.397 at 7, 0.114 and 0.439 at 6 (the wide stencils' 64
+// nodes a piece took 0.307 ms).  The quintic one is left to the compiler (0): 0.163
+// ms against 0.188 at 6 blocks, 0.244 at 8.
+#ifndef APRL_CHORD_MIN_BLOCKS
+#define APRL_CHORD_MIN_BLOCKS 8
 #endif
+#define APRL_CHORD_BOUNDS(S) __launch_bounds__(128, (S) == 0 ? APRL_CHORD_MIN_BLOCKS : 0)
+#define APRL_GATHER_BLOCKS(W, S, D, BLOCKS) \
+  ((S) != 0 ? APRL_QUINTIC_MIN_BLOCKS       \
+            : sizeof(W) == 4 && !(D) ? APRL_NARROW32_MIN_BLOCKS : BLOCKS)
+#define APRL_GATHER_BOUNDS(W, S, D) \
+  __launch_bounds__(128, APRL_GATHER_BLOCKS(W, S, D, APRL_GATHER_MIN_BLOCKS))
+#define APRL_RESIDUAL_BOUNDS(W, S, D) \
+  __launch_bounds__(128, APRL_GATHER_BLOCKS(W, S, D, APRL_RESIDUAL_MIN_BLOCKS))
+#define APRL_PUSH_BOUNDS __launch_bounds__(128, APRL_PUSH_MIN_BLOCKS)
 // W: arithmetic of the gathers (double, or float in the FP32-mixed mode).
 // S: the particle shape, 0 linear-binomial3, 1 quintic-compensated.
 // D, DB: read the wide stencils directly (linear-binomial3, sparse runs).
@@ -239,9 +246,9 @@ template <class F, int S, bool Q>
 __global__ void push_events_kernel(const __grid_constant__ PushArgs<F> a);
 template <class F, int S, bool Q> __global__ void carrier_kernel(const __grid_constant__ CarrierArgs<F> a);
 template <int S, bool Q>
-__global__ void APRL_CHORD_BOUNDS chord_deposit_kernel(const __grid_constant__ ChordArgs a);
+__global__ void APRL_CHORD_BOUNDS(S) chord_deposit_kernel(const __grid_constant__ ChordArgs a);
 template <class W, class F, int S, bool DB>
-__global__ void APRL_RESIDUAL_BOUNDS(S) residual_kernel(const __grid_constant__ ResidualArgs<F> a);
+__global__ void APRL_RESIDUAL_BOUNDS(W, S, DB) residual_kernel(const __grid_constant__ ResidualArgs<F> a);
 
 // RelativisticBorisPusher::push of `count` particles (SoA, in place) with
 // per-particle E and B (3 values each).
