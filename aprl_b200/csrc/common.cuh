@@ -298,10 +298,20 @@ constexpr double kFixedLimit = 4611686018427387904.0;  // 2^62
 // Returns false (and adds nothing) for a value outside the range.
 __device__ __forceinline__ bool fixed_add(unsigned long long* pair, double v, double scale) {
   const double s = v * scale;
-  if (!(fabs(s) < kFixedLimit)) return false;
-  const long long n = __double2ll_rn(s);
-  const unsigned long long lo = (unsigned long long)n & 0xffffffffull;
-  const long long hi = n >> 32;
+  // A warp's merged sum may hold 32 lanes' contributions.  From 2^53 on s is
+  // a whole number, so floor and remainder split it exactly without an int64.
+  if (!(fabs(s) < 64.0 * kFixedLimit)) return false;
+  unsigned long long lo;
+  long long hi;
+  if (fabs(s) < kFixedLimit) {
+    const long long n = __double2ll_rn(s);
+    lo = (unsigned long long)n & 0xffffffffull;
+    hi = n >> 32;
+  } else {
+    const double h = floor(s * 0x1p-32);
+    lo = (unsigned long long)(s - h * 0x1p32);
+    hi = (long long)h;
+  }
   if (lo) atomicAdd(&pair[0], lo);
   if (hi) atomicAdd(&pair[1], (unsigned long long)hi);
   return true;
