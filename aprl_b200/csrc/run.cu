@@ -395,6 +395,7 @@ struct aprl_run {
   int stage = 0;
   bool step_open = false;  // aprl_run_step_begin without its aprl_run_step_end yet
   unsigned trials = 0;
+  unsigned trials_unsettled = 0;  // issued ahead, slot fields not settled yet
   uint32_t last_iterations = 0, max_iterations = 0;
   uint64_t total_iterations = 0;
   double last_force = 0.0, last_work = 0.0;
@@ -1952,6 +1953,15 @@ void swap_slot_fields(aprl_run* r) {
   std::swap(r->used_b, r->next_b);
 }
 
+// The trials issued ahead exchanged the slot fields once each as they were
+// queued; those after the converged one did nothing, so the exchange is undone
+// for them.  Call once the step's read-back has landed, whoever asks first.
+void settle_slot_fields(aprl_run* r) {
+  const unsigned ran = r->h_block->stop ? (unsigned)r->h_block->stop : r->trials_unsettled;
+  if (r->np && (r->trials_unsettled - ran) % 2) swap_slot_fields(r);
+  r->trials_unsettled = 0;
+}
+
 // One coupling trial; W is the arithmetic of the gathers.
 template <class W>
 aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
@@ -3258,7 +3268,9 @@ aprl_status step_enqueue(aprl_run* r) {
   const unsigned ahead = trials_ahead(r);
   r->crop_ahead = true;
   for (unsigned t = 0; t < ahead; ++t) TRY(enqueue_trial(r, (int)t, true));
-  return read_block(r);
+  TRY(read_block(r));
+  r->trials_unsettled = ahead;
+  return APRL_OK;
 }
 
 aprl_status step_finish(aprl_run* r) {
@@ -3267,6 +3279,7 @@ aprl_status step_finish(aprl_run* r) {
   double force = 0.0, work = 0.0;
   const unsigned ahead = trials_ahead(r);
   TRY(wait_status(r));
+  if (r->trials_unsettled) settle_slot_fields(r);
   tune_harvest(r);
   unsigned t = 0;
   // forceHistory / workHistory of the reference's failure message.
@@ -3281,9 +3294,6 @@ aprl_status step_finish(aprl_run* r) {
   }
   if ((converged ? (int)iterations : 0) != r->h_block->stop)
     return fail(APRL_ERR_RUNTIME, "Device and host verdicts on the coupling trials differ");
-  // Trials issued beyond the converged one did nothing: the slot fields are
-  // where that one left them.
-  if (r->np && (ahead - t) % 2) swap_slot_fields(r);
   for (; !converged && t < r->cfg.max_trials; ++t) {
     double res[4];
     TRY(do_trial(r, res));
@@ -3459,6 +3469,7 @@ aprl_status aprl_run_get_slot_fields(aprl_run* r, size_t capacity, double* used_
   if (!used_e && !used_b && !next_e && !next_b) return APRL_OK;
   if (capacity < r->nslot) return fail(APRL_ERR_INVALID_ARGUMENT, "Slot buffer too small");
   CUDA_TRY(cudaStreamSynchronize(r->stream));
+  if (r->trials_unsettled) settle_slot_fields(r);  // inside an open step
   const size_t n = r->nslot;
   std::vector<size_t> perm;
   TRY(storage_permutation(r, r->slot_order, n, perm));
