@@ -1915,11 +1915,14 @@ aprl_status surface_current_prepare(aprl_run* r) {
   return APRL_OK;
 }
 
-// Into E* and S0 of the step (jz null), or into a read-out of Jz.
+// Into E* and S0 of the step (jz null), or into a read-out of Jz.  A read-out
+// adds what the step added: from the table as the step found it, which stands
+// until the next step's first trial prepares it again, also when the reference
+// has been replaced since.
 aprl_status surface_current_add(aprl_run* r, const GridT<double>& g, double* jz) {
-  TRY(surface_current_prepare(r));
   const aprl_run_config& c = r->cfg;
   if (!jz) {
+    TRY(surface_current_prepare(r));
     r->surface_offset = r->offset;
     r->surface_step = r->step + 1;
   }
@@ -1942,7 +1945,7 @@ aprl_status surface_current_add(aprl_run* r, const GridT<double>& g, double* jz)
   a.g = g;
   a.jz = jz;
   a.sum = r->np ? r->sum[2] : nullptr;
-  r->surface_in_j = true;
+  if (!jz) r->surface_in_j = true;
   return launch(r, kSurfaceCurrent, surface_add_kernel,
                 dim3(blocks_for(r->surface_count * c.nz, 256)), dim3(256), a);
 }

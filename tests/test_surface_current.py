@@ -105,3 +105,30 @@ def test_file_writer_matches_the_references_own_prepare(shape, tmp_path):
     assert reference.shape == tables.shape and np.abs(reference).max() > 0.0
     assert np.array_equal(reference, tables)
     assert not (tmp_path / "blocked").exists()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("planes", [False, True])
+def test_jz_is_the_steps_own_after_the_reference_is_replaced(planes):
+    """J is what the last step's trial deposited, whatever table the next
+    step will take its surface current from."""
+    w = case("linear-binomial3")
+    w.config = workloads.with_determinism(w.config)
+    g = native.Run(native.load(), w.config).load_workload(w)
+    other = native.Run(native.load(), w.config).load_workload(w)
+    g.step(1)
+    other.step(1)
+    jz = g.get_field(8)
+    doubled = [t if a not in (3, 4) else 2.0 * t for a, t in enumerate(w.reference)]
+    if planes:
+        for a in (3, 4):
+            g.set_reference_planes(a, 0, doubled[a])
+    else:
+        g.set_reference(doubled)
+    np.testing.assert_array_equal(g.get_field(8), jz)
+    # The next step takes the new table, the read-out between them or not.
+    other.set_reference(doubled)
+    g.step(1)
+    other.step(1)
+    np.testing.assert_array_equal(g.get_field(8), other.get_field(8))
+    assert checkers.max_relative(g.get_field(8), jz) > 1e-6
