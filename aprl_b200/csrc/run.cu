@@ -307,6 +307,7 @@ struct aprl_run {
   double* sum[3]{};
   void* filtered[3]{};
   void* bfilter[3]{};
+  bool never_steps = false;  // holds a bunch for its self-field only
   int zb_e[3]{}, zb_b[3]{};
   double* ref[6]{};
   bool ref_set[6]{};
@@ -1753,25 +1754,42 @@ aprl_status do_advance_magnetic(aprl_run* r) {
 // against 0.11, so the sides cross at one particle per 20 to 30 cells,
 // depending on the trials.  16 keeps what is near the crossing on the direct
 // reads, which need no memory of their own.  The quintic shape always gathers
-// from the filtered sum.  A run that cannot have the filtered B's memory reads
-// the wide stencils.
+// from the filtered sum.
+//
+// The two read the same terms in another order, so the choice must not hang on
+// how much memory is free when a step comes to it: the filtered B is reserved
+// with the particles (reserve_magnetic_filter), for all that the run can come
+// to hold.
 constexpr size_t kDenseCells = 16;
 
-bool dense_gathers(aprl_run* r) {
+bool dense_count(const aprl_run_config& c, size_t particles) {
+  return particles && (c.shape != APRL_SHAPE_LINEAR_BINOMIAL3 ||
+                       particles * kDenseCells >= (size_t)c.nx * c.ny * c.nz);
+}
+
+bool dense_gathers(const aprl_run* r) {
+  return dense_count(r->cfg, r->np) &&
+         (r->cfg.shape != APRL_SHAPE_LINEAR_BINOMIAL3 || r->bfilter[2]);
+}
+
+// A bit-reproducible run that cannot have the memory is refused; any other
+// keeps the wide stencils for as long as it holds these particles.
+aprl_status reserve_magnetic_filter(aprl_run* r, size_t particles) {
   const aprl_run_config& c = r->cfg;
-  if (!r->np) return false;
-  if (c.shape != APRL_SHAPE_LINEAR_BINOMIAL3) return true;
-  if (r->np * kDenseCells < (size_t)c.nx * c.ny * c.nz) return false;
-  const size_t w = r->fp32 ? sizeof(float) : sizeof(double);
-  for (int a = 0; a < 3; ++a)
-    if (!r->bfilter[a] &&
-        cudaMallocFromPoolAsync(&r->bfilter[a], bfilter_count(c, a) * w, r->pool, r->stream) !=
-            cudaSuccess) {
-      r->bfilter[a] = nullptr;
-      (void)cudaGetLastError();
-      return false;
-    }
-  return true;
+  if (r->bfilter[2] || r->never_steps || c.shape != APRL_SHAPE_LINEAR_BINOMIAL3) return APRL_OK;
+  if (r->queue.extracted) particles += r->queue.n - r->queue.cursor;
+  if (!dense_count(c, particles)) return APRL_OK;
+  aprl_status s = APRL_OK;
+  for (int a = 0; a < 3 && s == APRL_OK; ++a)
+    s = device_alloc_bytes(r, &r->bfilter[a],
+                           bfilter_count(c, a) * (r->fp32 ? sizeof(float) : sizeof(double)));
+  if (s == APRL_OK) return s;
+  (void)cudaGetLastError();
+  for (int a = 0; a < 3; ++a) {
+    device_free(r, r->bfilter[a]);
+    r->bfilter[a] = nullptr;
+  }
+  return r->deterministic ? s : APRL_OK;
 }
 
 // Launch grid of the filter kernels: `written` x nodes per warp, the z planes
@@ -2963,6 +2981,7 @@ aprl_status aprl_run_set_particles(aprl_run* r, size_t n, const double* x, const
         !std::isfinite(ux[i]) || !std::isfinite(uy[i]) || !std::isfinite(uz[i]) ||
         !std::isfinite(q[i]) || !(m[i] > 0.0))
       return fail(APRL_ERR_INVALID_ARGUMENT, "Particle %zu has a non-finite state or nonpositive mass", i);
+  TRY(reserve_magnetic_filter(r, n));
   TRY(reserve_particles(r, n));
   TRY(reserve_carriers(r, 1));
   note_charges(r, q, n);
@@ -4317,6 +4336,7 @@ aprl_status aprl_run_prepare_reference(aprl_run* r, size_t n, const double* x, c
   tc.initial_offset = 0;
   aprl_run* t = nullptr;
   TRY(aprl_run_create(&tc, r->stream, &t));
+  t->never_steps = true;
   std::vector<uint64_t> ids(n);
   for (size_t i = 0; i < n; ++i) ids[i] = i;
   aprl_status s = aprl_run_set_particles(t, n, x, y, z, ux, uy, uz, q, m, ids.data(), 1);

@@ -294,7 +294,10 @@ aprl_status aprl_run_get_history(aprl_run* run, unsigned index,
 /* Active particles: RelativisticParticleSI (src/eb_particles.h:12-25) as SoA.
  * position in m (box frame), proper velocity u = gamma v / c, charge and
  * mass of the macro-particle (weight already applied), id.  Replaces the
- * particle list, and resets the carrier list when reset_carriers != 0. */
+ * particle list, and resets the carrier list when reset_carriers != 0.
+ * Reserves the device memory that the list's steps need; a bit-reproducible
+ * run is refused here (APRL_ERR_CUDA) when it cannot have the filtered B of
+ * the dense gathers, any other then steps without it. */
 aprl_status aprl_run_set_particles(aprl_run* run, size_t count,
                                    const double* x, const double* y,
                                    const double* z, const double* ux,
