@@ -283,27 +283,32 @@ __device__ __forceinline__ float divide_by(float x, float h, float inv) {
 
 // ---------------------------------------------------------------------------
 // Order-free summation of binary64 contributions (the deterministic mode).
-// A contribution v becomes the integer n = round(v * scale), |n| < 2^62,
-// split into lo = n mod 2^32 (0 <= lo < 2^32) and hi = floor(n / 2^32), and
-// both parts are added with 64-bit integer reductions into a (lo, hi) word
-// pair.  Integer addition is associative, so after any interleaving of the
-// adds the pair holds the exact sum of the rounded contributions,
-// hi * 2^32 + lo (hi two's complement), and so does every other run: the
-// pair's value does not depend on the order of the adds.  lo stays below
-// 2^64 for fewer than 2^32 adds and hi below 2^63 in magnitude for fewer
-// than 2^33.  `scale` is a power of two chosen by the host so that the
-// largest contribution a run can make maps below 2^62.
+// An addend v -- one contribution, or a warp's sum of up to 32 of them --
+// becomes the integer n = round(v * scale), split into lo = n mod 2^32
+// (0 <= lo < 2^32) and hi = floor(n / 2^32), and both parts are added with
+// 64-bit integer reductions into a (lo, hi) word pair.  Integer addition is
+// associative, so after any interleaving of the adds the pair holds the exact
+// sum of the rounded addends, hi * 2^32 + lo (hi two's complement), and so
+// does every other run: the pair's value does not depend on the order of the
+// adds (which lanes a warp sums is a function of the storage order, itself
+// reproducible).  `scale` is a power of two chosen by the host so that the
+// largest contribution a run can make maps below 2^62, so a warp's sum stays
+// below 2^67.  lo stays below 2^64 for fewer than 2^32 adds, and hi, which
+// grows by less than 2^30 a contribution and 1 an add, below 2^63 in magnitude
+// for fewer than 2^32 contributions to one node.
 constexpr double kFixedLimit = 4611686018427387904.0;  // 2^62
 
+// MERGED: v is a warp's sum (the limit leaves room for that sum's rounding).
 // Returns false (and adds nothing) for a value outside the range.
+template <bool MERGED = false>
 __device__ __forceinline__ bool fixed_add(unsigned long long* pair, double v, double scale) {
   const double s = v * scale;
-  // A warp's merged sum may hold 32 lanes' contributions.  From 2^53 on s is
-  // a whole number, so floor and remainder split it exactly without an int64.
-  if (!(fabs(s) < 64.0 * kFixedLimit)) return false;
+  if (!(fabs(s) < (MERGED ? 64.0 * kFixedLimit : kFixedLimit))) return false;
   unsigned long long lo;
   long long hi;
-  if (fabs(s) < kFixedLimit) {
+  // From 2^53 on s is a whole number, so floor and remainder split it exactly
+  // without an int64.
+  if (!MERGED || fabs(s) < kFixedLimit) {
     const long long n = __double2ll_rn(s);
     lo = (unsigned long long)n & 0xffffffffull;
     hi = n >> 32;

@@ -1662,7 +1662,7 @@ __device__ __forceinline__ void chord_add(const DGrid& g, int a, unsigned at, do
                                           unsigned& err) {
   at = APRL_BOUNDED(g.status, at, j_count(g, a), 30 + a);
   if constexpr (Q) {
-    if (!fixed_add(g.jq[a] + 2 * (size_t)at, v, g.jq_scale)) err = kErrFixedRange;
+    if (!fixed_add<true>(g.jq[a] + 2 * (size_t)at, v, g.jq_scale)) err = kErrFixedRange;
   } else {
     atomicAdd(&g.j[a][at], v);
   }

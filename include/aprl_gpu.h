@@ -144,7 +144,8 @@ typedef struct {
   /* Bit-reproducible mode (no counterpart in the reference, whose deposit is
    * serial and therefore repeatable).  0: the current J is summed with FP64
    * atomics, whose order -- and so the last bits of J -- varies from run to
-   * run.  1: every deposit contribution is rounded once to a 128-bit fixed
+   * run.  1: every deposit contribution (or a warp's sum of neighbouring
+   * particles' contributions to one node) is rounded once to a 128-bit fixed
    * point (a power-of-two quantum below 2^-61 of the run's largest possible
    * single contribution, 4*max|q|*c/(dx*dy*dz)) and summed as integers, which is exact and
    * order-free, then converted to binary64 once per trial; the charge-matched

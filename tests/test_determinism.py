@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 import checkers
+import device_arithmetic
 from aprl_b200 import native, workloads
 from test_gpu_parity import compare_state
 
@@ -98,3 +99,55 @@ def test_held_injection_deterministic_matches_oracle():
         g.step(1)
         o.step(1)
         compare_state(g, o)
+
+
+@pytest.mark.parametrize("shape", ["linear-binomial3", "quintic-compensated"])
+def test_many_particles_of_one_charge_in_one_cell(shape):
+    """A warp whose lanes hold pieces of one cell adds their sum: 32 equal
+    weights near a node pass the range of a single contribution (2^62), in
+    either sign.  The fixed-point sum holds them exactly, so J stays within
+    the oracle's own rounding."""
+    w = deterministic(workloads.small_case(particles=1024, steps=2, shape=shape))
+    p = w.particles
+    n = p["x"].size
+    half = n // 2
+    cfg = w.config
+    rng = np.random.default_rng(7)
+    for k, at, h, o in (("x", 8, cfg.dx, 0), ("y", 8, cfg.dy, 1), ("z", 20, cfg.dz, 2)):
+        base = cfg.reference_origin[o] + (cfg.initial_offset * cfg.dz if o == 2 else 0.0)
+        p[k][:] = base + (at + 0.02 + 0.01 * rng.random(n)) * h
+    p["x"][half:] += 2 * cfg.dx
+    q = np.abs(p["charge"]).max()
+    p["charge"][:half], p["charge"][half:] = -q, q
+    g, o = gpu_run(w), checkers.run(checkers.oracle(), w)
+    for r in (g, o):
+        r.advance_magnetic()
+        r.preview_electric()
+    for _ in range(2):
+        g.coupling_trial()
+        o.coupling_trial()
+        for a in (6, 7, 8):
+            assert checkers.max_relative(g.get_field(a), o.get_field(a)) <= 1e-12, a
+    for r in (g, o):
+        r.commit_electric()
+        r.shift()
+    for a in range(6):
+        assert checkers.max_relative(g.get_field(a), o.get_field(a)) <= 1e-12, a
+
+
+@pytest.mark.parametrize("merged", [False, True])
+def test_fixed_point_addends_are_split_exactly(merged, tmp_path):
+    """One contribution: below 2^62; a warp's sum: below 2^68; each addend's
+    pair holds its nearest integer, ties to even."""
+    lib = device_arithmetic.load(tmp_path)
+    rng = np.random.default_rng(11)
+    edges = [2.0**e * m for e in (0, 31, 32, 33, 52, 53, 61, 62, 63, 64, 67)
+             for m in (1.0, 0.5, 1.0 - 2.0**-53, 1.0 + 2.0**-52, 0.75)]
+    v = np.array([0.0, 0.5, 1.5, 2.5] + edges + (2.0**rng.uniform(-2, 68, 4000)).tolist())
+    v = np.concatenate([v, -v])
+    scale = 2.0**7
+    accepted, values = device_arithmetic.fixed_add(lib, v / scale, scale, merged)
+    limit = 2.0**68 if merged else 2.0**62
+    for x, ok, n in zip(v.tolist(), accepted, values):
+        assert ok == (abs(x) < limit), x
+        assert n == (round(x) if ok else 0), x
