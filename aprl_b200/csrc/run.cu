@@ -2494,6 +2494,44 @@ namespace aprl_gpu {
 // The message of a run's failure in aprl_runs_step (the scan server).
 const char* run_error(const aprl_run* r) { return r->error.c_str(); }
 
+// Device bytes a run of `c` with `particles` particles holds while it steps:
+// the arrays of aprl_run_create, all six reference tables, the filtered B of a
+// dense run, and the storage of the particles, of as many pending entries when
+// some are held, and of its carriers (for which a quarter of the particles, and
+// at least one growth of the first reservation, is allowed).
+uint64_t run_device_bytes(const aprl_run_config& c, size_t particles, bool held) {
+  const uint64_t gather = c.precision == APRL_PRECISION_FP32_MIXED ? 4 : 8;
+  const bool filtered_b =
+      c.shape == APRL_SHAPE_LINEAR_BINOMIAL3 && dense_count(c, particles);
+  uint64_t bytes = 0;
+  for (int a = 0; a < 3; ++a) {
+    bytes += 3 * ::e_count(c, a) * 8;            // E^n, E*, S0
+    bytes += ::b_count(c, a) * 8;
+    bytes += raw_count(c, a) * (8 + gather);     // raw current, filtered sum
+    if (filtered_b) bytes += bfilter_count(c, a) * gather;
+    if (c.deterministic) bytes += raw_count(c, a) * 16;
+  }
+  for (unsigned a = 0; a < 6; ++a) {
+    size_t s[3];
+    comp_shape(c, a, s);
+    bytes += s[0] * s[1] * 8 *                   // reference table, inlet halo plane
+             (c.reference_nz + ((a == 0 || a == 1 || a == 5) ? 1 : 0) + (a < 3 ? 1 : 0));
+    // CPML histories: a slot per layer cell, along x except for E_x, B_x and
+    // along y except for E_y, B_y.
+    if (a % 3 != 0) bytes += std::min<uint64_t>(2 * c.cpml_cells_x, s[0]) * s[1] * s[2] * 8;
+    if (a % 3 != 1) bytes += std::min<uint64_t>(2 * c.cpml_cells_y, s[1]) * s[0] * s[2] * 8;
+  }
+  if (c.reference_surface_current)
+    bytes += 2 * (c.nx + c.ny + 2) * (std::max<uint64_t>(1, c.reference_nz) * 8 + 8);
+  bytes += 6 * c.nx * c.ny * 8;                  // detector plane
+  // Two particle states (89 B each), the trial's outputs and slots (184), flags,
+  // events and order (17), sort keys (16), newborn carriers (72), block counts.
+  bytes += (uint64_t)particles * (2 * 89 + 184 + 17 + 16 + 72 + 3);
+  if (held) bytes += (uint64_t)particles * 80;
+  bytes += std::max<uint64_t>(particles / 4, 2 * 4096) * (3 * 72 + 1);
+  return bytes + (16ull << 20);                  // the pool's rounding, small arrays
+}
+
 aprl_status report_error(aprl_status status, const char* message) {
   g_error = message;
   return status;

@@ -30,6 +30,7 @@
 namespace aprl_gpu {
 aprl_status report_error(aprl_status status, const char* message);
 const char* run_error(const aprl_run* r);
+uint64_t run_device_bytes(const aprl_run_config& c, size_t particles, bool held);
 }
 
 namespace {
@@ -47,44 +48,6 @@ struct Job {
 
 aprl_status scan_fail(aprl_status s, const char* message) {
   return aprl_gpu::report_error(s, message);
-}
-
-size_t component_count(const aprl_run_config& c, int a, bool electric) {
-  const uint64_t n[3] = {c.nx, c.ny, c.nz};
-  size_t count = 1;
-  for (int d = 0; d < 3; ++d) count *= (size_t)(n[d] + (electric ? (d != a) : (d == a)));
-  return count;
-}
-
-// Device bytes of one run, following aprl_run_create and the particle and
-// carrier capacities a step uses.
-uint64_t footprint(const aprl_run_config& c, size_t particles) {
-  const size_t fes = c.precision == APRL_PRECISION_FP32_MIXED ? 4 : 8;
-  uint64_t bytes = 0;
-  for (int a = 0; a < 3; ++a) {
-    bytes += 3 * component_count(c, a, true) * fes;   // E^n, E*, J
-    bytes += component_count(c, a, false) * fes;      // B
-    bytes += (c.nx + 1) * (c.ny + 1) * fes;           // inlet halo plane
-  }
-  // CPML histories: at most 2*cells slots of one plane row per layer, 8 terms.
-  const uint64_t cells = std::max(c.cpml_cells_x, c.cpml_cells_y);
-  bytes += 8 * 2 * cells * (std::max(c.nx, c.ny) + 1) * (c.nz + 1) * fes;
-  // Inlet reference table (binary64), six components.
-  for (int a = 0; a < 6; ++a) {
-    const bool electric = a < 3;
-    const int axis = a % 3;
-    const size_t plane = (size_t)(c.nx + (electric ? axis != 0 : axis == 0)) *
-                         (c.ny + (electric ? axis != 1 : axis == 1));
-    bytes += plane * (c.reference_nz + 1) * 8;
-  }
-  // Particles (two state copies, trial outputs, slots, newborn carriers,
-  // sort scratch) and a carrier allowance of a quarter of the particles (at
-  // least the 4096 carriers a run reserves up front).
-  bytes += (uint64_t)particles * 480 +
-           (std::max<uint64_t>(particles / 4, 4096) + 1024) * 3 * 80;
-  // Cell sort and scan scratch, reductions.
-  bytes += (uint64_t)c.nx * c.ny * c.nz * 8 + (32ull << 20);
-  return bytes;
 }
 
 double seconds_since(Clock::time_point origin, Clock::time_point t) {
@@ -256,7 +219,7 @@ extern "C" {
 aprl_status aprl_scan_footprint(const aprl_run_config* config, size_t particles,
                                 uint64_t* bytes) {
   if (!config || !bytes) return scan_fail(APRL_ERR_INVALID_ARGUMENT, "null argument");
-  *bytes = footprint(*config, particles);
+  *bytes = aprl_gpu::run_device_bytes(*config, particles, false);
   return APRL_OK;
 }
 
@@ -290,7 +253,8 @@ aprl_status aprl_scan_create(const aprl_scan_config* config, aprl_scan** out) {
 aprl_status aprl_scan_submit(aprl_scan* scan, const aprl_scan_request* request,
                              uint64_t* ticket) {
   if (!scan || !request || !ticket) return scan_fail(APRL_ERR_INVALID_ARGUMENT, "null argument");
-  const uint64_t bytes = footprint(request->config, request->particles);
+  const uint64_t bytes = aprl_gpu::run_device_bytes(request->config, request->particles,
+                                                    request->frozen != nullptr);
   auto job = std::make_shared<Job>();
   job->request = *request;
   job->footprint = bytes;

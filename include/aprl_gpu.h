@@ -735,8 +735,10 @@ typedef struct {
   char message[256];              /* aprl_last_error of a failed run */
 } aprl_scan_result;
 
-/* Estimated device bytes of one run: fields, histories, the inlet table,
- * particle and carrier storage. */
+/* Estimated device bytes of one run with no held particles: every array it
+ * holds while it steps (the filtered B of a dense run among them), with an
+ * allowance for its carriers.  A request with held particles is counted with
+ * its pending entries too (80 B a particle). */
 aprl_status aprl_scan_footprint(const aprl_run_config* config, size_t particles,
                                 uint64_t* bytes);
 /* Creates the scan on the current device and starts its worker threads. */

@@ -1,5 +1,6 @@
 """Device memory of a run: what its steps need is reserved with its particles,
-so that no step depends on the memory free when it comes.  Measured in a fresh
+so that no step depends on the memory free when it comes, and the scan server's
+estimate covers what the run holds.  Measured in a fresh
 process, as the growth of the device's memory in use (the runs' pool keeps
 what it was given, so the growth is its high-water mark)."""
 import subprocess
@@ -61,3 +62,22 @@ print(a, used())
 """)
     component = 129 * 128 * 257 * (8 if precision == "fp64" else 4)
     assert stepped - loaded < component, (stepped - loaded) / component
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32-mixed"])
+@pytest.mark.parametrize("shape,particles", [("linear-binomial3", 60000),
+                                             ("linear-binomial3", 600000),
+                                             ("quintic-compensated", 600000)])
+def test_the_scan_estimate_covers_a_run(precision, shape, particles):
+    estimate, held = child(f"""
+warm({precision!r}, {shape!r})
+cfg, bunch = case(128, 128, 256, {particles}, {precision!r}, {shape!r})
+a = used()
+r = loaded(cfg, bunch)
+r.step(2)
+b = used()
+scan = native.Scan(native.load(), slots=1)
+print(scan.footprint(cfg, {particles}), b - a)
+""")
+    # Neither short nor, beyond the margins for carriers and pool rounding, wasteful.
+    assert held <= estimate <= 1.25 * held, (estimate / 2**20, held / 2**20)
