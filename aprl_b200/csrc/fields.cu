@@ -617,6 +617,7 @@ __global__ void current_filter_kernel(FilterArgs a) {
   const double* sum = c == 0 ? a.sum[0] : (c == 1 ? a.sum[1] : a.sum[2]);
   double* star = c == 0 ? g.e_star[0] : (c == 1 ? g.e_star[1] : g.e_star[2]);
   void* out = c == 0 ? a.out[0] : (c == 1 ? a.out[1] : a.out[2]);
+  if (MODE == kFilterCurrent && !out) return;  // not the component asked for
   // Tiles: kFilterLanes nodes from -1 on for the orbit modes (lanes 2..29
   // write), 30 from 0 on otherwise (lanes 1..30).
   constexpr int kHalo = kOrbit ? 2 : 1, kWritten = 32 - 2 * kHalo;

@@ -2932,15 +2932,14 @@ aprl_status aprl_run_field_shape(const aprl_run* r, unsigned a, uint64_t shape[3
 // equivalent surface current that the step's E* holds.
 static aprl_status current_out(aprl_run* r, int c, double* out, size_t plane, size_t layers) {
   double* j[3] = {};
-  aprl_status s = APRL_OK;
-  for (int a = 0; a < 3 && s == APRL_OK; ++a) s = device_alloc(r, &j[a], e_count(r->cfg, a));
-  if (s == APRL_OK)
-    s = filter_pass<kFilterCurrent, double>(r, kOrbitSum, make_grid<double>(r), dim3(32, 8),
-                                            reinterpret_cast<void* const*>(j));
+  TRY(device_alloc(r, &j[c], e_count(r->cfg, c)));
+  aprl_status s = filter_pass<kFilterCurrent, double>(r, kOrbitSum, make_grid<double>(r),
+                                                      dim3(32, 8),
+                                                      reinterpret_cast<void* const*>(j));
   if (s == APRL_OK && c == 2 && r->surface_in_j)
     s = surface_current_add(r, make_grid<double>(r), j[2]);
   if (s == APRL_OK) s = copy_ring(r, j[c], nullptr, out, plane, layers, 0);
-  for (int a = 0; a < 3; ++a) device_free(r, j[a]);
+  device_free(r, j[c]);
   return s;
 }
 

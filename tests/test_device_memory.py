@@ -81,3 +81,16 @@ print(scan.footprint(cfg, {particles}), b - a)
 """)
     # Neither short nor, beyond the margins for carriers and pool rounding, wasteful.
     assert held <= estimate <= 1.25 * held, (estimate / 2**20, held / 2**20)
+
+
+def test_reading_one_component_of_j_allocates_one_array():
+    before, after = child("""
+warm("fp64", "linear-binomial3")
+cfg, bunch = case(128, 128, 256, 60000, "fp64", "linear-binomial3")
+r = loaded(cfg, bunch)
+r.step(1)
+a = used()
+r.get_field(6)
+print(a, used())
+""")
+    assert after - before <= 2 * 128 * 129 * 257 * 8
