@@ -612,16 +612,50 @@ struct HostCopy {
   size_t bytes;
 };
 
+// The run's device, current for the length of a call that only copies: such a
+// call may come from any thread, whatever its current device.
+class OnDevice {
+ public:
+  explicit OnDevice(int device) : device_(device), previous_(device) {
+    (void)cudaGetDevice(&previous_);
+    if (previous_ != device_) (void)cudaSetDevice(device_);
+  }
+  ~OnDevice() {
+    if (previous_ != device_) (void)cudaSetDevice(previous_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+
+ private:
+  int device_, previous_;
+};
+
+// Ordinary host memory, which the lanes may touch.  Page-locked and managed
+// memory is left to the driver, which copies it without staging (67 MB: 1.25 ms
+// against 1.75 over the lanes), and so is a pointer that is not the host's,
+// which the driver refuses.
+bool pageable(const void* host) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
 // Copies `list` after the work queued on the run's stream, and returns once
 // everything has landed.
 cudaError_t run_copies(aprl_run* r, const HostCopy* list, size_t count, bool to_host) {
+  const OnDevice device(r->device);
   std::vector<HostCopy> items;
   size_t total = 0;
   for (size_t i = 0; i < count; ++i) total += list[i].bytes;
+  bool staged = total >= kStagedFrom;
+  for (size_t i = 0; i < count && staged; ++i) staged = pageable(list[i].host);
   std::vector<CopyLane*> lanes;
   cudaEvent_t ready = nullptr;
   cudaError_t e = cudaSuccess;
-  if (total >= kStagedFrom) {
+  if (staged) {
     const size_t want = std::min<size_t>(kHostThreads, total / kLaneBytes);
     while (lanes.size() < want) {
       CopyLane* l = lane_take(r->device);
@@ -640,10 +674,8 @@ cudaError_t run_copies(aprl_run* r, const HostCopy* list, size_t count, bool to_
     std::vector<cudaError_t> status(lanes.size(), cudaSuccess);
     auto drive = [&](size_t n) {
       CopyLane& l = *lanes[n];
-      int previous = r->device;  // the caller's own thread drives a lane too
-      (void)cudaGetDevice(&previous);
-      cudaError_t x = cudaSetDevice(r->device);
-      if (x == cudaSuccess) x = cudaStreamWaitEvent(l.stream, ready, 0);
+      const OnDevice own(r->device);  // a driver's thread starts on device 0
+      cudaError_t x = cudaStreamWaitEvent(l.stream, ready, 0);
       const HostCopy* in_flight[2] = {nullptr, nullptr};
       auto land = [&](int b) {  // the copy out of (or the use of) buffer b is over
         if (!in_flight[b]) return;
@@ -670,7 +702,6 @@ cudaError_t run_copies(aprl_run* r, const HostCopy* list, size_t count, bool to_
       land(b ^ 1);
       const cudaError_t w = cudaStreamSynchronize(l.stream);
       status[n] = x == cudaSuccess ? w : x;
-      if (previous != r->device) (void)cudaSetDevice(previous);
     };
     if (e == cudaSuccess) {
       // one driver per lane; drivers that got no thread of their own find the
@@ -1449,6 +1480,7 @@ aprl_status sort_particles(aprl_run* r) {
 // read-out copies contiguous arrays instead of permuting them on the host.
 aprl_status ordered_particles(aprl_run* r) {
   if (!r->np) return APRL_OK;
+  const OnDevice device(r->device);
   const long long n = (long long)r->np;
   const dim3 grid(blocks_for(r->np, 256)), block(256);
   int from = 0;
@@ -2931,6 +2963,7 @@ aprl_status aprl_run_field_shape(const aprl_run* r, unsigned a, uint64_t shape[3
 // J of the last trial (component c): the filtered raw current, and for Jz the
 // equivalent surface current that the step's E* holds.
 static aprl_status current_out(aprl_run* r, int c, double* out, size_t plane, size_t layers) {
+  const OnDevice device(r->device);
   double* j[3] = {};
   TRY(device_alloc(r, &j[c], e_count(r->cfg, c)));
   aprl_status s = filter_pass<kFilterCurrent, double>(r, kOrbitSum, make_grid<double>(r),

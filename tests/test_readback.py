@@ -1,11 +1,14 @@
 """Uploads and read-outs: ring-ordered fields and histories in two runs of
 planes, particles ordered on the device, and large copies driven by several
 threads over page-locked lanes.  Everything is a copy, so equality is exact."""
+import subprocess
+import sys
 import threading
 
 import numpy as np
 import pytest
 
+import checkers
 from aprl_b200 import native, workloads
 
 pytestmark = pytest.mark.gpu
@@ -84,3 +87,61 @@ def test_concurrent_callers_share_the_lanes():
     for t in threads:
         t.join()
     assert not failed
+
+
+def test_page_locked_memory_round_trip():
+    """Memory the driver knows is left to it, at any size."""
+    torch = pytest.importorskip("torch")
+    w = large_case()
+    r = native.Run(native.load(), w.config)
+    r.set_reference(w.reference)
+    value = np.random.default_rng(5).standard_normal(r.get_field(0).shape)
+    locked = torch.from_numpy(value).pin_memory().numpy()
+    r.set_field(0, locked)
+    out = torch.empty(value.shape, dtype=torch.float64).pin_memory().numpy()
+    r.b("run_get_field", r.handle, 0, native._ptr(out), out.size)
+    np.testing.assert_array_equal(out, value)
+    np.testing.assert_array_equal(r.get_field(0), value)
+
+
+def test_a_device_pointer_does_not_end_the_process():
+    """A read-out into a device pointer is the driver's to refuse (or to copy,
+    where it takes the pointer's own word for its place)."""
+    code = f"""
+import ctypes, sys
+sys.path[:0] = [{checkers.REPO!r}, {checkers.REPO + "/tests"!r}]
+import torch
+import test_readback
+from aprl_b200 import native
+w = test_readback.large_case()
+r = native.Run(native.load(), w.config)
+r.set_reference(w.reference)
+t = torch.zeros(r.get_field(0).shape, dtype=torch.float64, device="cuda")
+p = ctypes.cast(t.data_ptr(), ctypes.POINTER(ctypes.c_double))
+try:
+    r.b("run_get_field", r.handle, 0, p, t.numel())
+    print("copied")
+except native.AprlError as e:
+    print("refused")
+torch.cuda.synchronize()
+"""
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert out.stdout.split() in (["refused"], ["copied"])
+
+
+def test_copies_from_a_thread_on_another_device():
+    torch = pytest.importorskip("torch")
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    w = large_case()
+    with torch.cuda.device(1):
+        r = native.Run(native.load(), w.config)
+        r.set_reference(w.reference)
+        r.set_particles(w.particles)
+    with torch.cuda.device(0):
+        value = np.random.default_rng(5).standard_normal(r.get_field(0).shape)
+        r.set_field(0, value)
+        np.testing.assert_array_equal(r.get_field(0), value)
+        np.testing.assert_array_equal(r.get_particles()["z"], w.particles["z"])
+        assert not np.any(r.get_field(8))
