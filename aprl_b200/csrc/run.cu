@@ -243,6 +243,7 @@ constexpr uint64_t kSortInterval = 4;
 struct TunePending {
   int kernel;
   int candidate;
+  unsigned trial;  // issued ahead as this trial (from 1), which may not have run; 0: ran
   cudaEvent_t start, stop;
 };
 
@@ -877,15 +878,16 @@ aprl_status launch(aprl_run* r, unsigned id, K kernel, dim3 grid, dim3 block, Ar
 // ---- autotuner -------------------------------------------------------------
 // The launch shapes of the grid kernels are chosen by measurement, per device
 // and grid extent: the Cowan magnetic kernel's z planes per block and the
-// thread-block shape of the preview, orbit-filter and commit kernels.  Every
-// candidate computes each node exactly as the others do (one thread per node,
-// or the same plane ring over a different split of z), so a choice changes
-// timing only, never a bit of a result.  While a grid extent has no choice
-// yet, the runs on it launch the candidates in turn -- each a real launch of
-// the step, timed with CUDA events and read after the step's own wait -- and
-// once every candidate has two samples the one with the smallest sample
-// becomes the choice for every later launch of every run of that extent in
-// the process.
+// thread-block shape of the preview, orbit-filter and commit kernels (the
+// filters' also per particle shape, the orbit filter's per precision: those are
+// kernels of their own).  Every candidate computes each node exactly as the
+// others do -- the same operations on the same values, over another split of
+// the columns or of z -- so a choice changes timing only, never a bit of a
+// result.  While a grid extent has no choice yet, the runs on it launch the
+// candidates in turn -- each a real launch of the step, timed with CUDA events
+// and read after the step's own wait -- and once every candidate has two
+// samples the one with the smallest sample becomes the choice for every later
+// launch of every run of that extent in the process.
 enum TunedKernel { kTuneCowan = 0, kTunePreview, kTuneOrbit, kTuneCommit, kTuneCount };
 constexpr int kTuneCandidates = 4;
 constexpr int kTuneSamples = 2;
@@ -893,11 +895,12 @@ constexpr int kCowanChunks[kTuneCandidates] = {2, 4, 8, 16};
 const dim3 kGridBlocks[kTuneCandidates] = {dim3(32, 4), dim3(32, 8), dim3(64, 2), dim3(64, 4)};
 
 struct TuneKey {
-  int device, kernel;
+  int device, kernel, variant;
   uint64_t nx, ny, nz;
   bool operator<(const TuneKey& o) const {
     if (device != o.device) return device < o.device;
     if (kernel != o.kernel) return kernel < o.kernel;
+    if (variant != o.variant) return variant < o.variant;
     if (nx != o.nx) return nx < o.nx;
     if (ny != o.ny) return ny < o.ny;
     return nz < o.nz;
@@ -920,7 +923,10 @@ std::map<TuneKey, TuneEntry>& tune_table() {
 }
 
 TuneKey tune_key(const aprl_run* r, int kernel) {
-  return TuneKey{r->device, kernel, r->cfg.nx, r->cfg.ny, r->cfg.nz};
+  int variant = 0;
+  if (kernel == kTuneOrbit || kernel == kTuneCommit) variant = 2 * (int)r->cfg.shape;
+  if (kernel == kTuneOrbit && r->fp32) variant += 1;
+  return TuneKey{r->device, kernel, variant, r->cfg.nx, r->cfg.ny, r->cfg.nz};
 }
 
 // The candidate for this launch of `kernel`; *timed is set when the launch
@@ -955,7 +961,9 @@ void tune_harvest(aprl_run* r) {
       continue;
     }
     float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, p.start, p.stop) == cudaSuccess) {
+    const int converged = r->h_block->stop;
+    const bool ran = !p.trial || !converged || p.trial <= (unsigned)converged;
+    if (ran && cudaEventElapsedTime(&ms, p.start, p.stop) == cudaSuccess) {
       TuneEntry& e = tune_table()[tune_key(r, p.kernel)];
       if (e.samples[p.candidate] == 0 || ms < e.best[p.candidate]) e.best[p.candidate] = ms;
       ++e.samples[p.candidate];
@@ -981,6 +989,7 @@ void tune_harvest(aprl_run* r) {
 // shape; tune_end closes the measurement.
 struct TuneLaunch {
   int kernel = 0, candidate = 0;
+  unsigned trial = 0;  // as in TunePending
   bool timed = false;
   cudaEvent_t start = nullptr, stop = nullptr;
 };
@@ -999,7 +1008,7 @@ aprl_status tune_begin(aprl_run* r, int kernel, TuneLaunch& t) {
 aprl_status tune_end(aprl_run* r, const TuneLaunch& t) {
   if (!t.timed) return APRL_OK;
   CUDA_TRY(cudaEventRecord(t.stop, r->stream));
-  r->tune_pending.push_back(TunePending{t.kernel, t.candidate, t.start, t.stop});
+  r->tune_pending.push_back(TunePending{t.kernel, t.candidate, t.trial, t.start, t.stop});
   return APRL_OK;
 }
 
@@ -2215,17 +2224,20 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     TRY(join_carriers());
     TRY(convert_current());
     {
-      // Measured only in a step's first trial: a trial issued ahead may be
-      // skipped (its kernels return at once), which would time nothing.
+      // Measured once a step, on a pass over the marked columns like nearly all
+      // of them: the first trial's, or the second's where the first, without a
+      // guess pass, forms the step's sum everywhere.  A trial issued ahead may
+      // not run, which would time nothing; such a sample is dropped.
+      const bool full = direct && r->trials == 0;
       TuneLaunch tl;
-      if (r->trials == 0) {
+      if (r->trials == (direct ? 1u : 0u)) {
         TRY(tune_begin(r, kTuneOrbit, tl));
+        tl.trial = ahead ? r->trials + 1 : 0;
       } else {
         tl.candidate = std::max(0, r->tune_choice[kTuneOrbit]);
       }
-      // Without a guess pass the step's first sum is formed everywhere.
       TRY((filter_pass<kFilterOrbit, W>(r, kOrbitSum, g, kGridBlocks[tl.candidate],
-                                        r->filtered, direct && r->trials == 0)));
+                                        r->filtered, full)));
       TRY(tune_end(r, tl));
     }
     ResidualArgs<F> ra{};

@@ -397,7 +397,8 @@ aprl_status aprl_run_get_stats(const aprl_run* run, aprl_step_stats* stats);
  * the reference).  The grid kernels' launch shapes -- the Cowan magnetic
  * kernel's z planes per block (2, 4, 8, 16) and the thread blocks of the
  * preview, orbit-filter and commit kernels (32x4, 32x8, 64x2, 64x4) -- are
- * chosen per device and grid extent by timing each candidate twice on the
+ * chosen per device and grid extent (the filters' also per particle shape,
+ * the orbit filter's per precision) by timing each candidate twice on the
  * first steps of the runs of that extent (real launches of those steps, with
  * CUDA events); every candidate gives the same bits, so tuning changes no
  * result.  Kernels in order: Cowan magnetic, preview, orbit filter, commit. */

@@ -41,3 +41,23 @@ def test_choices_are_made_and_change_no_bit():
     for k in a["particles"]:
         np.testing.assert_array_equal(a["particles"][k], b["particles"][k])
     assert a["stats"] == b["stats"]
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_the_filters_choices_are_per_kernel(dense):
+    """The filter kernels differ by particle shape, the orbit filter also by
+    precision: each is measured on its own launches."""
+    def run(shape, precision):
+        w = workloads.small_case(nx=22, ny=18, nz=44 + dense, particles=4000 if dense else 500,
+                                 steps=12, shape=shape)
+        w.config = workloads.with_precision(w.config, precision)
+        return native.Run(native.load(), w.config).load_workload(w)
+
+    first = run("linear-binomial3", "fp64")
+    first.step(12)
+    assert first.tuning()["decided"] == [True] * 4
+    quintic = run("quintic-compensated", "fp64")
+    assert quintic.tuning()["decided"] == [True, True, False, False]
+    quintic.step(12)
+    assert quintic.tuning()["decided"] == [True] * 4
+    assert run("linear-binomial3", "fp32-mixed").tuning()["decided"] == [True, True, False, True]
