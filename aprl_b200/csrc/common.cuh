@@ -88,7 +88,14 @@ __device__ __forceinline__ void raise_error(DeviceStatus* s, unsigned code,
 // access) in the top 16 bits of the recorded element and the index below,
 // and the access goes to element 0 instead: the kernel never touches memory
 // outside its arrays and never traps.  In the normal build the checks
-// compile to nothing.
+// compile to nothing.  Sites, plus the component: 1 E, 4 B, 7 raw current and
+// filtered sum by node, 10 Cowan tile, 16 history, 22 plane 0 before the inlet,
+// 24 filtered sum by offset, 27 filtered B by node, 30 chord deposit, 33 raw
+// current, 36 S0, 39 E* and 42 filtered sum of a filter pass, 45 B of the
+// magnetic filter, 48 visitor's deposit, 51 S0 of the wide gather, 54 B of the
+// wide gather, 57 output of the magnetic filter, 60 J read-out, 63 raw current
+// or its fixed-point pairs by marked column, 66 column marks, 67 E* and 70 S0 of
+// the preview.
 #ifdef APRL_GPU_BOUNDS_CHECK
 __device__ __forceinline__ size_t bounded(DeviceStatus* s, size_t index, size_t extent,
                                           unsigned site) {
@@ -231,13 +238,18 @@ __device__ __forceinline__ size_t j_count(const GridT<F>& g, int c) {
 constexpr int kMarkNodes = 8;
 __host__ __device__ __forceinline__ int mark_block(int i) { return (i + 1) / kMarkNodes; }
 template <class F>
+__device__ __forceinline__ size_t mark_index(const GridT<F>& g, int i, int j) {
+  return APRL_BOUNDED(g.status, (size_t)j * g.mark_pitch + mark_block(i),
+                      (size_t)(g.ny + 1) * g.mark_pitch, 66);
+}
+template <class F>
 __device__ __forceinline__ void mark_column(const GridT<F>& g, int i, int j) {
-  unsigned char* const m = g.mark + (size_t)j * g.mark_pitch + mark_block(i);
+  unsigned char* const m = g.mark + mark_index(g, i, j);
   if (!*m) *m = 1;
 }
 template <class F>
 __device__ __forceinline__ bool column_marked(const GridT<F>& g, int i, int j) {
-  return g.mark[(size_t)j * g.mark_pitch + mark_block(i)] != 0;
+  return g.mark[mark_index(g, i, j)] != 0;
 }
 
 // The filtered B of component c: nodes -1 <= i <= b_nx, 0 <= j < b_ny,
@@ -256,6 +268,11 @@ __device__ __forceinline__ size_t e_count(const GridT<F>& g, int c) {
 template <class F>
 __device__ __forceinline__ size_t b_count(const GridT<F>& g, int c) {
   return (size_t)b_nx(g, c) * b_ny(g, c) * b_nz(g, c);
+}
+
+template <class F>
+__device__ __forceinline__ size_t bf_count(const GridT<F>& g, int c) {
+  return (size_t)(b_nx(g, c) + 2) * b_ny(g, c) * (b_nz(g, c) + 2);
 }
 
 // applyCurrentSource's interior mask (src/source_coupling.cpp:87) at one rank.

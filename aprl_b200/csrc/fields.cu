@@ -341,8 +341,9 @@ __global__ void __launch_bounds__(256, 4) electric_preview_kernel(PreviewArgs<F>
         if (a.pre_inlet[0]) a.pre_inlet[0][APRL_BOUNDED(g.status, on, pe0, 22)] = v;
         v = inlet_value(a.inlet, 0, i, j);
       }
-      g.e_star[0][b0 + on] = v;
-      if (a.sum[0]) a.sum[0][b0 + on] = v + old0;
+      g.e_star[0][APRL_BOUNDED(g.status, b0 + on, e_count(g, 0), 67)] = v;
+      if (a.sum[0])
+        a.sum[0][APRL_BOUNDED(g.status, b0 + on, e_count(g, 0), 70)] = v + old0;
     }
     if (has_y) {  // Ey (nx+1, ny, nz+1)
       double v = old1;
@@ -357,8 +358,9 @@ __global__ void __launch_bounds__(256, 4) electric_preview_kernel(PreviewArgs<F>
         if (a.pre_inlet[1]) a.pre_inlet[1][APRL_BOUNDED(g.status, ow, pe1, 23)] = v;
         v = inlet_value(a.inlet, 1, i, j);
       }
-      g.e_star[1][b1 + ow] = v;
-      if (a.sum[0]) a.sum[1][b1 + ow] = v + old1;
+      g.e_star[1][APRL_BOUNDED(g.status, b1 + ow, e_count(g, 1), 68)] = v;
+      if (a.sum[0])
+        a.sum[1][APRL_BOUNDED(g.status, b1 + ow, e_count(g, 1), 71)] = v + old1;
     }
     if (has_z) {  // Ez (nx+1, ny+1, nz)
       double v = old2;
@@ -373,8 +375,9 @@ __global__ void __launch_bounds__(256, 4) electric_preview_kernel(PreviewArgs<F>
                                            history_at(a.h[3], slot_y, k, g.zb_e[2], i, g.status));
       }
       if (i == 0 || i == nx || j == 0 || j == ny) v = 0.0;
-      g.e_star[2][b2 + ow] = v;
-      if (a.sum[0]) a.sum[2][b2 + ow] = v + old2;
+      g.e_star[2][APRL_BOUNDED(g.status, b2 + ow, e_count(g, 2), 69)] = v;
+      if (a.sum[0])
+        a.sum[2][APRL_BOUNDED(g.status, b2 + ow, e_count(g, 2), 72)] = v + old2;
     }
     by_k = by;
     bx_k = bx;
@@ -581,7 +584,9 @@ __device__ __forceinline__ void filter_march(const GridT<double>& g, const Filte
         if (m.writes && masked && current != 0.)
           m.star[APRL_BOUNDED(g.status, star_off[u], e_count(g, c), 39 + c)] += g.jcoef * current;
       } else if constexpr (MODE == kFilterCurrent) {
-        if (m.writes) static_cast<double*>(m.out)[out_off] = current;
+        if (m.writes)
+          static_cast<double*>(m.out)[APRL_BOUNDED(g.status, out_off, e_count(g, c), 60 + c)] =
+              current;
         out_off += m.nplane;
       } else {
         double s = sum_v[u];
@@ -698,7 +703,7 @@ __global__ void magnetic_filter_kernel(BFilterArgs a) {
   w.clear();
   w.push(lane_filter(at(k0 - 1)));
   w.push(lane_filter(at(k0)));
-  W* to = out + (unsigned)((k0 + 1) * plane + row);
+  unsigned to = (unsigned)((k0 + 1) * plane + row);
   // Four planes' reads are issued together (one at a time left too few bytes
   // in flight: 0.117 against 0.100 ms on the 128x128x512 grid).
   constexpr int U = 4;
@@ -710,7 +715,7 @@ __global__ void magnetic_filter_kernel(BFilterArgs a) {
     for (int u = 0; u < U; ++u) {
       if (kb + u >= k1) break;
       w.push(lane_filter(v[u]));
-      if (writes) *to = W(w.value());
+      if (writes) out[APRL_BOUNDED(g.status, to, bf_count(g, c), 57 + c)] = W(w.value());
       to += plane;
     }
   }

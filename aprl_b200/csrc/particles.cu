@@ -587,7 +587,7 @@ struct DirectVisitor {
 
   // One accumulation .5*w*(E_new + E^n) at the ring offset n of a node.
   __device__ __forceinline__ W term(int d, unsigned n, W w) const {
-    return W(.5) * w * W(s.p[d][APRL_BOUNDED(g->status, n, e_count(*g, d), 24 + d)]);
+    return W(.5) * w * W(s.p[d][APRL_BOUNDED(g->status, n, e_count(*g, d), 51 + d)]);
   }
 
   // binomialXZSegment specialised for the gather.  When the whole 4x2x4
@@ -712,7 +712,7 @@ __device__ __forceinline__ void binomial_xz_magnetic(const GridT<F>& g, const do
           W r = W(0.);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            r += wx[i] * W(base[APRL_BOUNDED(g.status, row + i, b_count(g, a), 27 + a)]);
+            r += wx[i] * W(base[APRL_BOUNDED(g.status, row + i, b_count(g, a), 54 + a)]);
           v += wz[k] * wy[j] * r;
         }
       }
@@ -2535,7 +2535,8 @@ __device__ __forceinline__ void marked_nodes(const GridT<double>& g, Fn fn) {
     size_t at = (size_t)(chunk * kMarkPlanes) * plane + (size_t)j * (e_nx(g, c) + 2) + (i + 1);
 #pragma unroll
     for (int k = 0; k < kMarkPlanes; ++k)
-      if (chunk * kMarkPlanes + k < last) fn(c, at + k * plane);
+      if (chunk * kMarkPlanes + k < last)
+        fn(c, APRL_BOUNDED(g.status, at + k * plane, j_count(g, c), 63 + c));
   }
 }
 

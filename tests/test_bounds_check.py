@@ -19,6 +19,7 @@ import checkers
 from aprl_b200 import native, workloads
 from test_c1_parity import compare
 from test_gpu_parity import compare_state
+from test_grid_filter import EXTENTS
 
 CASES = {
     "binomial3": dict(nx=16, ny=16, nz=16, particles=300, steps=4),
@@ -62,3 +63,22 @@ def test_held_injection_stays_inside_every_array():
         g.step(1)
         o.step(1)
     compare_state(g, o)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ["linear-binomial3", "quintic-compensated"])
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("nx,ny,nz,particles", EXTENTS)
+def test_grid_passes_stay_inside_every_array(nx, ny, nz, particles, deterministic, shape):
+    """The filter passes' tiles, chunks and marked columns at their edges, the
+    fixed-point pairs and the read-out of J among them."""
+    w = workloads.small_case(nx=nx, ny=ny, nz=nz, particles=particles, steps=3, shape=shape)
+    w.config = workloads.with_determinism(w.config, deterministic)
+    g = native.Run(native.load_checked(), w.config).load_workload(w)
+    for _ in range(3):
+        g.step(1)
+        for a in (6, 7, 8):
+            g.get_field(a)
+    g.synchronize()
+    g.step(1)     # reads the device status after the last read-out too
+    assert g.stats()["device_error"] == 0
