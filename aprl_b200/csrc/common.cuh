@@ -285,10 +285,14 @@ __device__ __forceinline__ bool current_mask(const GridT<F>& g, int c, int i, in
 
 // x / h for a divisor whose reciprocal `inv` = RN(1/h) is at hand: Markstein's
 // correction (P. W. Markstein, IBM J. Res. Dev. 34, 1990).  q = x * inv is
-// within an ulp of the quotient, the remainder x - q h is exact in a fused
-// multiply-add, and adding its share gives the correctly rounded quotient --
-// the same bits as x / h away from overflow and the subnormal range, in three
-// operations instead of the division's loop.
+// within 1.5 ulp of the quotient; q + (x - q h) inv, each step fused, is
+// Q + (Q - q) e for the exact quotient Q and the reciprocal's relative error e,
+// an error below 2^-52 ulp before its one rounding.  Markstein's theorem
+// gives the correctly rounded quotient for a q within one ulp.  For the q here,
+// every pair of significands was compared at each precision from 3 to 13 bits,
+// and every binary32 significand over the splines' divisors, without a miss; a
+// miss would be one ulp.  So x / h's bits, away from overflow and the subnormal
+// range, in three operations instead of the division's loop.
 __device__ __forceinline__ double divide_by(double x, double h, double inv) {
   const double q = x * inv;
   return fma(fma(-q, h, x), inv, q);

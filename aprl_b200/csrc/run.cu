@@ -1077,6 +1077,9 @@ DGrid make_geometry(const aprl_run* r) {
   g.dy = r->cfg.dy;
   g.dz = r->cfg.dz;
   g.dt = r->cfg.dt;
+  g.inv_h[0] = 1. / g.dx;
+  g.inv_h[1] = 1. / g.dy;
+  g.inv_h[2] = 1. / g.dz;
   for (int a = 0; a < 3; ++a) g.origin[a] = r->origin[a];
   return g;
 }
