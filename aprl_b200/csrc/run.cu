@@ -1791,20 +1791,27 @@ aprl_status do_advance_magnetic(aprl_run* r) {
 }
 
 // Whether this step's linear-binomial3 gathers read the filtered B and, in
-// the first trial, the filtered current-free sum.  The two grid passes move
-// 96 B a cell: 0.165 ms a step on the 128x128x512 grid.  There the first-trial
-// gather takes 0.088 ms for 289k particles with the wide stencils and 0.068 ms
-// for 962k with the narrow ones, and the residual 0.22 ns a particle and trial
-// against 0.11, so the sides cross at one particle per 20 to 30 cells,
-// depending on the trials.  16 keeps what is near the crossing on the direct
-// reads, which need no memory of their own.  The quintic shape always gathers
-// from the filtered sum.
+// the first trial, the filtered current-free sum, from 12 (24) nodes a piece
+// and point instead of 64 (96).  The two grid passes that form them move 96 B a
+// cell: 0.165 ms a step on the 128x128x512 grid.  Step times with the narrow
+// and the wide gathers, ms, by cells per particle in the list:
+//   128x128x512   FP64        FP32-mixed      91x107x263   FP64        FP32-mixed
+//      17    1.790 1.842     1.431 1.498         14    0.937 0.950    0.735 0.745
+//      21    1.733 1.756     1.390 1.433         19    0.910 0.923    0.706 0.723
+//      25    1.692 1.708     1.368 1.394         24    0.866 0.869    0.684 0.681
+//      29    1.672 1.670     1.349 1.366         29    0.858 0.853    0.679 0.664
+//      42    1.612 1.590     1.320 1.301         38    0.834 0.833    0.657 0.653
+// so they cross at one particle per 24 to 36 cells.  (On 64x64x256 cells, where
+// the passes are short and the wide reads' latency is not, the narrow gathers
+// are 3 to 9 % faster at every density up to 64; such runs keep the wide ones,
+// and with them the reference's order of the sums, when they are sparse.)  The
+// quintic shape always gathers from the filtered sum.
 //
 // The two read the same terms in another order, so the choice must not hang on
 // how much memory is free when a step comes to it: the filtered B is reserved
 // with the particles (reserve_magnetic_filter), for all that the run can come
 // to hold.
-constexpr size_t kDenseCells = 16;
+constexpr size_t kDenseCells = 24;
 
 bool dense_count(const aprl_run_config& c, size_t particles) {
   return particles && (c.shape != APRL_SHAPE_LINEAR_BINOMIAL3 ||

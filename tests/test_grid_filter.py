@@ -3,7 +3,7 @@
 Particles deposit narrow weights into a raw current and gather from filtered
 arrays; the filter passes work in x tiles of 28 and 30 nodes, z chunks of 8 to
 32 planes and columns marked by the deposits, and a sparse linear-binomial3 run
-(under one particle per 16 cells) reads the wide stencils directly in its first
+(under one particle per 24 cells) reads the wide stencils directly in its first
 trial.  The extents below put the last tile, the last chunk and the ring's wrap
 at their edges, on either side of the sparse rule, and the read-out of J
 applies the filter on its own.  Bound: the terms are the oracle's in another
