@@ -65,9 +65,12 @@ enum Kernel : unsigned {
   kSfMoments, kSfFinish, kSfDeposit, kSfSource, kSfApply, kSfUpdate,
   kSfDirection, kSfSmooth, kSfElectric, kSfMagnetic, kSfClear, kSfGauss, kSfEnergy,
   kInletHalo, kInletCharge, kInletComplete, kRadixCount, kPermuteParticles,
-  kCurrentConvert, kFixedConvert, kChordDeposit, kSfModal, kSurfaceCurrent, kSfOpen, kPushEvents, kKernelCount
+  kCurrentConvert, kFixedConvert, kChordDeposit, kSfModal, kSurfaceCurrent, kSfOpen, kPushEvents,
+  kGuessFilter, kCurrentFilter, kKernelCount
 };
 
+// The profile's names.  "push_deposit" is the push (push_kernel): it deposits
+// nothing, which chord_deposit and push_events do.
 const char* kKernelNames[kKernelCount] = {
   "inlet_lower", "cowan_magnetic", "electric_preview", "carrier",
   "push_deposit", "residual", "electric_commit", "flag_count",
@@ -79,7 +82,8 @@ const char* kKernelNames[kKernelCount] = {
   "trial_verdict", "sf_moments", "sf_finish", "sf_deposit", "sf_source", "sf_apply",
   "sf_update", "sf_direction", "sf_smooth", "sf_electric", "sf_magnetic",
   "sf_clear", "sf_gauss", "sf_energy", "inlet_halo", "inlet_charge", "inlet_complete",
-  "radix_count", "permute_particles", "current_convert", "fixed_convert", "chord_deposit", "sf_modal", "surface_current", "sf_open", "push_events"};
+  "radix_count", "permute_particles", "current_convert", "fixed_convert", "chord_deposit", "sf_modal", "surface_current", "sf_open", "push_events",
+  "guess_filter", "current_filter"};
 
 const char* device_error_text(unsigned code) {
   switch (code) {
@@ -2193,7 +2197,7 @@ aprl_status trial_enqueue_t(aprl_run* r, int slot, bool ahead) {
     }
     if (r->trials == 0) {
       if (!direct)
-        TRY((filter_pass<kFilterGuess, W>(r, kOrbitSum, g, dim3(32, 8), r->filtered)));
+        TRY((filter_pass<kFilterGuess, W>(r, kGuessFilter, g, dim3(32, 8), r->filtered)));
       TRY(launch(r, kGuessGather,
                  binomial ? (direct ? guess_gather_kernel<W, F, 0, true>
                                     : guess_gather_kernel<W, F, 0, false>)
@@ -2988,7 +2992,7 @@ static aprl_status current_out(aprl_run* r, int c, double* out, size_t plane, si
   const OnDevice device(r->device);
   double* j[3] = {};
   TRY(device_alloc(r, &j[c], e_count(r->cfg, c)));
-  aprl_status s = filter_pass<kFilterCurrent, double>(r, kOrbitSum, make_grid<double>(r),
+  aprl_status s = filter_pass<kFilterCurrent, double>(r, kCurrentFilter, make_grid<double>(r),
                                                       dim3(32, 8),
                                                       reinterpret_cast<void* const*>(j));
   if (s == APRL_OK && c == 2 && r->surface_in_j)

@@ -187,10 +187,20 @@ def clock_sampler(index):
                        "reasons": sorted(reasons), "samples": len(sm)})
 
 
-def algorithmic_bytes(kernel, cfg, particles, carriers):
+def current_nodes(run):
+    """Nodes in the z columns that the last step's current reaches, per
+    component: the columns whose orbit sum a trial's filter pass forms anew."""
+    total = 0
+    for a in (6, 7, 8):
+        j = run.get_field(a)
+        total += int(np.count_nonzero(j.any(axis=0))) * j.shape[0]
+    return total
+
+
+def algorithmic_bytes(kernel, cfg, particles, carriers, reached):
     """Unique-state bytes one launch must move (FP64).  Gather/deposit
     stencil traffic is not counted: it is cache traffic for cell-local
-    particles."""
+    particles.  reached: current_nodes."""
     n_cells = cfg.nx * cfg.ny * cfg.nz
     if kernel == "cowan_magnetic":      # read 3 E, read+write 3 B
         return 9 * 8 * n_cells
@@ -206,8 +216,10 @@ def algorithmic_bytes(kernel, cfg, particles, carriers):
         return particles * (48 + 16 + 48 + 8 + 48)
     if kernel == "guess_gather":        # read x,u,flags; write nextE/B
         return particles * (48 + 1 + 48)
-    if kernel == "orbit_filter":        # the columns the bunch's deposits marked: their share of
-        return None                     # the grid is not known here
+    if kernel == "orbit_filter":        # a trial's: read the raw current and S0, write the
+        return 3 * 8 * reached          # filtered sum, in the columns the current reaches
+    if kernel == "guess_filter":        # read S0, write the filtered sum, everywhere
+        return 2 * 8 * 3 * n_cells
     if kernel == "magnetic_filter":     # read B, write the filtered B
         return 2 * 8 * 3 * n_cells
     if kernel == "carrier":             # read + write 8 words
@@ -388,6 +400,7 @@ def run_ours(args):
     profiled_ms = p_start.elapsed_time(p_stop)
     profile = run.profile_read()
     run.profile_enable(False)
+    reached = current_nodes(run)
 
     # ---- end to end through the C ABI with host buffers -------------------
     # A second run of the same workload, from the same start and warm-up, so
@@ -484,7 +497,7 @@ def run_ours(args):
         name, (ms, count) = dominant
         per_launch_ms = ms / max(count, 1)
         mean_particles = particle_steps / max(K, 1)
-        algo = algorithmic_bytes(name, cfg, mean_particles, stats["carriers"])
+        algo = algorithmic_bytes(name, cfg, mean_particles, stats["carriers"], reached)
         achieved = algo / (per_launch_ms * 1e-3) / 1e9 if algo else None
         roofline = {"bound": "hbm", "kernel": name,
                     "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -522,7 +535,7 @@ def run_ours(args):
     kernels = {}
     for k, v in profile.items():
         entry = {"ms": v[0], "launches": v[1], "share": v[0] / total_ms}
-        algo = algorithmic_bytes(k, cfg, particle_steps / max(K, 1), stats["carriers"])
+        algo = algorithmic_bytes(k, cfg, particle_steps / max(K, 1), stats["carriers"], reached)
         if algo and v[1]:
             gbs = algo / (v[0] / v[1] * 1e-3) / 1e9
             entry.update({"bytes_per_launch": algo, "achieved_gbs": gbs, "hbm_frac": gbs / peak})
