@@ -13,12 +13,12 @@
 // there the gathered fields are the reference's bits.  Deposition accumulates
 // with atomics; the summation order of J differs from the reference.
 //
-// The walkers are templated on the type F of J and of the weight
-// arithmetic.  Positions, chord cuts and cell indices are always binary64,
-// and so are the E and B arrays; the weights are evaluated in F from the
-// cell-relative offsets, the field values are rounded to F as they are read
-// and accumulated in F, and J is accumulated in F.  F = double is the FP64
-// drop-in, F = float the FP32-mixed mode.
+// Positions, chord cuts and cell indices are always binary64, and so are the
+// E, B and current arrays and the deposit's weights.  The gathers' walkers are
+// templated on the type W of their arithmetic: the weights are evaluated in W
+// from the cell-relative offsets, the field values -- filtered in binary64 and
+// rounded once to W, or rounded as they are read -- are accumulated in W.
+// W = double is the FP64 drop-in, W = float the FP32-mixed mode.
 #include "common.cuh"
 #include "particles.cuh"
 

@@ -189,8 +189,8 @@ struct ChordArgs {
 // one SM), measured on the 128x128x512 dipole grid with 1M particles (FP64),
 // on the 128x128x2048 undulator grid with 4M (FP32-mixed) and on smaller runs.
 //
-// push_deposit is bound by FP64 issue (Newton, divisions) with long serial
-// chains: 8 blocks (64 registers) 0.074 and 0.295 ms against 0.075 and 0.297
+// push_kernel (push_deposit in the profile) is bound by FP64 issue (Newton,
+// divisions) with long serial chains: 8 blocks (64 registers) 0.074 and 0.295 ms against 0.075 and 0.297
 // at 7, 0.078 and 0.323 at 6.  (While the kernel carried the boundary events'
 // pieces, 6 were best.)
 #ifndef APRL_PUSH_MIN_BLOCKS
@@ -222,8 +222,11 @@ struct ChordArgs {
 // chord_deposit is bound by issue and the scan's shuffles (6.5 L2 reductions a
 // particle, a quarter of their ceiling rate): 0.101 and 0.375 ms at 8 blocks
 // against 0.105 and 0.397 at 7, 0.114 and 0.439 at 6 (the wide stencils' 64
-// nodes a piece took 0.307 ms).  The quintic one is left to the compiler (0): 0.163
-// ms against 0.188 at 6 blocks, 0.244 at 8.
+// nodes a piece took 0.307 ms).  The quintic one is left to the compiler (0: 168
+// registers, 3 blocks).  Launches with 77k, 247k and 939k particles: 0.060, 0.157
+// and 0.539 ms; at 4 blocks (128 registers, 0.2 KB spilled) 0.061, 0.141 and
+// 0.475, at 5 0.063, 0.156 and 0.503, at 6 0.070, 0.172 and 0.544.  With the
+// fixed-point sum 0.105, 0.262 and 0.876; at 4 blocks 0.110, 0.237 and 0.768.
 #ifndef APRL_CHORD_MIN_BLOCKS
 #define APRL_CHORD_MIN_BLOCKS 8
 #endif

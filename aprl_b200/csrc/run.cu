@@ -2393,12 +2393,15 @@ aprl_status do_commit(aprl_run* r) {
     }
     r->np = kept;
     // Particles move about one cell per step, so the cell order survives a
-    // few steps: re-sorting every kSortInterval steps kept push_deposit and
-    // the residual at their sorted speed on the dipole and drift workloads
-    // (1M particles: step 4.24 -> 4.14 ms against sorting every step; never
-    // sorting, 8.4 ms).  Storage order changes no integer result; it changes
-    // J only to roundoff through the order of the FP64 atomics, and not at
-    // all in the deterministic mode, whose fixed-point sum is order-free.
+    // few steps: sorting every kSortInterval steps keeps the particle kernels
+    // at their sorted speed (chord deposit, residual, push and guess gather
+    // within 1 % at every interval from 1 to 16).  Step times at intervals 1, 2,
+    // 4, 8 and 16: dipole 128x128x512 with 1M particles, FP64, 2.280, 2.207,
+    // 2.174, 2.158 and 2.144 ms; 64x64x256 with 100k, 0.675, 0.640, 0.616, 0.599
+    // and 0.603.  Storage order changes no integer result.  It changes J only
+    // to roundoff, through the order of the FP64 atomics and through which
+    // lanes a warp adds together; the bit-reproducible mode sorts at the same
+    // steps in every run, so its bits stand.
     if (r->step % kSortInterval == 0) TRY(sort_particles(r));
   }
   add_counters(r->cumulative, tc);
