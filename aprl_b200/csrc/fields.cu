@@ -703,7 +703,7 @@ __global__ void magnetic_filter_kernel(BFilterArgs a) {
   w.clear();
   w.push(lane_filter(at(k0 - 1)));
   w.push(lane_filter(at(k0)));
-  unsigned to = (unsigned)((k0 + 1) * plane + row);
+  W* to = out + (unsigned)((k0 + 1) * plane + row);
   // Four planes' reads are issued together (one at a time left too few bytes
   // in flight: 0.117 against 0.100 ms on the 128x128x512 grid).
   constexpr int U = 4;
@@ -715,7 +715,7 @@ __global__ void magnetic_filter_kernel(BFilterArgs a) {
     for (int u = 0; u < U; ++u) {
       if (kb + u >= k1) break;
       w.push(lane_filter(v[u]));
-      if (writes) out[APRL_BOUNDED(g.status, to, bf_count(g, c), 57 + c)] = W(w.value());
+      if (writes) out[APRL_BOUNDED(g.status, to - out, bf_count(g, c), 57 + c)] = W(w.value());
       to += plane;
     }
   }
