@@ -14,7 +14,7 @@ positions and momenta (each array's max |a - b| / max |b|) of
 
 as one JSON object per line to `--out`.
 
-    python tests/divergence_curve.py --steps 200 --out gpurun_out/curve.jsonl
+    python tests/divergence_curve.py --steps 200 --out curve.jsonl
 """
 import argparse
 import json
