@@ -2019,6 +2019,8 @@ __global__ void APRL_RESIDUAL_BOUNDS(W, S, DB) residual_kernel(const __grid_cons
     }
     defect = fabs(wd);
     scale = abs_work + fabs(wn);
+  } else if (n < a.count) {  // no push: the slot stays as beginStep resets it
+    for (int d = 0; d < 3; ++d) a.next_e[3 * n + d] = a.next_b[3 * n + d] = 0.0;
   }
   __shared__ unsigned s_calls[32];
   const unsigned calls = __popc(__ballot_sync(0xffffffffu, seen != 0));
