@@ -152,11 +152,19 @@ def clock_sampler(index):
     proc = None
     try:
         proc = subprocess.Popen(["nvidia-smi", "-i", str(index), f"--query-gpu={fields}",
-                                 "--format=csv,noheader,nounits", "-lms", "200"],
+                                 "--format=csv,noheader,nounits", "-lms", "20"],
                                 stdout=out, stderr=subprocess.DEVNULL)
     except OSError:
         proc = None
     result = {}
+    # The timed region may last some tens of ms, less than nvidia-smi takes to
+    # start: it begins once the sampler's first row is there, and only later
+    # rows count.
+    waited = time.perf_counter()
+    while proc is not None and os.path.getsize(out.name) == 0 and \
+            time.perf_counter() - waited < 5.0 and proc.poll() is None:
+        time.sleep(0.005)
+    begun = os.path.getsize(out.name)
     try:
         yield result
     finally:
@@ -167,7 +175,7 @@ def clock_sampler(index):
             except subprocess.TimeoutExpired:
                 proc.kill()
         out.flush()
-        out.seek(0)
+        out.seek(begun)
         rows = [r for r in csv.reader(io.StringIO(out.read())) if len(r) >= 9]
         out.close()
         os.unlink(out.name)
